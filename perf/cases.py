@@ -154,9 +154,10 @@ def _tokens(batch, seq, vocab):
 
 
 def _gradient(count, m, n):
-    """Gradients as they come out of a backward pass: a decaying spectrum above a flat floor."""
+    """Gradients as they come out of a backward pass: a decaying spectrum, up to eight times as high as the largest
+    singular value of the flat floor of noise under it."""
     k = min(64, m, n)
-    scale = torch.logspace(0, -1.5, k, device="cuda")
+    scale = torch.logspace(0, -1.5, k, device="cuda") * (8 * (m ** 0.5 + n ** 0.5) / (m * n) ** 0.5)
     left = torch.randn(count, m, k, device="cuda") * scale
     g = torch.bmm(left, torch.randn(count, k, n, device="cuda"))
     return g.add_(torch.randn(count, m, n, device="cuda")).mul_(1e-3)
@@ -334,9 +335,9 @@ def tolerance(case):
         # rank the smallest directions of the momentum are below the gradients' own rounding: 0.013 / 0.19 seen
         if case["optimizer"] == "dion" and case["rank_fraction"] > 0.25:
             return dict(rel=0.03, max=0.8)
-        return dict(rel=2e-3, max=0.3)
+        return dict(rel=4e-3, max=0.3)               # 8e-4 / 0.06 seen
     if case["optimizer"] == "muon":  # the same bf16 iteration, of which the weights take a part: 5e-4 / 6e-3 seen
         return dict(rel=2e-3, max=0.025)
-    if case["mixed"]:                # bf16 states: an entry may round the other way
-        return dict(rel=1e-3, max=0.03)
-    return dict(rel=1e-4, max=2e-3)  # fp32 states, products in tf32, orthonormalisation close to fp32: 7e-6 / 1e-4 seen
+    # products in tf32 or bf16, orthonormalisation close to fp32; after two steps 3e-4 / 1.6e-3 seen (the columns of the
+    # smallest directions move).  bf16 states: an entry may round the other way
+    return dict(rel=1e-3, max=0.03 if case["mixed"] else 8e-3)

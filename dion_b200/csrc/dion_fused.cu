@@ -22,6 +22,7 @@
 // speed; only the flag words cross NVLink here.  Nothing in this file uses TMA.
 #include <cuda_bf16.h>
 #include <float.h>
+#include <string.h>
 
 #include "kernels.h"
 #include "symm_flags.cuh"
@@ -178,22 +179,41 @@ __device__ __forceinline__ void store_quad(void* p, int type, long long i, const
   }
 }
 
-// One CTA per (strip of kStrip columns, matrix): 8 warps take the rows in turn, a lane owns kV consecutive
-// columns, so that a warp moves kStrip * 4 contiguous bytes of a row per access.  kV = 4 (strips of 128
-// columns, 16-byte accesses) needs r, the pitches and the column offsets to be multiples of 4 and aligned
-// bases; kV = 1 (strips of 32 columns) takes everything else.
+// A cluster of CTAs per (strip of 32 * kV columns, matrix): the CTAs split the rows (of R, and of P for its guard)
+// into contiguous parts, the warps of a CTA take rows in groups of kRows with all loads of a group in flight, and
+// a lane owns kV consecutive columns, so that a warp moves kV * 128 contiguous bytes of a row per access.  The
+// column sums of squares are completed over the cluster through distributed shared memory, in rank order (the
+// result does not depend on timing).  kV = 4 needs r, the pitches and the column offsets to be multiples of 4 and
+// aligned bases; kV = 1 takes everything else.
+// Bound by HBM: R is read once from there and once more from L2, P once.  Why a cluster: with one CTA per strip
+// the kernel ran on B * r / 128 CTAs (16 for four 4096 x 512 matrices) and was bound by the latency of one row
+// after the other.  Measured with / without (B200): 72 r = 96 matrices of GPT-160M 72 / 663 us; fourteen fp32
+// matrices of two 8B-shaped layers (R up to 4096 x 512, P up to 14336 x 512) 273 us / 5.2 ms.
+constexpr int kPostThreads = 512;
+constexpr int kPostRows = 4;         // rows a warp has in flight
+constexpr int kPostMaxCluster = 8;   // portable cluster size
+
 template <int kV>
-__global__ void __launch_bounds__(256) r_post_kernel(const RPostArgs a) {
-  if (!exchange_ready(a.wait, a.status)) return;
-  __shared__ float red[8][32 * kV + 1];
+__global__ void __launch_bounds__(kPostThreads) r_post_kernel(const RPostArgs a, int strips) {
+  constexpr int kWarps = kPostThreads / 32;
+  __shared__ float red[kWarps][32 * kV + 1];
+  __shared__ float part[32 * kV];  // this CTA's sums, read by the cluster
   __shared__ float tot[32 * kV];
+  uint32_t csize;
+  asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(csize));
+  const uint32_t crank = cluster_ctarank();
+  const int strip = (int)(blockIdx.x / csize);
   const int b = blockIdx.y;
+  // a CTA whose peers did not arrive writes nothing, but stays with its cluster until the sums were exchanged
+  const bool ready = exchange_ready(a.wait, a.status);
   const int lane = threadIdx.x & 31;
-  const int rlane = threadIdx.x >> 5;
-  const int col = (blockIdx.x * 32 + lane) * kV;
-  const bool live = col < a.r;  // kV = 4: r is a multiple of 4, so a live lane owns four valid columns
+  const int warp = threadIdx.x >> 5;
+  const int col = (strip * 32 + lane) * kV;
+  const bool live = ready && strip < strips && col < a.r;  // kV = 4: r is a multiple of 4, a live lane owns four valid columns
   const bool nz = a.nonzero == nullptr || a.nonzero[b] != 0;
   const long long mat = (long long)b * a.n * a.r;
+  const int rows_per = (a.n + (int)csize - 1) / (int)csize;
+  const int i0 = (int)crank * rows_per, i1 = min(a.n, i0 + rows_per);
 
   // guarded R[b][i][col ..]: the rank-ordered sum of the slots, or the previous Q for an all-zero momentum
   auto guarded = [&](int i, float (&v)[kV]) {
@@ -214,13 +234,14 @@ __global__ void __launch_bounds__(256) r_post_kernel(const RPostArgs a) {
         const float4 x = *reinterpret_cast<const float4*>(a.slots + k * a.slot_stride + e);
         s.x += x.x; s.y += x.y; s.z += x.z; s.w += x.w;
       }
-      v[0] = nan_to_num(s.x * a.scale); v[1] = nan_to_num(s.y * a.scale);
-      v[2] = nan_to_num(s.z * a.scale); v[3] = nan_to_num(s.w * a.scale);
+      v[0] = s.x * a.scale; v[1] = s.y * a.scale; v[2] = s.z * a.scale; v[3] = s.w * a.scale;
     } else {
       float s = a.slots[e];
       for (int k = 1; k < a.nslots; ++k) s += a.slots[k * a.slot_stride + e];
-      v[0] = nan_to_num(s * a.scale);
+      v[0] = s * a.scale;
     }
+#pragma unroll
+    for (int k = 0; k < kV; ++k) v[k] = nan_to_num(v[k]);
   };
   auto put = [&](void* p, int type, long long e, const float (&v)[kV]) {
     if constexpr (kV == 4) store_quad(p, type, e, make_float4(v[0], v[1], v[2], v[3]));
@@ -231,79 +252,143 @@ __global__ void __launch_bounds__(256) r_post_kernel(const RPostArgs a) {
 #pragma unroll
   for (int k = 0; k < kV; ++k) ss[k] = 0.f;
   if (live) {
-    for (int i = rlane; i < a.n; i += 8) {
-      float v[kV];
-      guarded(i, v);
-      const long long e = mat + (long long)i * a.r + col;
-      if (a.R32) put(a.R32, kElemF32, e, v);
-      if (a.Rm) put(a.Rm, a.rm_type, e, v);
+    for (int i = i0 + warp * kPostRows; i < i1; i += kWarps * kPostRows) {
+      float v[kPostRows][kV];
 #pragma unroll
-      for (int k = 0; k < kV; ++k) ss[k] = fmaf(v[k], v[k], ss[k]);
+      for (int u = 0; u < kPostRows; ++u)
+        if (i + u < i1) guarded(i + u, v[u]);
+#pragma unroll
+      for (int u = 0; u < kPostRows; ++u) {
+        if (i + u < i1) {
+          const long long e = mat + (long long)(i + u) * a.r + col;
+          if (a.R32) put(a.R32, kElemF32, e, v[u]);
+          if (a.Rm) put(a.Rm, a.rm_type, e, v[u]);
+#pragma unroll
+          for (int k = 0; k < kV; ++k) ss[k] = fmaf(v[u][k], v[u][k], ss[k]);
+        }
+      }
     }
     // P[b][:, col ..]: zero for an all-zero momentum, NaN / inf replaced otherwise; written only where it changes
     if (a.P) {
-      for (long long i = rlane; i < a.p_rows; i += 8) {
-        const long long e = (long long)b * a.p_bs + i * a.p_ld + col;
-        float v[kV], w[kV];
-        if constexpr (kV == 4) {
-          const float4 q = load_quad(a.P, a.p_type, e);
-          v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
-        } else {
-          v[0] = load_elem(a.P, a.p_type, e);
-        }
-        bool same = true;
+      const long long p_per = (a.p_rows + csize - 1) / csize;
+      const long long p0 = crank * p_per, p1 = min(a.p_rows, p0 + p_per);
+      for (long long i = p0 + warp * kPostRows; i < p1; i += kWarps * kPostRows) {
+        float v[kPostRows][kV];
+        const long long e0 = (long long)b * a.p_bs + i * a.p_ld + col;
 #pragma unroll
-        for (int k = 0; k < kV; ++k) {
-          w[k] = nz ? nan_to_num(v[k]) : 0.f;
-          same = same && (w[k] == v[k]);
+        for (int u = 0; u < kPostRows; ++u) {
+          if (i + u < p1) {
+            if constexpr (kV == 4) {
+              const float4 q = load_quad(a.P, a.p_type, e0 + u * a.p_ld);
+              v[u][0] = q.x; v[u][1] = q.y; v[u][2] = q.z; v[u][3] = q.w;
+            } else {
+              v[u][0] = load_elem(a.P, a.p_type, e0 + u * a.p_ld);
+            }
+          }
         }
-        if (!same) put(a.P, a.p_type, e, w);
+#pragma unroll
+        for (int u = 0; u < kPostRows; ++u) {
+          if (i + u < p1) {
+            float w[kV];
+            bool same = true;
+#pragma unroll
+            for (int k = 0; k < kV; ++k) {
+              w[k] = nz ? nan_to_num(v[u][k]) : 0.f;
+              same = same && (w[k] == v[u][k]);
+            }
+            if (!same) put(a.P, a.p_type, e0 + u * a.p_ld, w);
+          }
+        }
       }
     }
   }
 #pragma unroll
-  for (int k = 0; k < kV; ++k) red[rlane][lane * kV + k] = ss[k];
+  for (int k = 0; k < kV; ++k) red[warp][lane * kV + k] = ss[k];
   __syncthreads();
   if (threadIdx.x < 32 * kV) {
     float t = 0.f;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) t += red[k][threadIdx.x];
-    tot[threadIdx.x] = t;
-    const int c = blockIdx.x * 32 * kV + threadIdx.x;
-    if (c < a.r && a.ss) a.ss[(long long)b * a.r + c] = t;
+    for (int k = 0; k < kWarps; ++k) t += red[k][threadIdx.x];
+    part[threadIdx.x] = t;
   }
-  if (!a.finish) return;
-  __syncthreads();
-  if (!live) return;
+  if (csize > 1) cluster_sync_all();
+  else __syncthreads();
+  if (threadIdx.x < 32 * kV) {
+    float t = 0.f;
+    if (csize > 1) {
+      const uint32_t addr = smem_u32(&part[threadIdx.x]);
+      for (uint32_t c = 0; c < csize; ++c) {
+        float x;
+        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(x) : "r"(mapa_shared(addr, c)) : "memory");
+        t += x;
+      }
+    } else {
+      t = part[threadIdx.x];
+    }
+    tot[threadIdx.x] = t;
+    const int c = strip * 32 * kV + threadIdx.x;
+    if (ready && crank == 0 && c < a.r && a.ss) a.ss[(long long)b * a.r + c] = t;
+  }
+  // nobody leaves while its sums may still be read
+  if (csize > 1) cluster_sync_all();
+  else __syncthreads();
+  if (!a.finish || !live) return;
   // new Q: column-normalised R; a column that came out zero keeps the previous Q
   float inv[kV];
   bool keep[kV];
+  bool any_keep = false;
 #pragma unroll
   for (int k = 0; k < kV; ++k) {
     const float t = tot[lane * kV + k];
     keep[k] = !(t > 0.f);
+    any_keep = any_keep || keep[k];
     inv[k] = 1.f / (sqrtf(t) + a.eps);
   }
   // the Q state holds columns [qs_col0, qs_col0 + qs_cols); kV = 4: both are multiples of 4
   const bool in_slice = col >= a.qs_col0 && col < a.qs_col0 + a.qs_cols;
-  for (int i = rlane; i < a.n; i += 8) {
-    float q[kV];
-    guarded(i, q);
-    bool any_keep = false;
+  for (int i = i0 + warp * kPostRows; i < i1; i += kWarps * kPostRows) {
+    float q[kPostRows][kV];
 #pragma unroll
-    for (int k = 0; k < kV; ++k) {
-      q[k] *= inv[k];
-      any_keep = any_keep || keep[k];
-    }
-    if (any_keep) {
-      const long long qe = (long long)b * a.q_bs + (long long)i * a.q_ld + col;
+    for (int u = 0; u < kPostRows; ++u)
+      if (i + u < i1) guarded(i + u, q[u]);
 #pragma unroll
-      for (int k = 0; k < kV; ++k)
-        if (keep[k]) q[k] = load_elem(a.Qm, a.q_type, qe + k);
+    for (int u = 0; u < kPostRows; ++u) {
+      if (i + u < i1) {
+#pragma unroll
+        for (int k = 0; k < kV; ++k) q[u][k] *= inv[k];
+        if (any_keep) {
+          const long long qe = (long long)b * a.q_bs + (long long)(i + u) * a.q_ld + col;
+#pragma unroll
+          for (int k = 0; k < kV; ++k)
+            if (keep[k]) q[u][k] = load_elem(a.Qm, a.q_type, qe + k);
+        }
+        if (a.Qn) put(a.Qn, a.qn_type, mat + (long long)(i + u) * a.r + col, q[u]);
+        if (a.Qs && in_slice) put(a.Qs, a.qs_type, ((long long)b * a.n + i + u) * a.qs_cols + (col - a.qs_col0), q[u]);
+      }
     }
-    if (a.Qn) put(a.Qn, a.qn_type, mat + (long long)i * a.r + col, q);
-    if (a.Qs && in_slice) put(a.Qs, a.qs_type, ((long long)b * a.n + i) * a.qs_cols + (col - a.qs_col0), q);
   }
+}
+
+template <int kV>
+cudaError_t r_post_launch_v(const RPostArgs& a, cudaStream_t s) {
+  const int strips = (a.r + 32 * kV - 1) / (32 * kV);
+  // Rows are split until the grid covers the chip twice or a CTA is down to one pass of its warps over R
+  const long long rows = a.n > a.p_rows ? a.n : a.p_rows;
+  int c = 1;
+  while (c < kPostMaxCluster && (long long)strips * a.B * c < 2 * 148 && rows > (long long)c * (kPostThreads / 32) * kPostRows) c *= 2;
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3((unsigned)(strips * c), (unsigned)a.B, 1);
+  cfg.blockDim = dim3(kPostThreads, 1, 1);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)c;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, r_post_kernel<kV>, a, strips);
 }
 
 template <int kV>
@@ -405,9 +490,7 @@ cudaError_t r_post_launch(const RPostArgs& a, cudaStream_t s) {
                     quad_ok(a.R32, kElemF32, a.r, mat) && quad_ok(a.Rm, a.rm_type, a.r, mat) &&
                     quad_ok(a.Qn, a.qn_type, a.r, mat) &&
                     (a.Qs == nullptr || (quad_ok(a.Qs, a.qs_type, a.qs_cols, (long long)a.n * a.qs_cols) && (a.qs_col0 & 3) == 0));
-  if (wide) r_post_kernel<4><<<dim3((a.r + 127) / 128, a.B), 256, 0, s>>>(a);
-  else r_post_kernel<1><<<dim3((a.r + 31) / 32, a.B), 256, 0, s>>>(a);
-  return cudaGetLastError();
+  return wide ? r_post_launch_v<4>(a, s) : r_post_launch_v<1>(a, s);
 }
 
 cudaError_t q_norm_launch(const QNormArgs& a, cudaStream_t s) {

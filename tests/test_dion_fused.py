@@ -20,8 +20,8 @@ def _case(device, dtype, B=5, n=70, r=45, m=52, nslots=3, seed=0):
     return slots, Qm, P, nonzero
 
 
-def _run(device, dtype, finish, qs_cols, qs_col0, r=45):
-    slots, Qm, P, nonzero = _case(device, dtype, r=r)
+def _run(device, dtype, finish, qs_cols, qs_col0, r=45, **sizes):
+    slots, Qm, P, nonzero = _case(device, dtype, r=r, **sizes)
     nsl, B, n, r = slots.shape
     scale, eps = 0.5, 1e-8
     Rr, Pr, ssr, Qr = ops.dion_r_post_reference(slots, scale, nonzero, Qm, P.clone(), eps, finish=True)
@@ -72,6 +72,15 @@ def test_r_post_kernel_wide_strips(dtype, finish, qs_cols, qs_col0, r):
     """Ranks that are multiples of four take the 128-column strips with 16-byte accesses (several strips,
     a ragged last one, and a Q slice whose offset is not a multiple of four, which falls back)."""
     _run("cuda", dtype, finish, qs_cols, qs_col0, r=r)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,m", [(64, 64), (65, 12), (129, 513), (515, 1027), (1024, 40)])
+@pytest.mark.parametrize("r", [45, 136])
+def test_r_post_kernel_splits_rows_over_a_cluster(n, m, r):
+    """One, two, four and eight CTAs per strip, with parts that do not divide the rows and ranks of the cluster
+    that are left without any."""
+    _run("cuda", torch.float32, True, r, 0, r=r, n=n, m=m)
 
 
 @pytest.mark.gpu

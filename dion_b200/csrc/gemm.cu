@@ -40,6 +40,7 @@ constexpr int kNumEpilogueWarps = 8;  // two per TMEM lane quadrant, each takes 
 constexpr int kNumThreads = 64 + 32 * kNumEpilogueWarps;
 constexpr int kNumGatherThreads = 64;  // two more warps in the all-gather variant (register budget of 384 threads)
 constexpr int kGatherUnitBytes = 64 * 1024;  // what one CTA's copier warps move at a time
+constexpr int kPartPitch = kBlockM + 4;  // row pitch (floats) of a partial tile in shared memory: no bank conflicts
 constexpr int kNumSplitThreads = 128;  // four converter warps in the variant that splits fp32 operands in shared memory
 
 // Operand A gathered from the ranks of a group while the product runs (GemmArgs::Gather).
@@ -85,6 +86,8 @@ struct KernelParams {
   void* const* scatter_ptrs;
   int vec_c, vec_d, vec_d2;  // 16-byte vector access allowed
   int stage;                 // turn epilogue accesses through shared memory (coalesced)
+  int b_is_a;                // symmetric product of one matrix with itself: diagonal tiles need one operand only
+  int cluster_k;             // kClusterK: CTAs of a cluster that share one output tile (each a K range)
   int* status;
   GatherParams g;            // used by the kGather instantiations only
 };
@@ -358,12 +361,18 @@ __device__ __forceinline__ bool mbar_wait_for(uint64_t* bar, uint32_t parity, vo
 // and write the remainders (lo) LO_OFFSET further on, same layout - an element-wise pass that does not
 // need to know the swizzle.  The MMA warp then issues hi*hi into the main accumulator and lo*hi, hi*lo
 // into the cross-term accumulator for every K-step.  Operand bytes cross L2 once instead of three times.
-template <bool kTf32, int kAMajor, int kBMajor, int kBlockN, bool kPair, bool kGather = false, bool kSplit = false>
+//
+// kClusterK (with kSplit): the CTAs of a cluster share one output tile, each multiplies a range of K; the partial
+// tiles meet in shared memory, where every CTA adds its 1 / cluster-size of the rows over all CTAs in rank order
+// (the same bits in every run) and stores them.  For Gram matrices of tall factors: few tiles, long K.
+template <bool kTf32, int kAMajor, int kBMajor, int kBlockN, bool kPair, bool kGather = false, bool kSplit = false,
+          bool kClusterK = false>
 __global__ void __launch_bounds__(kNumThreads + (kGather ? kNumGatherThreads : 0) + (kSplit ? kNumSplitThreads : 0), 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
             const __grid_constant__ CUtensorMap tmap_a_lo, const __grid_constant__ CUtensorMap tmap_b_lo,
             const KernelParams p) {
   static_assert(!(kSplit && kGather), "the converter warps and the copier warps use the same warp slots");
+  static_assert(!kClusterK || (kSplit && kBlockN == 128), "K ranges over a cluster: splitting variants, 128-column tiles");
   using C = Cfg<kTf32, kAMajor, kBMajor, kBlockN, kPair, kSplit>;
   extern __shared__ uint8_t smem_raw[];
   // 128B swizzle atoms need 1024-byte aligned tiles.
@@ -386,8 +395,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   // CTA pair: rank 0 leads (issues the MMAs, owns the full / tmem_empty barriers in use)
   uint32_t cta_rank = 0;
   if constexpr (kPair) cta_rank = cluster_ctarank();
-  const int worker = kPair ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
-  const int num_workers = kPair ? (int)(gridDim.x >> 1) : (int)gridDim.x;
+  int k_rank = 0;  // kClusterK: which K range of the cluster's tile this CTA multiplies
+  if constexpr (kClusterK) k_rank = (int)cluster_ctarank();
+  const int worker = kPair ? (int)(blockIdx.x >> 1) : kClusterK ? (int)blockIdx.x / p.cluster_k : (int)blockIdx.x;
+  // kClusterK: one tile per cluster
+  const int num_workers = kPair ? (int)(gridDim.x >> 1) : kClusterK ? p.total_tiles : (int)gridDim.x;
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmap_a);
@@ -428,6 +440,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   if (threadIdx.x == 0) (void)DION_DBG_OK((tmem_base & 0xffffu) + C::TMEM_COLS <= 512u, p.status);
 
   const int kb_per_split = p.kblocks_per_split;
+  // diagonal tile of x^T x with the same rows on both sides: B is A's tile, loaded and split once
+  auto one_operand = [&](const TileCoord& t) -> bool { return kSplit && kBlockN == kBlockM && p.b_is_a && t.m_blk == t.n_blk; };
   // every wait inside the pipeline; the all-gather variant allows for the time another GPU may take
   auto wait = [&](uint64_t* bar, uint32_t parity) -> bool {
     if constexpr (kGather) return mbar_wait_for(bar, parity, abort_flag, kWaitBudgetNs + p.g.budget_ns);
@@ -445,8 +459,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
         const TileCoord t = decode_tile<kGather>(p, tile);
         const int m0 = t.m_blk * C::TILE_M + (int)cta_rank * kBlockM;
         const int n0 = t.n_blk * kBlockN + (int)cta_rank * (kPair ? C::B_ROWS : 0);
-        const int kb0 = t.split * kb_per_split;
+        const int kb0 = (kClusterK ? k_rank : t.split) * kb_per_split;
         const int kb1 = min(kb0 + kb_per_split, p.kblocks_total);
+        const bool skip_b = one_operand(t);
         if constexpr (kGather) {
           // the rows of this tile are in place once every unit of their chunk has been counted
           const int chunk = m0 / p.g.chunk_rows;
@@ -475,7 +490,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
             break;
           }
           // the leader's full barrier collects the bytes of both CTAs
-          if (cta_rank == 0) mbar_arrive_expect_tx(&full_bar[stage], C::TX_BYTES);
+          if (cta_rank == 0) mbar_arrive_expect_tx(&full_bar[stage], skip_b ? C::A_BYTES : C::TX_BYTES);
           const uint32_t bar = kPair ? mapa_shared(smem_u32(&full_bar[stage]), 0) : smem_u32(&full_bar[stage]);
           auto load = [&](void* dst, const CUtensorMap* map, int c0, int c1) {
             if constexpr (kPair) tma_load_3d_pair(dst, map, bar, c0, c1, t.batch);
@@ -502,7 +517,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
 #pragma unroll
             for (int c = 0; c < kBlockM / C::CH; ++c) load(sa + c * (C::BK * 128), map_a, m0 + c * C::CH, k0);
           }
-          if constexpr (kBMajor == kMajorK) {
+          if (skip_b) {
+            // the multiply reads A's tile twice
+          } else if constexpr (kBMajor == kMajorK) {
             load(sb, map_b, k0, n0);
           } else {
 #pragma unroll
@@ -525,8 +542,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       bool ok = true;
       for (int tile = worker; tile < p.total_tiles && ok; tile += num_workers, ++it) {
         const TileCoord t = decode_tile<kGather>(p, tile);
-        const int kb0 = t.split * kb_per_split;
+        const int kb0 = (kClusterK ? k_rank : t.split) * kb_per_split;
         const int kb1 = min(kb0 + kb_per_split, p.kblocks_total);
+        const int b_off = one_operand(t) ? 0 : C::A_BYTES;
         const int acc = it & 1;
         const uint32_t acc_phase = (it >> 1) & 1;
         if (!wait(&tmem_empty[acc], acc_phase ^ 1u)) {
@@ -558,7 +576,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
           }
           tc_fence_after();
           const uint32_t sa = smem_u32(smem + stage * C::STAGE_STRIDE);
-          const uint32_t sb = sa + C::A_BYTES;
+          const uint32_t sb = sa + b_off;
 #pragma unroll
           for (int j = 0; j < C::KSTEPS; ++j) {
             const uint64_t da = make_smem_desc(sa + j * C::A_KSTEP, C::A_LBO, C::A_SBO, C::A_LAYOUT);
@@ -598,8 +616,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     bool ok = true;
     for (int tile = worker; tile < p.total_tiles && ok; tile += num_workers) {
       const TileCoord t = decode_tile<false>(p, tile);
-      const int kb0 = t.split * kb_per_split;
+      const int kb0 = (kClusterK ? k_rank : t.split) * kb_per_split;
       const int kb1 = min(kb0 + kb_per_split, p.kblocks_total);
+      const int nbytes = one_operand(t) ? C::A_BYTES : C::STAGE_BYTES;
       for (int kb = kb0; kb < kb1; ++kb) {
         if (!wait(&full_bar[stage], phase)) {
           ok = false;
@@ -609,7 +628,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
         }
         uint8_t* hi = smem + stage * C::STAGE_STRIDE;
 #pragma unroll 4
-        for (int off = ct * 16; off < C::STAGE_BYTES; off += kNumSplitThreads * 16) {
+        for (int off = ct * 16; off < nbytes; off += kNumSplitThreads * 16) {
           const float4 q = *reinterpret_cast<const float4*>(hi + off);
           float4 h, l;
           h.x = __int_as_float(__float_as_int(q.x) & 0xffffe000);
@@ -746,8 +765,34 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       const int n0 = t.n_blk * kBlockN;
       const int acc = it & 1;
       const uint32_t acc_phase = (it >> 1) & 1;
-      const int kb0 = t.split * kb_per_split;
+      const int kb0 = (kClusterK ? k_rank : t.split) * kb_per_split;
       const bool has_work = kb0 < p.kblocks_total;
+      if constexpr (kClusterK) {
+        // park this CTA's partial tile in the pipeline's shared memory (every load and multiply is done with it);
+        // the sum over the cluster follows behind the barrier at the end of the kernel
+        if (!wait(&tmem_full[0], 0)) {
+          *abort_flag = 1;
+          if (p.status) atomicCAS(p.status, 0, kStatusEpilogueTimeout);
+          break;
+        }
+        tc_fence_after();
+        float* part = reinterpret_cast<float*>(smem) + (quad * 32 + lane) * kPartPitch;
+#pragma unroll 1
+        for (int c = ((warp - 2) >> 2) * 2; c < ((warp - 2) >> 2) * 2 + 2; ++c) {
+          if (n0 + c * 32 >= p.N) break;
+          float v[32], x[32];
+          const uint32_t taddr = tmem_base + c * 32 + ((uint32_t)(quad * 32) << 16);
+          tmem_ld_32x32(taddr, v);
+          tmem_ld_32x32(taddr + kBlockN, x);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 32; i += 4)
+            *reinterpret_cast<float4*>(part + c * 32 + i) =
+                has_work ? make_float4(v[i] + x[i], v[i + 1] + x[i + 1], v[i + 2] + x[i + 2], v[i + 3] + x[i + 3])
+                         : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        break;  // one tile per cluster
+      }
       const int row = m0 + quad * 32 + lane;
       // debug build: the tile lies inside the problem and the output base is 16-byte aligned where vector stores go
       const bool row_ok = row < p.M && DION_DBG_OK(t.batch < p.batch && m0 < p.M + C::TILE_M && n0 < p.N, p.status);
@@ -1031,8 +1076,68 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     while (global_timer_ns() - t0 < 2000000ull) __nanosleep(1000);
     __syncthreads();
   }
-  // a CTA of a pair must outlive its peer's last access to its shared memory, barriers and TMEM
-  if constexpr (kPair) cluster_sync_all();
+  if constexpr (kClusterK) {
+    cluster_sync_all();  // all partial tiles are in place
+    const TileCoord t = decode_tile<false>(p, worker);
+    const int rows = kBlockM / p.cluster_k;  // rows of the tile this CTA adds up
+    const int r0 = k_rank * rows;
+    const int row0 = t.m_blk * kBlockM + r0;
+    const int col0 = t.n_blk * kBlockN;
+    const bool mirror = p.symmetric && t.m_blk != t.n_blk;
+    const float* part = reinterpret_cast<const float*>(smem);
+    float* sum = reinterpret_cast<float*>(smem) + kBlockM * kPartPitch;  // [rows][kPartPitch], for the transposed copy
+    float* D = reinterpret_cast<float*>(p.D) + (long long)t.batch * p.d_batch_stride;
+    for (int e = threadIdx.x; e < rows * (kBlockN / 4); e += blockDim.x) {
+      const int r = e >> 5, c = (e & 31) * 4;
+      if (col0 + c >= p.N) continue;
+      const uint32_t addr = smem_u32(part + (r0 + r) * kPartPitch + c);
+      float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int k = 0; k < p.cluster_k; ++k) {
+        float4 q;
+        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                     : "=f"(q.x), "=f"(q.y), "=f"(q.z), "=f"(q.w)
+                     : "r"(mapa_shared(addr, k))
+                     : "memory");
+        s.x += q.x;
+        s.y += q.y;
+        s.z += q.z;
+        s.w += q.w;
+      }
+      s = make_float4(s.x * p.alpha, s.y * p.alpha, s.z * p.alpha, s.w * p.alpha);
+      if (mirror) *reinterpret_cast<float4*>(sum + r * kPartPitch + c) = s;
+      if (row0 + r < p.M) {
+        float* dp = D + (long long)(row0 + r) * p.ldd + col0 + c;
+        if (p.vec_d && col0 + c + 4 <= p.N) {
+          *reinterpret_cast<float4*>(dp) = s;
+        } else {
+          const float sv[4] = {s.x, s.y, s.z, s.w};
+          for (int i = 0; i < 4; ++i)
+            if (col0 + c + i < p.N) dp[i] = sv[i];
+        }
+      }
+    }
+    if (mirror) {
+      __syncthreads();
+      const int segs = rows / 4;
+      for (int e = threadIdx.x; e < segs * kBlockN; e += blockDim.x) {
+        const int q = e % segs, c = e / segs;
+        if (col0 + c >= p.N) continue;
+        const float* sp = sum + (q * 4) * kPartPitch + c;
+        const float4 s = make_float4(sp[0], sp[kPartPitch], sp[2 * kPartPitch], sp[3 * kPartPitch]);
+        float* dp = D + (long long)(col0 + c) * p.ldd + row0 + q * 4;
+        if (p.vec_d && row0 + q * 4 + 4 <= p.M) {
+          *reinterpret_cast<float4*>(dp) = s;
+        } else {
+          const float sv[4] = {s.x, s.y, s.z, s.w};
+          for (int i = 0; i < 4; ++i)
+            if (row0 + q * 4 + i < p.M) dp[i] = sv[i];
+        }
+      }
+    }
+  }
+  // a CTA of a pair must outlive its peer's last access to its shared memory, barriers and TMEM; so must a CTA whose
+  // partial tile the others read
+  if constexpr (kPair || kClusterK) cluster_sync_all();
   if (warp == 1) {
     tc_fence_after();
     if constexpr (kPair) tmem_dealloc_pair(tmem_base, C::TMEM_COLS);
@@ -1155,7 +1260,8 @@ int num_sms() {
   return n;
 }
 
-template <bool kTf32, int kAMajor, int kBMajor, int kBlockN, bool kPair = false, bool kGather = false, bool kSplit = false>
+template <bool kTf32, int kAMajor, int kBMajor, int kBlockN, bool kPair = false, bool kGather = false, bool kSplit = false,
+          bool kClusterK = false>
 cudaError_t launch_cfg(const GemmArgs& a, const KernelParams& kp, cudaStream_t stream) {
   using C = Cfg<kTf32, kAMajor, kBMajor, kBlockN, kPair, kSplit>;
   CUtensorMap ta, tb, ta_lo, tb_lo;
@@ -1176,7 +1282,7 @@ cudaError_t launch_cfg(const GemmArgs& a, const KernelParams& kp, cudaStream_t s
     tb_lo = tb;
   }
 
-  auto kernel = gemm_kernel<kTf32, kAMajor, kBMajor, kBlockN, kPair, kGather, kSplit>;
+  auto kernel = gemm_kernel<kTf32, kAMajor, kBMajor, kBlockN, kPair, kGather, kSplit, kClusterK>;
   constexpr int kThreads = kNumThreads + (kGather ? kNumGatherThreads : 0) + (kSplit ? kNumSplitThreads : 0);
   static bool attr_set = false;
   if (!attr_set) {
@@ -1185,19 +1291,20 @@ cudaError_t launch_cfg(const GemmArgs& a, const KernelParams& kp, cudaStream_t s
     attr_set = true;
   }
   int grid = a.max_ctas > 0 ? a.max_ctas : num_sms();
-  if constexpr (kPair) {
-    grid /= 2;  // clusters of two CTAs, one tile per cluster at a time
-    if (grid > kp.total_tiles) grid = kp.total_tiles;
+  if constexpr (kPair || kClusterK) {
+    const int cluster = kPair ? 2 : kp.cluster_k;
+    grid /= cluster;  // one tile per cluster at a time
+    if (grid > kp.total_tiles || kClusterK) grid = kp.total_tiles;
     if (grid < 1) grid = 1;
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3(2 * grid, 1, 1);
+    cfg.gridDim = dim3(cluster * grid, 1, 1);
     cfg.blockDim = dim3(kThreads, 1, 1);
     cfg.dynamicSmemBytes = C::SMEM_BYTES;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.x = cluster;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
@@ -1227,7 +1334,40 @@ cudaError_t launch_split_bn(const GemmArgs& a, const KernelParams& kp, int bn, c
   return launch_cfg<true, kAMajor, kBMajor, 128, false, false, true>(a, kp, s);
 }
 
+// CTAs of a cluster that share one output tile of a Gram product (1: no sharing).  Time is taken as waves of tiles
+// times K blocks per CTA, plus what every tile costs besides (pipeline fill, the exchange of the partial tiles): about
+// kTileCost blocks.  One matrix of 14336 x 512 (10 tiles, 448 blocks) takes 8, as do twelve of 3072 x 96; 48 of
+// 768 x 768 (1008 tiles, 24 blocks) fill the chip by themselves and take 1.
+int choose_cluster_k(const GemmArgs& a, const KernelParams& kp, int bn) {
+  if (!a.symmetric || bn != 128 || a.a_major != kMajorMN || a.b_major != kMajorMN || a.d_dtype != kF32 ||
+      a.epilogue != kEpiStore || a.act != 0 || a.C || a.c_ptrs || a.D2 || a.d2_ptrs || a.d_ptrs || a.scatter_mode != 0 ||
+      a.max_ctas > 0)
+    return 1;
+  constexpr int kTileCost = 8;
+  // clusters live inside a GPC, whose SM count is not a multiple of 8 everywhere
+  const int sms = num_sms();
+  int best = 1;
+  long long best_cost = 0;
+  for (int s = 1; s <= 8; s *= 2) {
+    const long long slots = s == 8 ? sms / 8 * 7 / 8 : sms / s;
+    const long long waves = (kp.total_tiles + slots - 1) / (slots > 0 ? slots : 1);
+    const long long cost = waves * ((kp.kblocks_total + s - 1) / s + kTileCost);
+    if (s == 1 || cost < best_cost) {
+      best = s;
+      best_cost = cost;
+    }
+  }
+  return best;
+}
+
 cudaError_t launch_split(const GemmArgs& a, const KernelParams& kp, int bn, cudaStream_t s) {
+  const int ck = choose_cluster_k(a, kp, bn);
+  if (ck > 1) {
+    KernelParams kc = kp;
+    kc.cluster_k = ck;
+    kc.kblocks_per_split = (kp.kblocks_total + ck - 1) / ck;
+    return launch_cfg<true, kMajorMN, kMajorMN, 128, false, false, true, true>(a, kc, s);
+  }
   if (a.a_major == kMajorK) {
     if (a.b_major == kMajorK) return launch_split_bn<kMajorK, kMajorK>(a, kp, bn, s);
     return launch_split_bn<kMajorK, kMajorMN>(a, kp, bn, s);
@@ -1460,6 +1600,9 @@ cudaError_t gemm_launch(const GemmArgs& a, cudaStream_t stream) {
   kp.epilogue = a.epilogue;
   kp.act = a.act;
   kp.symmetric = a.symmetric;
+  kp.b_is_a = a.symmetric && a.A == a.B && a.a_major == kMajorMN && a.b_major == kMajorMN && a.lda == a.ldb &&
+              a.a_batch_stride == a.b_batch_stride;
+  kp.cluster_k = 1;
   kp.scatter_mode = a.scatter_mode;
   kp.scatter_block = a.scatter_block;
   kp.scatter_dests = a.scatter_dests;

@@ -121,7 +121,7 @@ struct Cfg {
   static constexpr bool CROSS_ACC = kTf32 && !kPair && kBlockN <= 128;
   static constexpr int ACC_STRIDE = CROSS_ACC ? 2 * kBlockN : kBlockN;
   static constexpr int TMEM_COLS = (2 * ACC_STRIDE <= 32) ? 32 : 2 * ACC_STRIDE;  // power of two
-  static constexpr int SMEM_BYTES = STAGES * STAGE_STRIDE + 1024 /*align*/ + 256 /*barriers*/ + 8 * 32 * 128 /*epilogue staging*/;
+  static constexpr int SMEM_BYTES = STAGES * STAGE_STRIDE + 1024 /*align*/ + 1024 /*barriers*/ + 8 * 32 * 128 /*epilogue staging*/;
   // descriptor strides
   static constexpr uint32_t A_LBO = (kAMajor == kMajorK) ? 16u : (uint32_t)BK * 128u;
   static constexpr uint32_t B_LBO = (kBMajor == kMajorK) ? 16u : (uint32_t)BK * 128u;
@@ -365,13 +365,20 @@ __device__ __forceinline__ bool mbar_wait_for(uint64_t* bar, uint32_t parity, vo
 // kClusterK (with kSplit): the CTAs of a cluster share one output tile, each multiplies a range of K; the partial
 // tiles meet in shared memory, where every CTA adds its 1 / cluster-size of the rows over all CTAs in rank order
 // (the same bits in every run) and stores them.  For Gram matrices of tall factors: few tiles, long K.
+//
+// kTmaEpi (bf16 operands, C and D): the epilogue moves C and D with TMA.  Every epilogue warp owns a 4 KB
+// buffer, one box of 32 rows x 64 columns: the C box is fetched into it (the first of a tile while the accumulator is
+// still being multiplied), replaced in place by the result and stored from it.  The path with generic loads and stores takes 4.6 us
+// for a 128 x 256 tile and 8.2 us with C, more than the multiply of K = 768 (5.6 us) that should hide it.
 template <bool kTf32, int kAMajor, int kBMajor, int kBlockN, bool kPair, bool kGather = false, bool kSplit = false,
-          bool kClusterK = false>
+          bool kClusterK = false, bool kTmaEpi = false>
 __global__ void __launch_bounds__(kNumThreads + (kGather ? kNumGatherThreads : 0) + (kSplit ? kNumSplitThreads : 0), 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
             const __grid_constant__ CUtensorMap tmap_a_lo, const __grid_constant__ CUtensorMap tmap_b_lo,
-            const KernelParams p) {
+            const __grid_constant__ CUtensorMap tmap_mirror, const KernelParams p) {
+  // kTmaEpi: the slots of the low halves hold the maps of D and C, tmap_mirror the map of D for transposed boxes
   static_assert(!(kSplit && kGather), "the converter warps and the copier warps use the same warp slots");
+  static_assert(!kTmaEpi || (!kTf32 && !kGather && kBlockN >= 128), "TMA epilogue: bf16, 128- and 256-column tiles");
   static_assert(!kClusterK || (kSplit && kBlockN == 128), "K ranges over a cluster: splitting variants, 128-column tiles");
   using C = Cfg<kTf32, kAMajor, kBMajor, kBlockN, kPair, kSplit>;
   extern __shared__ uint8_t smem_raw[];
@@ -384,11 +391,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   uint64_t* tmem_full = empty_bar + C::STAGES;
   uint64_t* tmem_empty = tmem_full + 2;
   uint64_t* conv_bar = tmem_empty + 2;  // kSplit: stage has been split (one arrival per converter warp)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(conv_bar + (kSplit ? C::STAGES : 0));
-  static_assert((2 * C::STAGES + 4 + (kSplit ? C::STAGES : 0)) * 8 + 16 <= 256, "barrier area");
+  uint64_t* c_bar = conv_bar + (kSplit ? C::STAGES : 0);  // kTmaEpi: C box has arrived, one per epilogue warp
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(c_bar + (kTmaEpi ? kNumEpilogueWarps : 0));
+  static_assert((2 * C::STAGES + 4 + (kSplit ? C::STAGES : 0) + (kTmaEpi ? kNumEpilogueWarps : 0)) * 8 + 16 <= 1024,
+                "barrier area");
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   volatile int* gather_word = abort_flag + 1;  // broadcast slot of the copier warps
-  uint8_t* stage_area = bar_area + 256;
+  uint8_t* stage_area = bar_area + 1024;  // 128B-swizzled boxes start on 1024 bytes
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -418,6 +427,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tmem_full[a], 1);
       mbar_init(&tmem_empty[a], kPair ? 2 * kNumEpilogueWarps : kNumEpilogueWarps);
+    }
+    if constexpr (kTmaEpi) {
+      tma_prefetch_desc(&tmap_a_lo);
+      for (int w = 0; w < kNumEpilogueWarps; ++w) mbar_init(&c_bar[w], 1);
     }
     *abort_flag = 0;
     mbar_fence_init();
@@ -754,6 +767,141 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
         }
       }
     }
+  } else if constexpr (kTmaEpi) {
+    // ------------------------------------------------------------------ epilogue, C and D by TMA
+    const int quad = warp & 3;
+    constexpr int kBoxes = kBlockN / 128;  // boxes of 64 columns per warp and tile
+    uint8_t* st = stage_area + (warp - 2) * kStageBytes;
+    uint64_t* cb = &c_bar[warp - 2];
+    uint32_t c_phase = 0;
+    const bool use_c = p.C != nullptr;
+    auto fetch_c = [&](int col, int row, int batch) {
+      if (lane == 0) {
+        tma_store_wait_read();  // the box stored last has left the buffer
+        mbar_arrive_expect_tx(cb, kStageBytes);
+        tma_load_3d(st, &tmap_b_lo, cb, col, row, batch);
+      }
+    };
+    auto buffer_free = [&] {
+      if (lane == 0) tma_store_wait_read();
+      __syncwarp();
+    };
+    int it = 0;
+    bool ok = true;
+    for (int tile = worker; tile < p.total_tiles && ok; tile += num_workers, ++it) {
+      const TileCoord t = decode_tile<false>(p, tile);
+      const int row0 = t.m_blk * C::TILE_M + (int)cta_rank * kBlockM + quad * 32;
+      const int col0 = t.n_blk * kBlockN + ((warp - 2) >> 2) * (kBlockN / 2);
+      const int acc = it & 1;
+      const bool mirror = p.symmetric && t.m_blk != t.n_blk;
+      // boxes of this warp that lie inside the matrix (a box that only overlaps it is clipped by the copy)
+      const int boxes = row0 < p.M ? min(kBoxes, max(0, (p.N - col0 + 63) / 64)) : 0;
+      if (use_c && boxes > 0) fetch_c(col0, row0, t.batch);
+      if (!wait(&tmem_full[acc], (it >> 1) & 1)) {
+        ok = false;
+        *abort_flag = 1;
+        if (p.status) atomicCAS(p.status, 0, kStatusEpilogueTimeout);
+        break;
+      }
+      tc_fence_after();
+      const uint32_t taddr = tmem_base + acc * C::ACC_STRIDE + ((warp - 2) >> 2) * (kBlockN / 2) + ((uint32_t)(quad * 32) << 16);
+#pragma unroll 1
+      for (int h = 0; h < boxes; ++h) {
+        const int col = col0 + h * 64;
+        if (!use_c) buffer_free();
+        else if (h > 0) fetch_c(col, row0, t.batch);
+        float v[64];
+        float(&lo)[32] = *reinterpret_cast<float(*)[32]>(&v[0]);
+        float(&hi)[32] = *reinterpret_cast<float(*)[32]>(&v[32]);
+        tmem_ld_32x32(taddr + h * 64, lo);
+        tmem_ld_32x32(taddr + h * 64 + 32, hi);
+        tmem_ld_wait();
+        if (h == boxes - 1) {
+          // the accumulator is in registers: hand its columns back to the MMA warp
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) {
+            if (cta_rank == 0) mbar_arrive(&tmem_empty[acc]);
+            else mbar_arrive_cluster(mapa_shared(smem_u32(&tmem_empty[acc]), 0));
+          }
+        }
+        if (p.alpha != 1.f) {
+#pragma unroll
+          for (int i = 0; i < 64; ++i) v[i] *= p.alpha;
+        }
+        if (p.act == kActRelu2) {
+#pragma unroll
+          for (int i = 0; i < 64; ++i) v[i] = apply_act(v[i], kActRelu2);
+        }
+        if (use_c) {
+          if (!wait(cb, c_phase)) {
+            ok = false;
+            *abort_flag = 1;
+            if (p.status) atomicCAS(p.status, 0, kStatusEpilogueTimeout);
+            break;
+          }
+          c_phase ^= 1u;
+#pragma unroll
+          for (int s = 0; s < 8; ++s) {
+            const uint4 q = *reinterpret_cast<const uint4*>(st + stage_off(lane, s));
+            const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&q);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const float2 f = __bfloat1622float2(h2[j]);
+              float& a = v[8 * s + 2 * j];
+              float& b = v[8 * s + 2 * j + 1];
+              if (p.act == kActMulRelu2GradSq) {
+                a *= 2.f * sqrt_approx(fmaxf(f.x, 0.f));
+                b *= 2.f * sqrt_approx(fmaxf(f.y, 0.f));
+              } else if (p.act == kActMulRelu2Grad) {
+                a *= 2.f * fmaxf(f.x, 0.f);
+                b *= 2.f * fmaxf(f.y, 0.f);
+              } else {
+                a += p.beta * f.x;
+                b += p.beta * f.y;
+              }
+            }
+          }
+        }
+        // this lane's row over the C row it has just read
+#pragma unroll
+        for (int s = 0; s < 8; ++s) {
+          uint4 q;
+          __nv_bfloat162* h2 = reinterpret_cast<__nv_bfloat162*>(&q);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) h2[j] = __floats2bfloat162_rn(v[8 * s + 2 * j], v[8 * s + 2 * j + 1]);
+          *reinterpret_cast<uint4*>(st + stage_off(lane, s)) = q;
+        }
+        fence_proxy_async_shared();
+        __syncwarp();
+        if (lane == 0) {
+          tma_store_3d(&tmap_a_lo, st, col, row0, t.batch);
+          tma_store_commit();
+        }
+        if (mirror) {
+          // the block transposed, 64 rows of 32: every lane parks its row as a column
+          buffer_free();
+          __nv_bfloat16* tb = reinterpret_cast<__nv_bfloat16*>(st);
+#pragma unroll
+          for (int i = 0; i < 64; ++i) tb[i * 32 + lane] = __float2bfloat16(v[i]);
+          fence_proxy_async_shared();
+          __syncwarp();
+          if (lane == 0) {
+            tma_store_3d(&tmap_mirror, st, row0, col, t.batch);
+            tma_store_commit();
+          }
+        }
+      }
+      if (boxes == 0) {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+          if (cta_rank == 0) mbar_arrive(&tmem_empty[acc]);
+          else mbar_arrive_cluster(mapa_shared(smem_u32(&tmem_empty[acc]), 0));
+        }
+      }
+    }
+    if (lane == 0) tma_store_wait_read();  // the buffers may go when the copies have read them
   } else {
     // ------------------------------------------------------------------ epilogue
     const int quad = warp & 3;  // TMEM lane quadrant this warp may read
@@ -1171,8 +1319,10 @@ struct TmapKey {
   const void* base;
   uint64_t inner, rows, batch, pitch, bstride;
   uint32_t box_inner, box_rows;
-  int32_t dtype, atom32;
+  int32_t dtype, swizzle;
 };
+// shared-memory layout of a box: 128-byte rows swizzled in 16-byte or 32-byte units, or plain rows
+enum { kSwizzle128 = 0, kSwizzle128Atom32 = 1, kSwizzleNone = 2 };
 struct TmapSlot {
   CUtensorMap map;
   TmapKey key;
@@ -1191,7 +1341,7 @@ bool tmap_cache_enabled() {  // DION_B200_TMAP_CACHE=0 encodes every map afresh
 // Tensor map over a row-major [batch][rows][inner] array with a [1][box_rows][box_inner] box.
 bool make_tmap(CUtensorMap* map, const void* base, int dtype, uint64_t inner, uint64_t rows, uint64_t batch,
                uint64_t row_pitch_elems, uint64_t batch_stride_elems, uint32_t box_inner, uint32_t box_rows,
-               bool atom32) {
+               int swizzle) {
   EncodeFn fn = get_encode_fn();
   if (!fn) {
     g_last_error = "cuTensorMapEncodeTiled is not available from this driver";
@@ -1218,7 +1368,7 @@ bool make_tmap(CUtensorMap* map, const void* base, int dtype, uint64_t inner, ui
     key.inner = inner; key.rows = rows; key.batch = batch;
     key.pitch = strides[0]; key.bstride = strides[1];
     key.box_inner = box_inner; key.box_rows = box_rows;
-    key.dtype = dtype; key.atom32 = atom32 ? 1 : 0;
+    key.dtype = dtype; key.swizzle = swizzle;
     uint64_t h = 1469598103934665603ull;
     const unsigned char* kb = reinterpret_cast<const unsigned char*>(&key);
     for (size_t i = 0; i < sizeof(key); ++i) h = (h ^ kb[i]) * 1099511628211ull;
@@ -1233,7 +1383,9 @@ bool make_tmap(CUtensorMap* map, const void* base, int dtype, uint64_t inner, ui
   }
   CUresult r = fn(map, dtype == kBF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3,
                   const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  atom32 ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B,
+                  swizzle == kSwizzleNone        ? CU_TENSOR_MAP_SWIZZLE_NONE
+                  : swizzle == kSwizzle128Atom32 ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B
+                                                 : CU_TENSOR_MAP_SWIZZLE_128B,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
@@ -1261,18 +1413,18 @@ int num_sms() {
 }
 
 template <bool kTf32, int kAMajor, int kBMajor, int kBlockN, bool kPair = false, bool kGather = false, bool kSplit = false,
-          bool kClusterK = false>
+          bool kClusterK = false, bool kTmaEpi = false>
 cudaError_t launch_cfg(const GemmArgs& a, const KernelParams& kp, cudaStream_t stream) {
   using C = Cfg<kTf32, kAMajor, kBMajor, kBlockN, kPair, kSplit>;
   CUtensorMap ta, tb, ta_lo, tb_lo;
   const int dt = kTf32 ? kF32 : kBF16;
   auto map_a = [&](CUtensorMap* m, const void* base) {
-    if (kAMajor == kMajorK) return make_tmap(m, base, dt, a.K, a.M, a.batch, a.lda, a.a_batch_stride, C::BK, kBlockM, false);
-    return make_tmap(m, base, dt, a.M, a.K, a.batch, a.lda, a.a_batch_stride, C::CH, C::BK, C::A_ATOM32);
+    if (kAMajor == kMajorK) return make_tmap(m, base, dt, a.K, a.M, a.batch, a.lda, a.a_batch_stride, C::BK, kBlockM, kSwizzle128);
+    return make_tmap(m, base, dt, a.M, a.K, a.batch, a.lda, a.a_batch_stride, C::CH, C::BK, C::A_ATOM32 ? kSwizzle128Atom32 : kSwizzle128);
   };
   auto map_b = [&](CUtensorMap* m, const void* base) {
-    if (kBMajor == kMajorK) return make_tmap(m, base, dt, a.K, a.N, a.batch, a.ldb, a.b_batch_stride, C::BK, C::B_ROWS, false);
-    return make_tmap(m, base, dt, a.N, a.K, a.batch, a.ldb, a.b_batch_stride, C::CH, C::BK, C::B_ATOM32);
+    if (kBMajor == kMajorK) return make_tmap(m, base, dt, a.K, a.N, a.batch, a.ldb, a.b_batch_stride, C::BK, C::B_ROWS, kSwizzle128);
+    return make_tmap(m, base, dt, a.N, a.K, a.batch, a.ldb, a.b_batch_stride, C::CH, C::BK, C::B_ATOM32 ? kSwizzle128Atom32 : kSwizzle128);
   };
   if (!map_a(&ta, a.A) || !map_b(&tb, a.B)) return cudaErrorInvalidValue;
   if (a.A_lo != nullptr) {
@@ -1281,8 +1433,16 @@ cudaError_t launch_cfg(const GemmArgs& a, const KernelParams& kp, cudaStream_t s
     ta_lo = ta;  // never read
     tb_lo = tb;
   }
+  CUtensorMap tm = ta;  // never read
+  if constexpr (kTmaEpi) {
+    if (!make_tmap(&ta_lo, a.D, kBF16, a.N, a.M, a.batch, a.ldd, a.d_batch_stride, 64, 32, kSwizzle128)) return cudaErrorInvalidValue;
+    if (a.C && !make_tmap(&tb_lo, a.C, kBF16, a.N, a.M, a.batch, a.ldc, a.c_batch_stride, 64, 32, kSwizzle128))
+      return cudaErrorInvalidValue;
+    if (a.symmetric && !make_tmap(&tm, a.D, kBF16, a.N, a.M, a.batch, a.ldd, a.d_batch_stride, 32, 64, kSwizzleNone))
+      return cudaErrorInvalidValue;
+  }
 
-  auto kernel = gemm_kernel<kTf32, kAMajor, kBMajor, kBlockN, kPair, kGather, kSplit, kClusterK>;
+  auto kernel = gemm_kernel<kTf32, kAMajor, kBMajor, kBlockN, kPair, kGather, kSplit, kClusterK, kTmaEpi>;
   constexpr int kThreads = kNumThreads + (kGather ? kNumGatherThreads : 0) + (kSplit ? kNumSplitThreads : 0);
   static bool attr_set = false;
   if (!attr_set) {
@@ -1309,16 +1469,37 @@ cudaError_t launch_cfg(const GemmArgs& a, const KernelParams& kp, cudaStream_t s
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, ta, tb, ta_lo, tb_lo, kp);
+    return cudaLaunchKernelEx(&cfg, kernel, ta, tb, ta_lo, tb_lo, tm, kp);
   } else {
     if (grid > kp.total_tiles) grid = kp.total_tiles;
-    kernel<<<grid, kThreads, C::SMEM_BYTES, stream>>>(ta, tb, ta_lo, tb_lo, kp);
+    kernel<<<grid, kThreads, C::SMEM_BYTES, stream>>>(ta, tb, ta_lo, tb_lo, tm, kp);
     return cudaGetLastError();
   }
 }
 
+// Problems whose epilogue moves C and D with TMA: bf16 in and out, one destination, operands K-major / any, 16-byte
+// aligned rows of whole 16 bytes (every box starts at a multiple of 64 columns; a row is clipped in units of 16 bytes, so
+// that 1001 columns would lose what lies behind the 1001st).  With fp32 outputs, pointer arrays, a second output or
+// scattered tiles, and for tiles of 64 columns, the generic epilogue remains.
+bool tma_epilogue(const GemmArgs& a, const KernelParams& kp, int bn) {
+  return kp.stage && a.ab_dtype == kBF16 && a.a_major == kMajorK && a.d_dtype == kBF16 && a.epilogue == kEpiStore && bn >= 128 &&
+         a.split_k == 1 && !a.c_ptrs && !a.d_ptrs && !a.D2 && !a.d2_ptrs && !a.c_col_scale && a.scatter_mode == 0 &&
+         a.act != kActRelu2SavePre && kp.vec_d && a.D && a.N % 8 == 0 &&
+         (!a.C || (a.c_dtype == kBF16 && kp.vec_c)) && (a.batch == 1 || (a.d_batch_stride != 0 && (!a.C || a.c_batch_stride != 0)));
+}
+
 template <bool kTf32, int kAMajor, int kBMajor>
 cudaError_t launch_bn(const GemmArgs& a, const KernelParams& kp, int bn, bool pair, cudaStream_t s) {
+  if constexpr (!kTf32 && kAMajor == kMajorK) {
+    if (tma_epilogue(a, kp, bn)) {
+      KernelParams kt = kp;
+      // C is read only where it counts
+      if (kp.beta == 0.f && kp.act != kActMulRelu2Grad && kp.act != kActMulRelu2GradSq) kt.C = nullptr;
+      if (pair) return launch_cfg<false, kAMajor, kBMajor, 256, true, false, false, false, true>(a, kt, s);
+      if (bn == 128) return launch_cfg<false, kAMajor, kBMajor, 128, false, false, false, false, true>(a, kt, s);
+      return launch_cfg<false, kAMajor, kBMajor, 256, false, false, false, false, true>(a, kt, s);
+    }
+  }
   if (pair) return launch_cfg<kTf32, kAMajor, kBMajor, 256, true>(a, kp, s);
   switch (bn) {
     case 64: return launch_cfg<kTf32, kAMajor, kBMajor, 64>(a, kp, s);
@@ -1435,8 +1616,12 @@ Tiling choose_tiling(const GemmArgs& a) {
   if (a.pair > 0 && !a.symmetric) bn = 256;
   if (!a.symmetric && bn == 256 && a.pair >= 0 && (pair_env || a.pair > 0)) {
     const long long t = (long long)((a.M + 255) / 256) * ((a.N + 255) / 256) * a.batch * a.split_k;
-    // short-K tiles are bound by the epilogue, which a pair does not speed up
-    pair = a.pair > 0 || (t >= 2 * (num_sms() / 2) && a.K / a.split_k >= 1024);
+    // Short-K tiles are bound by the epilogue, which a pair does not speed up.  Where C and D move by TMA the line lies
+    // lower: 50176 x 768, K = 768: 58 us unpaired, 52 us on pairs, with C 65 and 64; K = 256: 31 and 37 us.  The ReLU^2
+    // gradient's epilogue does more arithmetic (65536 x 3072, K = 768: 322 us unpaired, 348 us on pairs).
+    const bool light = a.ab_dtype == kBF16 && a.d_dtype == kBF16 && a.a_major == kMajorK && !a.d_ptrs && !a.D2 && !a.d2_ptrs &&
+                       a.scatter_mode == 0 && a.act != kActMulRelu2GradSq && a.act != kActMulRelu2Grad;
+    pair = a.pair > 0 || (t >= 2 * (num_sms() / 2) && a.K / a.split_k >= (light ? 512 : 1024));
   }
 
   if (sym_pair) pair = true;

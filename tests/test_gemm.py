@@ -227,6 +227,48 @@ def test_gemm_hi_lo_operands_and_column_scale_cpu():
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("mode", ["plain", "relu2", "addc", "inplace", "grad_sq", "symmetric"])
+@pytest.mark.parametrize("M,N,K,batch", [(1, 136, 64, 1), (24, 768, 768, 1), (300, 520, 72, 2), (129, 264, 200, 1),
+                                         (2049, 1000, 1096, 1), (4100, 2056, 1024, 1), (777, 200, 768, 3)])
+def test_tma_epilogue_moves_c_and_d_by_boxes(M, N, K, batch, mode):
+    """bf16 C and D go through 32 x 64 boxes: ragged rows and columns are clipped, a row pitch above N leaves what lies
+    between the rows alone, C may be D.  The result is the fp64 one rounded to bf16 once (2^-9) plus the error of the
+    fp32 sum, K / 16 truncations of at most 2^-23 of the sum of magnitudes (of order sqrt(K) times an entry)."""
+    if mode == "symmetric":
+        N = M
+    shape = lambda *s: s if batch == 1 else (batch, *s)
+    a = torch.randn(*shape(M, K), device="cuda").bfloat16()
+    w = a if mode == "symmetric" else torch.randn(*shape(N, K), device="cuda").bfloat16()
+    pitch = (N + 7) // 8 * 8 + 16
+    store = torch.full(shape(M, pitch), 7.0, device="cuda", dtype=torch.bfloat16)
+    out = store[..., :N]
+    c = torch.zeros(*shape(M, pitch), device="cuda", dtype=torch.bfloat16)[..., :N]
+    c.copy_(torch.randn(*shape(M, N), device="cuda").abs())
+    ref = a.double() @ w.double().transpose(-1, -2)
+    kw = {}
+    if mode == "relu2":
+        kw, ref = dict(act="relu2", alpha=0.5), torch.relu(0.5 * ref).square()
+    elif mode == "addc":
+        kw, ref = dict(c=c, beta=-1.5), ref - 1.5 * c.double()
+    elif mode == "inplace":
+        out.copy_(c)
+        kw, ref = dict(c=out, beta=1.0), ref + c.double()
+    elif mode == "grad_sq":
+        kw, ref = dict(c=c, act="mul_relu2_grad_sq"), ref * 2 * c.double().sqrt()
+    elif mode == "symmetric":
+        c = (c + c.transpose(-1, -2)).contiguous() if N % 8 == 0 else None
+        kw, ref = (dict(c=c, beta=2.0, symmetric=True), ref + 2 * c.double()) if c is not None else (dict(symmetric=True), ref)
+    gemm(a, w.transpose(-1, -2), out=out, **kw)
+    scale = ref.abs().amax().item()
+    err = (out.double() - ref).abs()
+    assert (err <= ref.abs() * 2 ** -8 + scale * 2 ** -14).all(), (err.max().item(), scale)
+    assert torch.equal(store[..., N:], torch.full_like(store[..., N:], 7.0))
+    from dion_b200 import ops
+
+    ops.check_status()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("batch,rows,r", [(1, 40, 128), (12, 3072, 96), (4, 2056, 512), (3, 5000, 200), (1, 4096, 130),
                                           (2, 776, 8), (40, 160, 96)])
 def test_gram_of_tall_factors_sums_k_ranges_over_a_cluster(batch, rows, r):

@@ -620,6 +620,17 @@ void rope_bwd(const Tensor& dout, const Tensor& x, Tensor dx, const Tensor& cos,
                                                at::cuda::getCurrentCUDAStream()));
 }
 
+void scale_by_scalar(const Tensor& x, Tensor y, const Tensor& scale) {
+  const c10::cuda::CUDAGuard guard(x.device());
+  TORCH_CHECK(x.is_contiguous() && y.is_contiguous() && x.numel() == y.numel() && x.scalar_type() == y.scalar_type(),
+              "scale_by_scalar: contiguous tensors of one size and type");
+  TORCH_CHECK(scale.numel() == 1 && scale.scalar_type() == at::kFloat && scale.device() == x.device(),
+              "scale_by_scalar: the scale is one fp32 value on the same device");
+  ++g_launches;
+  DION_CUDA_CHECK(dion::scale_by_scalar_launch(x.data_ptr(), y.data_ptr(), elem_type(x, "x"), x.numel(),
+                                               scale.data_ptr<float>(), at::cuda::getCurrentCUDAStream()));
+}
+
 void relu2_fwd(const Tensor& x, Tensor h) {
   check_bf16(x, "x");
   check_bf16(h, "h");
@@ -1111,6 +1122,7 @@ TORCH_LIBRARY(dion_b200, m) {
       "Tensor sin, int seq_len, int heads, int head_dim, float eps) -> ()");
   m.def("rope_fwd(Tensor x, Tensor(a!) out, Tensor cos, Tensor sin, int seq_len, int heads, int head_dim) -> ()");
   m.def("rope_bwd(Tensor dout, Tensor x, Tensor(a!) dx, Tensor cos, Tensor sin, int seq_len, int heads, int head_dim) -> ()");
+  m.def("scale_by_scalar(Tensor x, Tensor(a!) y, Tensor scale) -> ()");
   m.def("relu2_fwd(Tensor x, Tensor(a!) h) -> ()");
   m.def("relu2_bwd(Tensor dh, Tensor x, Tensor(a!) dx) -> ()");
   m.def(
@@ -1159,6 +1171,7 @@ TORCH_LIBRARY_IMPL(dion_b200, CUDA, m) {
   m.impl("rope_qknorm_bwd", &rope_qknorm_bwd);
   m.impl("rope_fwd", &rope_fwd);
   m.impl("rope_bwd", &rope_bwd);
+  m.impl("scale_by_scalar", &scale_by_scalar);
   m.impl("relu2_fwd", &relu2_fwd);
   m.impl("relu2_bwd", &relu2_bwd);
   m.impl("cross_entropy_fwd_bwd", &cross_entropy_fwd_bwd);

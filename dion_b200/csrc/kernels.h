@@ -83,6 +83,9 @@ cudaError_t rope_qknorm_bwd_launch(const void* dq_out, const void* dk_out, const
 // h = relu(x)^2 ; dx = dh * 2 * relu(x)
 cudaError_t relu2_fwd_launch(const void* x, void* h, long long n, cudaStream_t s);
 cudaError_t relu2_bwd_launch(const void* dh, const void* x, void* dx, long long n, cudaStream_t s);
+// y = x * (*scale) over n elements, fp32, or bf16 with the scale rounded to bf16 first.  With y == x nothing is read or
+// written when the scale is one.
+cudaError_t scale_by_scalar_launch(const void* x, void* y, int elem_type, long long n, const float* scale, cudaStream_t s);
 // Softmax cross-entropy over bf16 logits [rows, vocab] with row pitch `pitch`:
 //   row_loss[i] = lse_i - logit_i[target_i]  (0 for rows whose target == ignore_index)
 //   when write_grad: logits are overwritten with grad_scale * (*scale_ptr) * (softmax - onehot)

@@ -564,6 +564,40 @@ __global__ void __launch_bounds__(kCeThreads) cross_entropy_kernel(bf16* __restr
   }
 }
 
+// ------------------------------------------------------------------ scaling by a device scalar
+// The gradient of the loss multiplies what the forward pass kept.  It is one in a plain backward pass: in place that
+// costs a launch and no traffic; otherwise one pass in 16-byte accesses (525 M fp32 values to another buffer: 0.65 ms,
+// against 1.59 ms for a broadcasting multiply that moves 4 bytes per access).
+template <bool kBf16>
+__global__ void __launch_bounds__(256) scale_by_scalar_kernel(const void* x, void* y, long long n, int vec,
+                                                             const float* __restrict__ scale) {
+  const float s = kBf16 ? __bfloat162float(__float2bfloat16(*scale)) : *scale;
+  if (x == y && s == 1.f) return;
+  const long long t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long step = (long long)gridDim.x * blockDim.x;
+  constexpr int kPer = kBf16 ? 8 : 4;
+  const long long nvec = vec ? n / kPer : 0;
+#pragma unroll 4
+  for (long long i = t0; i < nvec; i += step) {
+    if constexpr (kBf16) {
+      float f[8];
+      unpack8(reinterpret_cast<const uint4*>(x)[i], f);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) f[j] *= s;
+      reinterpret_cast<uint4*>(y)[i] = pack8(f);
+    } else {
+      const float4 q = reinterpret_cast<const float4*>(x)[i];
+      reinterpret_cast<float4*>(y)[i] = make_float4(q.x * s, q.y * s, q.z * s, q.w * s);
+    }
+  }
+  for (long long i = nvec * kPer + t0; i < n; i += step) {
+    if constexpr (kBf16)
+      reinterpret_cast<bf16*>(y)[i] = __float2bfloat16(__bfloat162float(reinterpret_cast<const bf16*>(x)[i]) * s);
+    else
+      reinterpret_cast<float*>(y)[i] = reinterpret_cast<const float*>(x)[i] * s;
+  }
+}
+
 // ------------------------------------------------------------------ embedding
 __global__ void __launch_bounds__(256) embedding_fwd_kernel(const void* __restrict__ table, int table_type,
                                                            const long long* __restrict__ idx, bf16* __restrict__ out,
@@ -726,6 +760,19 @@ cudaError_t cross_entropy_fwd_bwd_launch(void* logits, const long long* targets,
   cross_entropy_kernel<<<(unsigned)rows, kCeThreads, 0, s>>>(reinterpret_cast<bf16*>(logits), targets, row_loss,
                                                             scale_ptr, vocab, pitch, grad_scale, ignore_index,
                                                             write_grad ? 1 : 0);
+  return cudaGetLastError();
+}
+
+cudaError_t scale_by_scalar_launch(const void* x, void* y, int elem_type, long long n, const float* scale,
+                                   cudaStream_t s) {
+  if (n == 0) return cudaSuccess;
+  const int vec = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0 ? 1 : 0;
+  long long grid = (n + 1023) / 1024;
+  if (grid > 148 * 8) grid = 148 * 8;
+  if (elem_type == kElemF32)
+    scale_by_scalar_kernel<false><<<(unsigned)grid, 256, 0, s>>>(x, y, n, vec, scale);
+  else
+    scale_by_scalar_kernel<true><<<(unsigned)grid, 256, 0, s>>>(x, y, n, vec, scale);
   return cudaGetLastError();
 }
 

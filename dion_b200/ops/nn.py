@@ -534,6 +534,16 @@ def embedding(idx: torch.Tensor, table: torch.Tensor, out_dtype: torch.dtype = t
 
 # --------------------------------------------------------------------------- lm_head + cross entropy
 
+def _times_scalar(x: torch.Tensor, s: torch.Tensor, in_place: bool) -> torch.Tensor:
+    """``x * s`` for a 0-dim fp32 ``s`` (rounded to the dtype of x first); in place if `in_place`."""
+    if (torch.is_grad_enabled() or s.dtype != torch.float32 or s.device != x.device or not x.is_contiguous()
+            or x.dtype not in (torch.float32, torch.bfloat16)):
+        return x * s.to(x.dtype)
+    out = x if in_place else torch.empty_like(x)
+    torch.ops.dion_b200.scale_by_scalar(x, out, s)
+    return out
+
+
 class _LinearCrossEntropyFn(torch.autograd.Function):
     """loss = mean CE(x @ W^T, targets) without keeping the logits: the token dimension is
     processed in chunks; each chunk's logits are turned into their gradient in place by the
@@ -549,7 +559,7 @@ class _LinearCrossEntropyFn(torch.autograd.Function):
         inv_valid = valid.reciprocal()
         row_loss = torch.empty(T, device=x.device, dtype=torch.float32)
         dx = torch.empty_like(x) if need_grad else None
-        dw = torch.zeros(V, K, device=x.device, dtype=torch.float32) if need_grad else None
+        dw = torch.empty(V, K, device=x.device, dtype=torch.float32) if need_grad else None
         chunk = min(chunk_tokens, T)
         logits = torch.empty(chunk, V, device=x.device, dtype=torch.bfloat16)
         for t0 in range(0, T, chunk):
@@ -561,20 +571,26 @@ class _LinearCrossEntropyFn(torch.autograd.Function):
                                                       ignore_index, need_grad)
             if need_grad:
                 gemm(lg, wb, out=dx[t0:t1])  # [n, V] @ [V, K]
-                gemm(lg.t(), x[t0:t1], out=dw, accumulate=True, split_k=1)  # [V, n] @ [n, K]
+                gemm(lg.t(), x[t0:t1], out=dw, accumulate=t0 > 0, split_k=1)  # [V, n] @ [n, K]
         loss = row_loss.sum() * inv_valid
         if need_grad:
             ctx.save_for_backward(dx, dw)
             ctx.w_dtype = weight.dtype
+            # with saved-tensor hooks what comes back in the backward pass may belong to whoever set them
+            ctx.plain_save = torch._C._autograd._top_saved_tensors_default_hooks(False) is None
         return loss
 
     @staticmethod
     def backward(ctx, dloss):
         dx, dw = ctx.saved_tensors
-        dxo = dx * dloss.to(dx.dtype) if ctx.needs_input_grad[0] else None
+        # When the graph is not kept, the kept gradients are scaled where they lie and handed on (a plain backward pass
+        # has dloss = 1 and moves nothing); otherwise they stay as they are for the next backward pass.
+        own = (ctx.plain_save and not torch.is_grad_enabled()
+               and not torch._C._autograd._get_current_graph_task_keep_graph())
+        dxo = _times_scalar(dx, dloss, own) if ctx.needs_input_grad[0] else None
         dwo = None
         if ctx.needs_input_grad[1]:
-            dwo = dw * dloss
+            dwo = _times_scalar(dw, dloss, own)
             if ctx.w_dtype != torch.float32:
                 dwo = dwo.to(ctx.w_dtype)
         return dxo, dwo, None, None, None

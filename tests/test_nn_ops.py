@@ -206,6 +206,36 @@ def test_linear_cross_entropy(vocab):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("tokens,chunk", [(256, 8192), (300, 128)])
+def test_linear_cross_entropy_backward_twice_and_scaled(tokens, chunk):
+    """The gradients kept by the forward pass are scaled in place only when nobody needs them again: a kept graph gives
+    the same gradients in every pass, and a scaled loss the scaled ones (bf16 dx: the scale is a power of two)."""
+    torch.manual_seed(3)
+    x = torch.randn(tokens, 64, device="cuda").bfloat16().requires_grad_()
+    # logits of about 0.8: rounded to bf16 they move by up to 2^-8, and so do the probabilities
+    w = (0.1 * torch.randn(512, 64, device="cuda")).requires_grad_()
+    t = torch.randint(0, 512, (tokens,), device="cuda")
+    t[5] = -1
+    run = lambda: N.linear_cross_entropy(x, w, t, chunk_tokens=chunk)
+    gx, gw = torch.autograd.grad(run(), (x, w))
+    logits = (x.detach().float() @ w.detach().bfloat16().float().t()).requires_grad_()
+    F.cross_entropy(logits, t, ignore_index=-1).backward()
+    _close(gw, logits.grad.t() @ x.detach().float(), 1e-2)
+    loss = run()
+    for _ in range(2):
+        a, b = torch.autograd.grad(0.25 * loss, (x, w), retain_graph=True)
+        assert torch.equal(a, 0.25 * gx) and torch.allclose(b, 0.25 * gw, rtol=1e-5, atol=1e-8)
+    a, b = torch.autograd.grad(0.25 * loss, (x, w))
+    assert torch.equal(a, 0.25 * gx) and torch.allclose(b, 0.25 * gw, rtol=1e-5, atol=1e-8)
+    held = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda v: held.append(v) or v, lambda v: v):
+        loss = run()
+    copies = [v.clone() for v in held]
+    torch.autograd.grad(0.25 * loss, (x, w))
+    assert all(torch.equal(a, b) for a, b in zip(held, copies))
+
+
+@pytest.mark.gpu
 def test_fused_mlp_matches_unfused_reference():
     T, D = 520, 256
     x = torch.randn(T, D, device="cuda").bfloat16().requires_grad_()

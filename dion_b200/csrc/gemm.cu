@@ -1575,7 +1575,8 @@ Tiling choose_tiling(const GemmArgs& a) {
   int bn = a.block_n;
   // symmetric products with long K and enough 256 x 256 tiles on and above the diagonal run on CTA pairs
   // as well (half the B traffic per CTA, wide MMAs); short K is bound by the epilogue, where 128-wide
-  // tiles spread the mirrored stores over more CTAs
+  // tiles spread the mirrored stores over more CTAs.  With bf16 results stored by TMA pairs pay from K = 512 on
+  // (48 x 768 x 768: 43 -> 37 us).
   bool sym_pair = false;
   if (a.symmetric) {
     const long long tn = (a.N + 255) / 256;
@@ -1584,7 +1585,7 @@ Tiling choose_tiling(const GemmArgs& a) {
       const char* e = getenv("DION_B200_GEMM_SYM_PAIR");
       return (e && e[0] == '0') ? 0 : 1;
     }();
-    sym_pair = sym_pair_env && a.pair >= 0 && a.split_k == 1 && a.K >= 1024 && a.N >= 512 && t >= num_sms() / 2 / 2 &&
+    sym_pair = sym_pair_env && a.pair >= 0 && a.split_k == 1 && a.K >= (a.ab_dtype == kBF16 && a.d_dtype == kBF16 ? 512 : 1024) && a.N >= 512 && t >= num_sms() / 2 / 2 &&
                a.A_lo == nullptr && !a.split3;
     bn = sym_pair ? 256 : 128;
   } else if (bn != 64 && bn != 128 && bn != 256) {

@@ -368,8 +368,8 @@ __device__ __forceinline__ bool mbar_wait_for(uint64_t* bar, uint32_t parity, vo
 // tiles meet in shared memory, where every CTA adds its 1 / cluster-size of the rows over all CTAs in rank order
 // (the same bits in every run) and stores them.  For Gram matrices of tall factors: few tiles, long K.
 //
-// kTmaEpi (bf16 operands, C and D): the epilogue moves C and D with TMA.  Every epilogue warp owns a 4 KB
-// buffer, one box of 32 rows x 64 columns: the C box is fetched into it (the first of a tile while the accumulator is
+// kTmaEpi (C and D both bf16, or both fp32 for fp32 operands): the epilogue moves C and D with TMA.  Every epilogue warp
+// owns a 4 KB buffer, one box of 32 rows x 128 bytes: the C box is fetched into it (the first of a tile while the accumulator is
 // still being multiplied), replaced in place by the result and stored from it.  The path with generic loads and stores takes 4.6 us
 // for a 128 x 256 tile and 8.2 us with C, more than the multiply of K = 768 (5.6 us) that should hide it.
 template <bool kTf32, int kAMajor, int kBMajor, int kBlockN, bool kPair, bool kGather = false, bool kSplit = false,
@@ -380,7 +380,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
             const __grid_constant__ CUtensorMap tmap_mirror, const KernelParams p) {
   // kTmaEpi: the slots of the low halves hold the maps of D and C, tmap_mirror the map of D for transposed boxes
   static_assert(!(kSplit && kGather), "the converter warps and the copier warps use the same warp slots");
-  static_assert(!kTmaEpi || (!kTf32 && !kGather && kBlockN >= 128), "TMA epilogue: bf16, 128- and 256-column tiles");
+  static_assert(!kTmaEpi || (!kGather && !kClusterK && kBlockN >= 128), "TMA epilogue: 128- and 256-column tiles");
   static_assert(!kClusterK || (kSplit && kBlockN == 128), "K ranges over a cluster: splitting variants, 128-column tiles");
   using C = Cfg<kTf32, kAMajor, kBMajor, kBlockN, kPair, kSplit>;
   extern __shared__ uint8_t smem_raw[];
@@ -767,7 +767,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   } else if constexpr (kTmaEpi) {
     // ------------------------------------------------------------------ epilogue, C and D by TMA
     const int quad = warp & 3;
-    constexpr int kBoxes = kBlockN / 128;  // boxes of 64 columns per warp and tile
+    constexpr int kBoxCols = 128 / C::ES;                // C and D have the operands' element size
+    constexpr int kBoxes = kBlockN / 2 / kBoxCols;       // per warp and tile
     uint8_t* st = stage_area + (warp - 2) * kStageBytes;
     uint64_t* cb = &c_bar[warp - 2];
     uint32_t c_phase = 0;
@@ -792,7 +793,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       const int acc = it & 1;
       const bool mirror = p.symmetric && t.m_blk != t.n_blk;
       // boxes of this warp that lie inside the matrix (a box that only overlaps it is clipped by the copy)
-      const int boxes = row0 < p.M ? min(kBoxes, max(0, (p.N - col0 + 63) / 64)) : 0;
+      const int boxes = row0 < p.M ? min(kBoxes, max(0, (p.N - col0 + kBoxCols - 1) / kBoxCols)) : 0;
       if (use_c && boxes > 0) fetch_c(col0, row0, t.batch);
       if (!wait(&tmem_full[acc], (it >> 1) & 1)) {
         ok = false;
@@ -804,14 +805,23 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       const uint32_t taddr = tmem_base + acc * C::ACC_STRIDE + ((warp - 2) >> 2) * (kBlockN / 2) + ((uint32_t)(quad * 32) << 16);
 #pragma unroll 1
       for (int h = 0; h < boxes; ++h) {
-        const int col = col0 + h * 64;
+        const int col = col0 + h * kBoxCols;
         if (!use_c) buffer_free();
         else if (h > 0) fetch_c(col, row0, t.batch);
-        float v[64];
-        float(&lo)[32] = *reinterpret_cast<float(*)[32]>(&v[0]);
-        float(&hi)[32] = *reinterpret_cast<float(*)[32]>(&v[32]);
-        tmem_ld_32x32(taddr + h * 64, lo);
-        tmem_ld_32x32(taddr + h * 64 + 32, hi);
+        float v[kBoxCols];
+        float(&v0)[32] = *reinterpret_cast<float(*)[32]>(&v[0]);
+        tmem_ld_32x32(taddr + h * kBoxCols, v0);
+        if constexpr (kBoxCols == 64) {
+          float(&v1)[32] = *reinterpret_cast<float(*)[32]>(&v[32]);
+          tmem_ld_32x32(taddr + h * kBoxCols + 32, v1);
+        }
+        if constexpr (kSplit) {  // the cross terms, summed on their own
+          float x[32];
+          tmem_ld_32x32(taddr + kBlockN + h * kBoxCols, x);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 32; ++i) v[i] += x[i];
+        }
         tmem_ld_wait();
         if (h == boxes - 1) {
           // the accumulator is in registers: hand its columns back to the MMA warp
@@ -824,11 +834,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
         }
         if (p.alpha != 1.f) {
 #pragma unroll
-          for (int i = 0; i < 64; ++i) v[i] *= p.alpha;
+          for (int i = 0; i < kBoxCols; ++i) v[i] *= p.alpha;
         }
         if (p.act == kActRelu2) {
 #pragma unroll
-          for (int i = 0; i < 64; ++i) v[i] = apply_act(v[i], kActRelu2);
+          for (int i = 0; i < kBoxCols; ++i) v[i] = apply_act(v[i], kActRelu2);
         }
         if (use_c) {
           if (!wait(cb, c_phase)) {
@@ -838,24 +848,45 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
             break;
           }
           c_phase ^= 1u;
+          if constexpr (kTf32) {
+            // every lane reads the same factors (a broadcast load per factor); the splitting variants have no registers to
+            // spare for them and leave such products to the generic epilogue
+            const float* cs =
+                !kSplit && p.c_col_scale != nullptr ? p.c_col_scale + (long long)t.batch * p.N + col : nullptr;
 #pragma unroll
-          for (int s = 0; s < 8; ++s) {
-            const uint4 q = *reinterpret_cast<const uint4*>(st + stage_off(lane, s));
-            const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&q);
+            for (int s = 0; s < 8; ++s) {
+              float4 q = *reinterpret_cast<const float4*>(st + stage_off(lane, s));
+              if (cs != nullptr && col + 4 * s < p.N) {
+                q.x *= cs[4 * s];
+                q.y *= cs[4 * s + 1];
+                q.z *= cs[4 * s + 2];
+                q.w *= cs[4 * s + 3];
+              }
+              v[4 * s] += p.beta * q.x;
+              v[4 * s + 1] += p.beta * q.y;
+              v[4 * s + 2] += p.beta * q.z;
+              v[4 * s + 3] += p.beta * q.w;
+            }
+          } else {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const float2 f = __bfloat1622float2(h2[j]);
-              float& a = v[8 * s + 2 * j];
-              float& b = v[8 * s + 2 * j + 1];
-              if (p.act == kActMulRelu2GradSq) {
-                a *= 2.f * sqrt_approx(fmaxf(f.x, 0.f));
-                b *= 2.f * sqrt_approx(fmaxf(f.y, 0.f));
-              } else if (p.act == kActMulRelu2Grad) {
-                a *= 2.f * fmaxf(f.x, 0.f);
-                b *= 2.f * fmaxf(f.y, 0.f);
-              } else {
-                a += p.beta * f.x;
-                b += p.beta * f.y;
+            for (int s = 0; s < 8; ++s) {
+              const uint4 q = *reinterpret_cast<const uint4*>(st + stage_off(lane, s));
+              const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&q);
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const float2 f = __bfloat1622float2(h2[j]);
+                float& a = v[8 * s + 2 * j];
+                float& b = v[8 * s + 2 * j + 1];
+                if (p.act == kActMulRelu2GradSq) {
+                  a *= 2.f * sqrt_approx(fmaxf(f.x, 0.f));
+                  b *= 2.f * sqrt_approx(fmaxf(f.y, 0.f));
+                } else if (p.act == kActMulRelu2Grad) {
+                  a *= 2.f * fmaxf(f.x, 0.f);
+                  b *= 2.f * fmaxf(f.y, 0.f);
+                } else {
+                  a += p.beta * f.x;
+                  b += p.beta * f.y;
+                }
               }
             }
           }
@@ -863,11 +894,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
         // this lane's row over the C row it has just read
 #pragma unroll
         for (int s = 0; s < 8; ++s) {
-          uint4 q;
-          __nv_bfloat162* h2 = reinterpret_cast<__nv_bfloat162*>(&q);
+          if constexpr (kTf32) {
+            *reinterpret_cast<float4*>(st + stage_off(lane, s)) = make_float4(v[4 * s], v[4 * s + 1], v[4 * s + 2], v[4 * s + 3]);
+          } else {
+            uint4 q;
+            __nv_bfloat162* h2 = reinterpret_cast<__nv_bfloat162*>(&q);
 #pragma unroll
-          for (int j = 0; j < 4; ++j) h2[j] = __floats2bfloat162_rn(v[8 * s + 2 * j], v[8 * s + 2 * j + 1]);
-          *reinterpret_cast<uint4*>(st + stage_off(lane, s)) = q;
+            for (int j = 0; j < 4; ++j) h2[j] = __floats2bfloat162_rn(v[8 * s + 2 * j], v[8 * s + 2 * j + 1]);
+            *reinterpret_cast<uint4*>(st + stage_off(lane, s)) = q;
+          }
         }
         fence_proxy_async_shared();
         __syncwarp();
@@ -876,15 +911,20 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
           tma_store_commit();
         }
         if (mirror) {
-          // the block transposed, 64 rows of 32: every lane parks its row as a column
+          // the block transposed, 64 (bf16) or 32 (fp32) rows of 32: every lane parks its row as a column
           buffer_free();
-          __nv_bfloat16* tb = reinterpret_cast<__nv_bfloat16*>(st);
+          if constexpr (kTf32) {
 #pragma unroll
-          for (int i = 0; i < 64; ++i) tb[i * 32 + lane] = __float2bfloat16(v[i]);
+            for (int i = 0; i < 32; ++i) *reinterpret_cast<float*>(st + stage_off(i, lane >> 2) + (lane & 3) * 4) = v[i];
+          } else {
+            __nv_bfloat16* tb = reinterpret_cast<__nv_bfloat16*>(st);
+#pragma unroll
+            for (int i = 0; i < 64; ++i) tb[i * 32 + lane] = __float2bfloat16(v[i]);
+          }
           fence_proxy_async_shared();
           __syncwarp();
           if (lane == 0) {
-            tma_store_3d(&tmap_mirror, st, row0, col, t.batch);
+            tma_store_3d(kTf32 ? &tmap_a_lo : &tmap_mirror, st, row0, col, t.batch);
             tma_store_commit();
           }
         }
@@ -1432,10 +1472,11 @@ cudaError_t launch_cfg(const GemmArgs& a, const KernelParams& kp, cudaStream_t s
   }
   CUtensorMap tm = ta;  // never read
   if constexpr (kTmaEpi) {
-    if (!make_tmap(&ta_lo, a.D, kBF16, a.N, a.M, a.batch, a.ldd, a.d_batch_stride, 64, 32, kSwizzle128)) return cudaErrorInvalidValue;
-    if (a.C && !make_tmap(&tb_lo, a.C, kBF16, a.N, a.M, a.batch, a.ldc, a.c_batch_stride, 64, 32, kSwizzle128))
+    if (!make_tmap(&ta_lo, a.D, dt, a.N, a.M, a.batch, a.ldd, a.d_batch_stride, 128 / C::ES, 32, kSwizzle128))
       return cudaErrorInvalidValue;
-    if (a.symmetric && !make_tmap(&tm, a.D, kBF16, a.N, a.M, a.batch, a.ldd, a.d_batch_stride, 32, 64, kSwizzleNone))
+    if (a.C && !make_tmap(&tb_lo, a.C, dt, a.N, a.M, a.batch, a.ldc, a.c_batch_stride, 128 / C::ES, 32, kSwizzle128))
+      return cudaErrorInvalidValue;
+    if (!kTf32 && a.symmetric && !make_tmap(&tm, a.D, kBF16, a.N, a.M, a.batch, a.ldd, a.d_batch_stride, 32, 64, kSwizzleNone))
       return cudaErrorInvalidValue;
   }
 
@@ -1474,27 +1515,33 @@ cudaError_t launch_cfg(const GemmArgs& a, const KernelParams& kp, cudaStream_t s
   }
 }
 
-// Problems whose epilogue moves C and D with TMA: bf16 in and out, one destination, operands K-major / any, 16-byte
-// aligned rows of whole 16 bytes (every box starts at a multiple of 64 columns; a row is clipped in units of 16 bytes, so
-// that 1001 columns would lose what lies behind the 1001st).  With fp32 outputs, pointer arrays, a second output or
-// scattered tiles, and for tiles of 64 columns, the generic epilogue remains.
+// Problems whose epilogue moves C and D with TMA: C and D of the operands' type, one destination, operands K-major / any,
+// 16-byte aligned rows of whole 16 bytes (every box starts at a multiple of 128 bytes; a row is clipped in units of 16
+// bytes, so that 1001 columns would lose what lies behind the 1001st).  With outputs of another type, pointer arrays, a
+// second output or scattered tiles, and for tiles of 64 columns, the generic epilogue remains.
 bool tma_epilogue(const GemmArgs& a, const KernelParams& kp, int bn) {
-  return kp.stage && a.ab_dtype == kBF16 && a.a_major == kMajorK && a.d_dtype == kBF16 && a.epilogue == kEpiStore && bn >= 128 &&
-         a.split_k == 1 && !a.c_ptrs && !a.d_ptrs && !a.D2 && !a.d2_ptrs && !a.c_col_scale && a.scatter_mode == 0 &&
-         a.act != kActRelu2SavePre && kp.vec_d && a.D && a.N % 8 == 0 &&
-         (!a.C || (a.c_dtype == kBF16 && kp.vec_c)) && (a.batch == 1 || (a.d_batch_stride != 0 && (!a.C || a.c_batch_stride != 0)));
+  const bool bf16 = a.ab_dtype == kBF16;
+  return kp.stage && a.a_major == kMajorK && a.d_dtype == a.ab_dtype && a.epilogue == kEpiStore && bn >= 128 &&
+         a.split_k == 1 && !a.A_lo && !a.c_ptrs && !a.d_ptrs && !a.D2 && !a.d2_ptrs && a.scatter_mode == 0 &&
+         (bf16 ? a.act != kActRelu2SavePre && !a.c_col_scale : a.act == 0 || a.act == kActRelu2) && kp.vec_d && a.D &&
+         a.N % (bf16 ? 8 : 4) == 0 && (!a.C || (a.c_dtype == a.ab_dtype && kp.vec_c)) &&
+         (a.batch == 1 || (a.d_batch_stride != 0 && (!a.C || a.c_batch_stride != 0)));
+}
+// C is read only where it counts
+KernelParams tma_params(const KernelParams& kp) {
+  KernelParams kt = kp;
+  if (kp.beta == 0.f && kp.act != kActMulRelu2Grad && kp.act != kActMulRelu2GradSq) kt.C = nullptr;
+  return kt;
 }
 
 template <bool kTf32, int kAMajor, int kBMajor>
 cudaError_t launch_bn(const GemmArgs& a, const KernelParams& kp, int bn, bool pair, cudaStream_t s) {
-  if constexpr (!kTf32 && kAMajor == kMajorK) {
+  if constexpr (kAMajor == kMajorK) {
     if (tma_epilogue(a, kp, bn)) {
-      KernelParams kt = kp;
-      // C is read only where it counts
-      if (kp.beta == 0.f && kp.act != kActMulRelu2Grad && kp.act != kActMulRelu2GradSq) kt.C = nullptr;
-      if (pair) return launch_cfg<false, kAMajor, kBMajor, 256, true, false, false, false, true>(a, kt, s);
-      if (bn == 128) return launch_cfg<false, kAMajor, kBMajor, 128, false, false, false, false, true>(a, kt, s);
-      return launch_cfg<false, kAMajor, kBMajor, 256, false, false, false, false, true>(a, kt, s);
+      const KernelParams kt = tma_params(kp);
+      if (pair) return launch_cfg<kTf32, kAMajor, kBMajor, 256, true, false, false, false, true>(a, kt, s);
+      if (bn == 128) return launch_cfg<kTf32, kAMajor, kBMajor, 128, false, false, false, false, true>(a, kt, s);
+      return launch_cfg<kTf32, kAMajor, kBMajor, 256, false, false, false, false, true>(a, kt, s);
     }
   }
   if (pair) return launch_cfg<kTf32, kAMajor, kBMajor, 256, true>(a, kp, s);
@@ -1508,6 +1555,10 @@ cudaError_t launch_bn(const GemmArgs& a, const KernelParams& kp, int bn, bool pa
 // fp32 operands split in shared memory: 64- and 128-column tiles
 template <int kAMajor, int kBMajor>
 cudaError_t launch_split_bn(const GemmArgs& a, const KernelParams& kp, int bn, cudaStream_t s) {
+  if constexpr (kAMajor == kMajorK) {
+    if (!a.c_col_scale && tma_epilogue(a, kp, bn))
+      return launch_cfg<true, kAMajor, kBMajor, 128, false, false, true, false, true>(a, tma_params(kp), s);
+  }
   if (bn == 64) return launch_cfg<true, kAMajor, kBMajor, 64, false, false, true>(a, kp, s);
   return launch_cfg<true, kAMajor, kBMajor, 128, false, false, true>(a, kp, s);
 }

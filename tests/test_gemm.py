@@ -269,6 +269,41 @@ def test_tma_epilogue_moves_c_and_d_by_boxes(M, N, K, batch, mode):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("mode", ["plain", "inplace", "col_scale", "symmetric"])
+@pytest.mark.parametrize("split3", [False, True])
+@pytest.mark.parametrize("M,N,K,batch", [(1, 132, 40, 1), (300, 516, 72, 2), (2049, 1000, 1096, 1), (4100, 2056, 1024, 1),
+                                         (777, 200, 768, 3)])
+def test_tma_epilogue_fp32(M, N, K, batch, split3, mode):
+    """The same for fp32 C and D.  tf32 operands lose up to 2^-10 of each factor (errors of K products add up like their
+    squares), split ones 2^-21; the accumulator drops up to 2^-23 of its value with each of K / 8 multiplies."""
+    if mode == "symmetric":
+        N = M = M // 4 * 4 + 4
+    shape = lambda *s: s if batch == 1 else (batch, *s)
+    a = torch.randn(*shape(M, K), device="cuda")
+    w = a if mode == "symmetric" else torch.randn(*shape(N, K), device="cuda")
+    store = torch.full(shape(M, N + 20), 7.0, device="cuda")
+    out = store[..., :N]
+    ref = a.double() @ w.double().transpose(-1, -2)
+    kw = {}
+    if mode == "inplace":
+        out.copy_(torch.randn_like(out))
+        kw, ref = dict(c=out, beta=-0.5, alpha=2.0), 2 * ref - 0.5 * out.double()
+    elif mode == "col_scale":
+        c, d = torch.randn(*shape(M, N), device="cuda"), torch.rand(batch, N, device="cuda")
+        kw, ref = dict(c=c, beta=1.0, alpha=-1.0, c_col_scale=d), c.double() * d.double().view(*shape(1, N)) - ref
+    elif mode == "symmetric":
+        kw = dict(symmetric=True)
+    gemm(a, w.transpose(-1, -2), out=out, split3=split3, **kw)
+    big = (a.double().norm(dim=-1).amax() * w.double().norm(dim=-1).amax()).item() * abs(kw.get("alpha", 1.0))
+    bound = big * ((2 ** -20 + K / 8 * 2 ** -23) if split3 else 2 ** -8)
+    assert (out.double() - ref).abs().amax().item() < bound + 1e-6
+    assert torch.equal(store[..., N:], torch.full_like(store[..., N:], 7.0))
+    from dion_b200 import ops
+
+    ops.check_status()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("batch,rows,r", [(1, 40, 128), (12, 3072, 96), (4, 2056, 512), (3, 5000, 200), (1, 4096, 130),
                                           (2, 776, 8), (40, 160, 96)])
 def test_gram_of_tall_factors_sums_k_ranges_over_a_cluster(batch, rows, r):

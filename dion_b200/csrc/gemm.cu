@@ -98,7 +98,7 @@ struct KernelParams {
 // kSplit: fp32 operands are split into tf32 hi / lo halves inside the kernel (see the converter warps).
 template <bool kTf32, int kAMajor, int kBMajor, int kBlockN, bool kPair = false, bool kSplit = false>
 struct Cfg {
-  static_assert(!kSplit || (kTf32 && !kPair && kBlockN <= 128), "in-kernel splitting: fp32 operands, unpaired tiles of up to 128 columns");
+  static_assert(!kSplit || (kTf32 && kBlockN <= (kPair ? 256 : 128)), "in-kernel splitting: fp32 operands, tiles of up to 128 columns per CTA");
   static constexpr int ES = kTf32 ? 4 : 2;
   static constexpr int BK = 128 / ES;      // K elements per stage (one 128B swizzle span)
   static constexpr int CH = 128 / ES;      // M/N elements per 128B chunk (MN-major tiles)
@@ -113,14 +113,17 @@ struct Cfg {
   // kSplit keeps the lo halves of a stage right behind its hi halves (same layout, LO_OFFSET further on)
   static constexpr int STAGE_STRIDE = kSplit ? 2 * STAGE_BYTES : STAGE_BYTES;
   static constexpr int LO_OFFSET = STAGE_BYTES;
-  static constexpr int STAGES = 196608 / STAGE_STRIDE;  // 4 / 6 / 8 stages in 192 KB (3 / 4 when splitting)
-  // Two accumulator buffers (the epilogue of one tile overlaps the main loop of the next).  fp32 operands
-  // on tiles up to 128 columns get a second accumulator per buffer, for the small cross terms of a
-  // hi / lo product: added into the large accumulator one by one they would lose their low bits at
+  static constexpr int STAGES = 196608 / STAGE_STRIDE;  // 4 / 6 / 8 stages in 192 KB (3 / 4 when splitting, 3 in pairs)
+  // fp32 operands on tiles up to 128 columns, and split ones on any, get a second accumulator for the small cross
+  // terms of a hi / lo product: added into the large accumulator one by one they would lose their low bits at
   // every step, summed on their own and added once in the epilogue they do not.
-  static constexpr bool CROSS_ACC = kTf32 && !kPair && kBlockN <= 128;
+  static constexpr bool CROSS_ACC = kTf32 && ((!kPair && kBlockN <= 128) || kSplit);
   static constexpr int ACC_STRIDE = CROSS_ACC ? 2 * kBlockN : kBlockN;
-  static constexpr int TMEM_COLS = (2 * ACC_STRIDE <= 32) ? 32 : 2 * ACC_STRIDE;  // power of two
+  // Two accumulator buffers (the epilogue of one tile overlaps the main loop of the next) where tensor memory holds them
+  static constexpr int ACC_BUFS = 2 * ACC_STRIDE <= 512 ? 2 : 1;
+  static constexpr int TMEM_COLS = (ACC_BUFS * ACC_STRIDE <= 32) ? 32 : ACC_BUFS * ACC_STRIDE;  // power of two
+  __device__ static int acc_of(int it) { return ACC_BUFS == 2 ? it & 1 : 0; }               // buffer of the it-th tile
+  __device__ static uint32_t acc_phase_of(int it) { return (ACC_BUFS == 2 ? it >> 1 : it) & 1; }
   static constexpr int SMEM_BYTES = STAGES * STAGE_STRIDE + 1024 /*align*/ + 1024 /*barriers*/ + 8 * 32 * 128 /*epilogue staging*/;
   // descriptor strides
   static constexpr uint32_t A_LBO = (kAMajor == kMajorK) ? 16u : (uint32_t)BK * 128u;
@@ -362,7 +365,9 @@ __device__ __forceinline__ bool mbar_wait_for(uint64_t* bar, uint32_t parity, vo
 // fp32 operands as tf32 by dropping their low 13 mantissa bits.  The MMA warp then issues hi*hi into the main accumulator
 // and lo*hi, hi*lo into the cross-term accumulator for every K-step.  Operand bytes cross L2 once instead of three times.
 // Bound by shared memory: per 32 KB stage 32 KB from TMA, 32 KB read and 32 KB written here and 96 KB read by the three
-// multiplies, about 1500 cycles against 768 of multiplying.
+// multiplies, about 1500 cycles against 768 of multiplying.  A CTA pair on a 256 x 256 tile moves the same bytes per CTA
+// for twice the products (1536 cycles of multiplying), but its main and cross-term accumulators fill tensor memory, so
+// that the epilogue does not overlap the next tile.
 //
 // kClusterK (with kSplit): the CTAs of a cluster share one output tile, each multiplies a range of K; the partial
 // tiles meet in shared memory, where every CTA adds its 1 / cluster-size of the rows over all CTAs in rank order
@@ -424,7 +429,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     for (int s = 0; s < C::STAGES; ++s) {
       mbar_init(&full_bar[s], 1);
       mbar_init(&empty_bar[s], 1);
-      if constexpr (kSplit) mbar_init(&conv_bar[s], kNumSplitThreads / 32);
+      if constexpr (kSplit) mbar_init(&conv_bar[s], (kPair ? 2 : 1) * kNumSplitThreads / 32);
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tmem_full[a], 1);
@@ -456,7 +461,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
 
   const int kb_per_split = p.kblocks_per_split;
   // diagonal tile of x^T x with the same rows on both sides: B is A's tile, loaded and split once
-  auto one_operand = [&](const TileCoord& t) -> bool { return kSplit && kBlockN == kBlockM && p.b_is_a && t.m_blk == t.n_blk; };
+  // (in a pair each CTA's half of B are its own rows of A)
+  auto one_operand = [&](const TileCoord& t) -> bool { return kSplit && kBlockN == C::TILE_M && p.b_is_a && t.m_blk == t.n_blk; };
   // every wait inside the pipeline; the all-gather variant allows for the time another GPU may take
   auto wait = [&](uint64_t* bar, uint32_t parity) -> bool {
     if constexpr (kGather) return mbar_wait_for(bar, parity, abort_flag, kWaitBudgetNs + p.g.budget_ns);
@@ -504,11 +510,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
             if (p.status) atomicCAS(p.status, 0, kStatusProducerTimeout);
             break;
           }
-          // the leader's full barrier collects the bytes of both CTAs
-          if (cta_rank == 0) mbar_arrive_expect_tx(&full_bar[stage], skip_b ? C::A_BYTES : C::TX_BYTES);
-          const uint32_t bar = kPair ? mapa_shared(smem_u32(&full_bar[stage]), 0) : smem_u32(&full_bar[stage]);
+          // the leader's full barrier collects the bytes of both CTAs; where operands are split every CTA waits for its own
+          constexpr bool kJoint = kPair && !kSplit;
+          if (!kJoint || cta_rank == 0)
+            mbar_arrive_expect_tx(&full_bar[stage], skip_b ? C::A_BYTES : kJoint ? C::TX_BYTES : C::STAGE_BYTES);
+          const uint32_t bar = kJoint ? mapa_shared(smem_u32(&full_bar[stage]), 0) : smem_u32(&full_bar[stage]);
           auto load = [&](void* dst, const CUtensorMap* map, int c0, int c1) {
-            if constexpr (kPair) tma_load_3d_pair(dst, map, bar, c0, c1, t.batch);
+            if constexpr (kJoint) tma_load_3d_pair(dst, map, bar, c0, c1, t.batch);
             else tma_load_3d(dst, map, &full_bar[stage], c0, c1, t.batch);
           };
           uint8_t* sa = smem + stage * C::STAGE_STRIDE;
@@ -560,8 +568,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
         const int kb0 = (kClusterK ? k_rank : t.split) * kb_per_split;
         const int kb1 = min(kb0 + kb_per_split, p.kblocks_total);
         const int b_off = one_operand(t) ? 0 : C::A_BYTES;
-        const int acc = it & 1;
-        const uint32_t acc_phase = (it >> 1) & 1;
+        const int acc = C::acc_of(it);
+        const uint32_t acc_phase = C::acc_phase_of(it);
         if (!wait(&tmem_empty[acc], acc_phase ^ 1u)) {
           ok = false;
           *abort_flag = 1;
@@ -583,7 +591,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
           }
           // the operands of a stage are ready when TMA delivered them - or, when they are split in
           // shared memory, when the converter warps are through with the stage
-          if (!wait(kSplit ? &conv_bar[stage] : &full_bar[stage], phase)) {
+          const bool there = kSplit && kPair ? mbar_wait<true>(&conv_bar[stage], phase, abort_flag)
+                                             : wait(kSplit ? &conv_bar[stage] : &full_bar[stage], phase);
+          if (!there) {
             ok = false;
             *abort_flag = 1;
             if (p.status) atomicCAS(p.status, 0, kStatusMmaTimeout);
@@ -600,9 +610,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
               const uint64_t da_lo = make_smem_desc(sa + C::LO_OFFSET + j * C::A_KSTEP, C::A_LBO, C::A_SBO, C::A_LAYOUT);
               const uint64_t db_lo = make_smem_desc(sb + C::LO_OFFSET + j * C::B_KSTEP, C::B_LBO, C::B_SBO, C::B_LAYOUT);
               const uint32_t first = (!fresh || j > 0) ? 1u : 0u;
-              umma_ss<true>(d_main, da, db, idesc, first);                 // hi * hi
-              umma_ss<true>(d_main + kBlockN, da_lo, db, idesc, first);    // lo * hi
-              umma_ss<true>(d_main + kBlockN, da, db_lo, idesc, 1u);       // hi * lo
+              auto mma = [&](uint32_t d, uint64_t x, uint64_t y, uint32_t accumulate) {
+                if constexpr (kPair) umma_ss_pair<true>(d, x, y, idesc, accumulate);
+                else umma_ss<true>(d, x, y, idesc, accumulate);
+              };
+              mma(d_main, da, db, first);                 // hi * hi
+              mma(d_main + kBlockN, da_lo, db, first);    // lo * hi
+              mma(d_main + kBlockN, da, db_lo, 1u);       // hi * lo
             } else if constexpr (kPair) {
               umma_ss_pair<kTf32>(d_tmem, da, db, idesc, (!fresh || j > 0) ? 1u : 0u);
             } else {
@@ -655,7 +669,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
         // these stores are read by the tensor core (async proxy)
         fence_proxy_async_all();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&conv_bar[stage]);
+        if (lane == 0) {  // the leader issues the multiplies
+          if (cta_rank == 0) mbar_arrive(&conv_bar[stage]);
+          else mbar_arrive_cluster(mapa_shared(smem_u32(&conv_bar[stage]), 0));
+        }
         if (++stage == C::STAGES) {
           stage = 0;
           phase ^= 1u;
@@ -790,12 +807,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       const TileCoord t = decode_tile<false>(p, tile);
       const int row0 = t.m_blk * C::TILE_M + (int)cta_rank * kBlockM + quad * 32;
       const int col0 = t.n_blk * kBlockN + ((warp - 2) >> 2) * (kBlockN / 2);
-      const int acc = it & 1;
+      const int acc = C::acc_of(it);
       const bool mirror = p.symmetric && t.m_blk != t.n_blk;
       // boxes of this warp that lie inside the matrix (a box that only overlaps it is clipped by the copy)
       const int boxes = row0 < p.M ? min(kBoxes, max(0, (p.N - col0 + kBoxCols - 1) / kBoxCols)) : 0;
       if (use_c && boxes > 0) fetch_c(col0, row0, t.batch);
-      if (!wait(&tmem_full[acc], (it >> 1) & 1)) {
+      if (!wait(&tmem_full[acc], C::acc_phase_of(it))) {
         ok = false;
         *abort_flag = 1;
         if (p.status) atomicCAS(p.status, 0, kStatusEpilogueTimeout);
@@ -948,8 +965,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       const TileCoord t = decode_tile<kGather>(p, tile);
       const int m0 = t.m_blk * C::TILE_M + (int)cta_rank * kBlockM;
       const int n0 = t.n_blk * kBlockN;
-      const int acc = it & 1;
-      const uint32_t acc_phase = (it >> 1) & 1;
+      const int acc = C::acc_of(it);
+      const uint32_t acc_phase = C::acc_phase_of(it);
       const int kb0 = (kClusterK ? k_rank : t.split) * kb_per_split;
       const bool has_work = kb0 < p.kblocks_total;
       if constexpr (kClusterK) {
@@ -1555,6 +1572,9 @@ cudaError_t launch_bn(const GemmArgs& a, const KernelParams& kp, int bn, bool pa
 // fp32 operands split in shared memory: 64- and 128-column tiles
 template <int kAMajor, int kBMajor>
 cudaError_t launch_split_bn(const GemmArgs& a, const KernelParams& kp, int bn, cudaStream_t s) {
+  if constexpr (kAMajor == kMajorK || kAMajor == kBMajor) {
+    if (bn == 256) return launch_cfg<true, kAMajor, kBMajor, 256, true, false, true, false, true>(a, tma_params(kp), s);
+  }
   if constexpr (kAMajor == kMajorK) {
     if (!a.c_col_scale && tma_epilogue(a, kp, bn))
       return launch_cfg<true, kAMajor, kBMajor, 128, false, false, true, false, true>(a, tma_params(kp), s);
@@ -1563,11 +1583,15 @@ cudaError_t launch_split_bn(const GemmArgs& a, const KernelParams& kp, int bn, c
   return launch_cfg<true, kAMajor, kBMajor, 128, false, false, true>(a, kp, s);
 }
 
+bool aligned16(const void* p, long long ld, int es) {
+  return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && ((ld * es) & 15) == 0;
+}
+
 // CTAs of a cluster that share one output tile of a Gram product (1: no sharing).  Time is taken as waves of tiles
 // times K blocks per CTA, plus what every tile costs besides (pipeline fill, the exchange of the partial tiles): about
 // kTileCost blocks.  One matrix of 14336 x 512 (10 tiles, 448 blocks) takes 8, as do twelve of 3072 x 96; 48 of
 // 768 x 768 (1008 tiles, 24 blocks) fill the chip by themselves and take 1.
-int choose_cluster_k(const GemmArgs& a, const KernelParams& kp, int bn) {
+int choose_cluster_k(const GemmArgs& a, const KernelParams& kp, int bn, long long* blocks = nullptr) {
   if (!a.symmetric || bn != 128 || a.a_major != kMajorMN || a.b_major != kMajorMN || a.d_dtype != kF32 ||
       a.epilogue != kEpiStore || a.act != 0 || a.C || a.c_ptrs || a.D2 || a.d2_ptrs || a.d_ptrs || a.scatter_mode != 0 ||
       a.max_ctas > 0)
@@ -1586,11 +1610,40 @@ int choose_cluster_k(const GemmArgs& a, const KernelParams& kp, int bn) {
       best_cost = cost;
     }
   }
+  if (blocks) *blocks = best_cost;
   return best;
 }
 
+// Split products on CTA pairs.  Cycles per K block: about 1500 for a 128 x 128 tile (shared memory), 1536 for a 256 x 256
+// tile of a pair (tensor core), which also shows about 5000 cycles of epilogue.  Both sides are counted in waves; where
+// few tiles share a long K (choose_cluster_k) the unpaired side is what that takes.
+bool split_pair(const GemmArgs& a) {
+  if (!a.split3 || a.pair < 0 || a.block_n != 0 || a.max_ctas > 0 || a.d_dtype != kF32 || a.epilogue != kEpiStore || a.act != 0 ||
+      a.c_ptrs || a.d_ptrs || a.D2 || a.d2_ptrs || a.c_col_scale || a.scatter_mode != 0 || !a.D || a.N % 4 != 0 || a.N <= 128 ||
+      a.M <= 128 || (a.C && a.c_dtype != kF32))
+    return false;
+  if (a.a_major != kMajorK && !(a.symmetric && a.b_major == kMajorMN)) return false;
+  if (!aligned16(a.D, a.ldd, 4) || (a.batch > 1 && (a.d_batch_stride == 0 || a.d_batch_stride % 4 != 0))) return false;
+  if (a.C && (!aligned16(a.C, a.ldc, 4) || (a.batch > 1 && (a.c_batch_stride == 0 || a.c_batch_stride % 4 != 0)))) return false;
+  const long long kb = (a.K + 31) / 32, sms = num_sms();
+  auto tiles = [&](long long t) {
+    const long long m = (a.M + t - 1) / t, n = (a.N + t - 1) / t;
+    return (a.symmetric ? n * (n + 1) / 2 : m * n) * a.batch;
+  };
+  const long long t128 = tiles(128);
+  long long unpaired = (t128 + sms - 1) / sms * kb * 1500;
+  KernelParams kp;
+  memset(&kp, 0, sizeof(kp));
+  kp.total_tiles = (int)(t128 < 0x7fffffff ? t128 : 0x7fffffff);
+  kp.kblocks_total = (int)kb;
+  long long shared_k = 0;
+  if (choose_cluster_k(a, kp, 128, &shared_k) > 1) unpaired = shared_k * 1500;
+  const long long paired = (tiles(256) + sms / 2 - 1) / (sms / 2) * (kb * 1536 + 5000);
+  return paired < unpaired;
+}
+
 cudaError_t launch_split(const GemmArgs& a, const KernelParams& kp, int bn, cudaStream_t s) {
-  const int ck = choose_cluster_k(a, kp, bn);
+  const int ck = bn == 256 ? 1 : choose_cluster_k(a, kp, bn);
   if (ck > 1) {
     KernelParams kc = kp;
     kc.cluster_k = ck;
@@ -1675,8 +1728,9 @@ Tiling choose_tiling(const GemmArgs& a) {
 
   if (sym_pair) pair = true;
   if (a.A_lo != nullptr || a.split3) {  // the cross-term accumulator exists on unpaired tiles of up to 128 columns
-    pair = false;
-    if (bn > 128) bn = 128;
+    pair = a.split3 && split_pair(a);
+    if (pair) bn = 256;
+    else if (bn > 128) bn = 128;
   }
   if (a.gather.world > 0 && bn == 64) bn = 128;  // the all-gather variant is built for 128- and 256-wide tiles
   Tiling t;
@@ -1717,10 +1771,6 @@ bool plan_gather(const GemmArgs& a, const Tiling& tl, GatherParams* g) {
   g->ready = ga.counters ? ga.counters + 2 : nullptr;
   g->budget_ns = (unsigned long long)(ga.budget_ns > 0 ? ga.budget_ns : (long long)kWaitBudgetNs);
   return true;
-}
-
-bool aligned16(const void* p, long long ld, int es) {
-  return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && ((ld * es) & 15) == 0;
 }
 
 }  // namespace

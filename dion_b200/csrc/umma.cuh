@@ -78,8 +78,20 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t by
       : "memory");
 }
 
+// kCluster: acquires what other CTAs of the cluster released by arriving here
+template <bool kCluster = false>
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
+  if constexpr (kCluster) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+  }
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
@@ -92,18 +104,19 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 
 // Bounded wait.  Returns false when the budget ran out or another role of this
 // CTA already gave up (`*abort_flag != 0`).
+template <bool kCluster = false>
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
                                           volatile int* abort_flag) {
 #pragma unroll 1
   for (int i = 0; i < 64; ++i) {
-    if (mbar_try_wait(bar, parity)) return true;
+    if (mbar_try_wait<kCluster>(bar, parity)) return true;
   }
   const unsigned long long t0 = global_timer_ns();
 #pragma unroll 1
   for (;;) {
 #pragma unroll 1
     for (int i = 0; i < 128; ++i) {
-      if (mbar_try_wait(bar, parity)) return true;
+      if (mbar_try_wait<kCluster>(bar, parity)) return true;
     }
     if (*abort_flag != 0) return false;
     if (global_timer_ns() - t0 > kWaitBudgetNs) return false;

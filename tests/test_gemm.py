@@ -305,11 +305,11 @@ def test_tma_epilogue_fp32(M, N, K, batch, split3, mode):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("batch,rows,r", [(1, 40, 128), (12, 3072, 96), (4, 2056, 512), (3, 5000, 200), (1, 4096, 130),
-                                          (2, 776, 8), (40, 160, 96)])
+                                          (2, 776, 8), (40, 160, 96), (48, 776, 520)])
 def test_gram_of_tall_factors_sums_k_ranges_over_a_cluster(batch, rows, r):
     """P^T P with few tiles and long K: the CTAs of a cluster take K ranges (2, 4 or 8 of them, some of them empty) and
-    add their partial tiles.  The tensor core's accumulator drops up to 2^-23 of its value with every multiply (8 rows
-    each), and the rows are divided by at least two; splitting the operands and adding the parts costs below 2^-21."""
+    add their partial tiles; the last shape has enough tiles for CTA pairs instead.  The tensor core's accumulator drops
+    up to 2^-23 of its value with every multiply (8 rows each); splitting the operands and adding parts costs below 2^-21."""
     x = torch.randn(batch, rows, r, device="cuda") + 0.25
     pitch = (r + 3) // 4 * 4
     buf = torch.zeros(batch, rows, pitch, device="cuda")
@@ -318,9 +318,9 @@ def test_gram_of_tall_factors_sums_k_ranges_over_a_cluster(batch, rows, r):
     out = torch.full((batch, r, r), float("nan"), device="cuda")
     gemm(p.transpose(-1, -2), p, out=out, symmetric=True, split3=True)
     ref = x.double().transpose(-1, -2) @ x.double()
-    assert ((out.double() - ref).abs().amax() / ref.abs().amax()).item() < rows / 16 * 2 ** -23 + 2 ** -21
-    if r > 128:  # blocks off the diagonal are mirrored (on it the two cross terms are added in either order)
-        assert torch.equal(out[:, :128, 128:], out[:, 128:, :128].transpose(-1, -2))
+    assert ((out.double() - ref).abs().amax() / ref.abs().amax()).item() < rows / 8 * 2 ** -23 + 2 ** -21
+    if r > 256:  # blocks off the diagonal are mirrored (on it the two cross terms are added in either order)
+        assert torch.equal(out[:, :256, 256:], out[:, 256:, :256].transpose(-1, -2))
     again = gemm(p.transpose(-1, -2), p, symmetric=True, split3=True)
     assert torch.equal(out, again)
 

@@ -560,6 +560,238 @@ chol_inverse_pair_kernel(const float* __restrict__ Gall, float* __restrict__ Zal
 }
 
 
+// ---------------------------------------------------------------------------------------------
+// Ranks up to 256: one CTA per matrix, everything in shared memory.  The matrix is kept as the 32 x 32 blocks of its lower
+// triangle, and the inverse is built in place: when block column k of the factor has been applied, its slots hold block
+// column k of Z.  Per block step k, with P_i = A_ik Linv^T (i > k) kept aside:
+//   A:  P_i;  Z_kj = Linv B_kj (j < k);  Z_kk = Linv
+//   B:  A_ij -= P_i P_j^T (k < j <= i);  Z_ij -= P_i Z_kj (j < k);  Z_ik = -P_i Linv
+// Every product is one warp's 32 x 32 x 32 outer-product loop; blocks of A are stored transposed (blk[col][row]) and those
+// of Z by rows, so that both operands of every product are read as vectors.  While phase B runs, warp 0 updates block
+// (k + 1, k + 1) first and factorises it (lane i owns row i), so that the serial part hides behind the products.
+// Bound by fp32 FMA and by that chain: 11 M FMA at rank 256.  72 matrices of rank 256: 117 us, of rank 96: 36 us; the kernel
+// with two CTAs per matrix below, which exchanges through global memory after every step, takes 448 and 152 us and
+// remains for larger ranks, whose triangle does not fit.
+constexpr int kTriMaxBlocks = 8;
+constexpr int kTriThreads = 512;
+constexpr int kTriLinvPitch = 36;  // Linv transposed: rows of whole 16 bytes that start in different banks
+
+// acc[4][8] += sum_q U[q][x0 + .] V[q][y0 + .]; the 32 lanes tile the 32 x 32 result
+__device__ __forceinline__ void tri_product(const float* __restrict__ U, int pu, const float* __restrict__ V, int pv, int lane,
+                                            float (&acc)[4][8]) {
+  const float* u = U + (lane >> 2) * 4;
+  const float* v = V + (lane & 3) * 8;
+#pragma unroll 8
+  for (int q = 0; q < 32; ++q) {
+    const float4 a = *reinterpret_cast<const float4*>(u + q * pu);
+    const float4 b0 = *reinterpret_cast<const float4*>(v + q * pv);
+    const float4 b1 = *reinterpret_cast<const float4*>(v + q * pv + 4);
+    const float av[4] = {a.x, a.y, a.z, a.w};
+    const float bv[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+  }
+}
+// blk[x][y] (pitch `p`) = or -= s * acc
+template <bool kSub>
+__device__ __forceinline__ void tri_store(float* blk, int p, int lane, const float (&acc)[4][8], float s) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    float4* o = reinterpret_cast<float4*>(blk + ((lane >> 2) * 4 + i) * p + (lane & 3) * 8);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float4 r = make_float4(s * acc[i][4 * h], s * acc[i][4 * h + 1], s * acc[i][4 * h + 2], s * acc[i][4 * h + 3]);
+      if constexpr (kSub) {
+        const float4 c = o[h];
+        r = make_float4(c.x - r.x, c.y - r.y, c.z - r.z, c.w - r.w);
+      }
+      o[h] = r;
+    }
+  }
+}
+
+// Cholesky factor of the block blk[col][row] and its inverse: linv[row][col] (pitch 32) and linv_t[col][row].  One warp,
+// lane i owns row i of the factor, then column i of the inverse.  A pivot that is not safely positive gets a unit pivot
+// and eliminates nothing.  Returns the number of such pivots among the first nb.
+__device__ __forceinline__ int tri_factor(const float* blk, float* lrow, float* dinv, float* linv, float* linv_t, int nb,
+                                          float pivot_floor, int lane, float* colmask) {
+  float a[32];
+#pragma unroll
+  for (int c = 0; c < 32; ++c) a[c] = blk[c * 32 + lane];
+  int clamped = 0;
+  float my_inv = 1.f;
+#pragma unroll
+  for (int j = 0; j < 32; ++j) {
+    const float d = __shfl_sync(0xffffffffu, a[j], j);
+    const bool bad = !(d > pivot_floor);
+    if (bad && j < nb) ++clamped;
+    if (colmask != nullptr && lane == 0 && j < nb) colmask[j] = bad ? 0.f : 1.f;
+    const float inv = bad ? 1.f : rsqrtf(d);
+    if (lane == j) my_inv = inv;
+    const float l = (lane > j && !bad) ? a[j] * inv : 0.f;
+    a[j] = l;
+#pragma unroll
+    for (int c = j + 1; c < 32; ++c) a[c] = fmaf(-l, __shfl_sync(0xffffffffu, l, c), a[c]);
+  }
+  // rows of L below the diagonal (entries at and above it are never read)
+#pragma unroll
+  for (int c = 0; c < 32; c += 4)
+    *reinterpret_cast<float4*>(lrow + lane * kTriLinvPitch + c) = make_float4(a[c], a[c + 1], a[c + 2], a[c + 3]);
+  dinv[lane] = my_inv;
+  __syncwarp();
+  // column `lane` of the inverse by forward substitution
+  float x[32];
+#pragma unroll
+  for (int i = 0; i < 32; ++i) {
+    float s0 = (i == lane) ? 1.f : 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+#pragma unroll
+    for (int k = 0; k < i; k += 4) {
+      const float4 l = *reinterpret_cast<const float4*>(lrow + i * kTriLinvPitch + k);
+      s0 = fmaf(-l.x, x[k], s0);
+      if (k + 1 < i) s1 = fmaf(-l.y, x[k + 1], s1);
+      if (k + 2 < i) s2 = fmaf(-l.z, x[k + 2], s2);
+      if (k + 3 < i) s3 = fmaf(-l.w, x[k + 3], s3);
+    }
+    x[i] = ((s0 + s1) + (s2 + s3)) * dinv[i];
+  }
+#pragma unroll
+  for (int i = 0; i < 32; ++i) linv[i * 32 + lane] = x[i];
+#pragma unroll
+  for (int i = 0; i < 32; i += 4)
+    *reinterpret_cast<float4*>(linv_t + lane * kTriLinvPitch + i) = make_float4(x[i], x[i + 1], x[i + 2], x[i + 3]);
+  __syncwarp();
+  return clamped;
+}
+
+// shared memory of n blocks per side, in floats
+__host__ __device__ constexpr int tri_smem_floats(int n) {
+  return n * (n + 1) / 2 * 1024        // the triangle
+         + 32 * 32 * n                 // P, transposed: [q][32 n]
+         + 2 * (1024 + 32 * kTriLinvPitch)  // Linv of this step and the next, both ways round
+         + 32 * kTriLinvPitch + 32     // rows of L, reciprocal pivots
+         + 32 * n;                     // Jacobi scaling
+}
+
+static_assert(tri_smem_floats(kTriMaxBlocks) * 4 <= 227 * 1024, "the triangle of rank 256 fits");
+
+__global__ void __launch_bounds__(kTriThreads, 1)
+chol_inverse_tri_kernel(const float* __restrict__ Gall, float* __restrict__ Zall, int* __restrict__ info, int r,
+                        long long ldg, long long g_batch_stride, float pivot_floor, int jacobi,
+                        float* __restrict__ colmask) {
+  extern __shared__ __align__(16) float sm[];
+  const int n = (r + 31) >> 5;
+  float* tri = sm;
+  float* PT = tri + n * (n + 1) / 2 * 1024;
+  const int pp = 32 * n;
+  float* linv_all = PT + 32 * pp;                      // [2][32][32]
+  float* linv_t_all = linv_all + 2 * 1024;             // [2][32][kTriLinvPitch]
+  float* lrow = linv_t_all + 2 * 32 * kTriLinvPitch;   // [32][kTriLinvPitch]
+  float* dinv = lrow + 32 * kTriLinvPitch;             // [32]
+  float* dscale = dinv + 32;                           // [32 n]
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, warps = blockDim.x >> 5;
+  const int b = blockIdx.x;
+  const float* G = Gall + (long long)b * g_batch_stride;
+  float* Z = Zall + (long long)b * r * r;
+  auto block = [&](int i, int j) { return tri + (i * (i + 1) / 2 + j) * 1024; };
+
+  for (int i = tid; i < pp; i += blockDim.x) {
+    float d = 0.f;
+    if (i < r) {
+      const float g = G[(long long)i * ldg + i];
+      d = !jacobi ? 1.f : ((g > 1e-30f) ? rsqrtf(g) : 0.f);
+    }
+    dscale[i] = d;
+  }
+  __syncthreads();
+  // A = D G D from the lower triangle, transposed by block; the identity in rows and columns from r on.  A warp covers
+  // 8 rows x 4 columns at a time: 16-byte pieces of G, four lanes to a bank on the way in.
+  for (int blk = warp; blk < n * (n + 1) / 2; blk += warps) {
+    int i = 0, j = blk;
+    while (j > i) j -= ++i;
+#pragma unroll 16
+    for (int part = 0; part < 32; ++part) {
+      const int row = (part & 3) * 8 + (lane >> 2), col = (part >> 2) * 4 + (lane & 3);
+      const int gr = i * 32 + row, gc = j * 32 + col;
+      float v = gr == gc ? 1.f : 0.f;
+      if (gr < r && gc <= gr) v = G[(long long)gr * ldg + gc] * dscale[gr] * dscale[gc];
+      tri[blk * 1024 + col * 32 + row] = v;
+    }
+  }
+  __syncthreads();
+
+  int clamped = 0;  // lane 0 of warp 0
+  auto factor = [&](int k) {
+    clamped += tri_factor(block(k, k), lrow, dinv, linv_all + (k & 1) * 1024, linv_t_all + (k & 1) * 32 * kTriLinvPitch,
+                          min(32, r - 32 * k), pivot_floor, lane,
+                          colmask != nullptr ? colmask + (long long)b * r + 32 * k : nullptr);
+  };
+  if (warp == 0) factor(0);
+  for (int k = 0; k < n; ++k) {
+    __syncthreads();  // Linv of step k, and all updates of step k - 1, are in place
+    const float* linv = linv_all + (k & 1) * 1024;
+    const float* linv_t = linv_t_all + (k & 1) * 32 * kTriLinvPitch;
+    const int m = n - 1 - k;  // block rows below
+    for (int it = warp; it < n; it += warps) {
+      float acc[4][8] = {};
+      if (it < m) {
+        const int i = k + 1 + it;
+        tri_product(linv_t, kTriLinvPitch, block(i, k), 32, lane, acc);  // P_i transposed: [q][row]
+        tri_store<false>(PT + i * 32, pp, lane, acc, 1.f);
+      } else if (it < n - 1) {
+        float* zk = block(k, it - m);
+        tri_product(linv_t, kTriLinvPitch, zk, 32, lane, acc);
+        __syncwarp();  // the block is this warp's alone
+        tri_store<false>(zk, 32, lane, acc, 1.f);
+      } else {
+        float4* d = reinterpret_cast<float4*>(block(k, k));
+        for (int q = lane; q < 256; q += 32) d[q] = reinterpret_cast<const float4*>(linv)[q];
+      }
+    }
+    __syncthreads();
+    if (m == 0) break;
+    const int nA = m * (m + 1) / 2, total = nA + m * (k + 1);
+    // warp 0 takes the next diagonal block and its factorisation, the others everything else (and warp 0 what is left
+    // over once there are fewer of them than work)
+    for (int it = warp == 0 ? 0 : warp; it < total; it += warps - 1) {
+      float acc[4][8] = {};
+      if (it < nA) {
+        int i = 0, j = it;
+        while (j > i) j -= ++i;
+        i += k + 1;
+        j += k + 1;
+        tri_product(PT + j * 32, pp, PT + i * 32, pp, lane, acc);
+        tri_store<true>(block(i, j), 32, lane, acc, 1.f);
+      } else {
+        const int q = it - nA;
+        const int i = k + 1 + q / (k + 1), j = q % (k + 1);
+        if (j < k) {
+          tri_product(PT + i * 32, pp, block(k, j), 32, lane, acc);
+          tri_store<true>(block(i, j), 32, lane, acc, 1.f);
+        } else {
+          tri_product(PT + i * 32, pp, linv, 32, lane, acc);
+          tri_store<false>(block(i, k), 32, lane, acc, -1.f);
+        }
+      }
+      if (warp == 0) {
+        __syncwarp();
+        factor(k + 1);
+        break;
+      }
+    }
+  }
+  // undo the Jacobi scaling: G = D^-1 L' L'^T D^-1  =>  L^{-1} = L'^{-1} D, i.e. scale column j by d_j
+  for (int i = warp; i < r; i += warps) {
+    for (int j = lane; j < r; j += 32) {
+      float v = 0.f;
+      if (j <= i) v = block(i >> 5, j >> 5)[(i & 31) * 32 + (j & 31)] * dscale[j];
+      Z[(long long)i * r + j] = v;
+    }
+  }
+  if (tid == 0 && info) info[b] = clamped;
+}
+
 // x = hi + lo with hi exactly representable in tf32 (low 13 mantissa bits cleared): the two
 // operands of a 3xTF32 product, written in one pass over x.
 __global__ void __launch_bounds__(256) split_tf32_kernel(const float4* __restrict__ x, float4* __restrict__ hi,
@@ -626,6 +858,21 @@ cudaError_t chol_inverse_launch(const float* G, float* Z, float* work, int* info
   constexpr int kMaxDevices = 64;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) dev = 0;
+  const int nblk = (r + 31) / 32;
+  if (nblk <= kTriMaxBlocks) {
+    const size_t smem = (size_t)tri_smem_floats(nblk) * sizeof(float);
+    static bool granted[kMaxDevices] = {};
+    if (!granted[dev]) {
+      cudaError_t e = cudaFuncSetAttribute(chol_inverse_tri_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)(tri_smem_floats(kTriMaxBlocks) * sizeof(float)));
+      if (e != cudaSuccess) return e;
+      granted[dev] = true;
+    }
+    // up to rank 128 no step has work for more than seven warps, and several matrices share an SM
+    chol_inverse_tri_kernel<<<batch, nblk <= 4 ? 256 : kTriThreads, smem, s>>>(G, Z, info, r, ldg, g_batch_stride, pivot_floor,
+                                                                             jac, colmask);
+    return cudaGetLastError();
+  }
   {
     // cluster-pair kernel (two CTAs per matrix); DION_B200_CHOL_PAIR=0 selects the single-CTA one
     static const int pair_env = [] {

@@ -50,6 +50,35 @@ def test_chol_inverse_kernel(r):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("r", [1, 8, 31, 32, 33, 72, 128, 129, 160, 250, 256])
+@pytest.mark.parametrize("jacobi", [True, False])
+def test_chol_inverse_of_a_triangle_in_shared_memory(r, jacobi):
+    """Ranks up to 256 at the edges of its 32 x 32 blocks: a strided view of well-conditioned matrices (the error of the
+    inverse is a small multiple of 2^-24 times the condition number, below 100, times the rank), one of them with a
+    column that depends on another: it gets a unit pivot, eliminates nothing and is counted."""
+    batch = 5
+    P = torch.randn(batch, 4 * r + 16, r, device="cuda", dtype=torch.float64)
+    if r > 8:
+        P[1, :, 7] = P[1, :, 3]
+    P = P / P.norm(dim=1, keepdim=True)
+    big = torch.full((batch, r + 4, r + 9), float("nan"), device="cuda")
+    G = big[:, 2:2 + r, 1:1 + r]
+    low = (P.transpose(1, 2) @ P).float()
+    G.copy_(torch.tril(low) + torch.triu(torch.full_like(low, float("nan")), 1))  # the upper triangle is not read
+    Z = torch.full((batch, r, r), float("nan"), device="cuda")
+    info = torch.full((batch,), -1, dtype=torch.int32, device="cuda")
+    mask = torch.full((batch, r), -1.0, device="cuda")
+    torch.ops.dion_b200.chol_inverse(G, Z, torch.empty_like(Z), info, 1e-5, jacobi, mask)
+    full = torch.tril(low.double()) + torch.tril(low.double(), -1).transpose(1, 2)
+    ref_mask = torch.empty(batch, r, device="cuda", dtype=torch.float64)
+    Zr, info_r = ops.chol_inverse_reference(full, 1e-5, jacobi=jacobi, colmask=ref_mask)
+    assert torch.equal(info.cpu(), info_r.cpu().int()) and int(info[1]) == (1 if r > 8 else 0)
+    assert torch.equal(mask.double(), ref_mask.double())
+    assert torch.equal(Z, torch.tril(Z))
+    assert ((Z.double() - Zr).norm() / Zr.norm()).item() < 100 * r * 2 ** -24 + 1e-6
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("r,batch", [(768, 80), (200, 7)])
 def test_chol_inverse_kernel_is_deterministic(r, batch):
     """The two CTAs that share a matrix exchange their updates through global memory; whichever of them

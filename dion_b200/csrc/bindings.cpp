@@ -71,8 +71,23 @@ void check_out(const Tensor& t, int64_t batch, int64_t M, int64_t N, const char*
   TORCH_CHECK(t.stride(-1) == 1, what, " must be row-major");
 }
 
-// d = act(alpha * a @ b) + beta * c   (a: [B,]M,K   b: [B,]K,N, any transposed views)
-void gemm(const Tensor& a, const Tensor& b, const std::optional<Tensor>& c, Tensor d,
+// A matrix view that TMA can address: a unit stride in one of its last two dimensions, base, pitch and batch stride
+// multiples of 16 bytes.
+bool tma_addressable(const Tensor& t) {
+  const int64_t es = t.element_size();
+  if (reinterpret_cast<uintptr_t>(t.data_ptr()) % 16) return false;
+  const int64_t s_row = t.stride(-2), s_col = t.stride(-1), rows = t.size(-2), cols = t.size(-1);
+  int64_t ld;
+  if (s_col == 1 && (s_row >= cols || rows == 1)) ld = rows > 1 ? s_row : std::max(s_row, cols);
+  else if (s_row == 1 && (s_col >= rows || cols == 1)) ld = cols > 1 ? s_col : std::max(s_col, rows);
+  else return false;
+  if ((ld * es) % 16) return false;
+  return !(t.dim() == 3 && t.size(0) > 1 && (t.stride(0) * es) % 16);
+}
+
+// d = act(alpha * a @ b) + beta * c   (a: [B,]M,K   b: [B,]K,N, any transposed views).  Returns false, and launches
+// nothing, for operands of other types, that TMA cannot address, or a d that is not row-major.
+bool gemm(const Tensor& a, const Tensor& b, const std::optional<Tensor>& c, Tensor d,
           const std::optional<Tensor>& d2, const std::optional<Tensor>& c_ptrs,
           const std::optional<Tensor>& d_ptrs, const std::optional<Tensor>& d2_ptrs, double alpha, double beta,
           int64_t act, int64_t epilogue, int64_t split_k, bool symmetric, int64_t block_n, int64_t pair,
@@ -81,6 +96,10 @@ void gemm(const Tensor& a, const Tensor& b, const std::optional<Tensor>& c, Tens
   TORCH_CHECK(a.is_cuda() && b.is_cuda(), "gemm operands must be CUDA tensors");
   TORCH_CHECK(a.scalar_type() == b.scalar_type(), "gemm operands must share a dtype");
   TORCH_CHECK(a.dim() == b.dim(), "gemm operands must both be 2-D or both 3-D");
+  if ((a.scalar_type() != at::kBFloat16 && a.scalar_type() != at::kFloat) || !tma_addressable(a) || !tma_addressable(b) ||
+      d.stride(-1) != 1)
+    return false;
+  TORCH_CHECK_VALUE(split_k <= 1 || epilogue == dion::kEpiAtomicAdd, "split_k > 1 needs accumulate=True");
   const c10::cuda::CUDAGuard guard(a.device());
   dion::GemmArgs g;
   g.ab_dtype = gemm_dtype(a, "a");
@@ -172,6 +191,7 @@ void gemm(const Tensor& a, const Tensor& b, const std::optional<Tensor>& c, Tens
   TORCH_CHECK(e == cudaSuccess, "dion_b200 gemm launch failed: ", cudaGetErrorString(e), " ",
               dion::gemm_last_error());
   g_launches.fetch_add(1, std::memory_order_relaxed);
+  return true;
 }
 
 
@@ -957,6 +977,74 @@ void attn_fwd(const Tensor& q, const Tensor& k, const Tensor& v, Tensor out, Ten
                                         at::cuda::getCurrentCUDAStream()));
 }
 
+// ----------------------------------------------------------------------------- launch sequences
+// The products of a whole Newton-Schulz call, or of a transformer block without autograd, issued from here: one after the
+// other through Python a launch costs 12 to 30 us of host time, more than most of these kernels run at small sizes.
+
+// d = alpha * a @ b + beta * c for operands that TMA can address
+void product(const Tensor& a, const Tensor& b, const std::optional<Tensor>& c, Tensor d, double alpha, double beta,
+             bool symmetric, const Tensor& status, int act = 0) {
+  TORCH_CHECK(gemm(a, b, c, d, {}, {}, {}, {}, alpha, beta, act, dion::kEpiStore, 1, symmetric, 0, 0, status, 1, {}, {}, {}, false),
+              "operand layout");
+}
+
+// X [B, m, n] bf16, contiguous: X / (|X|_F + eps), then for every triple (a, b, c) of coeffs
+//   A = X X^T,  X <- a X + (b A + c A A) X      (from the right with X^T X when m > n)
+Tensor newton_schulz_steps(const Tensor& X0, const std::optional<Tensor>& sumsq, double eps, std::vector<double> coeffs,
+                           Tensor status) {
+  TORCH_CHECK(X0.dim() == 3 && coeffs.size() % 3 == 0, "newton_schulz_steps: [B, m, n] and three coefficients per step");
+  const c10::cuda::CUDAGuard guard(X0.device());
+  const bool tall = X0.size(1) > X0.size(2);
+  const int64_t B = X0.size(0), k = tall ? X0.size(2) : X0.size(1);
+  Tensor X = at::empty_like(X0), Y = at::empty_like(X0);
+  frob_scale(X0, X, sumsq, eps);
+  Tensor A = at::empty({B, k, k}, X0.options()), P = at::empty_like(A);
+  for (size_t i = 0; i < coeffs.size(); i += 3) {
+    if (tall) product(X.transpose(1, 2), X, {}, A, 1., 0., true, status);
+    else product(X, X.transpose(1, 2), {}, A, 1., 0., true, status);
+    product(A, A.transpose(1, 2), A, P, coeffs[i + 2], coeffs[i + 1], true, status);
+    product(tall ? X : P, tall ? P : X, X, Y, 1., coeffs[i], false, status);
+    std::swap(X, Y);
+  }
+  return X;
+}
+
+// x [B, T, C] bf16 through one block of the GPT model: x + attention(norm(x)), then + MLP(norm(.)).  The kernels, their
+// order and their arguments are those of the differentiable functions; nothing is kept for a backward pass.
+Tensor gpt_block_fwd(const Tensor& x, const Tensor& wq, const Tensor& wk, const Tensor& wv, const Tensor& wo, const Tensor& wfc,
+                     const Tensor& wproj, const Tensor& cos, const Tensor& sin, int64_t D, double eps,
+                     bool kernel_attention, Tensor status) {
+  TORCH_CHECK(x.dim() == 3 && x.is_contiguous(), "gpt_block_fwd: x is [B, T, C], contiguous");
+  const c10::cuda::CUDAGuard guard(x.device());
+  const int64_t B = x.size(0), T = x.size(1), C = x.size(2), N = B * T, heads = wq.size(0) / D;
+  const Tensor x2 = x.view({N, C});
+  Tensor rstd = at::empty({N}, x.options().dtype(at::kFloat));
+  auto linear = [&](const Tensor& a, const Tensor& w, const std::optional<Tensor>& residual, int act) {
+    Tensor y = at::empty({N, w.size(0)}, x.options());
+    product(a, w.t(), residual, y, 1., residual.has_value() ? 1. : 0., false, status, act);
+    return y;
+  };
+  Tensor h = at::empty_like(x2);
+  rmsnorm_fwd(x2, {}, {}, h, rstd, eps);
+  Tensor q = linear(h, wq, {}, 0), k = linear(h, wk, {}, 0), v = linear(h, wv, {}, 0);
+  Tensor qo = at::empty_like(q), ko = at::empty_like(k);
+  rope_qknorm_fwd(q, k, qo, ko, cos, sin, T, heads, D, eps);
+  const Tensor q4 = qo.view({B, T, heads, D}), k4 = ko.view({B, T, heads, D}), v4 = v.view({B, T, heads, D});
+  Tensor y;
+  if (kernel_attention && T % 128 == 0 && B * heads <= 65535) {
+    y = at::empty_like(q4);
+    Tensor lse = at::empty({B, heads, T}, x.options().dtype(at::kFloat));
+    attn_fwd(q4, k4, v4, y, lse, 1. / std::sqrt((double)D), status);
+  } else {
+    y = at::scaled_dot_product_attention(q4.transpose(1, 2), k4.transpose(1, 2), v4.transpose(1, 2), {}, 0., true)
+            .transpose(1, 2);
+  }
+  const Tensor x3 = linear(y.reshape({N, C}), wo, x2, 0);
+  rmsnorm_fwd(x3, {}, {}, h, rstd, eps);
+  const Tensor u = linear(h, wfc, {}, dion::kActRelu2);
+  return linear(u, wproj, x3, 0).view({B, T, C});
+}
+
 void attn_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& d_o, const Tensor& lse,
               Tensor delta, Tensor dq, Tensor dk, Tensor dv, double scale, Tensor status) {
   const c10::cuda::CUDAGuard guard(q.device());
@@ -1096,7 +1184,12 @@ TORCH_LIBRARY(dion_b200, m) {
       "gemm(Tensor a, Tensor b, Tensor? c, Tensor(a!) d, Tensor(b!)? d2, Tensor? c_ptrs, Tensor? d_ptrs, "
       "Tensor? d2_ptrs, float alpha, float beta, int act, int epilogue, int split_k, bool symmetric, "
       "int block_n, int pair, Tensor? status, int d_dup=1, Tensor? a_lo=None, Tensor? b_lo=None, "
-      "Tensor? c_col_scale=None, bool split3=False) -> ()");
+      "Tensor? c_col_scale=None, bool split3=False) -> bool");
+  m.def(
+      "newton_schulz_steps(Tensor X, Tensor? sumsq, float eps, float[] coeffs, Tensor status) -> Tensor");
+  m.def(
+      "gpt_block_fwd(Tensor x, Tensor wq, Tensor wk, Tensor wv, Tensor wo, Tensor wfc, Tensor wproj, Tensor cos, "
+      "Tensor sin, int head_dim, float eps, bool kernel_attention, Tensor status) -> Tensor");
   m.def(
       "adamw_multi(Tensor(a!)[] X, Tensor[] G, Tensor(b!)[] M, Tensor(c!)[] V, Tensor(d!)[] shadow, float lr, "
       "float beta1, float beta2, float weight_decay, float eps, int step) -> ()");
@@ -1160,6 +1253,8 @@ TORCH_LIBRARY(dion_b200, m) {
 
 TORCH_LIBRARY_IMPL(dion_b200, CUDA, m) {
   m.impl("gemm", &gemm);
+  m.impl("newton_schulz_steps", &newton_schulz_steps);
+  m.impl("gpt_block_fwd", &gpt_block_fwd);
   m.impl("frob_scale", &frob_scale);
   m.impl("rmsnorm_fwd", &rmsnorm_fwd);
   m.impl("rmsnorm_bwd", &rmsnorm_bwd);

@@ -130,13 +130,41 @@ class MLP(nn.Module):
         return K.mlp(h, _local(self.c_fc.weight), _local(self.c_proj.weight), residual)
 
 
+def _plain(module: nn.Module, cls: type) -> bool:
+    """`module` is a `cls` as it was built: calling it runs that class's forward and nothing else."""
+    return (type(module) is cls and "forward" not in module.__dict__ and not module._forward_hooks
+            and not module._forward_pre_hooks and not module._backward_hooks and not module._backward_pre_hooks)
+
+
 class Block(nn.Module):
     def __init__(self, config: GPTConfig):
         super().__init__()
         self.attn = CausalSelfAttention(config)
         self.mlp = MLP(config)
 
+    def _forward_native(self, x: torch.Tensor):
+        """The block as one native call, for passes that record no gradients; None where the general path has to run
+        (hooks or replaced parts, tensor-parallel weights, other types and sizes than the kernels take).  Same kernels in
+        the same order, so the same bits."""
+        attn, mlp = self.attn, self.mlp
+        if not (K.native_forward_ok(x) and _plain(attn, CausalSelfAttention) and _plain(mlp, MLP)
+                and _plain(attn.rotary, Rotary) and attn.head_dim in (64, 128) and x.shape[-1] <= 4096):
+            return None
+        weights = (attn.c_q.weight, attn.c_k.weight, attn.c_v.weight, attn.c_proj.weight, mlp.c_fc.weight, mlp.c_proj.weight)
+        if any(type(w) is not nn.Parameter or not w.is_contiguous() or w.device != x.device for w in weights):
+            return None
+        shadows = [K.bf16_weight(w) for w in weights]
+        if any(w.data_ptr() % 16 for w in shadows) or not (weights[0].shape == weights[1].shape == weights[2].shape):
+            return None
+        cos, sin = attn.rotary.tables(x.shape[1], x.device)
+        return torch.ops.dion_b200.gpt_block_fwd(x, *shadows, cos, sin, attn.head_dim, K.RMS_EPS,
+                                                 K.ATTENTION_IMPL == "kernel", K.runtime.status_tensor(x.device))
+
     def forward(self, x: torch.Tensor, bt=None) -> torch.Tensor:
+        if bt is None and not torch.is_grad_enabled():
+            y = self._forward_native(x)
+            if y is not None:
+                return y
         x, h = K.norm_branch(x)
         x = self.attn(h, x, bt)
         x, h = K.norm_branch(x)
@@ -228,7 +256,7 @@ class GPT(nn.Module):
         if targets is None:
             if not return_logits:
                 return None  # no targets, no logits requested: there is no loss to report
-            x = x[:, [-1], :]  # only the last position is needed for sampling
+            x = x[:, -1:, :].contiguous()  # only the last position is needed for sampling
         if group is not None:
             logits = TP.gather_from_tp_region(K.linear(TP.copy_to_tp_region(x, group), _local(w)), group)
         else:

@@ -130,17 +130,13 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, c: Optional[torch.Tensor] = None, 
         return gemm_reference(a, b, c=c, out=out, alpha=alpha, beta=beta, act=act, accumulate=accumulate,
                               shadow=shadow)
 
-    if a.dtype not in (torch.bfloat16, torch.float32) or not (_tma_ok(a) and _tma_ok(b)) or out.stride(-1) != 1:
-        # shapes TMA cannot address (pitch not a multiple of 16 bytes): library GEMM
-        if out_ptrs is not None or c_ptrs is not None or shadow_ptrs is not None:
-            raise ValueError("unaligned operands cannot be combined with pointer-array outputs")
-        cd = torch.float32 if a.dtype == torch.float32 else a.dtype
-        return gemm_reference(a, b, c=c, out=out, alpha=alpha, beta=beta, act=act, accumulate=accumulate,
-                              shadow=shadow, compute_dtype=cd)
-
-    if split_k > 1 and not accumulate:
-        raise ValueError("split_k > 1 needs accumulate=True")
-    torch.ops.dion_b200.gemm(a, b, c, out, shadow, c_ptrs, out_ptrs, shadow_ptrs, float(alpha), float(beta),
-                             _ACT[act], 1 if accumulate else 0, int(split_k), bool(symmetric), int(block_n), int(pair),
-                             runtime.status_tensor(a.device), int(out_dup), a_lo, b_lo, c_col_scale, bool(split3))
-    return out
+    if torch.ops.dion_b200.gemm(a, b, c, out, shadow, c_ptrs, out_ptrs, shadow_ptrs, float(alpha), float(beta),
+                                _ACT[act], 1 if accumulate else 0, int(split_k), bool(symmetric), int(block_n), int(pair),
+                                runtime.status_tensor(a.device), int(out_dup), a_lo, b_lo, c_col_scale, bool(split3)):
+        return out
+    # shapes TMA cannot address (pitch not a multiple of 16 bytes): library GEMM
+    if out_ptrs is not None or c_ptrs is not None or shadow_ptrs is not None:
+        raise ValueError("unaligned operands cannot be combined with pointer-array outputs")
+    cd = torch.float32 if a.dtype == torch.float32 else a.dtype
+    return gemm_reference(a, b, c=c, out=out, alpha=alpha, beta=beta, act=act, accumulate=accumulate, shadow=shadow,
+                          compute_dtype=cd)

@@ -29,6 +29,15 @@ def _fast(x: torch.Tensor) -> bool:
     return x.is_cuda and x.dtype == torch.bfloat16 and runtime.use_cuda_kernels(x)
 
 
+def native_forward_ok(x: torch.Tensor) -> bool:
+    """May a pass over ``x: [B, T, C]`` run as one native call?  Plain bf16 activations on a GPU, no gradients recorded, and
+    no transform (vmap, forward-mode derivatives) or module-wide hook that would have to see the single operations."""
+    return (type(x) is torch.Tensor and x.dim() == 3 and _fast(x) and x.is_contiguous() and x.numel() > 0
+            and x.shape[-1] % 8 == 0 and x.data_ptr() % 16 == 0 and not torch.is_grad_enabled()
+            and torch._C._functorch.peek_interpreter_stack() is None
+            and torch.autograd.forward_ad._current_level < 0 and not torch.nn.modules.module._has_any_global_hook())
+
+
 # --------------------------------------------------------------------------- weights in bf16
 
 def bf16_weight(w: torch.Tensor) -> torch.Tensor:

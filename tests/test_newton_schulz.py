@@ -41,6 +41,30 @@ def test_kernel_matches_torch_iteration(shape):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(333, 1001), (1001, 333), (2, 130, 64), (3, 64, 130), (7, 9), (1, 8), (2, 8, 1)])
+def test_sides_that_are_no_multiple_of_eight_are_padded(shape):
+    """Zero rows and columns stay zero in every product: the result is the iteration's, as close to its fp64 form as the
+    same bf16 iteration on PyTorch's products is (whose roundings differ; small singular values amplify them)."""
+    g = torch.randn(*shape, device="cuda").bfloat16()
+    out = newton_schulz(g)
+    assert out.shape == g.shape and out.is_contiguous() and out.dtype == torch.bfloat16
+
+    def iterate(dtype):
+        X = g.to(dtype)
+        X = X.mT if g.size(-2) > g.size(-1) else X
+        X = X / (X.norm(dim=(-2, -1), keepdim=True) + 1e-7)
+        for a, b, c in NS_COEFFS:
+            A = X @ X.mT
+            X = a * X + (b * A + c * (A @ A)) @ X
+        return X.mT if g.size(-2) > g.size(-1) else X
+
+    ref = iterate(torch.float64)
+    err = ((out.double() - ref).norm() / ref.norm()).item()
+    lib = ((iterate(torch.bfloat16).double() - ref).norm() / ref.norm()).item()
+    assert err < 1.5 * lib + 4e-3, (err, lib)  # one rounding of the result is 2^-9
+
+
+@pytest.mark.gpu
 def test_kernel_handles_zero_and_tiny_inputs():
     Z = torch.zeros(2, 128, 256, device="cuda")
     out = newton_schulz(Z)

@@ -388,3 +388,30 @@ def test_swiglu_kernels():
     _close(h, hr, 2e-2)
     _close(g.grad, gr.grad, 2e-2)
     _close(u.grad, ur.grad, 2e-2)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,T,heads,head_dim", [(1, 24, 6, 128), (3, 77, 2, 64), (2, 256, 4, 64)])
+def test_block_without_gradients_runs_natively_with_the_same_bits(B, T, heads, head_dim):
+    """A pass that records no gradients takes one native call per block; a hook on a part of the block, and recorded
+    gradients, take the general path.  Same kernels, same bits."""
+    from dion_b200 import ops
+    from dion_b200.models import GPT, GPTConfig
+
+    with torch.device("cuda"):
+        model = GPT(GPTConfig(sequence_len=T, vocab_size=512, n_layer=2, n_head=heads, n_embd=heads * head_dim))
+    model.init_weights()
+    idx = torch.randint(0, 512, (B, T), device="cuda")
+    general = model(idx, return_logits=True)
+    assert general.requires_grad
+    with torch.no_grad():
+        native = model(idx, return_logits=True)
+        x = torch.randn(B, T, heads * head_dim, device="cuda").bfloat16()
+        assert model.transformer.h[0]._forward_native(x) is not None
+        seen = []
+        handle = model.transformer.h[0].attn.register_forward_hook(lambda *a: seen.append(1))
+        assert model.transformer.h[0]._forward_native(x) is None
+        hooked = model(idx, return_logits=True)
+        handle.remove()
+    assert torch.equal(native, general) and torch.equal(hooked, general) and seen == [1]
+    ops.check_status()

@@ -19,6 +19,7 @@
 #include <string.h>
 
 #include <mutex>
+#include <type_traits>
 
 #include "gemm.h"
 #include "kernels.h"
@@ -127,6 +128,31 @@ __device__ __forceinline__ float fast_exp2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+
+// Two fp32 operations in one instruction.  The softmax loops issue 7 to 14 instructions per score without them and are
+// what the tensor core waits for; with them 3 to 5, of which one is the exponential.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
 }
 
 template <int D>
@@ -340,23 +366,27 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         m_used = m_new;
       }
       const float neg_m = (m_used == -INFINITY) ? 0.f : -m_used;
-      float sum4[4] = {0.f, 0.f, 0.f, 0.f};
+      const f32x2 s2 = pack2(p.scale_log2, p.scale_log2), nm2 = pack2(neg_m, neg_m);
+      f32x2 sums[2] = {pack2(0.f, 0.f), pack2(0.f, 0.f)};
       // exponentials, packed to bf16 pairs and stored over the first half of this row of S_j
       float pk[32];
 #pragma unroll
       for (int c = 0; c < kBN / 8; ++c) {
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
-          const float e0 = fast_exp2(fmaf(sc[8 * c + 2 * t], p.scale_log2, neg_m));
-          const float e1 = fast_exp2(fmaf(sc[8 * c + 2 * t + 1], p.scale_log2, neg_m));
+          float e0, e1;
+          unpack2(fma2(pack2(sc[8 * c + 2 * t], sc[8 * c + 2 * t + 1]), s2, nm2), e0, e1);
+          e0 = fast_exp2(e0);
+          e1 = fast_exp2(e1);
           const __nv_bfloat162 h2 = __floats2bfloat162_rn(e0, e1);
           pk[4 * c + t] = __uint_as_float(*reinterpret_cast<const uint32_t*>(&h2));
-          sum4[t] += e0 + e1;
+          sums[t & 1] = add2(sums[t & 1], pack2(e0, e1));
         }
       }
       tmem_st_32x32(lane_base + s * C::S_COLS, pk);
-      const float sum = (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
-      l += sum;
+      float sum0, sum1;
+      unpack2(add2(sums[0], sums[1]), sum0, sum1);
+      l += sum0 + sum1;
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
@@ -650,6 +680,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     const long long stat_idx = ((long long)b * p.H + h) * p.T + q_pos;
     const float neg_lse2 = -p.lse[stat_idx] * 1.4426950408889634f;
     const float dlt = p.delta[stat_idx];
+    const f32x2 scale2 = pack2(p.scale_log2, p.scale_log2), neg_lse2x2 = pack2(neg_lse2, neg_lse2), neg_dlt2 = pack2(-dlt, -dlt),
+                out_scale2 = pack2(p.scale, p.scale);
     bool ok = true;
     for (int j = 0; j < n_tiles && ok; ++j) {
       if (!mbar_wait(sdp_full, j & 1, abort_flag)) {
@@ -660,24 +692,33 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
       const int col0 = j * kBN;
       const bool diag = col0 + kBN - 1 > q_tile * kBM;
       float pk[32];
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
+      // dS = P o (dP - delta) * scale
+      auto half_tile = [&](int half, auto masked) {
         float sc[32], dp[32];
         tmem_ld_32x32(lane_base + C::S_COL + half * 32, sc);
         tmem_ld_32x32(lane_base + C::DP_COL + half * 32, dp);
         tmem_ld_wait();
 #pragma unroll
         for (int i = 0; i < 32; i += 2) {
-          float p0 = fast_exp2(fmaf(sc[i], p.scale_log2, neg_lse2));
-          float p1 = fast_exp2(fmaf(sc[i + 1], p.scale_log2, neg_lse2));
-          if (diag) {
+          float p0, p1;
+          unpack2(fma2(pack2(sc[i], sc[i + 1]), scale2, neg_lse2x2), p0, p1);
+          p0 = fast_exp2(p0);
+          p1 = fast_exp2(p1);
+          if constexpr (decltype(masked)::value) {
             if (col0 + half * 32 + i > q_pos) p0 = 0.f;
             if (col0 + half * 32 + i + 1 > q_pos) p1 = 0.f;
           }
-          const float d0 = p0 * (dp[i] - dlt) * p.scale;
-          const float d1 = p1 * (dp[i + 1] - dlt) * p.scale;
+          float d0, d1;
+          unpack2(mul2(mul2(pack2(p0, p1), add2(pack2(dp[i], dp[i + 1]), neg_dlt2)), out_scale2), d0, d1);
           pk[half * 16 + (i >> 1)] = __uint_as_float(pack_bf16x2(d0, d1));
         }
+      };
+      if (diag) {
+        half_tile(0, std::true_type());
+        half_tile(1, std::true_type());
+      } else {
+        half_tile(0, std::false_type());
+        half_tile(1, std::false_type());
       }
       tmem_st_32x32(lane_base + C::S_COL, pk);
       tmem_st_wait();
@@ -914,6 +955,8 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     const int row_in_tile = quad * 32 + lane;
     const int kv_pos = kv0 + row_in_tile;
     const uint32_t lane_base = tmem_base + ((uint32_t)(quad * 32) << 16);
+    const f32x2 scale2 = pack2(p.scale_log2, p.scale_log2), neg_log2e = pack2(-1.4426950408889634f, -1.4426950408889634f),
+                minus1 = pack2(-1.f, -1.f), out_scale2 = pack2(p.scale, p.scale);
     bool ok = true;
     // A failed wait clears `ok` but the loop keeps its shape: both warps of a quadrant must reach
     // the named barrier the same number of times.
@@ -936,25 +979,32 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
       const int qcol0 = i * kBQ + half * 32;           // sequence position of this thread's first column
       const bool diag = qcol0 < kv0 + kBM;             // some query of this block precedes some kv row
       uint32_t pp[16], dd[16];
+      // P and dS = P o (dP - delta) * scale
+      auto columns = [&](auto masked) {
 #pragma unroll
-      for (int c = 0; c < 32; c += 4) {
-        const float4 l4 = *reinterpret_cast<const float4*>(lse_s + c);
-        const float4 d4 = *reinterpret_cast<const float4*>(dlt_s + c);
-        const float ls[4] = {l4.x, l4.y, l4.z, l4.w};
-        const float dl[4] = {d4.x, d4.y, d4.z, d4.w};
-        float pv[4], dv[4];
+        for (int c = 0; c < 32; c += 4) {
+          const float4 l4 = *reinterpret_cast<const float4*>(lse_s + c);
+          const float4 d4 = *reinterpret_cast<const float4*>(dlt_s + c);
 #pragma unroll
-        for (int t = 0; t < 4; ++t) {
-          float e = fast_exp2(fmaf(sc[c + t], p.scale_log2, -ls[t] * 1.4426950408889634f));
-          if (diag && qcol0 + c + t < kv_pos) e = 0.f;
-          pv[t] = e;
-          dv[t] = e * (dp[c + t] - dl[t]) * p.scale;
+          for (int t = 0; t < 4; t += 2) {
+            const f32x2 neg_lse2 = mul2(t ? pack2(l4.z, l4.w) : pack2(l4.x, l4.y), neg_log2e);
+            float e0, e1, g0, g1;
+            unpack2(fma2(pack2(sc[c + t], sc[c + t + 1]), scale2, neg_lse2), e0, e1);
+            e0 = fast_exp2(e0);
+            e1 = fast_exp2(e1);
+            if constexpr (decltype(masked)::value) {
+              if (qcol0 + c + t < kv_pos) e0 = 0.f;
+              if (qcol0 + c + t + 1 < kv_pos) e1 = 0.f;
+            }
+            const f32x2 d = fma2(t ? pack2(d4.z, d4.w) : pack2(d4.x, d4.y), minus1, pack2(dp[c + t], dp[c + t + 1]));
+            unpack2(mul2(mul2(pack2(e0, e1), d), out_scale2), g0, g1);
+            pp[(c + t) >> 1] = pack_bf16x2(e0, e1);
+            dd[(c + t) >> 1] = pack_bf16x2(g0, g1);
+          }
         }
-        pp[c >> 1] = pack_bf16x2(pv[0], pv[1]);
-        pp[(c >> 1) + 1] = pack_bf16x2(pv[2], pv[3]);
-        dd[c >> 1] = pack_bf16x2(dv[0], dv[1]);
-        dd[(c >> 1) + 1] = pack_bf16x2(dv[2], dv[3]);
-      }
+      };
+      if (diag) columns(std::true_type());
+      else columns(std::false_type());
       // both warps of a quadrant must have read S^T / dP^T before either overwrites its part: the
       // packed halves land in columns [0, 32) of the buffers, which the other warp may still be loading
       pair_barrier(quad);

@@ -1052,18 +1052,27 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       constexpr int kChunksPerWarp = kBlockN / 32 / (kNumEpilogueWarps / 4);
       const int c_first = ((warp - 2) >> 2) * kChunksPerWarp;
 
-      // A staged bf16 C operand is fetched one chunk ahead: the loads of the first chunk go out before this
+      // A staged C operand is fetched one chunk ahead: the loads of the first chunk go out before this
       // warp waits for the accumulator, those of chunk c + 1 while chunk c is converted and stored, so that
       // their latency does not add to every chunk (with 8 epilogue warps per CTA nothing else hides it).
-      // Same lane mapping as stage_fetch<4>: 4 lanes per row, 8 rows per instruction.
-      const bool prefetch_c = !kSplit && stage_c && p.c_is_bf16;  // the splitting variants have no registers to spare
-      uint4 cq[4];
+      // Same lane mapping as stage_fetch: 4 (bf16) or 8 (fp32) lanes per row, 8 or 4 rows per instruction.
+      const bool prefetch_c = !kSplit && stage_c;  // the splitting variants have no registers to spare
+      uint4 cq[8];
       auto c_prefetch = [&](int chunk) {
-        const char* cp = c_base + ((long long)(row_first + (lane >> 2)) * p.ldc + n0 + chunk * 32) * 2 + (lane & 3) * 16;
+        if (p.c_is_bf16) {
+          const char* cp = c_base + ((long long)(row_first + (lane >> 2)) * p.ldc + n0 + chunk * 32) * 2 + (lane & 3) * 16;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          cq[i] = make_uint4(0u, 0u, 0u, 0u);
-          if (row_first + i * 8 + (lane >> 2) < p.M) cq[i] = *reinterpret_cast<const uint4*>(cp + (long long)i * 8 * p.ldc * 2);
+          for (int i = 0; i < 4; ++i) {
+            cq[i] = make_uint4(0u, 0u, 0u, 0u);
+            if (row_first + i * 8 + (lane >> 2) < p.M) cq[i] = *reinterpret_cast<const uint4*>(cp + (long long)i * 8 * p.ldc * 2);
+          }
+        } else {
+          const char* cp = c_base + ((long long)(row_first + (lane >> 3)) * p.ldc + n0 + chunk * 32) * 4 + (lane & 7) * 16;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            cq[i] = make_uint4(0u, 0u, 0u, 0u);
+            if (row_first + i * 4 + (lane >> 3) < p.M) cq[i] = *reinterpret_cast<const uint4*>(cp + (long long)i * 4 * p.ldc * 4);
+          }
         }
       };
       if (prefetch_c) c_prefetch(c_first);
@@ -1148,10 +1157,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
           if (use_c) {
             float cv[32];
             if (prefetch_c) {
+              if (p.c_is_bf16) {
 #pragma unroll
-              for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(st + stage_off(i * 8 + (lane >> 2), lane & 3)) = cq[i];
+                for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(st + stage_off(i * 8 + (lane >> 2), lane & 3)) = cq[i];
+              } else {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) *reinterpret_cast<uint4*>(st + stage_off(i * 4 + (lane >> 3), lane & 7)) = cq[i];
+              }
               __syncwarp();
-              stage_get(st, lane, true, cv);
+              stage_get(st, lane, p.c_is_bf16 != 0, cv);
               __syncwarp();
               if (c + 1 < c_first + kChunksPerWarp) c_prefetch(c + 1);  // a full tile: every chunk is in range
             } else if (stage_c) {

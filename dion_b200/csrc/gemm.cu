@@ -808,9 +808,19 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       const int row0 = t.m_blk * C::TILE_M + (int)cta_rank * kBlockM + quad * 32;
       const int col0 = t.n_blk * kBlockN + ((warp - 2) >> 2) * (kBlockN / 2);
       const int acc = C::acc_of(it);
-      const bool mirror = p.symmetric && t.m_blk != t.n_blk;
+      bool mirror = p.symmetric && t.m_blk != t.n_blk;
       // boxes of this warp that lie inside the matrix (a box that only overlaps it is clipped by the copy)
-      const int boxes = row0 < p.M ? min(kBoxes, max(0, (p.N - col0 + kBoxCols - 1) / kBoxCols)) : 0;
+      int boxes = row0 < p.M ? min(kBoxes, max(0, (p.N - col0 + kBoxCols - 1) / kBoxCols)) : 0;
+      if constexpr (kSplit && kPair) {
+        // On a diagonal tile the lower left quarter (the peer's rows, the first half of the columns) is the mirror of the
+        // upper right one, as it is between 128 x 128 tiles: computed by itself its cross terms would be added the other
+        // way round, which leaves the result symmetric to the last bit but one.
+        if (p.symmetric && t.m_blk == t.n_blk) {
+          const bool second_half = ((warp - 2) >> 2) == 1;
+          if (cta_rank == 1 && !second_half) boxes = 0;
+          mirror = cta_rank == 0 && second_half;
+        }
+      }
       if (use_c && boxes > 0) fetch_c(col0, row0, t.batch);
       if (!wait(&tmem_full[acc], C::acc_phase_of(it))) {
         ok = false;
@@ -872,17 +882,20 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
                 !kSplit && p.c_col_scale != nullptr ? p.c_col_scale + (long long)t.batch * p.N + col : nullptr;
 #pragma unroll
             for (int s = 0; s < 8; ++s) {
-              float4 q = *reinterpret_cast<const float4*>(st + stage_off(lane, s));
-              if (cs != nullptr && col + 4 * s < p.N) {
-                q.x *= cs[4 * s];
-                q.y *= cs[4 * s + 1];
-                q.z *= cs[4 * s + 2];
-                q.w *= cs[4 * s + 3];
+              const float4 q = *reinterpret_cast<const float4*>(st + stage_off(lane, s));
+              if (cs != nullptr) {
+                if (col + 4 * s < p.N) {  // scaled and added with one rounding
+                  v[4 * s] = fmaf(p.beta * q.x, cs[4 * s], v[4 * s]);
+                  v[4 * s + 1] = fmaf(p.beta * q.y, cs[4 * s + 1], v[4 * s + 1]);
+                  v[4 * s + 2] = fmaf(p.beta * q.z, cs[4 * s + 2], v[4 * s + 2]);
+                  v[4 * s + 3] = fmaf(p.beta * q.w, cs[4 * s + 3], v[4 * s + 3]);
+                }
+              } else {
+                v[4 * s] += p.beta * q.x;
+                v[4 * s + 1] += p.beta * q.y;
+                v[4 * s + 2] += p.beta * q.z;
+                v[4 * s + 3] += p.beta * q.w;
               }
-              v[4 * s] += p.beta * q.x;
-              v[4 * s + 1] += p.beta * q.y;
-              v[4 * s + 2] += p.beta * q.z;
-              v[4 * s + 3] += p.beta * q.w;
             }
           } else {
 #pragma unroll
@@ -1606,7 +1619,7 @@ bool aligned16(const void* p, long long ld, int es) {
 // kTileCost blocks.  One matrix of 14336 x 512 (10 tiles, 448 blocks) takes 8, as do twelve of 3072 x 96; 48 of
 // 768 x 768 (1008 tiles, 24 blocks) fill the chip by themselves and take 1.
 int choose_cluster_k(const GemmArgs& a, const KernelParams& kp, int bn, long long* blocks = nullptr) {
-  if (!a.symmetric || bn != 128 || a.a_major != kMajorMN || a.b_major != kMajorMN || a.d_dtype != kF32 ||
+  if (a.pair == 2 || a.pair < 0 || !a.symmetric || bn != 128 || a.a_major != kMajorMN || a.b_major != kMajorMN || a.d_dtype != kF32 ||
       a.epilogue != kEpiStore || a.act != 0 || a.C || a.c_ptrs || a.D2 || a.d2_ptrs || a.d_ptrs || a.scatter_mode != 0 ||
       a.max_ctas > 0)
     return 1;

@@ -645,16 +645,16 @@ __device__ __forceinline__ int tri_factor(const float* blk, float* lrow, float* 
   float x[32];
 #pragma unroll
   for (int i = 0; i < 32; ++i) {
-    float s0 = (i == lane) ? 1.f : 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+    float s = (i == lane) ? 1.f : 0.f;  // one chain: the order of sums of the kernel for larger ranks, the same bits
 #pragma unroll
     for (int k = 0; k < i; k += 4) {
       const float4 l = *reinterpret_cast<const float4*>(lrow + i * kTriLinvPitch + k);
-      s0 = fmaf(-l.x, x[k], s0);
-      if (k + 1 < i) s1 = fmaf(-l.y, x[k + 1], s1);
-      if (k + 2 < i) s2 = fmaf(-l.z, x[k + 2], s2);
-      if (k + 3 < i) s3 = fmaf(-l.w, x[k + 3], s3);
+      s = fmaf(-l.x, x[k], s);
+      if (k + 1 < i) s = fmaf(-l.y, x[k + 1], s);
+      if (k + 2 < i) s = fmaf(-l.z, x[k + 2], s);
+      if (k + 3 < i) s = fmaf(-l.w, x[k + 3], s);
     }
-    x[i] = ((s0 + s1) + (s2 + s3)) * dinv[i];
+    x[i] = s * dinv[i];
   }
 #pragma unroll
   for (int i = 0; i < 32; ++i) linv[i * 32 + lane] = x[i];

@@ -553,6 +553,15 @@ def _times_scalar(x: torch.Tensor, s: torch.Tensor, in_place: bool) -> torch.Ten
     return out
 
 
+def _halve_contraction(M: int, N: int, K: int) -> bool:
+    """Should a product with a very long contraction be cut in two halves that are added in fp32 (two summands onto zero:
+    the same bits in any order)?  Where the 256 x 256 tiles leave most of a wave of CTA pairs idle: 8192 x 768 has 96
+    tiles for 74 pairs, two waves where one and a half do (K = 50304: 590 -> 476 us with the clearing and the cast)."""
+    tiles = ((M + 255) // 256) * ((N + 255) // 256)
+    pairs = 74
+    return K >= 16384 and tiles * 2 >= 2 * pairs and 2 * (-(-tiles // pairs)) * 9 >= (-(-2 * tiles // pairs)) * 10
+
+
 class _LinearCrossEntropyFn(torch.autograd.Function):
     """loss = mean CE(x @ W^T, targets) without keeping the logits: the token dimension is
     processed in chunks; each chunk's logits are turned into their gradient in place by the
@@ -579,7 +588,12 @@ class _LinearCrossEntropyFn(torch.autograd.Function):
             torch.ops.dion_b200.cross_entropy_fwd_bwd(lg, targets[t0:t1], row_loss[t0:t1], inv_valid, 1.0,
                                                       ignore_index, need_grad)
             if need_grad:
-                gemm(lg, wb, out=dx[t0:t1])  # [n, V] @ [V, K]
+                if _halve_contraction(n, K, V):  # [n, V] @ [V, K]
+                    acc = torch.zeros(n, K, device=x.device, dtype=torch.float32)
+                    gemm(lg, wb, out=acc, accumulate=True, split_k=2)
+                    dx[t0:t1].copy_(acc)
+                else:
+                    gemm(lg, wb, out=dx[t0:t1])
                 gemm(lg.t(), x[t0:t1], out=dw, accumulate=t0 > 0, split_k=1)  # [V, n] @ [n, K]
         loss = row_loss.sum() * inv_valid
         if need_grad:

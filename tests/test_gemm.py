@@ -319,8 +319,12 @@ def test_gram_of_tall_factors_sums_k_ranges_over_a_cluster(batch, rows, r):
     gemm(p.transpose(-1, -2), p, out=out, symmetric=True, split3=True)
     ref = x.double().transpose(-1, -2) @ x.double()
     assert ((out.double() - ref).abs().amax() / ref.abs().amax()).item() < rows / 8 * 2 ** -23 + 2 ** -21
-    if r > 256:  # blocks off the diagonal are mirrored (on it the two cross terms are added in either order)
-        assert torch.equal(out[:, :256, 256:], out[:, 256:, :256].transpose(-1, -2))
+    # 128 x 128 blocks off the diagonal are mirrored (on it the two cross terms are added in either order)
+    for i in range(0, r, 128):
+        assert torch.equal(out[:, i:i + 128, i + 128:], out[:, i + 128:, i:i + 128].transpose(-1, -2))
+    # every K sum in one pass: the same bits from CTA pairs and from single tiles
+    p2 = gemm(p.transpose(-1, -2), p, symmetric=True, split3=True, pair=2)
+    assert torch.equal(p2, gemm(p.transpose(-1, -2), p, symmetric=True, split3=True, pair=-1, block_n=128))
     again = gemm(p.transpose(-1, -2), p, symmetric=True, split3=True)
     assert torch.equal(out, again)
 

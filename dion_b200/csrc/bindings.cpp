@@ -1015,6 +1015,9 @@ Tensor gpt_block_fwd(const Tensor& x, const Tensor& wq, const Tensor& wk, const 
                      const Tensor& wproj, const Tensor& cos, const Tensor& sin, int64_t D, double eps,
                      bool kernel_attention, Tensor status) {
   TORCH_CHECK(x.dim() == 3 && x.is_contiguous(), "gpt_block_fwd: x is [B, T, C], contiguous");
+  for (const Tensor& w : {wq, wk, wv})
+    TORCH_CHECK(w.scalar_type() == at::kBFloat16 && w.is_cuda() && w.is_contiguous() && w.sizes() == wq.sizes() && w.size(1) == x.size(2),
+                "gpt_block_fwd: q, k and v weights are bf16, contiguous and of one shape");
   const c10::cuda::CUDAGuard guard(x.device());
   const int64_t B = x.size(0), T = x.size(1), C = x.size(2), N = B * T, heads = wq.size(0) / D;
   const Tensor x2 = x.view({N, C});
@@ -1026,7 +1029,32 @@ Tensor gpt_block_fwd(const Tensor& x, const Tensor& wq, const Tensor& wk, const 
   };
   Tensor h = at::empty_like(x2);
   rmsnorm_fwd(x2, {}, {}, h, rstd, eps);
-  Tensor q = linear(h, wq, {}, 0), k = linear(h, wk, {}, 0), v = linear(h, wv, {}, 0);
+  Tensor q, k, v;
+  if (const char* env = getenv("DION_B200_GEMM_STAGE"); wq.size(0) > 64 && N > 0 && !(env && env[0] == '0')) {
+    // one launch for the three projections
+    Tensor qkv = at::empty({3, N, wq.size(0)}, x.options());
+    dion::GemmArgs g;
+    g.ab_dtype = g.d_dtype = dion::kBF16;
+    g.M = (int)N;
+    g.N = (int)wq.size(0);
+    g.K = (int)C;
+    g.batch = 3;
+    g.A = h.data_ptr();
+    g.B = wq.data_ptr();
+    g.B_more[0] = wk.data_ptr();
+    g.B_more[1] = wv.data_ptr();
+    g.lda = g.ldb = C;
+    g.D = qkv.data_ptr();
+    g.ldd = g.N;
+    g.d_batch_stride = N * g.N;
+    g.status = status.data_ptr<int>();
+    const cudaError_t e = dion::gemm_launch(g, at::cuda::getCurrentCUDAStream());
+    TORCH_CHECK(e == cudaSuccess, "projections: ", cudaGetErrorString(e), " ", dion::gemm_last_error());
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    q = qkv[0], k = qkv[1], v = qkv[2];
+  } else {
+    q = linear(h, wq, {}, 0), k = linear(h, wk, {}, 0), v = linear(h, wv, {}, 0);
+  }
   Tensor qo = at::empty_like(q), ko = at::empty_like(k);
   rope_qknorm_fwd(q, k, qo, ko, cos, sin, T, heads, D, eps);
   const Tensor q4 = qo.view({B, T, heads, D}), k4 = ko.view({B, T, heads, D}), v4 = v.view({B, T, heads, D});

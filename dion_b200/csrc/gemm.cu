@@ -87,6 +87,7 @@ struct KernelParams {
   int vec_c, vec_d, vec_d2;  // 16-byte vector access allowed
   int stage;                 // turn epilogue accesses through shared memory (coalesced)
   int b_is_a;                // symmetric product of one matrix with itself: diagonal tiles need one operand only
+  int b_separate;            // kTmaEpi: one A, the B of batch elements 1 and 2 in the map slots of C and of mirrored boxes
   int cluster_k;             // kClusterK: CTAs of a cluster that share one output tile (each a K range)
   int* status;
   GatherParams g;            // used by the kGather instantiations only
@@ -515,15 +516,19 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
           if (!kJoint || cta_rank == 0)
             mbar_arrive_expect_tx(&full_bar[stage], skip_b ? C::A_BYTES : kJoint ? C::TX_BYTES : C::STAGE_BYTES);
           const uint32_t bar = kJoint ? mapa_shared(smem_u32(&full_bar[stage]), 0) : smem_u32(&full_bar[stage]);
+          const int z = kTmaEpi && p.b_separate ? 0 : t.batch;
           auto load = [&](void* dst, const CUtensorMap* map, int c0, int c1) {
-            if constexpr (kJoint) tma_load_3d_pair(dst, map, bar, c0, c1, t.batch);
-            else tma_load_3d(dst, map, &full_bar[stage], c0, c1, t.batch);
+            if constexpr (kJoint) tma_load_3d_pair(dst, map, bar, c0, c1, z);
+            else tma_load_3d(dst, map, &full_bar[stage], c0, c1, z);
           };
           uint8_t* sa = smem + stage * C::STAGE_STRIDE;
           uint8_t* sb = sa + C::A_BYTES;
           // hi / lo operands: the K range is walked three times, as A B, A_lo B and A B_lo
           const CUtensorMap* map_a = &tmap_a;
           const CUtensorMap* map_b = &tmap_b;
+          if constexpr (kTmaEpi) {
+            if (p.b_separate && t.batch > 0) map_b = t.batch == 1 ? &tmap_b_lo : &tmap_mirror;
+          }
           int kk = kb;
           if constexpr (kTf32) {
             if (kb >= p.kblocks_seg) {
@@ -1499,13 +1504,14 @@ cudaError_t launch_cfg(const GemmArgs& a, const KernelParams& kp, cudaStream_t s
   using C = Cfg<kTf32, kAMajor, kBMajor, kBlockN, kPair, kSplit>;
   CUtensorMap ta, tb, ta_lo, tb_lo;
   const int dt = kTf32 ? kF32 : kBF16;
+  const int batch = a.B_more[0] ? 1 : a.batch;  // of the operands' maps
   auto map_a = [&](CUtensorMap* m, const void* base) {
-    if (kAMajor == kMajorK) return make_tmap(m, base, dt, a.K, a.M, a.batch, a.lda, a.a_batch_stride, C::BK, kBlockM, kSwizzle128);
-    return make_tmap(m, base, dt, a.M, a.K, a.batch, a.lda, a.a_batch_stride, C::CH, C::BK, C::A_ATOM32 ? kSwizzle128Atom32 : kSwizzle128);
+    if (kAMajor == kMajorK) return make_tmap(m, base, dt, a.K, a.M, batch, a.lda, a.a_batch_stride, C::BK, kBlockM, kSwizzle128);
+    return make_tmap(m, base, dt, a.M, a.K, batch, a.lda, a.a_batch_stride, C::CH, C::BK, C::A_ATOM32 ? kSwizzle128Atom32 : kSwizzle128);
   };
   auto map_b = [&](CUtensorMap* m, const void* base) {
-    if (kBMajor == kMajorK) return make_tmap(m, base, dt, a.K, a.N, a.batch, a.ldb, a.b_batch_stride, C::BK, C::B_ROWS, kSwizzle128);
-    return make_tmap(m, base, dt, a.N, a.K, a.batch, a.ldb, a.b_batch_stride, C::CH, C::BK, C::B_ATOM32 ? kSwizzle128Atom32 : kSwizzle128);
+    if (kBMajor == kMajorK) return make_tmap(m, base, dt, a.K, a.N, batch, a.ldb, a.b_batch_stride, C::BK, C::B_ROWS, kSwizzle128);
+    return make_tmap(m, base, dt, a.N, a.K, batch, a.ldb, a.b_batch_stride, C::CH, C::BK, C::B_ATOM32 ? kSwizzle128Atom32 : kSwizzle128);
   };
   if (!map_a(&ta, a.A) || !map_b(&tb, a.B)) return cudaErrorInvalidValue;
   if (a.A_lo != nullptr) {
@@ -1520,6 +1526,7 @@ cudaError_t launch_cfg(const GemmArgs& a, const KernelParams& kp, cudaStream_t s
       return cudaErrorInvalidValue;
     if (a.C && !make_tmap(&tb_lo, a.C, dt, a.N, a.M, a.batch, a.ldc, a.c_batch_stride, 128 / C::ES, 32, kSwizzle128))
       return cudaErrorInvalidValue;
+    if (a.B_more[0] && (!map_b(&tb_lo, a.B_more[0]) || !map_b(&tm, a.B_more[1]))) return cudaErrorInvalidValue;
     if (!kTf32 && a.symmetric && !make_tmap(&tm, a.D, kBF16, a.N, a.M, a.batch, a.ldd, a.d_batch_stride, 32, 64, kSwizzleNone))
       return cudaErrorInvalidValue;
   }
@@ -1848,6 +1855,13 @@ cudaError_t gemm_launch(const GemmArgs& a, cudaStream_t stream) {
     g_last_error = "symmetric mode needs M == N";
     return cudaErrorInvalidValue;
   }
+  if (a.B_more[0] && (!a.B_more[1] || a.batch != 3 || a.ab_dtype != kBF16 || a.d_dtype != kBF16 || a.a_major != kMajorK ||
+                      a.b_major != kMajorK || a.C || a.symmetric || a.N <= 64 || a.N % 8 != 0 || a.block_n == 64 ||
+                      a.epilogue != kEpiStore || !a.D || a.d_batch_stride <= 0 || a.d_batch_stride % 8 != 0 ||
+                      !aligned16(a.D, a.ldd, 2) || a.gather.world > 0)) {
+    g_last_error = "three products of one operand: bf16, K-major, no addend, aligned outputs of more than 64 columns";
+    return cudaErrorInvalidValue;
+  }
   if (!a.D && !a.d_ptrs && !a.scatter_ptrs) {
     g_last_error = "GEMM output missing";
     return cudaErrorInvalidValue;
@@ -1916,6 +1930,7 @@ cudaError_t gemm_launch(const GemmArgs& a, cudaStream_t stream) {
   kp.b_is_a = a.symmetric && a.A == a.B && a.a_major == kMajorMN && a.b_major == kMajorMN && a.lda == a.ldb &&
               a.a_batch_stride == a.b_batch_stride;
   kp.cluster_k = 1;
+  kp.b_separate = a.B_more[0] != nullptr;
   kp.scatter_mode = a.scatter_mode;
   kp.scatter_block = a.scatter_block;
   kp.scatter_dests = a.scatter_dests;
@@ -1955,6 +1970,10 @@ cudaError_t gemm_launch(const GemmArgs& a, cudaStream_t stream) {
     if (pair) return launch_cfg<false, kMajorK, kMajorK, 256, true, true>(a, kp, stream);
     if (bn == 128) return launch_cfg<false, kMajorK, kMajorK, 128, false, true>(a, kp, stream);
     return launch_cfg<false, kMajorK, kMajorK, 256, false, true>(a, kp, stream);
+  }
+  if (a.B_more[0] && !tma_epilogue(a, kp, bn)) {
+    g_last_error = "three products of one operand need the TMA epilogue";
+    return cudaErrorInvalidValue;
   }
   if (a.split3) return launch_split(a, kp, bn, stream);
   return tf32 ? launch_major<true>(a, kp, bn, pair, stream) : launch_major<false>(a, kp, bn, pair, stream);

@@ -90,6 +90,9 @@ struct GemmArgs {
   void* const* scatter_ptrs = nullptr;
   int block_n = 0;  // 0 = choose automatically (64 / 128 / 256)
   int max_ctas = 0;  // 0 = one CTA per SM
+  // Three products of one A with three matrices laid out like B (bf16, K-major both, no C): batch is 3, B belongs to batch
+  // element 0, these to 1 and 2, and D holds the three results d_batch_stride apart.
+  const void* B_more[2] = {nullptr, nullptr};
   int pair = 0;      // CTA pairs (256-row tiles): 0 = choose automatically, 1 = force (needs block_n 256), -1 = never
 
   int* status = nullptr;  // device int, set to a non-zero code on a device-side failure

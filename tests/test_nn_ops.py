@@ -391,7 +391,7 @@ def test_swiglu_kernels():
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("B,T,heads,head_dim", [(1, 24, 6, 128), (3, 77, 2, 64), (2, 256, 4, 64)])
+@pytest.mark.parametrize("B,T,heads,head_dim", [(1, 24, 6, 128), (3, 77, 2, 64), (2, 256, 4, 64), (1, 40, 1, 64), (8, 640, 5, 64)])
 def test_block_without_gradients_runs_natively_with_the_same_bits(B, T, heads, head_dim):
     """A pass that records no gradients takes one native call per block; a hook on a part of the block, and recorded
     gradients, take the general path.  Same kernels, same bits."""

@@ -543,10 +543,17 @@ def embedding(idx: torch.Tensor, table: torch.Tensor, out_dtype: torch.dtype = t
 
 # --------------------------------------------------------------------------- lm_head + cross entropy
 
+def _transformed(t: torch.Tensor) -> bool:
+    """Does `t` stand for more than its values: a batch of several gradients, a dual number, a subclass?"""
+    return (type(t) is not torch.Tensor or torch._C._functorch.is_batchedtensor(t)
+            or torch._C._functorch.is_legacy_batchedtensor(t) or torch._C._functorch.peek_interpreter_stack() is not None
+            or torch.autograd.forward_ad._current_level >= 0)
+
+
 def _times_scalar(x: torch.Tensor, s: torch.Tensor, in_place: bool) -> torch.Tensor:
     """``x * s`` for a 0-dim fp32 ``s`` (rounded to the dtype of x first); in place if `in_place`."""
     if (torch.is_grad_enabled() or s.dtype != torch.float32 or s.device != x.device or not x.is_contiguous()
-            or x.dtype not in (torch.float32, torch.bfloat16)):
+            or x.dtype not in (torch.float32, torch.bfloat16) or _transformed(s)):
         return x * s.to(x.dtype)
     out = x if in_place else torch.empty_like(x)
     torch.ops.dion_b200.scale_by_scalar(x, out, s)
@@ -608,7 +615,7 @@ class _LinearCrossEntropyFn(torch.autograd.Function):
         dx, dw = ctx.saved_tensors
         # When the graph is not kept, the kept gradients are scaled where they lie and handed on (a plain backward pass
         # has dloss = 1 and moves nothing); otherwise they stay as they are for the next backward pass.
-        own = (ctx.plain_save and not torch.is_grad_enabled()
+        own = (ctx.plain_save and not torch.is_grad_enabled() and not _transformed(dloss)
                and not torch._C._autograd._get_current_graph_task_keep_graph())
         dxo = _times_scalar(dx, dloss, own) if ctx.needs_input_grad[0] else None
         dwo = None

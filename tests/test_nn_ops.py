@@ -227,6 +227,8 @@ def test_linear_cross_entropy_backward_twice_and_scaled(tokens, chunk):
         assert torch.equal(a, 0.25 * gx) and torch.allclose(b, 0.25 * gw, rtol=1e-5, atol=1e-8)
     a, b = torch.autograd.grad(0.25 * loss, (x, w))
     assert torch.equal(a, 0.25 * gx) and torch.allclose(b, 0.25 * gw, rtol=1e-5, atol=1e-8)
+    a, b = torch.autograd.grad(run(), (x, w), grad_outputs=torch.tensor([1.0, 0.25], device="cuda"), is_grads_batched=True)
+    assert torch.equal(a[1], 0.25 * gx) and torch.allclose(b[1], 0.25 * gw, rtol=1e-5, atol=1e-8) and torch.equal(a[0], gx)
     held = []
     with torch.autograd.graph.saved_tensors_hooks(lambda v: held.append(v) or v, lambda v: v):
         loss = run()

@@ -1569,13 +1569,13 @@ cudaError_t launch_cfg(const GemmArgs& a, const KernelParams& kp, cudaStream_t s
 // Problems whose epilogue moves C and D with TMA: C and D of the operands' type, one destination, operands K-major / any,
 // 16-byte aligned rows of whole 16 bytes (every box starts at a multiple of 128 bytes; a row is clipped in units of 16
 // bytes, so that 1001 columns would lose what lies behind the 1001st).  With outputs of another type, pointer arrays, a
-// second output or scattered tiles, and for tiles of 64 columns, the generic epilogue remains.
+// second output or scattered tiles, addends with broadcast rows, and for tiles of 64 columns, the generic epilogue remains.
 bool tma_epilogue(const GemmArgs& a, const KernelParams& kp, int bn) {
   const bool bf16 = a.ab_dtype == kBF16;
   return kp.stage && a.a_major == kMajorK && a.d_dtype == a.ab_dtype && a.epilogue == kEpiStore && bn >= 128 &&
          a.split_k == 1 && !a.A_lo && !a.c_ptrs && !a.d_ptrs && !a.D2 && !a.d2_ptrs && a.scatter_mode == 0 &&
          (bf16 ? a.act != kActRelu2SavePre && !a.c_col_scale : a.act == 0 || a.act == kActRelu2) && kp.vec_d && a.D &&
-         a.N % (bf16 ? 8 : 4) == 0 && (!a.C || (a.c_dtype == a.ab_dtype && kp.vec_c)) &&
+         a.ldd >= a.N && (!a.C || a.ldc >= a.N) && a.N % (bf16 ? 8 : 4) == 0 && (!a.C || (a.c_dtype == a.ab_dtype && kp.vec_c)) &&
          (a.batch == 1 || (a.d_batch_stride != 0 && (!a.C || a.c_batch_stride != 0)));
 }
 // C is read only where it counts
@@ -1657,6 +1657,7 @@ bool split_pair(const GemmArgs& a) {
       a.M <= 128 || (a.C && a.c_dtype != kF32))
     return false;
   if (a.a_major != kMajorK && !(a.symmetric && a.b_major == kMajorMN)) return false;
+  if (a.ldd < a.N || (a.C && a.ldc < a.N)) return false;  // broadcast rows have no tensor map
   if (!aligned16(a.D, a.ldd, 4) || (a.batch > 1 && (a.d_batch_stride == 0 || a.d_batch_stride % 4 != 0))) return false;
   if (a.C && (!aligned16(a.C, a.ldc, 4) || (a.batch > 1 && (a.c_batch_stride == 0 || a.c_batch_stride % 4 != 0)))) return false;
   const long long kb = (a.K + 31) / 32, sms = num_sms();

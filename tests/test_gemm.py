@@ -304,6 +304,26 @@ def test_tma_epilogue_fp32(M, N, K, batch, split3, mode):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("dtype,split3", [(torch.bfloat16, False), (torch.float32, False), (torch.float32, True)])
+@pytest.mark.parametrize("M,N,K,batch", [(300, 520, 72, 1), (4100, 2056, 1024, 1), (1300, 1032, 512, 6)])
+def test_addend_with_broadcast_rows(dtype, split3, M, N, K, batch):
+    """One row (or one matrix) added everywhere: a pitch of zero, which no tensor map describes.  The result is close to
+    that with the addend written out (the same kernel arithmetic, one rounding to the result's type apart)."""
+    shape = lambda *s: s if batch == 1 else (batch, *s)
+    a = torch.randn(*shape(M, K), device="cuda").to(dtype)
+    b = torch.randn(*shape(N, K), device="cuda").to(dtype).transpose(-1, -2)
+    row = torch.randn(N, device="cuda").to(dtype)
+    full = gemm(a, b, c=row.expand(*shape(M, N)).contiguous(), beta=2.0, split3=split3)
+    eps = 2 ** -8 if dtype == torch.bfloat16 else 2 ** -22
+    for c in ([row.expand(M, N)] if batch == 1 else [row.expand(batch, M, N), row.expand(M, N).contiguous().expand(batch, M, N)]):
+        out = gemm(a, b, c=c, beta=2.0, split3=split3)
+        assert ((out - full).abs() <= eps * full.abs() + eps).all()
+    from dion_b200 import ops
+
+    ops.check_status()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("batch,rows,r", [(1, 40, 128), (12, 3072, 96), (4, 2056, 512), (3, 5000, 200), (1, 4096, 130),
                                           (2, 776, 8), (40, 160, 96), (48, 776, 520)])
 def test_gram_of_tall_factors_sums_k_ranges_over_a_cluster(batch, rows, r):

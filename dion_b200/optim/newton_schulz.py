@@ -82,7 +82,9 @@ def newton_schulz(G: Tensor, epsilon: float = 1e-7, coeffs: Sequence[Tuple[float
             Xp = torch.zeros(Bn, mp, np_, device=X.device, dtype=torch.bfloat16)
             Xp[:, :m, :n].copy_(X)
             X = Xp
-        out = torch.ops.dion_b200.newton_schulz_steps(X, ss, float(epsilon), flat, ops.runtime.status_tensor(X.device))
+        # the result is no part of an autograd graph, whatever G is
+        out = torch.ops.dion_b200.newton_schulz_steps(X.detach(), None if ss is None else ss.detach(), float(epsilon), flat,
+                                                      ops.runtime.status_tensor(X.device))
         if (mp, np_) != (m, n):
             out = out[:, :m, :n].contiguous()
         return (out[0] if squeeze else out).view(G.shape)

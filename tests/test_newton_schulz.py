@@ -48,6 +48,7 @@ def test_sides_that_are_no_multiple_of_eight_are_padded(shape):
     g = torch.randn(*shape, device="cuda").bfloat16()
     out = newton_schulz(g)
     assert out.shape == g.shape and out.is_contiguous() and out.dtype == torch.bfloat16
+    assert not newton_schulz(g.clone().requires_grad_()).requires_grad
 
     def iterate(dtype):
         X = g.to(dtype)

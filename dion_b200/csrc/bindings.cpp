@@ -989,12 +989,12 @@ void product(const Tensor& a, const Tensor& b, const std::optional<Tensor>& c, T
 }
 
 // X [B, m, n] bf16, contiguous: X / (|X|_F + eps), then for every triple (a, b, c) of coeffs
-//   A = X X^T,  X <- a X + (b A + c A A) X      (from the right with X^T X when m > n)
+//   A = X X^T,  X <- a X + (b A + c A A) X      (from the right with X^T X when `tall`)
+// The caller decides `tall`: padding may have made the columns of a tall matrix as many as its rows.
 Tensor newton_schulz_steps(const Tensor& X0, const std::optional<Tensor>& sumsq, double eps, std::vector<double> coeffs,
-                           Tensor status) {
+                           bool tall, Tensor status) {
   TORCH_CHECK(X0.dim() == 3 && coeffs.size() % 3 == 0, "newton_schulz_steps: [B, m, n] and three coefficients per step");
   const c10::cuda::CUDAGuard guard(X0.device());
-  const bool tall = X0.size(1) > X0.size(2);
   const int64_t B = X0.size(0), k = tall ? X0.size(2) : X0.size(1);
   Tensor X = at::empty_like(X0), Y = at::empty_like(X0);
   frob_scale(X0, X, sumsq, eps);
@@ -1214,7 +1214,7 @@ TORCH_LIBRARY(dion_b200, m) {
       "int block_n, int pair, Tensor? status, int d_dup=1, Tensor? a_lo=None, Tensor? b_lo=None, "
       "Tensor? c_col_scale=None, bool split3=False) -> bool");
   m.def(
-      "newton_schulz_steps(Tensor X, Tensor? sumsq, float eps, float[] coeffs, Tensor status) -> Tensor");
+      "newton_schulz_steps(Tensor X, Tensor? sumsq, float eps, float[] coeffs, bool tall, Tensor status) -> Tensor");
   m.def(
       "gpt_block_fwd(Tensor x, Tensor wq, Tensor wk, Tensor wv, Tensor wo, Tensor wfc, Tensor wproj, Tensor cos, "
       "Tensor sin, int head_dim, float eps, bool kernel_attention, Tensor status) -> Tensor");

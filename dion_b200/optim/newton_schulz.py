@@ -75,8 +75,10 @@ def newton_schulz(G: Tensor, epsilon: float = 1e-7, coeffs: Sequence[Tuple[float
         flat = [float(v) for step in coeffs for v in step]
         # rows of X and of the k x k products have to be whole 16 bytes: other sides are padded with zero rows and
         # columns, which stay zero in every product (the products of 2 x 333 x 1001: 0.30 ms on the library's unaligned
-        # kernels, with 0.2 ms of casts and copies around them; 0.12 ms padded)
-        mp = m if m > n else (m + 7) // 8 * 8
+        # kernels, with 0.2 ms of casts and copies around them; 0.12 ms padded).  The rows of a tall matrix are no side of
+        # a k x k product and stay as they are; tall is what it was before padding.
+        tall = m > n
+        mp = m if tall else (m + 7) // 8 * 8
         np_ = (n + 7) // 8 * 8
         if (mp, np_) != (m, n):
             Xp = torch.zeros(Bn, mp, np_, device=X.device, dtype=torch.bfloat16)
@@ -84,7 +86,7 @@ def newton_schulz(G: Tensor, epsilon: float = 1e-7, coeffs: Sequence[Tuple[float
             X = Xp
         # the result is no part of an autograd graph, whatever G is
         out = torch.ops.dion_b200.newton_schulz_steps(X.detach(), None if ss is None else ss.detach(), float(epsilon), flat,
-                                                      ops.runtime.status_tensor(X.device))
+                                                      tall, ops.runtime.status_tensor(X.device))
         if (mp, np_) != (m, n):
             out = out[:, :m, :n].contiguous()
         return (out[0] if squeeze else out).view(G.shape)

@@ -41,7 +41,9 @@ def test_kernel_matches_torch_iteration(shape):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("shape", [(333, 1001), (1001, 333), (2, 130, 64), (3, 64, 130), (7, 9), (1, 8), (2, 8, 1)])
+@pytest.mark.parametrize("shape", [(333, 1001), (1001, 333), (2, 130, 64), (3, 64, 130), (7, 9), (1, 8), (2, 8, 1),
+                                   (10, 9), (333, 330), (3, 1003, 1002), (1007, 1001), (64, 3, 2), (64, 2, 1),
+                                   (16, 9, 10), (330, 333)])
 def test_sides_that_are_no_multiple_of_eight_are_padded(shape):
     """Zero rows and columns stay zero in every product: the result is the iteration's, as close to its fp64 form as the
     same bf16 iteration on PyTorch's products is (whose roundings differ; small singular values amplify them)."""
@@ -63,6 +65,18 @@ def test_sides_that_are_no_multiple_of_eight_are_padded(shape):
     err = ((out.double() - ref).norm() / ref.norm()).item()
     lib = ((iterate(torch.bfloat16).double() - ref).norm() / ref.norm()).item()
     assert err < 1.5 * lib + 4e-3, (err, lib)  # one rounding of the result is 2^-9
+
+
+@pytest.mark.gpu
+def test_muon_steps_a_slightly_tall_matrix():
+    """Ten rows and nine columns: padded to sixteen columns the matrix is still multiplied from the right."""
+    from dion_b200 import Muon
+
+    p = torch.nn.Parameter(torch.randn(10, 9, device="cuda"))
+    before = p.detach().clone()
+    p.grad = torch.randn_like(p)
+    Muon([dict(params=[p])], lr=0.02).step()
+    assert torch.isfinite(p).all() and not torch.equal(p.detach(), before)
 
 
 @pytest.mark.gpu

@@ -72,7 +72,7 @@ def newton_schulz(G: Tensor, epsilon: float = 1e-7, coeffs: Sequence[Tuple[float
     Bn, m, n = X.shape
     if scatter is None and X.numel() > 0:
         ss = None if sumsq is None else sumsq.float().contiguous()
-        flat = [float(v) for step in coeffs for v in step]
+        flat = [float(v) for a, b, c in coeffs for v in (a, b, c)]
         # rows of X and of the k x k products have to be whole 16 bytes: other sides are padded with zero rows and
         # columns, which stay zero in every product (the products of 2 x 333 x 1001: 0.30 ms on the library's unaligned
         # kernels, with 0.2 ms of casts and copies around them; 0.12 ms padded).  The rows of a tall matrix are no side of

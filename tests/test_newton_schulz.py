@@ -68,6 +68,15 @@ def test_sides_that_are_no_multiple_of_eight_are_padded(shape):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("coeffs", [[(1.0, 2.0), (3.0, 4.0), (5.0, 6.0)], [(1.0, 2.0, 3.0, 4.0)] * 3])
+def test_a_step_takes_three_coefficients(coeffs):
+    with pytest.raises(ValueError):
+        newton_schulz(torch.randn(16, 24, device="cuda"), coeffs=coeffs)
+    with pytest.raises(ValueError):
+        newton_schulz_torch(torch.randn(16, 24), coeffs=coeffs)
+
+
+@pytest.mark.gpu
 def test_muon_steps_a_slightly_tall_matrix():
     """Ten rows and nine columns: padded to sixteen columns the matrix is still multiplied from the right."""
     from dion_b200 import Muon

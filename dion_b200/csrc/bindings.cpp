@@ -195,6 +195,41 @@ bool gemm(const Tensor& a, const Tensor& b, const std::optional<Tensor>& c, Tens
 }
 
 
+// host only: how such a product would run, {tile columns, CTA pairs, CTAs that share a tile's K}; the tensors give types, sizes,
+// strides and alignment and may lie on the CPU
+std::vector<int64_t> gemm_plan(const Tensor& a, const Tensor& b, const std::optional<Tensor>& c, const Tensor& d, double beta,
+                               int64_t act, bool symmetric, int64_t block_n, int64_t pair, bool split3) {
+  dion::GemmArgs g;
+  g.ab_dtype = gemm_dtype(a, "a");
+  g.d_dtype = gemm_dtype(d, "d");
+  g.M = (int)a.size(-2);
+  g.K = (int)a.size(-1);
+  g.N = (int)b.size(-1);
+  g.batch = a.dim() == 3 ? (int)a.size(0) : 1;
+  describe_operand(a, /*contract_last=*/true, &g.a_major, &g.lda, &g.a_batch_stride, "a");
+  describe_operand(b, /*contract_last=*/false, &g.b_major, &g.ldb, &g.b_batch_stride, "b");
+  g.A = a.data_ptr();
+  g.B = b.data_ptr();
+  g.D = d.data_ptr();
+  g.ldd = d.stride(-2);
+  g.d_batch_stride = d.dim() == 3 ? d.stride(0) : 0;
+  if (c.has_value()) {
+    g.c_dtype = gemm_dtype(*c, "c");
+    g.C = c->data_ptr();
+    g.ldc = c->stride(-2);
+    g.c_batch_stride = c->dim() == 3 ? c->stride(0) : 0;
+  }
+  g.beta = (float)beta;
+  g.act = (int)act;
+  g.symmetric = symmetric ? 1 : 0;
+  g.block_n = (int)block_n;
+  g.pair = (int)pair;
+  g.split3 = split3 ? 1 : 0;
+  int out[3];
+  dion::gemm_plan(g, out);
+  return std::vector<int64_t>(out, out + 3);
+}
+
 // out-of-place product whose result tiles are scattered to per-destination blocks:
 //   mode 1: block k = rows [k*block, (k+1)*block), mode 2: block k = columns [k*block, (k+1)*block).
 // `block_like` gives dtype and row pitch of one block; `scatter_ptrs` holds batch * dests addresses.
@@ -1276,6 +1311,10 @@ TORCH_LIBRARY(dion_b200, m) {
       "int channel, int rank, int epoch, int budget_ns, Tensor(g!) status) -> ()");
   m.def("dion_q_norm(Tensor R32, Tensor ss, Tensor Qm, float eps, Tensor(a!)? Qn, Tensor(b!)? Qs, int qs_col0) -> ()");
   m.def("launch_count() -> int", &launch_count);
+  m.def(
+      "gemm_plan(Tensor a, Tensor b, Tensor? c, Tensor d, float beta=0, int act=0, bool symmetric=False, int block_n=0, int pair=0, "
+      "bool split3=False) -> int[]",
+      &gemm_plan);
   m.def("gemm_gather_plan(int M, int N, int K, int rows, int world, int rank) -> int[]", &gemm_gather_plan);
 }
 

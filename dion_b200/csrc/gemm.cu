@@ -1625,8 +1625,8 @@ bool aligned16(const void* p, long long ld, int es) {
 // times K blocks per CTA, plus what every tile costs besides (pipeline fill, the exchange of the partial tiles): about
 // kTileCost blocks.  One matrix of 14336 x 512 (10 tiles, 448 blocks) takes 8, as do twelve of 3072 x 96; 48 of
 // 768 x 768 (1008 tiles, 24 blocks) fill the chip by themselves and take 1.
-int choose_cluster_k(const GemmArgs& a, const KernelParams& kp, int bn, long long* blocks = nullptr) {
-  if (a.pair == 2 || a.pair < 0 || !a.symmetric || bn != 128 || a.a_major != kMajorMN || a.b_major != kMajorMN || a.d_dtype != kF32 ||
+int choose_cluster_k(const GemmArgs& a, int bn, long long tiles, int kblocks, long long* blocks = nullptr) {
+  if (a.pair == kPairInOrder || a.pair < 0 || !a.symmetric || bn != 128 || a.a_major != kMajorMN || a.b_major != kMajorMN || a.d_dtype != kF32 ||
       a.epilogue != kEpiStore || a.act != 0 || a.C || a.c_ptrs || a.D2 || a.d2_ptrs || a.d_ptrs || a.scatter_mode != 0 ||
       a.max_ctas > 0)
     return 1;
@@ -1637,8 +1637,8 @@ int choose_cluster_k(const GemmArgs& a, const KernelParams& kp, int bn, long lon
   long long best_cost = 0;
   for (int s = 1; s <= 8; s *= 2) {
     const long long slots = s == 8 ? sms / 8 * 7 / 8 : sms / s;
-    const long long waves = (kp.total_tiles + slots - 1) / (slots > 0 ? slots : 1);
-    const long long cost = waves * ((kp.kblocks_total + s - 1) / s + kTileCost);
+    const long long waves = (tiles + slots - 1) / (slots > 0 ? slots : 1);
+    const long long cost = waves * ((kblocks + s - 1) / s + kTileCost);
     if (s == 1 || cost < best_cost) {
       best = s;
       best_cost = cost;
@@ -1667,18 +1667,14 @@ bool split_pair(const GemmArgs& a) {
   };
   const long long t128 = tiles(128);
   long long unpaired = (t128 + sms - 1) / sms * kb * 1500;
-  KernelParams kp;
-  memset(&kp, 0, sizeof(kp));
-  kp.total_tiles = (int)(t128 < 0x7fffffff ? t128 : 0x7fffffff);
-  kp.kblocks_total = (int)kb;
   long long shared_k = 0;
-  if (choose_cluster_k(a, kp, 128, &shared_k) > 1) unpaired = shared_k * 1500;
+  if (choose_cluster_k(a, 128, t128, (int)kb, &shared_k) > 1) unpaired = shared_k * 1500;
   const long long paired = (tiles(256) + sms / 2 - 1) / (sms / 2) * (kb * 1536 + 5000);
   return paired < unpaired;
 }
 
 cudaError_t launch_split(const GemmArgs& a, const KernelParams& kp, int bn, cudaStream_t s) {
-  const int ck = bn == 256 ? 1 : choose_cluster_k(a, kp, bn);
+  const int ck = bn == 256 ? 1 : choose_cluster_k(a, bn, kp.total_tiles, kp.kblocks_total);
   if (ck > 1) {
     KernelParams kc = kp;
     kc.cluster_k = ck;
@@ -1746,21 +1742,22 @@ Tiling choose_tiling(const GemmArgs& a) {
   }
 
   // CTA pairs (256-row tiles, half the B traffic per CTA) for GEMMs with enough 256 x 256 tiles to
-  // keep every pair busy; DION_B200_GEMM_PAIR=0 turns them off, a.pair = 1 / -1 forces / forbids.
+  // keep every pair busy; DION_B200_GEMM_PAIR=0 turns them off, a.pair = 1 / -1 forces / forbids (kPairInOrder does neither).
   static const int pair_env = [] {
     const char* e = getenv("DION_B200_GEMM_PAIR");
     return (e && e[0] == '0') ? 0 : 1;
   }();
   bool pair = false;
-  if (a.pair > 0 && !a.symmetric) bn = 256;
-  if (!a.symmetric && bn == 256 && a.pair >= 0 && (pair_env || a.pair > 0)) {
+  const bool force = a.pair > 0 && a.pair != kPairInOrder;
+  if (force && !a.symmetric) bn = 256;
+  if (!a.symmetric && bn == 256 && a.pair >= 0 && (pair_env || force)) {
     const long long t = (long long)((a.M + 255) / 256) * ((a.N + 255) / 256) * a.batch * a.split_k;
     // Short-K tiles are bound by the epilogue, which a pair does not speed up.  Where C and D move by TMA the line lies
     // lower: 50176 x 768, K = 768: 58 us unpaired, 52 us on pairs, with C 65 and 64; K = 256: 31 and 37 us.  The ReLU^2
     // gradient's epilogue does more arithmetic (65536 x 3072, K = 768: 322 us unpaired, 348 us on pairs).
     const bool light = a.ab_dtype == kBF16 && a.d_dtype == kBF16 && a.a_major == kMajorK && !a.d_ptrs && !a.D2 && !a.d2_ptrs &&
                        a.scatter_mode == 0 && a.act != kActMulRelu2GradSq && a.act != kActMulRelu2Grad;
-    pair = a.pair > 0 || (t >= 2 * (num_sms() / 2) && a.K / a.split_k >= (light ? 512 : 1024));
+    pair = force || (t >= 2 * (num_sms() / 2) && a.K / a.split_k >= (light ? 512 : 1024));
   }
 
   if (sym_pair) pair = true;
@@ -1813,6 +1810,15 @@ bool plan_gather(const GemmArgs& a, const Tiling& tl, GatherParams* g) {
 }  // namespace
 
 const char* gemm_last_error() { return g_last_error.c_str(); }
+
+void gemm_plan(const GemmArgs& a, int (&out)[3]) {
+  const Tiling tl = choose_tiling(a);
+  const long long tm = (a.M + tl.tile_m - 1) / tl.tile_m, tn = (a.N + tl.bn - 1) / tl.bn;
+  const long long tiles = (a.symmetric ? tn * (tn + 1) / 2 : tm * tn) * a.batch;
+  out[0] = tl.bn;
+  out[1] = tl.pair ? 1 : 0;
+  out[2] = a.split3 && !tl.pair ? choose_cluster_k(a, tl.bn, tiles, (a.K + 31) / 32) : 1;
+}
 
 bool gemm_gather_plan(const GemmArgs& a, int (&out)[8]) {
   const Tiling tl = choose_tiling(a);

@@ -32,6 +32,8 @@ enum GemmAct : int {
 //   b_major == kMajorMN : B is stored K x N row-major (N contiguous), row pitch ldb
 // Pitches and batch strides are in elements.  Base pointers must be 16-byte
 // aligned and pitches a multiple of 16 bytes (TMA requirement).
+enum { kPairInOrder = 2 };  // GemmArgs::pair
+
 struct GemmArgs {
   const void* A = nullptr;
   const void* B = nullptr;
@@ -93,7 +95,9 @@ struct GemmArgs {
   // Three products of one A with three matrices laid out like B (bf16, K-major both, no C): batch is 3, B belongs to batch
   // element 0, these to 1 and 2, and D holds the three results d_batch_stride apart.
   const void* B_more[2] = {nullptr, nullptr};
-  int pair = 0;      // CTA pairs (256-row tiles): 0 = choose automatically, 1 = force (needs block_n 256), -1 = never
+  // CTA pairs (256-row tiles): 0 = choose automatically, 1 = force (needs block_n 256), -1 = never, and no K range shared by a
+  // cluster either; kPairInOrder = choose automatically, but every K sum is taken in one pass (no sharing by a cluster)
+  int pair = 0;
 
   int* status = nullptr;  // device int, set to a non-zero code on a device-side failure
 
@@ -125,6 +129,9 @@ struct GemmArgs {
 // and write a message retrievable with gemm_last_error().
 cudaError_t gemm_launch(const GemmArgs& args, cudaStream_t stream);
 const char* gemm_last_error();
+
+// Host only, no launch: how gemm_launch would run `args`.  out = {tile columns, CTA pairs (0 / 1), CTAs that share a tile's K}.
+void gemm_plan(const GemmArgs& args, int (&out)[3]);
 
 // Host only, no launch: what the all-gather variant would do for `args` (sizes, majors and the
 // `gather` fields world / rank / rows are read).  out = {tile rows, tile columns, CTA pairs (0 / 1),

@@ -96,7 +96,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, c: Optional[torch.Tensor] = None, 
     over three K-segments - a 3xTF32 product in a single launch.
     ``c_col_scale`` (fp32 ``[B, N]``) scales the columns of the addend: ``beta * c * diag(c_col_scale)``.
     ``pair``: 1 forces and -1 forbids CTA pairs, 0 leaves both them and the sharing of a long K by a cluster (symmetric
-    ``split3`` products with few tiles) to the kernel, 2 forbids the sharing: every K sum is taken in one pass.
+    ``split3`` products with few tiles) to the kernel, 2 leaves CTA pairs to it but forbids the sharing: every K sum is
+    taken in one pass.
     ``split3=True`` (fp32 operands): the same 3xTF32 product without any hi / lo tensors - the kernel splits
     every operand tile in shared memory, so the operands are read once.  On CPU tensors, and for operands
     the kernel cannot address, the product is taken in plain fp32.

@@ -456,3 +456,37 @@ def test_gemm_split3_splits_fp32_operands_in_shared_memory(ta, tb, shape, symmet
     from dion_b200 import ops
 
     ops.check_status()
+
+
+def _plan(a, b, d, c=None, **kw):
+    from dion_b200.ops import _ext
+
+    if not _ext.load(required=False):
+        pytest.skip("extension not built")
+    return list(torch.ops.dion_b200.gemm_plan(a, b, c, d, **kw))
+
+
+def _shapes(B, M, N, K, dtype=torch.bfloat16, out=None, a_mn=False, b_mn=True):
+    """Operands and result of a product, for their sizes and layouts alone (host memory that nothing touches)."""
+    lead = (B,) if B else ()
+    a = torch.empty(*lead, K, M, dtype=dtype).mT if a_mn else torch.empty(*lead, M, K, dtype=dtype)
+    b = torch.empty(*lead, K, N, dtype=dtype) if b_mn else torch.empty(*lead, N, K, dtype=dtype).mT
+    return a, b, torch.empty(*lead, M, N, dtype=out or dtype)
+
+
+def test_sums_in_order_forbid_the_sharing_of_k_and_nothing_else():
+    """pair=2: the tiling is the one the kernel takes by itself, for every kind of product; only a K range that CTAs of a
+    cluster would share is summed by one of them."""
+    for block_n in (0, 64, 128, 256):
+        for B, M, N, K in [(0, 512, 768, 768), (0, 8192, 768, 768), (0, 24, 96, 3072), (0, 8192, 3072, 4096), (12, 768, 3072, 768)]:
+            for dtype in (torch.bfloat16, torch.float32):
+                t = _shapes(B, M, N, K, dtype)
+                assert _plan(*t, block_n=block_n, pair=2) == _plan(*t, block_n=block_n), (B, M, N, K, block_n)
+    p = torch.empty(4, 14336, 512)
+    g = torch.empty(4, 512, 512)
+    shared = _plan(p.mT, p, g, symmetric=True, split3=True)
+    in_order = _plan(p.mT, p, g, symmetric=True, split3=True, pair=2)
+    assert in_order[2] == 1 and (shared[2] > 1 or shared[1] == 1)
+    p, g = torch.empty(12, 3072, 96), torch.empty(12, 96, 96)
+    assert _plan(p.mT, p, g, symmetric=True, split3=True)[2] > 1
+    assert _plan(p.mT, p, g, symmetric=True, split3=True, pair=2)[2] == 1

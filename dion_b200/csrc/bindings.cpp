@@ -195,8 +195,8 @@ bool gemm(const Tensor& a, const Tensor& b, const std::optional<Tensor>& c, Tens
 }
 
 
-// host only: how such a product would run, {tile columns, CTA pairs, CTAs that share a tile's K}; the tensors give types, sizes,
-// strides and alignment and may lie on the CPU
+// host only: how such a product would run, {tile columns, CTA pairs, CTAs that share a tile's K, C and D moved by TMA}; the tensors
+// give types, sizes, strides and alignment and may lie on the CPU
 std::vector<int64_t> gemm_plan(const Tensor& a, const Tensor& b, const std::optional<Tensor>& c, const Tensor& d, double beta,
                                int64_t act, bool symmetric, int64_t block_n, int64_t pair, bool split3) {
   dion::GemmArgs g;
@@ -225,9 +225,9 @@ std::vector<int64_t> gemm_plan(const Tensor& a, const Tensor& b, const std::opti
   g.block_n = (int)block_n;
   g.pair = (int)pair;
   g.split3 = split3 ? 1 : 0;
-  int out[3];
+  int out[4];
   dion::gemm_plan(g, out);
-  return std::vector<int64_t>(out, out + 3);
+  return std::vector<int64_t>(out, out + 4);
 }
 
 // out-of-place product whose result tiles are scattered to per-destination blocks:

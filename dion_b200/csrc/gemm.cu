@@ -1566,16 +1566,40 @@ cudaError_t launch_cfg(const GemmArgs& a, const KernelParams& kp, cudaStream_t s
   }
 }
 
-// Problems whose epilogue moves C and D with TMA: C and D of the operands' type, one destination, operands K-major / any,
-// 16-byte aligned rows of whole 16 bytes (every box starts at a multiple of 128 bytes; a row is clipped in units of 16
-// bytes, so that 1001 columns would lose what lies behind the 1001st).  With outputs of another type, pointer arrays, a
-// second output or scattered tiles, addends with broadcast rows, and for tiles of 64 columns, the generic epilogue remains.
-bool tma_epilogue(const GemmArgs& a, const KernelParams& kp, int bn) {
+bool aligned16(const void* p, long long ld, int es) {
+  return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && ((ld * es) & 15) == 0;
+}
+// 16-byte vector access to C and D: aligned bases and pitches.  Per-batch pointer arrays and scattered blocks satisfy
+// this by contract (checked by the Python wrapper).
+bool vec_c_ok(const GemmArgs& a) {
+  const int es = a.c_dtype == kBF16 ? 2 : 4;
+  return (a.c_ptrs || aligned16(a.C, a.ldc, es)) && (a.c_batch_stride * es) % 16 == 0;
+}
+bool vec_d_ok(const GemmArgs& a) {
+  const int es = a.d_dtype == kBF16 ? 2 : 4;
+  if (a.scatter_mode != 0) return (a.ldd * es) % 16 == 0;
+  return (a.d_ptrs || aligned16(a.D, a.ldd, es)) && (a.d_batch_stride * es) % 16 == 0;
+}
+// DION_B200_GEMM_STAGE=0: every epilogue with direct accesses
+bool stage_enabled() {
+  static const bool on = [] {
+    const char* e = getenv("DION_B200_GEMM_STAGE");
+    return !(e && e[0] == '0');
+  }();
+  return on;
+}
+
+// Problems whose epilogue moves C and D with TMA on tiles of 128 and 256 columns: C and D of the operands' type, one
+// destination, operands K-major / any, 16-byte aligned rows of whole 16 bytes (every box starts at a multiple of 128
+// bytes; a row is clipped in units of 16 bytes, so that 1001 columns would lose what lies behind the 1001st).  With outputs
+// of another type, pointer arrays, a second output or scattered tiles, addends with broadcast rows, a gathered A, and
+// for tiles of 64 columns, the generic epilogue remains.
+bool tma_epilogue(const GemmArgs& a) {
   const bool bf16 = a.ab_dtype == kBF16;
-  return kp.stage && a.a_major == kMajorK && a.d_dtype == a.ab_dtype && a.epilogue == kEpiStore && bn >= 128 &&
-         a.split_k == 1 && !a.A_lo && !a.c_ptrs && !a.d_ptrs && !a.D2 && !a.d2_ptrs && a.scatter_mode == 0 &&
-         (bf16 ? a.act != kActRelu2SavePre && !a.c_col_scale : a.act == 0 || a.act == kActRelu2) && kp.vec_d && a.D &&
-         a.ldd >= a.N && (!a.C || a.ldc >= a.N) && a.N % (bf16 ? 8 : 4) == 0 && (!a.C || (a.c_dtype == a.ab_dtype && kp.vec_c)) &&
+  return stage_enabled() && a.a_major == kMajorK && a.d_dtype == a.ab_dtype && a.epilogue == kEpiStore && a.split_k == 1 &&
+         !a.A_lo && !a.c_ptrs && !a.d_ptrs && !a.D2 && !a.d2_ptrs && a.scatter_mode == 0 && a.gather.world == 0 &&
+         (bf16 ? a.act != kActRelu2SavePre && !a.c_col_scale : a.act == 0 || a.act == kActRelu2) && vec_d_ok(a) && a.D &&
+         a.ldd >= a.N && (!a.C || a.ldc >= a.N) && a.N % (bf16 ? 8 : 4) == 0 && (!a.C || (a.c_dtype == a.ab_dtype && vec_c_ok(a))) &&
          (a.batch == 1 || (a.d_batch_stride != 0 && (!a.C || a.c_batch_stride != 0)));
 }
 // C is read only where it counts
@@ -1588,7 +1612,7 @@ KernelParams tma_params(const KernelParams& kp) {
 template <bool kTf32, int kAMajor, int kBMajor>
 cudaError_t launch_bn(const GemmArgs& a, const KernelParams& kp, int bn, bool pair, cudaStream_t s) {
   if constexpr (kAMajor == kMajorK) {
-    if (tma_epilogue(a, kp, bn)) {
+    if (bn >= 128 && tma_epilogue(a)) {
       const KernelParams kt = tma_params(kp);
       if (pair) return launch_cfg<kTf32, kAMajor, kBMajor, 256, true, false, false, false, true>(a, kt, s);
       if (bn == 128) return launch_cfg<kTf32, kAMajor, kBMajor, 128, false, false, false, false, true>(a, kt, s);
@@ -1610,15 +1634,11 @@ cudaError_t launch_split_bn(const GemmArgs& a, const KernelParams& kp, int bn, c
     if (bn == 256) return launch_cfg<true, kAMajor, kBMajor, 256, true, false, true, false, true>(a, tma_params(kp), s);
   }
   if constexpr (kAMajor == kMajorK) {
-    if (!a.c_col_scale && tma_epilogue(a, kp, bn))
+    if (bn >= 128 && !a.c_col_scale && tma_epilogue(a))
       return launch_cfg<true, kAMajor, kBMajor, 128, false, false, true, false, true>(a, tma_params(kp), s);
   }
   if (bn == 64) return launch_cfg<true, kAMajor, kBMajor, 64, false, false, true>(a, kp, s);
   return launch_cfg<true, kAMajor, kBMajor, 128, false, false, true>(a, kp, s);
-}
-
-bool aligned16(const void* p, long long ld, int es) {
-  return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && ((ld * es) & 15) == 0;
 }
 
 // CTAs of a cluster that share one output tile of a Gram product (1: no sharing).  Time is taken as waves of tiles
@@ -1752,11 +1772,12 @@ Tiling choose_tiling(const GemmArgs& a) {
   if (force && !a.symmetric) bn = 256;
   if (!a.symmetric && bn == 256 && a.pair >= 0 && (pair_env || force)) {
     const long long t = (long long)((a.M + 255) / 256) * ((a.N + 255) / 256) * a.batch * a.split_k;
-    // Short-K tiles are bound by the epilogue, which a pair does not speed up.  Where C and D move by TMA the line lies
-    // lower: 50176 x 768, K = 768: 58 us unpaired, 52 us on pairs, with C 65 and 64; K = 256: 31 and 37 us.  The ReLU^2
-    // gradient's epilogue does more arithmetic (65536 x 3072, K = 768: 322 us unpaired, 348 us on pairs).
-    const bool light = a.ab_dtype == kBF16 && a.d_dtype == kBF16 && a.a_major == kMajorK && !a.d_ptrs && !a.D2 && !a.d2_ptrs &&
-                       a.scatter_mode == 0 && a.act != kActMulRelu2GradSq && a.act != kActMulRelu2Grad;
+    // Short-K tiles are bound by the epilogue, which a pair does not speed up: from K = 1024 on.  Where C and D move by TMA
+    // (tma_epilogue) the line lies lower: 50176 x 768, K = 768: 58 us unpaired, 52 us on pairs, with C 65 and 64; K = 256: 31
+    // and 37 us.  With generic loads and stores pairs lose there: 50176 x 1004, K = 768, with C: 691 us unpaired, 845 us on
+    // pairs; 6216 x 3068: 255 and 331.  So does the ReLU^2 gradient, whose epilogue does more arithmetic (65536 x 3072,
+    // K = 768: 322 and 348).
+    const bool light = a.ab_dtype == kBF16 && tma_epilogue(a) && a.act != kActMulRelu2GradSq && a.act != kActMulRelu2Grad;
     pair = force || (t >= 2 * (num_sms() / 2) && a.K / a.split_k >= (light ? 512 : 1024));
   }
 
@@ -1811,13 +1832,14 @@ bool plan_gather(const GemmArgs& a, const Tiling& tl, GatherParams* g) {
 
 const char* gemm_last_error() { return g_last_error.c_str(); }
 
-void gemm_plan(const GemmArgs& a, int (&out)[3]) {
+void gemm_plan(const GemmArgs& a, int (&out)[4]) {
   const Tiling tl = choose_tiling(a);
   const long long tm = (a.M + tl.tile_m - 1) / tl.tile_m, tn = (a.N + tl.bn - 1) / tl.bn;
   const long long tiles = (a.symmetric ? tn * (tn + 1) / 2 : tm * tn) * a.batch;
   out[0] = tl.bn;
   out[1] = tl.pair ? 1 : 0;
   out[2] = a.split3 && !tl.pair ? choose_cluster_k(a, tl.bn, tiles, (a.K + 31) / 32) : 1;
+  out[3] = tl.bn >= 128 && out[2] == 1 && (tma_epilogue(a) || (a.split3 && tl.pair)) ? 1 : 0;
 }
 
 bool gemm_gather_plan(const GemmArgs& a, int (&out)[8]) {
@@ -1943,20 +1965,10 @@ cudaError_t gemm_launch(const GemmArgs& a, cudaStream_t stream) {
   kp.scatter_dests = a.scatter_dests;
   kp.scatter_ptrs = a.scatter_ptrs;
   kp.status = a.status;
-  // Vector access needs aligned bases and pitches; per-batch pointer arrays are
-  // required to satisfy this by contract (checked by the Python wrapper).
-  const int ces = kp.c_is_bf16 ? 2 : 4, des = kp.d_is_bf16 ? 2 : 4;
-  kp.vec_c = (a.c_ptrs || aligned16(a.C, a.ldc, ces)) && ((a.c_batch_stride * ces) % 16 == 0);
-  kp.vec_d = (a.d_ptrs || aligned16(a.D, a.ldd, des)) && ((a.d_batch_stride * des) % 16 == 0);
-  if (a.scatter_mode != 0) kp.vec_d = ((a.ldd * des) % 16 == 0);  // block bases are 16-byte aligned by contract
+  kp.vec_c = vec_c_ok(a);
+  kp.vec_d = vec_d_ok(a);
   kp.vec_d2 = (a.d2_ptrs || aligned16(a.D2, a.ldd2, 2)) && ((a.d2_batch_stride * 2) % 16 == 0);
-  {
-    static const int stage_env = [] {
-      const char* e = getenv("DION_B200_GEMM_STAGE");
-      return (e && e[0] == '0') ? 0 : 1;
-    }();
-    kp.stage = stage_env;
-  }
+  kp.stage = stage_enabled();
 
   if (a.gather.world > 0) {
     // operand A is gathered from the group inside the kernel
@@ -1978,7 +1990,7 @@ cudaError_t gemm_launch(const GemmArgs& a, cudaStream_t stream) {
     if (bn == 128) return launch_cfg<false, kMajorK, kMajorK, 128, false, true>(a, kp, stream);
     return launch_cfg<false, kMajorK, kMajorK, 256, false, true>(a, kp, stream);
   }
-  if (a.B_more[0] && !tma_epilogue(a, kp, bn)) {
+  if (a.B_more[0] && (bn < 128 || !tma_epilogue(a))) {
     g_last_error = "three products of one operand need the TMA epilogue";
     return cudaErrorInvalidValue;
   }

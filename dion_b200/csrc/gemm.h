@@ -130,8 +130,9 @@ struct GemmArgs {
 cudaError_t gemm_launch(const GemmArgs& args, cudaStream_t stream);
 const char* gemm_last_error();
 
-// Host only, no launch: how gemm_launch would run `args`.  out = {tile columns, CTA pairs (0 / 1), CTAs that share a tile's K}.
-void gemm_plan(const GemmArgs& args, int (&out)[3]);
+// Host only, no launch: how gemm_launch would run `args`.  out = {tile columns, CTA pairs (0 / 1), CTAs that share a tile's K,
+// C and D moved by TMA (0 / 1)}.
+void gemm_plan(const GemmArgs& args, int (&out)[4]);
 
 // Host only, no launch: what the all-gather variant would do for `args` (sizes, majors and the
 // `gather` fields world / rank / rows are read).  out = {tile rows, tile columns, CTA pairs (0 / 1),

@@ -490,3 +490,29 @@ def test_sums_in_order_forbid_the_sharing_of_k_and_nothing_else():
     p, g = torch.empty(12, 3072, 96), torch.empty(12, 96, 96)
     assert _plan(p.mT, p, g, symmetric=True, split3=True)[2] > 1
     assert _plan(p.mT, p, g, symmetric=True, split3=True, pair=2)[2] == 1
+
+
+def test_short_k_takes_pairs_only_where_c_and_d_move_by_tma():
+    """K from 512 to 1023: pairs pay behind the TMA epilogue and lose behind the generic one, whatever keeps a product from
+    the former; from K = 1024 on both take them."""
+    M, N, f32 = 50176, 1000, torch.float32
+    a, b, d = _shapes(0, M, N, 768)
+    assert _plan(a, b, d) == [256, 1, 1, 1] and _plan(a, b, d, torch.empty_like(d), beta=1.0) == [256, 1, 1, 1]
+    generic = [(a, b, torch.empty(M, N + 3, dtype=d.dtype)[:, :N], None),               # pitch no multiple of 16 bytes
+               (a, b, torch.empty(M, N, dtype=f32), None),                              # results of another type
+               (a, b, d, torch.empty(M, N, dtype=f32)),                                 # addend of another type
+               (a, b, d, torch.empty(1, N, dtype=d.dtype).expand(M, N)),                # addend with broadcast rows
+               (*_shapes(0, M, N + 4, 768), None),                                      # rows that end inside 16 bytes
+               (*_shapes(0, M, N, 768, a_mn=True), None)]
+    for x, y, out, c in generic:
+        assert _plan(x, y, out, c, beta=1.0)[1::2] == [0, 0], (out.shape, out.stride(), out.dtype)
+    for x, y, out, c in [(*_shapes(0, M, N + 4, 1024), None), (*_shapes(0, M, N, 1024, a_mn=True), None)]:
+        assert _plan(x, y, out, c)[1::2] == [1, 0]
+
+
+def test_gather_plan_takes_row_blocks_of_128_at_short_k():
+    """The all-gather variant stores with the generic epilogue: at K = 768 it is not paired, and row blocks that are a
+    multiple of 128 but not of 256 are taken."""
+    _plan(*_shapes(0, 64, 64, 64))
+    plan = list(torch.ops.dion_b200.gemm_gather_plan(8 * 7808, 768, 768, 7808, 8, 3))
+    assert plan and plan[0] == 128 and plan[2] == 0

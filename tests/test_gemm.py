@@ -516,3 +516,29 @@ def test_gather_plan_takes_row_blocks_of_128_at_short_k():
     _plan(*_shapes(0, 64, 64, 64))
     plan = list(torch.ops.dion_b200.gemm_gather_plan(8 * 7808, 768, 768, 7808, 8, 3))
     assert plan and plan[0] == 128 and plan[2] == 0
+
+
+@pytest.mark.parametrize("B,n,k,tall,pair", [(48, 768, 768, False, 1), (48, 768, 768, True, 1), (24, 768, 768, True, 1),
+                                             (8, 1024, 768, False, 0), (8, 1024, 768, True, 0), (8, 520, 1000, False, 0),
+                                             (8, 520, 1000, True, 0), (30, 512, 600, False, 1), (30, 512, 600, True, 0),
+                                             (48, 512, 500, False, 0), (12, 768, 3072, True, 1), (1, 768, 3072, False, 0)])
+def test_symmetric_products_with_short_k_take_pairs_for_fewer_waves(B, n, k, tall, pair):
+    """K from 512 to 1023: pairs where their waves are few enough, which depends on the epilogue (X^T X has the generic one)."""
+    x = torch.empty(B, n, k, dtype=torch.bfloat16) if not tall else torch.empty(B, k, n, dtype=torch.bfloat16).mT
+    plan = _plan(x, x.mT, torch.empty(B, n, n, dtype=torch.bfloat16), symmetric=True)
+    assert plan == [256 if pair else 128, pair, 1, 0 if tall else 1]
+    # results of another type are not stored by TMA: pairs from K = 1024 on
+    plan = _plan(x, x.mT, torch.empty(B, n, n), symmetric=True)
+    assert plan[1] == (pair if k >= 1024 else 0) and plan[3] == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,n,k", [(24, 768, 768), (40, 520, 600), (16, 512, 512)])
+def test_symmetric_products_of_tall_matrices_with_short_k(B, n, k):
+    """X^T X (MN-major operands, generic mirrored epilogue) on CTA pairs and on single tiles: the same bits, symmetric, within
+    the rounding of the bf16 result."""
+    x = torch.randn(B, k, n, device="cuda").bfloat16()
+    got = gemm(x.mT, x, symmetric=True)
+    assert torch.equal(got, gemm(x.mT, x, symmetric=True, pair=-1)) and torch.equal(got, got.mT)
+    want = x.double().mT @ x.double()
+    assert ((got.double() - want).norm() / want.norm()).item() < 2.0 ** -8

@@ -198,14 +198,18 @@ __global__ void __launch_bounds__(kPostThreads) r_post_kernel(const RPostArgs a,
   constexpr int kWarps = kPostThreads / 32;
   __shared__ float red[kWarps][32 * kV + 1];
   __shared__ float part[32 * kV];  // this CTA's sums, read by the cluster
+  __shared__ int part_ready;       // and whether its peers arrived
+  __shared__ int all_ready;        // whether those of the whole cluster did
   __shared__ float tot[32 * kV];
   uint32_t csize;
   asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(csize));
   const uint32_t crank = cluster_ctarank();
   const int strip = (int)(blockIdx.x / csize);
   const int b = blockIdx.y;
-  // a CTA whose peers did not arrive writes nothing, but stays with its cluster until the sums were exchanged
+  // A CTA whose peers did not arrive reads and writes nothing, but stays with its cluster until the sums were exchanged;
+  // without its part they are incomplete, and no CTA of the cluster stores them or the Q they scale.
   const bool ready = exchange_ready(a.wait, a.status);
+  if (threadIdx.x == 0) part_ready = ready ? 1 : 0;
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const int col = (strip * 32 + lane) * kV;
@@ -313,6 +317,13 @@ __global__ void __launch_bounds__(kPostThreads) r_post_kernel(const RPostArgs a,
   }
   if (csize > 1) cluster_sync_all();
   else __syncthreads();
+  if (warp == 0) {
+    int x = part_ready;
+    if (lane < (int)csize && csize > 1)
+      asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(x) : "r"(mapa_shared(smem_u32(&part_ready), lane)) : "memory");
+    x = __all_sync(0xffffffffu, x != 0);
+    if (lane == 0) all_ready = x;
+  }
   if (threadIdx.x < 32 * kV) {
     float t = 0.f;
     if (csize > 1) {
@@ -326,12 +337,15 @@ __global__ void __launch_bounds__(kPostThreads) r_post_kernel(const RPostArgs a,
       t = part[threadIdx.x];
     }
     tot[threadIdx.x] = t;
-    const int c = strip * 32 * kV + threadIdx.x;
-    if (ready && crank == 0 && c < a.r && a.ss) a.ss[(long long)b * a.r + c] = t;
   }
   // nobody leaves while its sums may still be read
   if (csize > 1) cluster_sync_all();
   else __syncthreads();
+  if (!all_ready) return;
+  if (threadIdx.x < 32 * kV && crank == 0 && a.ss) {
+    const int c = strip * 32 * kV + threadIdx.x;
+    if (c < a.r) a.ss[(long long)b * a.r + c] = tot[threadIdx.x];
+  }
   if (!a.finish || !live) return;
   // new Q: column-normalised R; a column that came out zero keeps the previous Q
   float inv[kV];

@@ -95,6 +95,39 @@ def test_r_post_kernel_may_write_the_new_q_over_the_previous_one():
     torch.testing.assert_close(Q[ok], Qr[ok], rtol=1e-5, atol=1e-5)
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("r", [128, 45])
+def test_r_post_kernel_stores_no_q_from_incomplete_sums(r):
+    """The eight CTAs of a strip wait for their peers one by one.  Here the word of the other rank is set beforehand, and this
+    rank's own word is set by the first CTA of the grid when it announces itself, so that with a wait of a nanosecond it
+    sees both and the others of its cluster do not.  Whatever the timing, a strip is right or untouched, and the status
+    tells of the wait that ran out."""
+    n, strip = 1024, 128 if r % 4 == 0 else 32
+    slots = torch.randn(1, 1, n, r, device="cuda")
+    Qm = torch.randn(1, n, r, device="cuda")
+    want = ops.dion_r_post_reference(slots, 1.0, None, Qm, None, 1e-8)[3]
+    flags, other = (torch.zeros(1024, dtype=torch.int32, device="cuda") for _ in range(2))
+    status = ops.runtime.status_tensor(torch.device("cuda", torch.cuda.current_device()))
+    ran_out = 0
+    for _ in range(10):
+        flags.zero_()
+        flags[1] = 1
+        Qn, ss = torch.full_like(Qm, -7.0), torch.full((1, r), -7.0, device="cuda")
+        ops.dion_r_post(slots, 1.0, None, Qm, None, None, None, ss, True, 1e-8, Qn, None, 0,
+                        wait=([flags.data_ptr(), other.data_ptr()], 0, 0, 0, 1, 1))
+        code = int(status.item())
+        status.zero_()
+        assert code in (0, 4)
+        ran_out += code == 4
+        for c in range(0, r, strip):
+            q, w = Qn[..., c:c + strip], want[..., c:c + strip]
+            untouched, right = bool((q == -7.0).all()), torch.allclose(q, w, rtol=1e-4, atol=1e-6)
+            assert untouched or right
+            assert bool((ss[:, c:c + strip] == -7.0).all()) == untouched
+            assert right or code == 4
+    assert ran_out > 0
+
+
 def _slot_reduce_case(device, nslots=4, shape=(3, 40, 24)):
     g = torch.Generator().manual_seed(1)
     slots = torch.randn(nslots, *shape, generator=g).to(device)

@@ -17,6 +17,7 @@ from typing import Optional, Tuple
 
 import torch
 import torch.nn.functional as F
+from torch.utils._device import DeviceContext
 
 from . import runtime
 from .gemm import gemm
@@ -29,13 +30,23 @@ def _fast(x: torch.Tensor) -> bool:
     return x.is_cuda and x.dtype == torch.bfloat16 and runtime.use_cuda_kernels(x)
 
 
+def _observed() -> bool:
+    """Does anything around this call have to see the single operations?  A dispatch or function mode, a tracer, a transform
+    (vmap, forward-mode derivatives) or a module-wide hook.  A default device is a function mode too, but acts on the creation
+    of tensors only."""
+    if (torch._C._len_torch_dispatch_stack() > 0 or torch._C._functorch.peek_interpreter_stack() is not None
+            or torch.autograd.forward_ad._current_level >= 0 or torch.nn.modules.module._has_any_global_hook()
+            or torch.jit.is_tracing() or torch.compiler.is_compiling()):
+        return True
+    return torch._C._len_torch_function_stack() > 0 and any(
+        type(m) is not DeviceContext for m in torch.overrides._get_current_function_mode_stack())
+
+
 def native_forward_ok(x: torch.Tensor) -> bool:
     """May a pass over ``x: [B, T, C]`` run as one native call?  Plain bf16 activations on a GPU, no gradients recorded, and
-    no transform (vmap, forward-mode derivatives) or module-wide hook that would have to see the single operations."""
+    nothing around it that would have to see the single operations."""
     return (type(x) is torch.Tensor and x.dim() == 3 and _fast(x) and x.is_contiguous() and x.numel() > 0
-            and x.shape[-1] % 8 == 0 and x.data_ptr() % 16 == 0 and not torch.is_grad_enabled()
-            and torch._C._functorch.peek_interpreter_stack() is None
-            and torch.autograd.forward_ad._current_level < 0 and not torch.nn.modules.module._has_any_global_hook())
+            and x.shape[-1] % 8 == 0 and x.data_ptr() % 16 == 0 and not torch.is_grad_enabled() and not _observed())
 
 
 # --------------------------------------------------------------------------- weights in bf16

@@ -417,3 +417,63 @@ def test_block_without_gradients_runs_natively_with_the_same_bits(B, T, heads, h
         handle.remove()
     assert torch.equal(native, general) and torch.equal(hooked, general) and seen == [1]
     ops.check_status()
+
+
+class _SeenDispatch(torch.utils._python_dispatch.TorchDispatchMode):
+    def __init__(self):
+        super().__init__()
+        self.seen = []
+
+    def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+        self.seen.append(str(func))
+        return func(*args, **(kwargs or {}))
+
+
+class _SeenFunction(torch.overrides.TorchFunctionMode):
+    def __init__(self):
+        super().__init__()
+        self.seen = []
+
+    def __torch_function__(self, func, types, args=(), kwargs=None):
+        self.seen.append(str(func))
+        return func(*args, **(kwargs or {}))
+
+
+def test_modes_tracers_and_transforms_observe_a_call():
+    assert not N._observed()
+    with torch.device("cpu"):  # a default device only acts on the creation of tensors
+        assert not N._observed()
+        with _SeenFunction():
+            assert N._observed()
+    for mode in (_SeenDispatch(), _SeenFunction(), torch.autograd.forward_ad.dual_level()):
+        with mode:
+            assert N._observed()
+        assert not N._observed()
+    answers = []
+    torch.vmap(lambda v: answers.append(N._observed()) or v)(torch.zeros(2))
+    torch.jit.trace(lambda v: answers.append(N._observed()) or v + 1, torch.zeros(2), check_trace=False)
+    handle = torch.nn.modules.module.register_module_forward_hook(lambda *a: None)
+    answers.append(N._observed())
+    handle.remove()
+    assert answers == [True, True, True] and not N._observed()
+
+
+@pytest.mark.gpu
+def test_modes_see_the_operations_of_a_block_without_gradients():
+    """A dispatch or function mode around a pass that records no gradients sees its products and norms, not one opaque call."""
+    from dion_b200.models import GPT, GPTConfig
+
+    with torch.device("cuda"):
+        model = GPT(GPTConfig(sequence_len=40, vocab_size=512, n_layer=1, n_head=2, n_embd=128))
+    model.init_weights()
+    block, x = model.transformer.h[0], torch.randn(2, 40, 128, device="cuda").bfloat16()
+    with torch.no_grad():
+        plain = block(x)
+        with _SeenDispatch() as d:
+            assert torch.equal(block(x), plain)
+        with _SeenFunction() as f:
+            assert torch.equal(block(x), plain)
+        with torch.device("cuda"):
+            assert block._forward_native(x) is not None
+    assert sum("dion_b200.gemm" in s for s in d.seen) >= 6 and not any("gpt_block_fwd" in s for s in d.seen)
+    assert any("view" in s or "reshape" in s for s in f.seen) and not any("gpt_block_fwd" in s for s in f.seen)

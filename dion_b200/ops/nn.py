@@ -30,16 +30,32 @@ def _fast(x: torch.Tensor) -> bool:
     return x.is_cuda and x.dtype == torch.bfloat16 and runtime.use_cuda_kernels(x)
 
 
+def _ask(owner, name: str, *args, unknown):
+    """What an interface that PyTorch keeps to itself answers; `unknown` where this version has none of that name or one that
+    takes other arguments.  Every caller names the answer that makes it take the general path."""
+    try:
+        return getattr(owner, name)(*args)
+    except (AttributeError, TypeError):
+        return unknown
+
+
+def _transforming() -> bool:
+    """Is a transform (vmap, grad, ...) or a forward-mode derivative under way?"""
+    return (_ask(getattr(torch._C, "_functorch", None), "peek_interpreter_stack", unknown=True) is not None
+            or getattr(torch.autograd.forward_ad, "_current_level", 0) >= 0)
+
+
 def _observed() -> bool:
     """Does anything around this call have to see the single operations?  A dispatch or function mode, a tracer, a transform
-    (vmap, forward-mode derivatives) or a module-wide hook.  A default device is a function mode too, but acts on the creation
-    of tensors only."""
-    if (torch._C._len_torch_dispatch_stack() > 0 or torch._C._functorch.peek_interpreter_stack() is not None
-            or torch.autograd.forward_ad._current_level >= 0 or torch.nn.modules.module._has_any_global_hook()
+    or a module-wide hook.  A default device is a function mode too, but acts on the creation of tensors only."""
+    if (_transforming() or _ask(torch._C, "_len_torch_dispatch_stack", unknown=1) > 0
+            or _ask(torch.nn.modules.module, "_has_any_global_hook", unknown=True)
             or torch.jit.is_tracing() or torch.compiler.is_compiling()):
         return True
-    return torch._C._len_torch_function_stack() > 0 and any(
-        type(m) is not DeviceContext for m in torch.overrides._get_current_function_mode_stack())
+    if _ask(torch._C, "_len_torch_function_stack", unknown=1) == 0:
+        return False
+    modes = _ask(torch.overrides, "_get_current_function_mode_stack", unknown=[None])
+    return any(type(m) is not DeviceContext for m in modes)
 
 
 def native_forward_ok(x: torch.Tensor) -> bool:
@@ -556,9 +572,9 @@ def embedding(idx: torch.Tensor, table: torch.Tensor, out_dtype: torch.dtype = t
 
 def _transformed(t: torch.Tensor) -> bool:
     """Does `t` stand for more than its values: a batch of several gradients, a dual number, a subclass?"""
-    return (type(t) is not torch.Tensor or torch._C._functorch.is_batchedtensor(t)
-            or torch._C._functorch.is_legacy_batchedtensor(t) or torch._C._functorch.peek_interpreter_stack() is not None
-            or torch.autograd.forward_ad._current_level >= 0)
+    functorch = getattr(torch._C, "_functorch", None)
+    return (type(t) is not torch.Tensor or _transforming() or _ask(functorch, "is_batchedtensor", t, unknown=True)
+            or _ask(functorch, "is_legacy_batchedtensor", t, unknown=True))
 
 
 def _times_scalar(x: torch.Tensor, s: torch.Tensor, in_place: bool) -> torch.Tensor:
@@ -618,16 +634,17 @@ class _LinearCrossEntropyFn(torch.autograd.Function):
             ctx.save_for_backward(dx, dw)
             ctx.w_dtype = weight.dtype
             # with saved-tensor hooks what comes back in the backward pass may belong to whoever set them
-            ctx.plain_save = torch._C._autograd._top_saved_tensors_default_hooks(False) is None
+            ctx.plain_save = _ask(torch._C._autograd, "_top_saved_tensors_default_hooks", False, unknown=True) is None
         return loss
 
     @staticmethod
     def backward(ctx, dloss):
         dx, dw = ctx.saved_tensors
         # When the graph is not kept, the kept gradients are scaled where they lie and handed on (a plain backward pass
-        # has dloss = 1 and moves nothing); otherwise they stay as they are for the next backward pass.
+        # has dloss = 1 and moves nothing); otherwise, and where PyTorch cannot tell, they stay as they are for the next
+        # backward pass.
         own = (ctx.plain_save and not torch.is_grad_enabled() and not _transformed(dloss)
-               and not torch._C._autograd._get_current_graph_task_keep_graph())
+               and not _ask(torch._C._autograd, "_get_current_graph_task_keep_graph", unknown=True))
         dxo = _times_scalar(dx, dloss, own) if ctx.needs_input_grad[0] else None
         dwo = None
         if ctx.needs_input_grad[1]:

@@ -477,3 +477,54 @@ def test_modes_see_the_operations_of_a_block_without_gradients():
             assert block._forward_native(x) is not None
     assert sum("dion_b200.gemm" in s for s in d.seen) >= 6 and not any("gpt_block_fwd" in s for s in d.seen)
     assert any("view" in s or "reshape" in s for s in f.seen) and not any("gpt_block_fwd" in s for s in f.seen)
+
+
+_PRIVATE = [(torch._C._functorch, "peek_interpreter_stack"), (torch._C._functorch, "is_batchedtensor"),
+            (torch._C._functorch, "is_legacy_batchedtensor"), (torch._C._autograd, "_top_saved_tensors_default_hooks"),
+            (torch._C._autograd, "_get_current_graph_task_keep_graph")]
+
+
+@pytest.mark.parametrize("how", ["missing", "other arguments"])
+def test_interfaces_that_another_pytorch_lacks_mean_the_general_path(monkeypatch, how):
+    """Every private interface that decides about a native call or a write in place may be absent or take other arguments."""
+    def without(owner, name):
+        if how == "missing":
+            m.delattr(owner, name)
+        else:
+            m.setattr(owner, name, lambda one, two, three: None)
+
+    t = torch.zeros(2)
+    assert not N._observed() and not N._transformed(t)
+    for owner, name in [(torch._C._functorch, "peek_interpreter_stack"), (torch._C, "_len_torch_dispatch_stack"),
+                        (torch.nn.modules.module, "_has_any_global_hook")]:
+        with monkeypatch.context() as m:
+            without(owner, name)
+            assert N._observed()
+    with _SeenFunction():
+        with monkeypatch.context() as m:  # either of the two tells of the mode
+            without(torch._C, "_len_torch_function_stack")
+            assert N._observed()
+        with monkeypatch.context() as m:
+            without(torch.overrides, "_get_current_function_mode_stack")
+            assert N._observed()
+    for name in ("peek_interpreter_stack", "is_batchedtensor", "is_legacy_batchedtensor"):
+        with monkeypatch.context() as m:
+            without(torch._C._functorch, name)
+            assert N._transformed(t)
+    assert not N._observed() and not N._transformed(t)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("owner,name", _PRIVATE)
+def test_loss_gradients_where_pytorch_lacks_an_interface(monkeypatch, owner, name):
+    x = torch.randn(256, 64, device="cuda").bfloat16().requires_grad_()
+    w = (0.1 * torch.randn(512, 64, device="cuda")).requires_grad_()
+    t = torch.randint(0, 512, (256,), device="cuda")
+    want = torch.autograd.grad(0.25 * N.linear_cross_entropy(x, w, t), (x, w))
+    kept = N.linear_cross_entropy(x, w, t)
+    with monkeypatch.context() as m:
+        m.delattr(owner, name)
+        got = torch.autograd.grad(0.25 * N.linear_cross_entropy(x, w, t), (x, w))
+        again = [torch.autograd.grad(0.25 * kept, (x, w), retain_graph=True) for _ in range(2)]
+    for g in (got, *again):
+        assert all(torch.equal(a, b) for a, b in zip(g, want))

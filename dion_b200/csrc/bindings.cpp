@@ -1044,8 +1044,9 @@ Tensor newton_schulz_steps(const Tensor& X0, const std::optional<Tensor>& sumsq,
   return X;
 }
 
-// x [B, T, C] bf16 through one block of the GPT model: x + attention(norm(x)), then + MLP(norm(.)).  The kernels, their
-// order and their arguments are those of the differentiable functions; nothing is kept for a backward pass.
+// x [B, T, C] bf16 through one block of the GPT model: x + attention(norm(x)), then + MLP(norm(.)).  The kernels and their
+// arguments are those of the differentiable functions, except that q, k and v come from one launch where that can take them
+// (the same bits); nothing is kept for a backward pass, and every intermediate is given back once its last reader is issued.
 Tensor gpt_block_fwd(const Tensor& x, const Tensor& wq, const Tensor& wk, const Tensor& wv, const Tensor& wo, const Tensor& wfc,
                      const Tensor& wproj, const Tensor& cos, const Tensor& sin, int64_t D, double eps,
                      bool kernel_attention, Tensor status) {
@@ -1056,17 +1057,19 @@ Tensor gpt_block_fwd(const Tensor& x, const Tensor& wq, const Tensor& wk, const 
   const c10::cuda::CUDAGuard guard(x.device());
   const int64_t B = x.size(0), T = x.size(1), C = x.size(2), N = B * T, heads = wq.size(0) / D;
   const Tensor x2 = x.view({N, C});
-  Tensor rstd = at::empty({N}, x.options().dtype(at::kFloat));
   auto linear = [&](const Tensor& a, const Tensor& w, const std::optional<Tensor>& residual, int act) {
     Tensor y = at::empty({N, w.size(0)}, x.options());
     product(a, w.t(), residual, y, 1., residual.has_value() ? 1. : 0., false, status, act);
     return y;
   };
-  Tensor h = at::empty_like(x2);
-  rmsnorm_fwd(x2, {}, {}, h, rstd, eps);
+  auto norm = [&](const Tensor& a) {
+    Tensor h = at::empty_like(a), rstd = at::empty({N}, x.options().dtype(at::kFloat));
+    rmsnorm_fwd(a, {}, {}, h, rstd, eps);
+    return h;
+  };
   Tensor q, k, v;
-  if (const char* env = getenv("DION_B200_GEMM_STAGE"); wq.size(0) > 64 && N > 0 && !(env && env[0] == '0')) {
-    // one launch for the three projections
+  {
+    const Tensor h = norm(x2);
     Tensor qkv = at::empty({3, N, wq.size(0)}, x.options());
     dion::GemmArgs g;
     g.ab_dtype = g.d_dtype = dion::kBF16;
@@ -1083,28 +1086,34 @@ Tensor gpt_block_fwd(const Tensor& x, const Tensor& wq, const Tensor& wk, const 
     g.ldd = g.N;
     g.d_batch_stride = N * g.N;
     g.status = status.data_ptr<int>();
-    const cudaError_t e = dion::gemm_launch(g, at::cuda::getCurrentCUDAStream());
-    TORCH_CHECK(e == cudaSuccess, "projections: ", cudaGetErrorString(e), " ", dion::gemm_last_error());
-    g_launches.fetch_add(1, std::memory_order_relaxed);
     q = qkv[0], k = qkv[1], v = qkv[2];
-  } else {
-    q = linear(h, wq, {}, 0), k = linear(h, wk, {}, 0), v = linear(h, wv, {}, 0);
+    if (dion::gemm_takes_three(g)) {
+      const cudaError_t e = dion::gemm_launch(g, at::cuda::getCurrentCUDAStream());
+      TORCH_CHECK(e == cudaSuccess, "projections: ", cudaGetErrorString(e), " ", dion::gemm_last_error());
+      g_launches.fetch_add(1, std::memory_order_relaxed);
+    } else {
+      for (auto [y, w] : {std::pair(q, wq), std::pair(k, wk), std::pair(v, wv)})
+        product(h, w.t(), {}, y, 1., 0., false, status);
+    }
   }
-  Tensor qo = at::empty_like(q), ko = at::empty_like(k);
-  rope_qknorm_fwd(q, k, qo, ko, cos, sin, T, heads, D, eps);
-  const Tensor q4 = qo.view({B, T, heads, D}), k4 = ko.view({B, T, heads, D}), v4 = v.view({B, T, heads, D});
   Tensor y;
-  if (kernel_attention && T % 128 == 0 && B * heads <= 65535) {
-    y = at::empty_like(q4);
-    Tensor lse = at::empty({B, heads, T}, x.options().dtype(at::kFloat));
-    attn_fwd(q4, k4, v4, y, lse, 1. / std::sqrt((double)D), status);
-  } else {
-    y = at::scaled_dot_product_attention(q4.transpose(1, 2), k4.transpose(1, 2), v4.transpose(1, 2), {}, 0., true)
-            .transpose(1, 2);
+  {
+    Tensor qo = at::empty_like(q), ko = at::empty_like(k);
+    rope_qknorm_fwd(q, k, qo, ko, cos, sin, T, heads, D, eps);
+    const Tensor q4 = qo.view({B, T, heads, D}), k4 = ko.view({B, T, heads, D}), v4 = v.view({B, T, heads, D});
+    if (kernel_attention && T % 128 == 0 && B * heads <= 65535) {
+      y = at::empty_like(q4);
+      Tensor lse = at::empty({B, heads, T}, x.options().dtype(at::kFloat));
+      attn_fwd(q4, k4, v4, y, lse, 1. / std::sqrt((double)D), status);
+    } else {
+      y = at::scaled_dot_product_attention(q4.transpose(1, 2), k4.transpose(1, 2), v4.transpose(1, 2), {}, 0., true)
+              .transpose(1, 2);
+    }
+    q = k = v = Tensor();
   }
   const Tensor x3 = linear(y.reshape({N, C}), wo, x2, 0);
-  rmsnorm_fwd(x3, {}, {}, h, rstd, eps);
-  const Tensor u = linear(h, wfc, {}, dion::kActRelu2);
+  y = Tensor();
+  const Tensor u = linear(norm(x3), wfc, {}, dion::kActRelu2);
   return linear(u, wproj, x3, 0).view({B, T, C});
 }
 

@@ -1847,6 +1847,12 @@ void gemm_plan(const GemmArgs& a, int (&out)[4]) {
   out[3] = tl.bn >= 128 && out[2] == 1 && (tma_epilogue(a) || (a.split3 && tl.pair)) ? 1 : 0;
 }
 
+// The maps of the second and third B take the slots that only the TMA epilogue leaves free without C and mirrored boxes.
+bool gemm_takes_three(const GemmArgs& a) {
+  return a.B_more[0] && a.B_more[1] && a.batch == 3 && a.ab_dtype == kBF16 && a.b_major == kMajorK && !a.C && !a.symmetric &&
+         a.d_batch_stride > 0 && tma_epilogue(a) && choose_tiling(a).bn >= 128;
+}
+
 bool gemm_gather_plan(const GemmArgs& a, int (&out)[8]) {
   const Tiling tl = choose_tiling(a);
   GatherParams g;
@@ -1889,10 +1895,7 @@ cudaError_t gemm_launch(const GemmArgs& a, cudaStream_t stream) {
     g_last_error = "symmetric mode needs M == N";
     return cudaErrorInvalidValue;
   }
-  if (a.B_more[0] && (!a.B_more[1] || a.batch != 3 || a.ab_dtype != kBF16 || a.d_dtype != kBF16 || a.a_major != kMajorK ||
-                      a.b_major != kMajorK || a.C || a.symmetric || a.N <= 64 || a.N % 8 != 0 || a.block_n == 64 ||
-                      a.epilogue != kEpiStore || !a.D || a.d_batch_stride <= 0 || a.d_batch_stride % 8 != 0 ||
-                      !aligned16(a.D, a.ldd, 2) || a.gather.world > 0)) {
+  if (a.B_more[0] && !gemm_takes_three(a)) {
     g_last_error = "three products of one operand: bf16, K-major, no addend, aligned outputs of more than 64 columns";
     return cudaErrorInvalidValue;
   }
@@ -1994,10 +1997,6 @@ cudaError_t gemm_launch(const GemmArgs& a, cudaStream_t stream) {
     if (pair) return launch_cfg<false, kMajorK, kMajorK, 256, true, true>(a, kp, stream);
     if (bn == 128) return launch_cfg<false, kMajorK, kMajorK, 128, false, true>(a, kp, stream);
     return launch_cfg<false, kMajorK, kMajorK, 256, false, true>(a, kp, stream);
-  }
-  if (a.B_more[0] && (bn < 128 || !tma_epilogue(a))) {
-    g_last_error = "three products of one operand need the TMA epilogue";
-    return cudaErrorInvalidValue;
   }
   if (a.split3) return launch_split(a, kp, bn, stream);
   return tf32 ? launch_major<true>(a, kp, bn, pair, stream) : launch_major<false>(a, kp, bn, pair, stream);

@@ -130,6 +130,9 @@ struct GemmArgs {
 cudaError_t gemm_launch(const GemmArgs& args, cudaStream_t stream);
 const char* gemm_last_error();
 
+// Host only, no launch: can one launch take the three products of `args` (GemmArgs::B_more)?
+bool gemm_takes_three(const GemmArgs& args);
+
 // Host only, no launch: how gemm_launch would run `args`.  out = {tile columns, CTA pairs (0 / 1), CTAs that share a tile's K,
 // C and D moved by TMA (0 / 1)}.
 void gemm_plan(const GemmArgs& args, int (&out)[4]);

@@ -144,8 +144,8 @@ class Block(nn.Module):
 
     def _forward_native(self, x: torch.Tensor):
         """The block as one native call, for passes that record no gradients; None where the general path has to run
-        (hooks or replaced parts, tensor-parallel weights, other types and sizes than the kernels take).  Same kernels in
-        the same order, so the same bits."""
+        (hooks or replaced parts, tensor-parallel weights, other types and sizes than the kernels take).  The products and
+        kernels of the general path, with q, k and v in one launch: the same bits, and no more memory."""
         attn, mlp = self.attn, self.mlp
         if not (K.native_forward_ok(x) and _plain(attn, CausalSelfAttention) and _plain(mlp, MLP)
                 and _plain(attn.rotary, Rotary) and attn.head_dim in (64, 128) and x.shape[-1] <= 4096):

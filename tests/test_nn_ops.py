@@ -528,3 +528,32 @@ def test_loss_gradients_where_pytorch_lacks_an_interface(monkeypatch, owner, nam
         again = [torch.autograd.grad(0.25 * kept, (x, w), retain_graph=True) for _ in range(2)]
     for g in (got, *again):
         assert all(torch.equal(a, b) for a, b in zip(g, want))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T", [256, 200])
+def test_block_without_gradients_holds_no_more_than_its_single_operations(T):
+    """The native block gives every intermediate back once its last reader is issued: its peak is at most that of the general
+    path, which a hook selects."""
+    from dion_b200.models import GPT, GPTConfig
+
+    with torch.device("cuda"):
+        model = GPT(GPTConfig(sequence_len=T, vocab_size=512, n_layer=1, n_head=4, n_embd=512))
+    model.init_weights()
+    block, x = model.transformer.h[0], torch.randn(8, T, 512, device="cuda").bfloat16()
+
+    def peak():
+        block(x)
+        torch.cuda.synchronize()
+        held = torch.cuda.memory_allocated()
+        torch.cuda.reset_peak_memory_stats()
+        block(x)
+        return torch.cuda.max_memory_allocated() - held
+
+    with torch.no_grad():
+        assert block._forward_native(x) is not None
+        native = peak()
+        block.attn.register_forward_hook(lambda *a: None)
+        assert block._forward_native(x) is None
+        general = peak()
+    assert native <= general

@@ -542,3 +542,38 @@ def test_symmetric_products_of_tall_matrices_with_short_k(B, n, k):
     assert torch.equal(got, gemm(x.mT, x, symmetric=True, pair=-1)) and torch.equal(got, got.mT)
     want = x.double().mT @ x.double()
     assert ((got.double() - want).norm() / want.norm()).item() < 2.0 ** -8
+
+
+_LAYOUTS = {  # out, addend (or None) for an M x N product, B of them where the first is 3-D
+    "slices of wider rows": lambda z, r: (z(256, 3, 256).transpose(0, 1), None),
+    "slices of wider rows, addend too": lambda z, r: (z(256, 3, 256).transpose(0, 1), r(256, 3, 256).transpose(0, 1)),
+    "slices with a gap": lambda z, r: (z(200, 3, 272)[:, :, :264].transpose(0, 1), None),
+    "one row, odd pitch": lambda z, r: (torch.as_strided(z(512), (1, 256), (257, 1)), torch.as_strided(r(512), (1, 256), (259, 1))),
+    "one row, pitch 1": lambda z, r: (torch.as_strided(z(512), (1, 256), (1, 1)), None),
+    "one row each, odd pitch": lambda z, r: (torch.as_strided(z(1024), (2, 1, 256), (256, 257, 1)), None),
+    "addend of one row": lambda z, r: (z(256, 256), r(256).expand(256, 256)),
+    "addend of one matrix": lambda z, r: (z(3, 256, 256), r(256, 256).expand(3, 256, 256)),
+    "batch of one, odd stride": lambda z, r: (torch.as_strided(z(65536), (1, 256, 256), (7, 256, 1)),
+                                             torch.as_strided(r(65536), (1, 256, 256), (9, 256, 1))),
+    "addend beside the result": lambda z, r: (lambda buf: (buf[:, :256], buf[:, 512:768]))(r(256, 1024)),
+}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("layout", list(_LAYOUTS))
+def test_results_and_addends_in_any_layout(layout, dtype):
+    """Batch strides below the row pitch, single rows of any pitch, broadcast addends, result and addend in one buffer: the
+    epilogue that the layout selects stores what it should and nothing else."""
+    out, c = _LAYOUTS[layout](lambda *s: torch.zeros(*s, device="cuda", dtype=dtype),
+                              lambda *s: torch.randn(*s, device="cuda").to(dtype))
+    lead, (M, N), K = out.shape[:-2], out.shape[-2:], 128
+    a, b = torch.randn(*lead, M, K, device="cuda").to(dtype), torch.randn(*lead, K, N, device="cuda").to(dtype)
+    want = a.double() @ b.double() + (0.0 if c is None else c.double())
+    base = out if out._base is None else out._base
+    before = base.clone()
+    gemm(a, b, c=c, beta=0.0 if c is None else 1.0, out=out)
+    # one rounding of the result to bf16 (2^-9), tf32 operands with 10 bits of mantissa
+    assert ((out.double() - want).norm() / want.norm()).item() < 2.0 ** -8
+    out.copy_(torch.as_strided(before, out.shape, out.stride(), out.storage_offset()))
+    assert torch.equal(base, before)

@@ -569,9 +569,9 @@ chol_inverse_pair_kernel(const float* __restrict__ Gall, float* __restrict__ Zal
 // Every product is one warp's 32 x 32 x 32 outer-product loop; blocks of A are stored transposed (blk[col][row]) and those
 // of Z by rows, so that both operands of every product are read as vectors.  While phase B runs, warp 0 updates block
 // (k + 1, k + 1) first and factorises it (lane i owns row i), so that the serial part hides behind the products.
-// Bound by fp32 FMA and by that chain: 11 M FMA at rank 256.  72 matrices of rank 256: 117 us, of rank 96: 36 us; the kernel
-// with two CTAs per matrix below, which exchanges through global memory after every step, takes 448 and 152 us and
-// remains for larger ranks, whose triangle does not fit.
+// Bound by fp32 FMA and by that chain: 11 M FMA at rank 256.  72 matrices of rank 256, calls in a row: 109 us, of rank 96:
+// 27 us; the kernel with two CTAs per matrix below, which exchanges through global memory after every step, takes 439 and
+// 143 us and remains for larger ranks, whose triangle does not fit.
 constexpr int kTriMaxBlocks = 8;
 constexpr int kTriThreads = 512;
 constexpr int kTriLinvPitch = 36;  // Linv transposed: rows of whole 16 bytes that start in different banks
@@ -752,9 +752,16 @@ chol_inverse_tri_kernel(const float* __restrict__ Gall, float* __restrict__ Zall
     __syncthreads();
     if (m == 0) break;
     const int nA = m * (m + 1) / 2, total = nA + m * (k + 1);
-    // warp 0 takes the next diagonal block and its factorisation, the others everything else (and warp 0 what is left
-    // over once there are fewer of them than work)
-    for (int it = warp == 0 ? 0 : warp; it < total; it += warps - 1) {
+    if (warp == 0) {
+      // the next diagonal block (the first of the nA) and its factorisation
+      float acc[4][8] = {};
+      tri_product(PT + (k + 1) * 32, pp, PT + (k + 1) * 32, pp, lane, acc);
+      tri_store<true>(block(k + 1, k + 1), 32, lane, acc, 1.f);
+      __syncwarp();
+      factor(k + 1);
+      continue;
+    }
+    for (int it = warp; it < total; it += warps - 1) {  // everything else
       float acc[4][8] = {};
       if (it < nA) {
         int i = 0, j = it;
@@ -773,11 +780,6 @@ chol_inverse_tri_kernel(const float* __restrict__ Gall, float* __restrict__ Zall
           tri_product(PT + i * 32, pp, linv, 32, lane, acc);
           tri_store<false>(block(i, k), 32, lane, acc, -1.f);
         }
-      }
-      if (warp == 0) {
-        __syncwarp();
-        factor(k + 1);
-        break;
       }
     }
   }

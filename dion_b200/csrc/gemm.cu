@@ -1627,7 +1627,7 @@ cudaError_t launch_bn(const GemmArgs& a, const KernelParams& kp, int bn, bool pa
   }
 }
 
-// fp32 operands split in shared memory: 64- and 128-column tiles
+// fp32 operands split in shared memory: 64- and 128-column tiles, and 256-column tiles on CTA pairs (TMA epilogue only)
 template <int kAMajor, int kBMajor>
 cudaError_t launch_split_bn(const GemmArgs& a, const KernelParams& kp, int bn, cudaStream_t s) {
   if constexpr (kAMajor == kMajorK || kAMajor == kBMajor) {
@@ -1787,7 +1787,8 @@ Tiling choose_tiling(const GemmArgs& a) {
   }
 
   if (sym_pair) pair = true;
-  if (a.A_lo != nullptr || a.split3) {  // the cross-term accumulator exists on unpaired tiles of up to 128 columns
+  // the cross-term accumulator exists on unpaired tiles of up to 128 columns and, for split3, on 256-column tiles of pairs
+  if (a.A_lo != nullptr || a.split3) {
     pair = a.split3 && split_pair(a);
     if (pair) bn = 256;
     else if (bn > 128) bn = 128;

@@ -273,7 +273,8 @@ def _orthonormalize_many(Ps, row_groups, refine_passes, pivot_floor, shard_group
     Xs = [P.float() for P in Ps]
     # What is consumed in 16 bits keeps the order of the row sums.  Summed in parts the Gram matrices are closer to exact
     # (12 x 3072 x 96: 2e-6 instead of 2e-5), but P then differs in the fifth digit, after which 3 % of the entries of a
-    # bf16 Q round to the neighbouring value, 30 % after two steps: more than a resumed run's states may differ by.
+    # bf16 Q round to the neighbouring value, 30 % after two steps: 1.6e-3 to 2.3e-3 of the states' norm, where two correct
+    # runs are taken to agree within 1e-3 (the optimizer cases of perf/cases.py).  fp32 states take the parts (2e-4).
     in_order = [dt == torch.bfloat16 for dt in dtypes]
     first_info = [None] * n
     last_info = [None] * n  # pivots the last factorisation of each batch gave up on

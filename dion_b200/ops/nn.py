@@ -587,13 +587,16 @@ def _times_scalar(x: torch.Tensor, s: torch.Tensor, in_place: bool) -> torch.Ten
     return out
 
 
-def _halve_contraction(M: int, N: int, K: int) -> bool:
+def _halve_contraction(M: int, N: int, K: int, pairs: int) -> bool:
     """Should a product with a very long contraction be cut in two halves that are added in fp32 (two summands onto zero:
-    the same bits in any order)?  Where the 256 x 256 tiles leave most of a wave of CTA pairs idle: 8192 x 768 has 96
-    tiles for 74 pairs, two waves where one and a half do (K = 50304: 590 -> 476 us with the clearing and the cast)."""
+    the same bits in any order)?  Where its 256 x 256 tiles, of which `pairs` run at a time, take at least a sixth fewer
+    waves when cut: the last wave is nearly empty.  With the clearing and the cast, K = 50304: 8192 x 768 (96 tiles for 74
+    pairs, two waves or one and a half) 580 and 489 us, 6144 x 1024 802 and 509, 8192 x 1280 (3 and 2.5) 1168 and 878; at
+    K = 16384, the shortest measured, 8192 x 768 220 and 181.  Four waves and three and a half no longer pay for the second
+    pass: 4096 x 4096, K = 128256: 3644 and 3714 us; 8192 x 2048, K = 16384: 386 and 405."""
     tiles = ((M + 255) // 256) * ((N + 255) // 256)
-    pairs = 74
-    return K >= 16384 and tiles * 2 >= 2 * pairs and 2 * (-(-tiles // pairs)) * 9 >= (-(-2 * tiles // pairs)) * 10
+    whole, halves = -(-tiles // pairs), -(-2 * tiles // pairs)
+    return K >= 16384 and tiles >= pairs and halves * 6 <= 2 * whole * 5
 
 
 class _LinearCrossEntropyFn(torch.autograd.Function):
@@ -614,6 +617,7 @@ class _LinearCrossEntropyFn(torch.autograd.Function):
         dw = torch.empty(V, K, device=x.device, dtype=torch.float32) if need_grad else None
         chunk = min(chunk_tokens, T)
         logits = torch.empty(chunk, V, device=x.device, dtype=torch.bfloat16)
+        pairs = torch.cuda.get_device_properties(x.device).multi_processor_count // 2
         for t0 in range(0, T, chunk):
             t1 = min(t0 + chunk, T)
             n = t1 - t0
@@ -622,7 +626,7 @@ class _LinearCrossEntropyFn(torch.autograd.Function):
             torch.ops.dion_b200.cross_entropy_fwd_bwd(lg, targets[t0:t1], row_loss[t0:t1], inv_valid, 1.0,
                                                       ignore_index, need_grad)
             if need_grad:
-                if _halve_contraction(n, K, V):  # [n, V] @ [V, K]
+                if _halve_contraction(n, K, V, pairs):  # [n, V] @ [V, K]
                     acc = torch.zeros(n, K, device=x.device, dtype=torch.float32)
                     gemm(lg, wb, out=acc, accumulate=True, split_k=2)
                     dx[t0:t1].copy_(acc)

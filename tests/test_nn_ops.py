@@ -557,3 +557,32 @@ def test_block_without_gradients_holds_no_more_than_its_single_operations(T):
         assert block._forward_native(x) is None
         general = peak()
     assert native <= general
+
+
+def test_long_contractions_are_halved_where_the_last_wave_is_nearly_empty():
+    halved = [(8192, 768, 50304), (8192, 640, 50304), (6144, 1024, 50304), (8192, 1280, 50304), (7000, 768, 50304),
+              (8192, 768, 16384), (4096, 1280, 50304)]
+    whole = [(8192, 512, 50304), (8192, 1024, 50304), (4096, 2048, 32000), (8192, 2048, 16384), (4096, 4096, 128256),
+             (8192, 4096, 128256), (8192, 1536, 50304), (8192, 768, 16376), (300, 256, 50304)]
+    assert all(N._halve_contraction(*s, 74) for s in halved) and not any(N._halve_contraction(*s, 74) for s in whole)
+    assert not N._halve_contraction(8192, 768, 50304, 96)  # a device on which one wave takes the tiles
+
+
+@pytest.mark.gpu
+def test_halved_input_gradient_of_the_loss():
+    """A whole and a ragged chunk whose gradient products are cut in two: dx against the fp32 statement, the same bits again."""
+    T, K, V, chunk = 8192 + 6100, 768, 16384, 8192
+    pairs = torch.cuda.get_device_properties(0).multi_processor_count // 2
+    assert N._halve_contraction(chunk, K, V, pairs) and -(-(T - chunk) // 256) * 3 < pairs  # the second chunk is not cut
+    x = torch.randn(T, K, device="cuda").bfloat16().requires_grad_()
+    w = (0.02 * torch.randn(V, K, device="cuda")).requires_grad_()
+    t = torch.randint(0, V, (T,), device="cuda")
+    runs = [torch.autograd.grad(N.linear_cross_entropy(x, w, t, chunk_tokens=chunk), (x, w)) for _ in range(3)]
+    assert all(torch.equal(a, b) for r in runs[1:] for a, b in zip(r, runs[0]))
+    wb = w.detach().bfloat16().float()
+    logits = x.detach().float() @ wb.t()
+    p = torch.softmax(logits, -1)
+    p[torch.arange(T, device="cuda"), t] -= 1.0
+    want = (p / T) @ wb
+    # logits of about 0.55, the probabilities and dx are rounded to bf16 once each (2^-9 relative)
+    assert ((runs[0][0].float() - want).norm() / want.norm()).item() < 3 * 2.0 ** -9

@@ -2,6 +2,7 @@
 import pytest
 import torch
 
+from dion_b200 import ops
 from dion_b200.ops.gemm import gemm
 
 
@@ -577,3 +578,37 @@ def test_results_and_addends_in_any_layout(layout, dtype):
     assert ((out.double() - want).norm() / want.norm()).item() < 2.0 ** -8
     out.copy_(torch.as_strided(before, out.shape, out.stride(), out.storage_offset()))
     assert torch.equal(base, before)
+
+
+@pytest.mark.gpu
+def test_two_streams_at_a_time_give_the_bits_of_one():
+    """Clusters that share K, split pairs, the TMA epilogue with mirrored boxes, the Cholesky inverse and the launch sequence
+    of Newton-Schulz issued on two streams at once, each with inputs of its own: the kernels keep nothing between calls and
+    what one stream holds on an SM never blocks the other for good."""
+    from dion_b200.optim.newton_schulz import newton_schulz
+
+    def inputs(seed):
+        g = torch.Generator("cuda").manual_seed(seed)
+        r = lambda *s: torch.randn(*s, generator=g, device="cuda")
+        return r(12, 3072, 96), r(6, 768, 768), r(24, 768, 768).bfloat16(), r(2, 333, 330).bfloat16()
+
+    def work(p, f, x, odd):
+        G = gemm(p.mT, p, symmetric=True, split3=True)
+        return [G, ops.linalg.chol_inverse(G)[0], gemm(f, f, split3=True), gemm(x, x.mT, symmetric=True),
+                gemm(x, x, c=x, beta=1.0), newton_schulz(x), newton_schulz(odd)]
+
+    sets = [inputs(1), inputs(2)]
+    want = [work(*s) for s in sets]
+    streams = [torch.cuda.Stream() for _ in sets]
+    for s in streams:
+        s.wait_stream(torch.cuda.current_stream())
+    got = [[], []]
+    for _ in range(4):
+        for i, s in enumerate(streams):
+            with torch.cuda.stream(s):
+                got[i].append(work(*sets[i]))
+    torch.cuda.synchronize()
+    for i in range(2):
+        for outs in got[i]:
+            assert all(torch.equal(a, b) for a, b in zip(outs, want[i]))
+    ops.check_status()

@@ -1074,17 +1074,22 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       // warp waits for the accumulator, those of chunk c + 1 while chunk c is converted and stored, so that
       // their latency does not add to every chunk (with 8 epilogue warps per CTA nothing else hides it).
       // Same lane mapping as stage_fetch: 4 (bf16) or 8 (fp32) lanes per row, 8 or 4 rows per instruction.
-      const bool prefetch_c = !kSplit && stage_c;  // the splitting variants have no registers to spare
-      uint4 cq[8];
+      // fp32 addends only with fp32 operands (weight updates, 4 x 14336 x 4096, rank 512: 722 -> 698 us): bf16 products run
+      // this epilogue at the limit of its instructions, and the mere code of a second kind of addend costs those that have
+      // none 3 to 5 % (to fp32, 8192 x 3072, K = 768, MN-major: 52.6 -> 54.6 us; with a chunk loop of their own 56 us).
+      // The splitting variants have no registers to spare.
+      constexpr bool kFetchF32 = kTf32;
+      const bool prefetch_c = !kSplit && stage_c && (kFetchF32 || p.c_is_bf16);
+      uint4 cq[kFetchF32 ? 8 : 4];
       auto c_prefetch = [&](int chunk) {
-        if (p.c_is_bf16) {
+        if (!kFetchF32 || p.c_is_bf16) {
           const char* cp = c_base + ((long long)(row_first + (lane >> 2)) * p.ldc + n0 + chunk * 32) * 2 + (lane & 3) * 16;
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             cq[i] = make_uint4(0u, 0u, 0u, 0u);
             if (row_first + i * 8 + (lane >> 2) < p.M) cq[i] = *reinterpret_cast<const uint4*>(cp + (long long)i * 8 * p.ldc * 2);
           }
-        } else {
+        } else if constexpr (kFetchF32) {
           const char* cp = c_base + ((long long)(row_first + (lane >> 3)) * p.ldc + n0 + chunk * 32) * 4 + (lane & 7) * 16;
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
@@ -1175,15 +1180,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
           if (use_c) {
             float cv[32];
             if (prefetch_c) {
-              if (p.c_is_bf16) {
+              if (!kFetchF32 || p.c_is_bf16) {
 #pragma unroll
                 for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(st + stage_off(i * 8 + (lane >> 2), lane & 3)) = cq[i];
-              } else {
+              } else if constexpr (kFetchF32) {
 #pragma unroll
                 for (int i = 0; i < 8; ++i) *reinterpret_cast<uint4*>(st + stage_off(i * 4 + (lane >> 3), lane & 7)) = cq[i];
               }
               __syncwarp();
-              stage_get(st, lane, p.c_is_bf16 != 0, cv);
+              stage_get(st, lane, !kFetchF32 || p.c_is_bf16 != 0, cv);
               __syncwarp();
               if (c + 1 < c_first + kChunksPerWarp) c_prefetch(c + 1);  // a full tile: every chunk is in range
             } else if (stage_c) {

@@ -1736,9 +1736,10 @@ Tiling choose_tiling(const GemmArgs& a) {
   // Symmetric products with long K and enough 256 x 256 tiles on and above the diagonal run on CTA pairs as well (half the B
   // traffic per CTA, wide MMAs).  Short K is bound by the epilogue, where 128-wide tiles spread the mirrored stores over more
   // CTAs: bf16 products with K from 512 to 1023 go by the waves that each takes, of which a wave of pairs takes about 1.4
-  // times as long with C and D moved by TMA, and 1.6 times with the generic epilogue.  48 x 768, K = 768 (7 waves or 4 of
-  // pairs): 36 and 31 us, X^T X (generic): 38 and 36 us.  8 x 1024, K = 768 (2 and 2): 13.5 and 16.7 us, X^T X: 14.9 and 20.7;
-  // 8 x 520, K = 1000 (1 and 1): 12.3 and 15.3; 30 x 512, K = 600 (3 and 2): 19.4 and 17.7, X^T X: 17.4 and 18.2.
+  // times as long with C and D moved by TMA, and 1.6 times with the generic epilogue (1.4 from K = 960 on).
+  // 48 x 768, K = 768 (7 waves or 4 of pairs): 36 and 31 us, X^T X (generic): 38 and 36 us.  8 x 1024, K = 768 (2 and 2): 13.5
+  // and 16.7 us, X^T X: 14.9 and 20.7; 8 x 520, K = 1000 (1 and 1): 12.3 and 15.3; 30 x 512, K = 600 (3 and 2): 19.4 and 17.7,
+  // X^T X: 17.4 and 18.2, with K = 1000 22.1 and 20.8.
   bool sym_pair = false;
   if (a.symmetric) {
     const long long sms = num_sms();
@@ -1749,7 +1750,7 @@ Tiling choose_tiling(const GemmArgs& a) {
       return (e && e[0] == '0') ? 0 : 1;
     }();
     const bool fewer_waves = a.ab_dtype == kBF16 && a.d_dtype == kBF16 && a.K >= 512 &&
-                             (t + sms / 2 - 1) / (sms / 2) * 10 < (t128 + sms - 1) / sms * (tma_epilogue(a) ? 7 : 6);
+                             (t + sms / 2 - 1) / (sms / 2) * 10 < (t128 + sms - 1) / sms * (tma_epilogue(a) || a.K >= 960 ? 7 : 6);
     sym_pair = sym_pair_env && a.pair >= 0 && a.split_k == 1 && a.N >= 512 && a.A_lo == nullptr && !a.split3 &&
                (a.K >= 1024 ? t >= sms / 4 : fewer_waves);
     bn = sym_pair ? 256 : 128;

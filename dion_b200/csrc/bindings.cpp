@@ -1062,14 +1062,11 @@ Tensor gpt_block_fwd(const Tensor& x, const Tensor& wq, const Tensor& wk, const 
     product(a, w.t(), residual, y, 1., residual.has_value() ? 1. : 0., false, status, act);
     return y;
   };
-  auto norm = [&](const Tensor& a) {
-    Tensor h = at::empty_like(a), rstd = at::empty({N}, x.options().dtype(at::kFloat));
-    rmsnorm_fwd(a, {}, {}, h, rstd, eps);
-    return h;
-  };
+  Tensor rstd = at::empty({N}, x.options().dtype(at::kFloat));
   Tensor q, k, v;
   {
-    const Tensor h = norm(x2);
+    Tensor h = at::empty_like(x2);
+    rmsnorm_fwd(x2, {}, {}, h, rstd, eps);
     Tensor qkv = at::empty({3, N, wq.size(0)}, x.options());
     dion::GemmArgs g;
     g.ab_dtype = g.d_dtype = dion::kBF16;
@@ -1096,7 +1093,7 @@ Tensor gpt_block_fwd(const Tensor& x, const Tensor& wq, const Tensor& wk, const 
         product(h, w.t(), {}, y, 1., 0., false, status);
     }
   }
-  Tensor y;
+  Tensor y, h;
   {
     Tensor qo = at::empty_like(q), ko = at::empty_like(k);
     rope_qknorm_fwd(q, k, qo, ko, cos, sin, T, heads, D, eps);
@@ -1110,10 +1107,13 @@ Tensor gpt_block_fwd(const Tensor& x, const Tensor& wq, const Tensor& wk, const 
               .transpose(1, 2);
     }
     q = k = v = Tensor();
+    h = qo.numel() == x2.numel() ? qo.view_as(x2) : at::empty_like(x2);  // the rotated q is not needed any more
   }
   const Tensor x3 = linear(y.reshape({N, C}), wo, x2, 0);
   y = Tensor();
-  const Tensor u = linear(norm(x3), wfc, {}, dion::kActRelu2);
+  rmsnorm_fwd(x3, {}, {}, h, rstd, eps);
+  const Tensor u = linear(h, wfc, {}, dion::kActRelu2);
+  h = Tensor();
   return linear(u, wproj, x3, 0).view({B, T, C});
 }
 

@@ -47,15 +47,18 @@ def _transforming() -> bool:
 
 def _observed() -> bool:
     """Does anything around this call have to see the single operations?  A dispatch or function mode, a tracer, a transform
-    or a module-wide hook.  A default device is a function mode too, but acts on the creation of tensors only."""
-    if (_transforming() or _ask(torch._C, "_len_torch_dispatch_stack", unknown=1) > 0
-            or _ask(torch.nn.modules.module, "_has_any_global_hook", unknown=True)
-            or torch.jit.is_tracing() or torch.compiler.is_compiling()):
+    or a module-wide hook.  A default device is a function mode too, but acts on the creation of tensors only.  One guard
+    around all questions: this runs for every block of a model (1.2 us with a guard each, 0.7 us so)."""
+    c = torch._C
+    try:
+        if (c._len_torch_dispatch_stack() > 0 or c._functorch.peek_interpreter_stack() is not None
+                or torch.autograd.forward_ad._current_level >= 0 or torch.nn.modules.module._has_any_global_hook()
+                or torch.jit.is_tracing() or torch.compiler.is_compiling()):
+            return True
+        return c._len_torch_function_stack() > 0 and any(
+            type(m) is not DeviceContext for m in torch.overrides._get_current_function_mode_stack())
+    except (AttributeError, TypeError):
         return True
-    if _ask(torch._C, "_len_torch_function_stack", unknown=1) == 0:
-        return False
-    modes = _ask(torch.overrides, "_get_current_function_mode_stack", unknown=[None])
-    return any(type(m) is not DeviceContext for m in modes)
 
 
 def native_forward_ok(x: torch.Tensor) -> bool:

@@ -3,13 +3,14 @@
 // thread, read from tensor memory with tcgen05.ld).  It stands in for the fused attention the
 // reference gets from F.scaled_dot_product_attention (models/gpt_model.py:90-92).
 //
-// Forward, one CTA per (128 query rows, batch, head); two CTAs share an SM so that one CTA's
-// softmax overlaps the other's MMAs:
-//   warp 0      TMA: Q once, then K_j and V_j (two stages each) for every 64-row kv tile
-//   warp 1      MMA issue: S_j = Q K_j^T into one of two S buffers, O (+)= P_j V_j
-//   warps 2-5   softmax: running max / sum in the log2 domain, P_j as bf16 back into tensor memory
-//               over S_j (the second MMA reads its A operand from there), lazy rescaling of O (only
-//               when the running max grew by more than 2^8), final O / l and the log-sum-exp
+// All three large kernels (forward, dQ, dK / dV) are persistent, one CTA per SM, and work on tiles of 128 queries by 128
+// keys: one warp issues the TMA loads, one elected lane of a warp each stream of MMAs, and eight or sixteen warps do the
+// softmax with S, dP (fp32), P and dS (bf16) in tensor memory.  What bounds them is the special function unit (16 exponentials per
+// cycle and SM: 1024 cycles per pair of tiles) and, at D = 128, the tensor core (2048 cycles in dK / dV); what costs time on
+// top are the waits between the roles, 200 to 300 cycles from an arrival to what it sets off.  So every product is issued as early
+// as its operands allow, and nothing waits for a buffer that could be another one.
+//   64 x 1024 x 12 heads of 64 (us, this against 128 x 64 tiles with two CTAs per SM): forward 183 / 250, dQ 237 / 368,
+//   dK and dV 261 / 579; 32 heads of 128 with 8 kv heads at T = 4096: 133 / 170, 165 / 301, 250 / 473.
 // Layouts: q [B*T, H*D], k / v [B*T, Hkv*D], out [B*T, H*D] (bf16, row-major), lse [B, H, T] fp32.
 // Every mbarrier wait is bounded; a wait that gives up sets the status word and the CTA drains.
 #include <cuda.h>
@@ -18,6 +19,7 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <atomic>
 #include <mutex>
 #include <type_traits>
 
@@ -29,40 +31,8 @@ namespace dion {
 
 namespace {
 
-constexpr int kAttnThreads = 192;
-constexpr int kBM = 128;  // query rows per CTA
-constexpr int kBN = 64;   // kv rows per iteration
+constexpr int kBM = 128;  // rows of a tile, of queries and of keys
 constexpr float kRescaleThreshold = 8.f;  // log2 units
-
-template <int D>
-struct AttnCfg {
-  static constexpr int PANELS = D / 64;             // 128-byte panels along the head dimension
-  static constexpr int Q_BYTES = kBM * D * 2;
-  static constexpr int K_BYTES = kBN * D * 2;
-  static constexpr int V_BYTES = kBN * D * 2;
-  // two CTAs per SM: 2 * (SMEM + 1 KB reserved) must fit in 228 KB; the 896 bytes of slack cover the
-  // alignment of the (128-byte aligned) dynamic shared memory base to 1024
-  static constexpr int SMEM = Q_BYTES + 2 * K_BYTES + 2 * V_BYTES + 128 + 896;
-  static constexpr int S_COLS = kBN;                // fp32 columns of one S buffer
-  static constexpr int O_COL = 2 * kBN;             // O starts after the two S buffers
-  static constexpr int TMEM_COLS = 256;             // 2 * 64 + D <= 256
-};
-
-struct AttnParams {
-  __nv_bfloat16* out;
-  float* lse;
-  int T, H, Hkv;
-  float scale_log2;  // softmax scale * log2(e)
-  int* status;
-};
-
-__device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
-          smem_u32(smem_dst)),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0), "r"(c1)
-      : "memory");
-}
 
 __device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const float (&v)[32]) {
   const uint32_t* r = reinterpret_cast<const uint32_t*>(v);
@@ -113,15 +83,20 @@ __device__ __forceinline__ void umma_ts_h(uint32_t tmem_d, uint32_t tmem_a, Desc
       : "memory");
 }
 
-// barrier of the two warps (64 threads) that share TMEM lane quadrant `quad`; immediate barrier
-// numbers, so that the kernel reserves five named barriers instead of all sixteen
-__device__ __forceinline__ void pair_barrier(int quad) {
-  switch (quad) {
-    case 0: asm volatile("bar.sync 1, 64;" ::: "memory"); break;
-    case 1: asm volatile("bar.sync 2, 64;" ::: "memory"); break;
-    case 2: asm volatile("bar.sync 3, 64;" ::: "memory"); break;
-    default: asm volatile("bar.sync 4, 64;" ::: "memory"); break;
-  }
+// One lane of a converged warp.  tcgen05.mma takes its descriptors from uniform registers: issued by a thread of a
+// divergent branch (`if (lane == 0)`) every MMA costs about 63 cycles, whatever its shape; with the whole warp running
+// the loop and one elected lane issuing, 8 MMAs of 128 x 64 x 16 go out in 285 cycles (48 each when both operands
+// come from shared memory, 32 when A comes from tensor memory: the rates of the tensor core itself).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(p));
+  return p != 0;
+}
+// a value that is the same in all lanes, in a form the compiler can keep in a uniform register
+__device__ __forceinline__ uint32_t warp_uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
+// mbar_wait by a whole warp, with one answer for all lanes
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
 }
 
 __device__ __forceinline__ float fast_exp2(float x) {
@@ -155,310 +130,6 @@ __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
   return r;
 }
 
-template <int D>
-__global__ void __launch_bounds__(kAttnThreads, 2)
-attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
-                const __grid_constant__ CUtensorMap tmap_v, const AttnParams p) {
-  using C = AttnCfg<D>;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
-                                             ~static_cast<uintptr_t>(1023));
-  uint8_t* sQ = smem;
-  uint8_t* sK = sQ + C::Q_BYTES;          // two stages
-  uint8_t* sV = sK + 2 * C::K_BYTES;      // two stages
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sV + 2 * C::V_BYTES);
-  uint64_t* q_full = bars;          // 1
-  uint64_t* k_full = bars + 1;      // 2
-  uint64_t* k_empty = bars + 3;     // 2
-  uint64_t* v_full = bars + 5;      // 2
-  uint64_t* v_empty = bars + 7;     // 2   PV_j retired: V stage j & 1 and the P buffer free, O stable
-  uint64_t* s_full = bars + 9;      // 2
-  uint64_t* p_full = bars + 11;     // 2
-  // (bars + 13 unused)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-
-  const int warp = threadIdx.x >> 5;
-  const int lane = threadIdx.x & 31;
-  // heavy (late) query tiles first, so that the tail of the grid is made of short CTAs
-  const int q_tile = (int)gridDim.x - 1 - (int)blockIdx.x;
-  const int bh = blockIdx.y;
-  const int b = bh / p.H, h = bh - b * p.H;
-  const int hk = h / (p.H / p.Hkv);
-  const int q_row0 = b * p.T + q_tile * kBM;      // row in the [B*T, .] matrices
-  const int n_tiles = min((q_tile * kBM + kBM + kBN - 1) / kBN, (p.T + kBN - 1) / kBN);  // causal
-
-  if (threadIdx.x == 0) {
-    tma_prefetch_desc(&tmap_q);
-    tma_prefetch_desc(&tmap_k);
-    tma_prefetch_desc(&tmap_v);
-    mbar_init(q_full, 1);
-    for (int s = 0; s < 2; ++s) {
-      mbar_init(&k_full[s], 1);
-      mbar_init(&k_empty[s], 1);
-      mbar_init(&s_full[s], 1);
-      mbar_init(&p_full[s], 4);
-      mbar_init(&v_full[s], 1);
-      mbar_init(&v_empty[s], 1);
-    }
-    *abort_flag = 0;
-    mbar_fence_init();
-  }
-  if (warp == 1) {
-    tmem_alloc(tmem_slot, C::TMEM_COLS);
-    tmem_relinquish();
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
-
-  if (warp == 0) {
-    // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      mbar_arrive_expect_tx(q_full, C::Q_BYTES);
-#pragma unroll
-      for (int c = 0; c < C::PANELS; ++c) tma_load_2d(sQ + c * (kBM * 128), &tmap_q, q_full, h * D + c * 64, q_row0);
-      bool ok = true;
-      for (int j = 0; j < n_tiles && ok; ++j) {
-        const int s = j & 1;
-        const int kv_row = b * p.T + j * kBN;
-        if (!mbar_wait(&k_empty[s], ((j >> 1) & 1) ^ 1u, abort_flag)) {
-          ok = false;
-          break;
-        }
-        mbar_arrive_expect_tx(&k_full[s], C::K_BYTES);
-#pragma unroll
-        for (int c = 0; c < C::PANELS; ++c)
-          tma_load_2d(sK + s * C::K_BYTES + c * (kBN * 128), &tmap_k, &k_full[s], hk * D + c * 64, kv_row);
-        if (!mbar_wait(&v_empty[s], ((j >> 1) & 1) ^ 1u, abort_flag)) {
-          ok = false;
-          break;
-        }
-        mbar_arrive_expect_tx(&v_full[s], C::V_BYTES);
-#pragma unroll
-        for (int c = 0; c < C::PANELS; ++c)
-          tma_load_2d(sV + s * C::V_BYTES + c * (kBN * 128), &tmap_v, &v_full[s], hk * D + c * 64, kv_row);
-      }
-      if (!ok) {
-        *abort_flag = 1;
-        if (p.status) atomicCAS(p.status, 0, kStatusProducerTimeout);
-      }
-    }
-  } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc_qk = make_instr_desc(1, kMajorK, kMajorK, kBM, kBN);
-      constexpr uint32_t idesc_pv = make_instr_desc(1, kMajorK, kMajorMN, kBM, D);
-      const DescHalves dq_ = desc_halves(smem_u32(sQ), 16, 1024);
-      const DescHalves dk0 = desc_halves(smem_u32(sK), 16, 1024), dk1 = desc_halves(smem_u32(sK + C::K_BYTES), 16, 1024);
-      const DescHalves dv0 = desc_halves(smem_u32(sV), kBN * 128, 1024),
-                       dv1 = desc_halves(smem_u32(sV + C::V_BYTES), kBN * 128, 1024);
-      bool ok = mbar_wait(q_full, 0, abort_flag);
-      // S_j and P_j share tensor-memory columns (P_j overwrites the first half of S_j), and the
-      // tensor core executes this thread's MMAs in issue order, so S_{j+2} = Q K_{j+2}^T, issued after
-      // P_j V_j, cannot overtake it; the softmax has finished reading S_j once p_full[j & 1] completed.
-      auto issue_qk = [&](int j) -> bool {
-        const int s = j & 1;
-        if (!mbar_wait(&k_full[s], (j >> 1) & 1, abort_flag)) return false;
-        tc_fence_after();
-        const DescHalves dk_s = s ? dk1 : dk0;
-#pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-          const uint32_t off_a = (kk >> 2) * (kBM * 128) + (kk & 3) * 32;
-          const uint32_t off_b = (kk >> 2) * (kBN * 128) + (kk & 3) * 32;
-          umma_ss_h(tmem_base + s * C::S_COLS, dq_, off_a, dk_s, off_b, idesc_qk, kk > 0 ? 1u : 0u);
-        }
-        umma_commit(&k_empty[s]);
-        umma_commit(&s_full[s]);
-        return true;
-      };
-      if (ok) ok = issue_qk(0);
-      if (ok && n_tiles > 1) ok = issue_qk(1);
-      for (int j = 0; j < n_tiles && ok; ++j) {
-        const int s = j & 1;
-        if (!mbar_wait(&v_full[s], (j >> 1) & 1, abort_flag) || !mbar_wait(&p_full[s], (j >> 1) & 1, abort_flag)) {
-          ok = false;
-          break;
-        }
-        tc_fence_after();
-        const DescHalves dv_s = s ? dv1 : dv0;
-#pragma unroll
-        for (int kk = 0; kk < kBN / 16; ++kk) {
-          // P from tensor memory: 16 bf16 of a row = 8 columns per step; V: MN-major, PANELS chunks of
-          // 64 head columns, 16 kv rows per step
-          umma_ts_h(tmem_base + C::O_COL, tmem_base + s * C::S_COLS + kk * 8, dv_s, kk * (16 * 128), idesc_pv,
-                    (j > 0 || kk > 0) ? 1u : 0u);
-        }
-        umma_commit(&v_empty[s]);
-        if (j + 2 < n_tiles) ok = issue_qk(j + 2);
-      }
-      if (!ok) {
-        *abort_flag = 1;
-        if (p.status) atomicCAS(p.status, 0, kStatusMmaTimeout);
-      }
-    }
-  } else {
-    // ------------------------------------------------------------------ softmax / epilogue
-    const int quad = warp & 3;
-    const int row_in_tile = quad * 32 + lane;
-    const int q_pos = q_tile * kBM + row_in_tile;            // position in the sequence
-    const uint32_t lane_base = tmem_base + ((uint32_t)(quad * 32) << 16);
-    float m_used = -INFINITY;  // reference max of the exponentials accumulated so far (log2 domain)
-    float l = 0.f;
-    bool ok = true;
-    for (int j = 0; j < n_tiles && ok; ++j) {
-      const int s = j & 1;
-      if (!mbar_wait(&s_full[s], (j >> 1) & 1, abort_flag)) {
-        ok = false;
-        break;
-      }
-      tc_fence_after();
-      float sc[kBN];
-      {
-        float(&lo)[32] = *reinterpret_cast<float(*)[32]>(&sc[0]);
-        float(&hi)[32] = *reinterpret_cast<float(*)[32]>(&sc[32]);
-        tmem_ld_32x32(lane_base + s * C::S_COLS, lo);
-        tmem_ld_32x32(lane_base + s * C::S_COLS + 32, hi);
-        tmem_ld_wait();
-      }
-
-      const int col0 = j * kBN;
-      const bool diag = col0 + kBN - 1 > q_tile * kBM;  // some column of this tile may exceed some row
-      if (diag) {
-#pragma unroll
-        for (int i = 0; i < kBN; ++i)
-          if (col0 + i > q_pos) sc[i] = -INFINITY;
-      }
-      // row maximum of the raw scores (the scale is positive), four independent chains
-      float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-      for (int i = 0; i < kBN; i += 8) {
-#pragma unroll
-        for (int t = 0; t < 4; ++t) mx4[t] = fmaxf(mx4[t], fmaxf(sc[i + 2 * t], sc[i + 2 * t + 1]));
-      }
-      const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * p.scale_log2;
-      const float m_new = fmaxf(m_used, mx);
-      const bool need = (j == 0) || (m_new - m_used > kRescaleThreshold);
-      if (__any_sync(0xffffffffu, need)) {
-        if (j > 0) {
-          // O may only be touched between two PV products: P_{j-1} V_{j-1} must have retired, and
-          // P_j V_j cannot start before this warp delivered P_j
-          if (!mbar_wait(&v_empty[(j - 1) & 1], ((j - 1) >> 1) & 1, abort_flag)) {
-            ok = false;
-            break;
-          }
-          const float alpha = (m_new == -INFINITY) ? 1.f : fast_exp2(m_used - m_new);
-          l *= alpha;
-          tc_fence_after();
-#pragma unroll 1
-          for (int c = 0; c < D / 32; ++c) {
-            float o[32];
-            tmem_ld_32x32(lane_base + C::O_COL + c * 32, o);
-            tmem_ld_wait();
-#pragma unroll
-            for (int i = 0; i < 32; ++i) o[i] *= alpha;
-            tmem_st_32x32(lane_base + C::O_COL + c * 32, o);
-          }
-          tmem_st_wait();
-          tc_fence_before();
-        }
-        m_used = m_new;
-      }
-      const float neg_m = (m_used == -INFINITY) ? 0.f : -m_used;
-      const f32x2 s2 = pack2(p.scale_log2, p.scale_log2), nm2 = pack2(neg_m, neg_m);
-      f32x2 sums[2] = {pack2(0.f, 0.f), pack2(0.f, 0.f)};
-      // exponentials, packed to bf16 pairs and stored over the first half of this row of S_j
-      float pk[32];
-#pragma unroll
-      for (int c = 0; c < kBN / 8; ++c) {
-#pragma unroll
-        for (int t = 0; t < 4; ++t) {
-          float e0, e1;
-          unpack2(fma2(pack2(sc[8 * c + 2 * t], sc[8 * c + 2 * t + 1]), s2, nm2), e0, e1);
-          e0 = fast_exp2(e0);
-          e1 = fast_exp2(e1);
-          const __nv_bfloat162 h2 = __floats2bfloat162_rn(e0, e1);
-          pk[4 * c + t] = __uint_as_float(*reinterpret_cast<const uint32_t*>(&h2));
-          sums[t & 1] = add2(sums[t & 1], pack2(e0, e1));
-        }
-      }
-      tmem_st_32x32(lane_base + s * C::S_COLS, pk);
-      float sum0, sum1;
-      unpack2(add2(sums[0], sums[1]), sum0, sum1);
-      l += sum0 + sum1;
-      tmem_st_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&p_full[s]);
-    }
-    // final: wait for the last PV, normalise, write out and the log-sum-exp
-    if (ok && !mbar_wait(&v_empty[(n_tiles - 1) & 1], ((n_tiles - 1) >> 1) & 1, abort_flag)) ok = false;
-    if (ok) {
-      tc_fence_after();
-      const float inv_l = l > 0.f ? 1.f / l : 0.f;
-      const bool row_ok = q_pos < p.T;
-      __nv_bfloat16* orow = p.out + ((long long)(b * p.T + q_pos) * p.H + h) * D;
-#pragma unroll 1
-      for (int c = 0; c < D / 32; ++c) {
-        float o[32];
-        tmem_ld_32x32(lane_base + C::O_COL + c * 32, o);
-        tmem_ld_wait();
-        if (row_ok) {
-#pragma unroll
-          for (int i = 0; i < 32; i += 8) {
-            uint4 q;
-            __nv_bfloat162* hh = reinterpret_cast<__nv_bfloat162*>(&q);
-#pragma unroll
-            for (int t = 0; t < 4; ++t) hh[t] = __floats2bfloat162_rn(o[i + 2 * t] * inv_l, o[i + 2 * t + 1] * inv_l);
-            *reinterpret_cast<uint4*>(orow + c * 32 + i) = q;
-          }
-        }
-      }
-      if (row_ok && p.lse)
-        p.lse[((long long)b * p.H + h) * p.T + q_pos] = (l > 0.f) ? (m_used + log2f(l)) * 0.6931471805599453f : -INFINITY;
-    } else {
-      *abort_flag = 1;
-      if (p.status) atomicCAS(p.status, 0, kStatusEpilogueTimeout);
-    }
-  }
-
-  tc_fence_before();
-  __syncthreads();
-  if (*abort_flag != 0) {
-    // a wait gave up: let copies that are still in flight land before the CTA retires
-    const unsigned long long t0 = global_timer_ns();
-    while (global_timer_ns() - t0 < 2000000ull) __nanosleep(1000);
-    __syncthreads();
-  }
-  if (warp == 1) {
-    tc_fence_after();
-    tmem_dealloc(tmem_base, C::TMEM_COLS);
-  }
-}
-
-// ============================================================================================ backward
-// dQ, dK, dV of causal attention from q, k, v, dO, the forward's log-sum-exp and
-// delta_i = sum_d O_id dO_id (`attn_delta_kernel`).  With S = scale * Q K^T, P = exp(S - lse):
-//   dV = P^T dO,  dP = dO V^T,  dS = P o (dP - delta) * scale,  dQ = dS K,  dK = dS^T Q.
-// Two kernels, neither needs atomics:
-//   attn_bwd_dq_kernel   one CTA per 128 query rows, loops over kv tiles (S, dP, dQ in tensor memory)
-//   attn_bwd_dkv_kernel  one CTA per 128 kv rows, loops over query tiles and over the query heads
-//                        that share the kv head (S^T, dP^T double buffered, dV, dK in tensor memory)
-// P and dS are rebuilt in registers from S and dP and handed to the next MMA as bf16 through tensor
-// memory, over the columns they were read from.
-
-struct AttnBwdParams {
-  __nv_bfloat16* dq;
-  __nv_bfloat16* dk;
-  __nv_bfloat16* dv;
-  const float* lse;
-  const float* delta;
-  int T, H, Hkv;
-  float scale, scale_log2;
-  int* status;
-};
-
 __device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&r)[16]) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
@@ -481,96 +152,249 @@ __device__ __forceinline__ void bulk_load_1d(void* smem_dst, const void* gsrc, u
                : "memory");
 }
 
-// delta[b, h, t] = sum_d O[b, t, h, d] * dO[b, t, h, d]; D / 8 lanes per (b, t, h) row, 16 bytes per lane
-template <int D>
-__global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __restrict__ o,
-                                                        const __nv_bfloat16* __restrict__ d_o,
-                                                        float* __restrict__ delta, long long rows, int T, int H) {
-  constexpr int LPR = D / 8;  // lanes per row: 16 (D = 128) or 8 (D = 64)
-  const long long row = ((long long)blockIdx.x * 256 + threadIdx.x) / LPR;  // index into [B, T, H]
-  const int sub = threadIdx.x % LPR;
-  float s = 0.f;
-  if (row < rows) {
-    const uint4 a = *reinterpret_cast<const uint4*>(o + row * D + sub * 8);
-    const uint4 g = *reinterpret_cast<const uint4*>(d_o + row * D + sub * 8);
-    const __nv_bfloat162* ah = reinterpret_cast<const __nv_bfloat162*>(&a);
-    const __nv_bfloat162* gh = reinterpret_cast<const __nv_bfloat162*>(&g);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float2 x = __bfloat1622float2(ah[i]), y = __bfloat1622float2(gh[i]);
-      s = fmaf(x.x, y.x, fmaf(x.y, y.y, s));
+// n / d for 0 <= n < 2^31 by a multiplication (Granlund and Montgomery, 1994); the integer division of the device takes some
+// hundred cycles, and a role does several of them before it can start on a tile
+struct FastDiv {
+  uint32_t d, m, s;
+  FastDiv() = default;
+  explicit FastDiv(int divisor) : d((uint32_t)divisor), m(0), s(0) {
+    while (s < 31 && (1u << s) < d) ++s;
+    m = (uint32_t)(((1ull << 32) * ((1ull << s) - d)) / d + 1);
+  }
+  __device__ __forceinline__ int operator()(int n) const { return (int)((__umulhi((uint32_t)n, m) + (uint32_t)n) >> s); }
+};
+
+// What a persistent CTA works through: (sequence and head, tile) pairs, tile `level` 0 being the one with the most work.
+// The pairs are taken in groups of as many heads as there are CTAs: a CTA then runs all tiles of one head, so every CTA
+// does the same work per group and what it reads again is still in L2.  The heads that are left over are dealt out tile
+// by tile, heaviest first, back and forth over the CTAs.
+struct WorkPlan {  // made on the host
+  int levels, whole, first, rem, total;  // tiles per head; rounds with a head for every CTA; the heads after them, their pairs
+  FastDiv by_rem;
+  WorkPlan() = default;
+  WorkPlan(int levels_, int heads, int ctas)
+      : levels(levels_), whole(heads / ctas * levels_), first(heads / ctas * ctas), rem(heads % ctas), total(rem * levels_),
+        by_rem(rem > 0 ? rem : 1) {}
+};
+struct WorkList {
+  const WorkPlan& plan;
+  int head, level;  // the current pair
+  int round = 0;
+  bool valid = true;
+  __device__ __forceinline__ explicit WorkList(const WorkPlan& p) : plan(p), head((int)blockIdx.x), level(0) {
+    if (plan.whole == 0) leftover();
+  }
+  __device__ __forceinline__ void next() {
+    ++round;
+    if (round < plan.whole) {
+      if (++level == plan.levels) {
+        level = 0;
+        head += (int)gridDim.x;
+      }
+    } else {
+      leftover();
     }
   }
+  __device__ __forceinline__ void leftover() {
+    const int g = (int)gridDim.x, c = (int)blockIdx.x;
+    const int r = round - plan.whole;
+    const int k = r * g + ((r & 1) ? g - 1 - c : c);
+    valid = k < plan.total;
+    level = plan.by_rem(k);
+    head = plan.first + (k - level * plan.rem);
+  }
+};
+
+// Position in a ring of N stages and the parity of the barrier phase that fills it next
+template <int N>
+struct Ring {
+  int s = 0;
+  uint32_t ph = 0;
+  __device__ __forceinline__ void next() {
+    if (++s == N) {
+      s = 0;
+      ph ^= 1u;
+    }
+  }
+};
+
+// 16 lanes x 32 fp32 columns: lane t receives, for k = 0..3, columns 8k + 2 (t & 3) and + 1 of row t >> 2 (v[4k], v[4k + 1])
+// and of row (t >> 2) + 8 (v[4k + 2], v[4k + 3])
+__device__ __forceinline__ void tmem_ld_16x256b_x4(uint32_t taddr, float (&v)[16]) {
+  uint32_t* r = reinterpret_cast<uint32_t*>(v);
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+// 128 rows x 32 bytes from shared memory (a K-major operand tile) to 8 columns of tensor memory
+__device__ __forceinline__ void tmem_cp_128x32b(uint32_t taddr, DescHalves d, uint32_t off) {
+  asm volatile("{\n\t.reg .b64 d;\n\tmov.b64 d, {%1, %2};\n\ttcgen05.cp.cta_group::1.128x256b [%0], d;\n\t}" ::"r"(taddr),
+               "r"(d.lo + (off >> 4)), "r"(d.hi)
+               : "memory");
+}
+// v[k] of lane q of each group of four becomes v[q] of lane k
+__device__ __forceinline__ void quad_transpose(uint32_t (&v)[4], int lane) {
 #pragma unroll
-  for (int off = LPR / 2; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-  if (sub == 0 && row < rows) {
-    const long long bt = row / H;
-    const int h = (int)(row - bt * H);
-    const long long b = bt / T;
-    const int t = (int)(bt - b * T);
-    delta[(b * H + h) * T + t] = s;
+  for (int b = 1; b <= 2; b <<= 1) {
+    const bool up = lane & b;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (i & b) continue;
+      const uint32_t got = __shfl_xor_sync(0xffffffffu, up ? v[i] : v[i | b], b);
+      if (up) v[i] = got;
+      else v[i | b] = got;
+    }
+  }
+}
+// 32 accumulator rows (lane quadrant `quad`, COLS fp32 columns from `taddr`) to `out` as bf16, row r at out + (quad * 32 + r) *
+// pitch, rows from `rows` on left out; kScaled: times the factor that the lane of the row holds.  Eight rows of 64 bytes per store instruction: with a row per lane each one touches
+// 32 lines, and the stores of dV and dK took 3000 cycles per kv tile.
+template <int COLS, bool kScaled = false>
+__device__ __forceinline__ void store_rows(uint32_t taddr, int quad, int lane, __nv_bfloat16* out, long long pitch, int rows,
+                                           float scale_of_lane = 1.f) {
+#pragma unroll
+  for (int c0 = 0; c0 < COLS; c0 += 64) {  // all loads of 64 columns first: they take as long as one
+    constexpr int CH = COLS < 64 ? COLS / 32 : 2;
+    float v[2][CH][16];
+#pragma unroll
+    for (int hh = 0; hh < 2; ++hh)
+#pragma unroll
+      for (int c = 0; c < CH; ++c)
+        tmem_ld_16x256b_x4(taddr + ((uint32_t)(quad * 32 + hh * 16) << 16) + c0 + c * 32, v[hh][c]);
+    tmem_ld_wait();
+#pragma unroll
+    for (int hh = 0; hh < 2; ++hh) {
+      const int row = quad * 32 + hh * 16 + (lane >> 2);
+      __nv_bfloat16* dst = out + row * pitch + c0 + (lane & 3) * 8;
+      float f0 = 1.f, f1 = 1.f;  // of this lane's two rows
+      if constexpr (kScaled) {
+        f0 = __shfl_sync(0xffffffffu, scale_of_lane, hh * 16 + (lane >> 2));
+        f1 = __shfl_sync(0xffffffffu, scale_of_lane, hh * 16 + 8 + (lane >> 2));
+      }
+#pragma unroll
+      for (int c = 0; c < CH; ++c) {
+        uint32_t lo[4], hi[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const float* w = &v[hh][c][4 * k];
+          lo[k] = kScaled ? pack_bf16x2(w[0] * f0, w[1] * f0) : pack_bf16x2(w[0], w[1]);
+          hi[k] = kScaled ? pack_bf16x2(w[2] * f1, w[3] * f1) : pack_bf16x2(w[2], w[3]);
+        }
+        quad_transpose(lo, lane);
+        quad_transpose(hi, lane);
+        if (row < rows) *reinterpret_cast<uint4*>(dst + c * 32) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+        if (row + 8 < rows) *reinterpret_cast<uint4*>(dst + 8 * pitch + c * 32) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+      }
+    }
   }
 }
 
+// D[128 x 128] = A B^T over the head dimension, both K-major tiles; A from tensor memory (a_col) where kTmemA
+template <int D, bool kTmemA>
+__device__ __forceinline__ void scores(uint32_t d_col, DescHalves a, uint32_t a_col, DescHalves b, uint32_t b_off) {
+  constexpr uint32_t idesc = make_instr_desc(1, kMajorK, kMajorK, kBM, kBM);
+#pragma unroll
+  for (int kk = 0; kk < D / 16; ++kk) {
+    const uint32_t off = (kk >> 2) * (kBM * 128) + (kk & 3) * 32;
+    if constexpr (kTmemA) umma_ts_h(d_col, a_col + kk * 8, b, b_off + off, idesc, kk > 0 ? 1u : 0u);
+    else umma_ss_h(d_col, a, off, b, b_off + off, idesc, kk > 0 ? 1u : 0u);
+  }
+}
+// a K-major tile of 128 rows into tensor memory as the A operand of `scores`
 template <int D>
-struct BwdQCfg {
-  static constexpr int PANELS = D / 64;
-  static constexpr int Q_BYTES = kBM * D * 2;
-  static constexpr int K_BYTES = kBN * D * 2;
-  static constexpr int SMEM = 2 * Q_BYTES + 3 * K_BYTES + 128 + 896;  // Q, dO, K x 2, V
-  static constexpr int S_COL = 0, DP_COL = kBN, DQ_COL = 2 * kBN;
-  static constexpr int TMEM_COLS = 256;
+__device__ __forceinline__ void keep_tile(uint32_t col, DescHalves a) {
+#pragma unroll
+  for (int kk = 0; kk < D / 16; ++kk) tmem_cp_128x32b(col + kk * 8, a, (kk >> 2) * (kBM * 128) + (kk & 3) * 32);
+}
+
+// ---------------------------------------------------------------------------------- forward
+struct AttnParams {
+  __nv_bfloat16* out;
+  float* lse;
+  int B, T, H, Hkv;
+  float scale_log2;  // softmax scale * log2(e)
+  int pair;          // query tiles per work item: 2, or 1 where there are SMs to spare
+  WorkPlan plan;
+  FastDiv by_heads, by_group;
+  int* status;
 };
 
+
+// Register shares of the first warpgroup and of the eight softmax warps after it: together no more than the 384 x 168 that
+// the launch has, or the larger share waits forever
+template <int kFirst, int kSoftmax>
+__device__ __forceinline__ void give_registers() {
+  static_assert(128 * kFirst + 256 * kSoftmax <= 384 * 168 && kFirst % 8 == 0 && kSoftmax % 8 == 0);
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kFirst));
+}
+template <int kFirst, int kSoftmax>
+__device__ __forceinline__ void take_registers() {
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSoftmax));
+}
+constexpr int kFwdThreads = 32 * 12;  // TMA; products of either query tile; a spare; four softmax warps per query tile
+
 template <int D>
-__global__ void __launch_bounds__(kAttnThreads, 2)
-attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_do,
-                   const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
-                   const AttnBwdParams p) {
-  using C = BwdQCfg<D>;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
-                                             ~static_cast<uintptr_t>(1023));
-  uint8_t* sQ = smem;
-  uint8_t* sDO = sQ + C::Q_BYTES;
-  uint8_t* sK = sDO + C::Q_BYTES;      // two stages
-  uint8_t* sV = sK + 2 * C::K_BYTES;   // one stage
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sV + C::K_BYTES);
-  uint64_t* q_full = bars;         // 1
-  uint64_t* k_full = bars + 1;     // 2
-  uint64_t* k_empty = bars + 3;    // 2
-  uint64_t* v_full = bars + 5;     // 1
-  uint64_t* v_empty = bars + 6;    // 1
-  uint64_t* sdp_full = bars + 7;   // 1
-  uint64_t* ds_full = bars + 8;    // 1 (four warps arrive)
-  uint64_t* dq_full = bars + 9;    // 1
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 10);
+struct AttnCfg {
+  static constexpr int PANELS = D / 64;             // 128-byte panels along the head dimension
+  static constexpr int TILE_BYTES = kBM * D * 2;    // 128 rows of Q, K or V
+  static constexpr int K_STAGES = D == 128 ? 3 : 4, V_STAGES = D == 128 ? 2 : 4;
+  static constexpr int SMEM = (2 + K_STAGES + V_STAGES) * TILE_BYTES + 256;
+  // tensor memory: S and O of both query tiles; D = 64 has room for P beside S, D = 128 writes P over S
+  static constexpr bool P_APART = D == 64;
+  static constexpr int S_COL = 0;                   // + 128 per query tile
+  static constexpr int O_COL = 2 * kBM;             // + D
+  static constexpr int P_COL = P_APART ? 2 * kBM + 2 * D : S_COL;
+  static constexpr int P_TILE = P_APART ? 64 : kBM;  // columns from one query tile's P to the other's
+  static constexpr int TMEM_COLS = 512;
+  static_assert(P_COL + 2 * 64 <= TMEM_COLS && O_COL + 2 * D <= TMEM_COLS && SMEM <= 232448, "one CTA per SM");
+};
+
+// One CTA per SM runs through pairs of query tiles; both share the K and V tiles, each has four softmax warps with one
+// query row per thread.  While one pair of warps per scheduler takes exponentials (1024 cycles of the special function
+// unit per tile, what bounds the kernel at D = 64), the other tile's row maximum, stores and products run.  At D = 64 the
+// next S of a tile is multiplied as soon as this one is in registers.
+template <int D>
+__global__ void __launch_bounds__(kFwdThreads, 1)
+attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
+                const __grid_constant__ CUtensorMap tmap_v, const AttnParams p) {
+  using C = AttnCfg<D>;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  uint8_t* sQ = smem;                                  // two tiles
+  uint8_t* sK = sQ + 2 * C::TILE_BYTES;
+  uint8_t* sV = sK + C::K_STAGES * C::TILE_BYTES;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sV + C::V_STAGES * C::TILE_BYTES);
+  uint64_t* q_full = bars;       // one per query tile, as the next five
+  uint64_t* q_empty = bars + 2;
+  uint64_t* s_full = bars + 4;
+  uint64_t* s_free = bars + 6;   // four warps: S is in registers (P_APART)
+  uint64_t* p_full = bars + 8;   // four warps
+  uint64_t* pv_done = bars + 10;  // O += P V retired: O stable, P free
+  uint64_t* k_full = bars + 12;  // K_STAGES each
+  uint64_t* k_empty = k_full + C::K_STAGES;
+  uint64_t* v_full = k_empty + C::K_STAGES;  // V_STAGES each
+  uint64_t* v_empty = v_full + C::V_STAGES;
+  uint64_t* bars_end = v_empty + C::V_STAGES;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars_end);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = (int)warp_uniform(threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
-  const int q_tile = (int)gridDim.x - 1 - (int)blockIdx.x;
-  const int bh = blockIdx.y;
-  const int b = bh / p.H, h = bh - b * p.H;
-  const int hk = h / (p.H / p.Hkv);
-  const int q_row0 = b * p.T + q_tile * kBM;
-  const int n_tiles = min((q_tile * kBM + kBM + kBN - 1) / kBN, (p.T + kBN - 1) / kBN);
+  const int tiles = (p.T + kBM - 1) / kBM;
+  const int items = (tiles + p.pair - 1) / p.pair;  // per head
+  WorkList work(p.plan);                            // level 0 = the last query tiles, which see all kv tiles
+  if (smem_u32(smem) & 1023) {                      // the 128-byte swizzle repeats every 1024 bytes
+    if (threadIdx.x == 0 && p.status) atomicCAS(p.status, 0, kStatusBadArgument);
+    return;
+  }
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmap_q);
-    tma_prefetch_desc(&tmap_do);
     tma_prefetch_desc(&tmap_k);
     tma_prefetch_desc(&tmap_v);
-    mbar_init(q_full, 1);
-    for (int s = 0; s < 2; ++s) {
-      mbar_init(&k_full[s], 1);
-      mbar_init(&k_empty[s], 1);
-    }
-    mbar_init(v_full, 1);
-    mbar_init(v_empty, 1);
-    mbar_init(sdp_full, 1);
-    mbar_init(ds_full, 4);
-    mbar_init(dq_full, 1);
+    for (uint64_t* b = bars; b < bars_end; ++b) mbar_init(b, (b >= s_free && b < pv_done) ? 4 : ((b >= k_empty && b < v_full) || b >= v_empty) ? 2 : 1);
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -581,181 +405,570 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
 
-  if (warp == 0) {
-    if (lane == 0) {
-      mbar_arrive_expect_tx(q_full, 2 * C::Q_BYTES);
+  if (warp < 4) {
+    give_registers<96, 200>();
+    if (warp == 0) {
+      // ---------------------------------------------------------------- TMA producer
+      if (lane == 0) {
+        bool ok = true;
+        Ring<C::K_STAGES> ks;
+        Ring<C::V_STAGES> vs;
+        int nq[2] = {0, 0};  // loads of each query tile's buffer
+        auto load = [&](uint8_t* dst, const CUtensorMap* map, uint64_t* bar, int col, int row, int seq) {
 #pragma unroll
-      for (int c = 0; c < C::PANELS; ++c) {
-        tma_load_2d(sQ + c * (kBM * 128), &tmap_q, q_full, h * D + c * 64, q_row0);
-        tma_load_2d(sDO + c * (kBM * 128), &tmap_do, q_full, h * D + c * 64, q_row0);
+          for (int c = 0; c < C::PANELS; ++c) tma_load_3d(dst + c * (kBM * 128), map, bar, col + c * 64, row, seq);
+        };
+        for (; ok && work.valid; work.next()) {
+          const int q0 = (items - 1 - work.level) * p.pair, q1 = min(q0 + p.pair, tiles);
+          const int b = p.by_heads(work.head), h = work.head - b * p.H, hk = p.by_group(h);
+          for (int j = 0; j < q1 && ok; ++j) {
+            if (j == 0) {
+#pragma unroll
+              for (int x = 0; x < 2; ++x) {
+                if (q0 + x >= q1) continue;
+                ok = ok && mbar_wait(&q_empty[x], (nq[x] & 1) ^ 1u, abort_flag);
+                if (!ok) break;
+                mbar_arrive_expect_tx(&q_full[x], C::TILE_BYTES);
+                load(sQ + x * C::TILE_BYTES, &tmap_q, &q_full[x], h * D, (q0 + x) * kBM, b);
+                ++nq[x];
+              }
+              if (!ok) break;
+            }
+            ok = mbar_wait(&k_empty[ks.s], ks.ph ^ 1u, abort_flag);
+            if (!ok) break;
+            mbar_arrive_expect_tx(&k_full[ks.s], C::TILE_BYTES);
+            load(sK + ks.s * C::TILE_BYTES, &tmap_k, &k_full[ks.s], hk * D, j * kBM, b);
+            ok = mbar_wait(&v_empty[vs.s], vs.ph ^ 1u, abort_flag);
+            if (!ok) break;
+            mbar_arrive_expect_tx(&v_full[vs.s], C::TILE_BYTES);
+            load(sV + vs.s * C::TILE_BYTES, &tmap_v, &v_full[vs.s], hk * D, j * kBM, b);
+            ks.next();
+            vs.next();
+          }
+        }
+        if (!ok) {
+          *abort_flag = 1;
+          if (p.status) atomicCAS(p.status, 0, kStatusProducerTimeout);
+        }
       }
-      bool ok = true;
-      for (int j = 0; j < n_tiles && ok; ++j) {
-        const int s = j & 1;
-        const int kv_row = b * p.T + j * kBN;
-        if (!mbar_wait(&k_empty[s], ((j >> 1) & 1) ^ 1u, abort_flag)) {
-          ok = false;
-          break;
-        }
-        mbar_arrive_expect_tx(&k_full[s], C::K_BYTES);
+    } else if (warp < 3) {
+      // ---------------------------------------------------------------- S = Q K^T and O += P V of one query tile
+      // Each tile has an issuing warp of its own: with one for both, a tile that is ahead waits for the other's softmax.
+      if (elect_one()) {
+        const int x = warp - 1;
+        constexpr uint32_t idesc = make_instr_desc(1, kMajorK, kMajorMN, kBM, D);
+        const DescHalves dq_ = desc_halves(smem_u32(sQ) + x * C::TILE_BYTES, 16, 1024), dk_ = desc_halves(smem_u32(sK), 16, 1024);
+        const DescHalves dv_ = desc_halves(smem_u32(sV), kBM * 128, 1024);
+        const uint32_t s_col = tmem_base + C::S_COL + x * kBM, p_col = tmem_base + C::P_COL + x * C::P_TILE;
+        const uint32_t o_col = tmem_base + C::O_COL + x * D;
+        bool ok = true;
+        Ring<C::K_STAGES> ks;
+        Ring<C::V_STAGES> vs;
+        uint32_t ph = 0;    // of the tile whose P is awaited
+        uint32_t nq = 0;    // query tiles so far
+        // S of kv tile j of the item that `w` stands at; `last` is the tile's last one
+        auto issue_s = [&](int j, int last) {
+          ok = ok && mbar_wait(&k_full[ks.s], ks.ph, abort_flag) && (j > 0 || mbar_wait(&q_full[x], nq & 1, abort_flag));
+          if (!ok) return;
+          tc_fence_after();
+          scores<D, false>(s_col, dq_, 0, dk_, ks.s * C::TILE_BYTES);
+          umma_commit(&s_full[x]);
+          umma_commit(&k_empty[ks.s]);
+          if (j == last) {
+            umma_commit(&q_empty[x]);
+            ++nq;
+          }
+          ks.next();
+        };
+        // a pair of K and V tiles that this query tile does not see: passed on once it has arrived
+        auto skip = [&]() {
+          ok = ok && mbar_wait(&k_full[ks.s], ks.ph, abort_flag);
+          if (ok) mbar_arrive(&k_empty[ks.s]);
+          ok = ok && mbar_wait(&v_full[vs.s], vs.ph, abort_flag);
+          if (ok) mbar_arrive(&v_empty[vs.s]);
+          ks.next();
+          vs.next();
+        };
+        auto last_of = [&](const WorkList& w) {  // this tile's last kv tile; -1: the item has no such tile
+          const int qt = (items - 1 - w.level) * p.pair + x;
+          return x < p.pair && qt < tiles ? qt : -1;
+        };
+        int last = last_of(work);
+        if (last >= 0) issue_s(0, last);
+        while (ok && work.valid) {
+          const int q1 = min((items - 1 - work.level) * p.pair + p.pair, tiles);
+          for (int j = 0; j <= last && ok; ++j) {
+            if (C::P_APART && j < last) {
+              ok = mbar_wait(&s_free[x], ph, abort_flag);
+              issue_s(j + 1, last);
+            }
+            ok = ok && mbar_wait(&v_full[vs.s], vs.ph, abort_flag) && mbar_wait(&p_full[x], ph, abort_flag);
+            if (!ok) break;
+            tc_fence_after();
 #pragma unroll
-        for (int c = 0; c < C::PANELS; ++c)
-          tma_load_2d(sK + s * C::K_BYTES + c * (kBN * 128), &tmap_k, &k_full[s], hk * D + c * 64, kv_row);
-        if (!mbar_wait(v_empty, (j & 1) ^ 1u, abort_flag)) {
-          ok = false;
-          break;
+            for (int kk = 0; kk < kBM / 16; ++kk)
+              umma_ts_h(o_col, p_col + kk * 8, dv_, vs.s * C::TILE_BYTES + kk * (16 * 128), idesc, (j > 0 || kk > 0) ? 1u : 0u);
+            umma_commit(&pv_done[x]);
+            umma_commit(&v_empty[vs.s]);
+            vs.next();
+            if (!C::P_APART && j < last) issue_s(j + 1, last);  // over the P just read: the tensor core keeps the order
+            ph ^= 1u;
+          }
+          for (int j = last + 1; j < q1 && ok; ++j) skip();
+          work.next();
+          last = work.valid ? last_of(work) : -1;
+          if (last >= 0) issue_s(0, last);  // S has been read: P of it has been multiplied
         }
-        mbar_arrive_expect_tx(v_full, C::K_BYTES);
-#pragma unroll
-        for (int c = 0; c < C::PANELS; ++c) tma_load_2d(sV + c * (kBN * 128), &tmap_v, v_full, hk * D + c * 64, kv_row);
-      }
-      if (!ok) {
-        *abort_flag = 1;
-        if (p.status) atomicCAS(p.status, 0, kStatusProducerTimeout);
-      }
-    }
-  } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc_s = make_instr_desc(1, kMajorK, kMajorK, kBM, kBN);
-      constexpr uint32_t idesc_dq = make_instr_desc(1, kMajorK, kMajorMN, kBM, D);
-      const DescHalves dq_ = desc_halves(smem_u32(sQ), 16, 1024), ddo_ = desc_halves(smem_u32(sDO), 16, 1024);
-      const DescHalves dk0 = desc_halves(smem_u32(sK), 16, 1024), dk1 = desc_halves(smem_u32(sK + C::K_BYTES), 16, 1024);
-      const DescHalves dv_ = desc_halves(smem_u32(sV), 16, 1024);
-      // K_j once more, read as [64 kv rows (K) x D (N)], MN-major, for dQ += dS K_j
-      const DescHalves dkm0 = desc_halves(smem_u32(sK), kBN * 128, 1024),
-                       dkm1 = desc_halves(smem_u32(sK + C::K_BYTES), kBN * 128, 1024);
-      bool ok = mbar_wait(q_full, 0, abort_flag);
-      // S_j = Q K_j^T and dP_j = dO V_j^T.  Both overwrite columns the previous dS lives in; they are
-      // issued after dS_{j-1} K_{j-1}, which the tensor core therefore finishes first.
-      auto issue_sdp = [&](int j) -> bool {
-        const int s = j & 1;
-        if (!mbar_wait(&k_full[s], (j >> 1) & 1, abort_flag) || !mbar_wait(v_full, j & 1, abort_flag)) return false;
-        tc_fence_after();
-        const DescHalves dk_s = s ? dk1 : dk0;
-#pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-          const uint32_t off_a = (kk >> 2) * (kBM * 128) + (kk & 3) * 32;
-          const uint32_t off_b = (kk >> 2) * (kBN * 128) + (kk & 3) * 32;
-          umma_ss_h(tmem_base + C::S_COL, dq_, off_a, dk_s, off_b, idesc_s, kk > 0 ? 1u : 0u);
+        if (!ok) {
+          *abort_flag = 1;
+          if (p.status) atomicCAS(p.status, 0, kStatusMmaTimeout);
         }
-#pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-          const uint32_t off_a = (kk >> 2) * (kBM * 128) + (kk & 3) * 32;
-          const uint32_t off_b = (kk >> 2) * (kBN * 128) + (kk & 3) * 32;
-          umma_ss_h(tmem_base + C::DP_COL, ddo_, off_a, dv_, off_b, idesc_s, kk > 0 ? 1u : 0u);
-        }
-        umma_commit(v_empty);
-        umma_commit(sdp_full);
-        return true;
-      };
-      if (ok) ok = issue_sdp(0);
-      for (int j = 0; j < n_tiles && ok; ++j) {
-        const int s = j & 1;
-        if (!mbar_wait(ds_full, j & 1, abort_flag)) {
-          ok = false;
-          break;
-        }
-        tc_fence_after();
-        const DescHalves dkm_s = s ? dkm1 : dkm0;
-#pragma unroll
-        for (int kk = 0; kk < kBN / 16; ++kk)
-          umma_ts_h(tmem_base + C::DQ_COL, tmem_base + C::S_COL + kk * 8, dkm_s, kk * (16 * 128), idesc_dq,
-                    (j > 0 || kk > 0) ? 1u : 0u);
-        umma_commit(&k_empty[s]);
-        if (j + 1 < n_tiles) ok = issue_sdp(j + 1);
-      }
-      if (ok) umma_commit(dq_full);
-      else {
-        *abort_flag = 1;
-        if (p.status) atomicCAS(p.status, 0, kStatusMmaTimeout);
       }
     }
   } else {
+    // ------------------------------------------------------------------ softmax, stores
+    // Quadrant = warp & 3 (query rows), x = which query tile.  A wait that gives up raises the abort flag for all roles
+    // and the warp goes on (its lanes stay together); nothing is stored then.
+    take_registers<96, 200>();
     const int quad = warp & 3;
+    const int x = (warp - 4) >> 2;
     const int row_in_tile = quad * 32 + lane;
-    const int q_pos = q_tile * kBM + row_in_tile;
     const uint32_t lane_base = tmem_base + ((uint32_t)(quad * 32) << 16);
-    const long long stat_idx = ((long long)b * p.H + h) * p.T + q_pos;
-    const float neg_lse2 = -p.lse[stat_idx] * 1.4426950408889634f;
-    const float dlt = p.delta[stat_idx];
-    const f32x2 scale2 = pack2(p.scale_log2, p.scale_log2), neg_lse2x2 = pack2(neg_lse2, neg_lse2), neg_dlt2 = pack2(-dlt, -dlt),
-                out_scale2 = pack2(p.scale, p.scale);
-    bool ok = true;
-    for (int j = 0; j < n_tiles && ok; ++j) {
-      if (!mbar_wait(sdp_full, j & 1, abort_flag)) {
-        ok = false;
-        break;
-      }
-      tc_fence_after();
-      const int col0 = j * kBN;
-      const bool diag = col0 + kBN - 1 > q_tile * kBM;
-      float pk[32];
-      // dS = P o (dP - delta) * scale
-      auto half_tile = [&](int half, auto masked) {
-        float sc[32], dp[32];
-        tmem_ld_32x32(lane_base + C::S_COL + half * 32, sc);
-        tmem_ld_32x32(lane_base + C::DP_COL + half * 32, dp);
-        tmem_ld_wait();
+    const uint32_t s_col = lane_base + C::S_COL + x * kBM, p_col = lane_base + C::P_COL + x * C::P_TILE;
+    const uint32_t o_col = C::O_COL + x * D;
+    const f32x2 s2 = pack2(p.scale_log2, p.scale_log2);
+    auto wait = [&](uint64_t* bar, uint32_t parity) {
+      if (!mbar_wait(bar, parity, abort_flag)) *abort_flag = 1;
+    };
+    uint32_t ph = 0;  // of the tile at hand: s_full, s_free, p_full, pv_done
+    for (; work.valid;) {
+      const int qt = (items - 1 - work.level) * p.pair + x;
+      const int b = p.by_heads(work.head), h = work.head - b * p.H;
+      work.next();
+      if (x >= p.pair || qt >= tiles) continue;
+      float m_used = -INFINITY;  // reference max of the exponentials accumulated so far (log2 domain)
+      float l = 0.f;
+      for (int j = 0; j <= qt; ++j) {
+        wait(&s_full[x], ph);
+        tc_fence_after();
+        float sc[kBM];
 #pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          float p0, p1;
-          unpack2(fma2(pack2(sc[i], sc[i + 1]), scale2, neg_lse2x2), p0, p1);
-          p0 = fast_exp2(p0);
-          p1 = fast_exp2(p1);
-          if constexpr (decltype(masked)::value) {
-            if (col0 + half * 32 + i > q_pos) p0 = 0.f;
-            if (col0 + half * 32 + i + 1 > q_pos) p1 = 0.f;
-          }
-          float d0, d1;
-          unpack2(mul2(mul2(pack2(p0, p1), add2(pack2(dp[i], dp[i + 1]), neg_dlt2)), out_scale2), d0, d1);
-          pk[half * 16 + (i >> 1)] = __uint_as_float(pack_bf16x2(d0, d1));
+        for (int c = 0; c < 4; ++c) tmem_ld_32x32(s_col + c * 32, *reinterpret_cast<float(*)[32]>(&sc[c * 32]));
+        tmem_ld_wait();
+        if (C::P_APART) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&s_free[x]);
         }
-      };
-      if (diag) {
-        half_tile(0, std::true_type());
-        half_tile(1, std::true_type());
-      } else {
-        half_tile(0, std::false_type());
-        half_tile(1, std::false_type());
-      }
-      tmem_st_32x32(lane_base + C::S_COL, pk);
-      tmem_st_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(ds_full);
-    }
-    if (ok && !mbar_wait(dq_full, 0, abort_flag)) ok = false;
-    if (ok) {
-      tc_fence_after();
-      __nv_bfloat16* orow = p.dq + ((long long)(b * p.T + q_pos) * p.H + h) * D;
+        if (j == qt) {
+#pragma unroll
+          for (int i = 0; i < kBM; ++i)
+            if (i > row_in_tile) sc[i] = -INFINITY;
+        }
+        // row maximum of the raw scores (the scale is positive), four independent chains
+        float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+        for (int i = 0; i < kBM; i += 8) {
+#pragma unroll
+          for (int t = 0; t < 4; ++t) mx4[t] = fmaxf(mx4[t], fmaxf(sc[i + 2 * t], sc[i + 2 * t + 1]));
+        }
+        const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * p.scale_log2;
+        const float m_new = fmaxf(m_used, mx);
+        const bool need = (j == 0) || (m_new - m_used > kRescaleThreshold);
+        if (__any_sync(0xffffffffu, need)) {
+          if (j > 0) {
+            // O may only be touched between two products: the one before must have retired, the next one cannot start
+            // before this warp delivered its P
+            wait(&pv_done[x], ph ^ 1u);
+            tc_fence_after();
+            const float alpha = (m_new == -INFINITY) ? 1.f : fast_exp2(m_used - m_new);
+            l *= alpha;
 #pragma unroll 1
-      for (int c = 0; c < D / 32; ++c) {
-        float o[32];
-        tmem_ld_32x32(lane_base + C::DQ_COL + c * 32, o);
-        tmem_ld_wait();
-        if (q_pos < p.T) {
+            for (int c = 0; c < D / 32; ++c) {
+              float o[32];
+              tmem_ld_32x32(lane_base + o_col + c * 32, o);
+              tmem_ld_wait();
 #pragma unroll
-          for (int i = 0; i < 32; i += 8) {
-            uint4 q;
-            q.x = pack_bf16x2(o[i], o[i + 1]);
-            q.y = pack_bf16x2(o[i + 2], o[i + 3]);
-            q.z = pack_bf16x2(o[i + 4], o[i + 5]);
-            q.w = pack_bf16x2(o[i + 6], o[i + 7]);
-            *reinterpret_cast<uint4*>(orow + c * 32 + i) = q;
+              for (int i = 0; i < 32; ++i) o[i] *= alpha;
+              tmem_st_32x32(lane_base + o_col + c * 32, o);
+            }
+            tmem_st_wait();
           }
+          m_used = m_new;
         }
+        const float neg_m = (m_used == -INFINITY) ? 0.f : -m_used;
+        const f32x2 nm2 = pack2(neg_m, neg_m);
+        f32x2 sums[2] = {pack2(0.f, 0.f), pack2(0.f, 0.f)};
+        // exponentials, packed to bf16 pairs
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          uint32_t pk[16];
+#pragma unroll
+          for (int i = 0; i < 32; i += 2) {
+            float e0, e1;
+            unpack2(fma2(pack2(sc[c * 32 + i], sc[c * 32 + i + 1]), s2, nm2), e0, e1);
+            e0 = fast_exp2(e0);
+            e1 = fast_exp2(e1);
+            pk[i >> 1] = pack_bf16x2(e0, e1);
+            sums[(i >> 1) & 1] = add2(sums[(i >> 1) & 1], pack2(e0, e1));
+          }
+          if (C::P_APART && c == 0) wait(&pv_done[x], ph ^ 1u);  // the P before this one
+          tmem_st_32x16(p_col + c * 16, pk);
+        }
+        float sum0, sum1;
+        unpack2(add2(sums[0], sums[1]), sum0, sum1);
+        l += sum0 + sum1;
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&p_full[x]);
+        ph ^= 1u;
       }
-    } else {
-      *abort_flag = 1;
-      if (p.status) atomicCAS(p.status, 0, kStatusEpilogueTimeout);
+      // normalise, write out and the log-sum-exp.  The next item's first product overwrites O only after these warps
+      // delivered its P.
+      wait(&pv_done[x], ph ^ 1u);
+      tc_fence_after();
+      if (__any_sync(0xffffffffu, *abort_flag != 0)) break;
+      const int rows = p.T - qt * kBM;
+      store_rows<D, true>(tmem_base + o_col, quad, lane, p.out + (((long long)b * p.T + qt * kBM) * p.H + h) * D,
+                          (long long)p.H * D, rows, l > 0.f ? 1.f / l : 0.f);
+      if (row_in_tile < rows)
+        p.lse[((long long)b * p.H + h) * p.T + qt * kBM + row_in_tile] =
+            (l > 0.f) ? (m_used + log2f(l)) * 0.6931471805599453f : -INFINITY;
     }
+    if (*abort_flag != 0 && lane == 0 && p.status) atomicCAS(p.status, 0, kStatusEpilogueTimeout);
   }
 
   tc_fence_before();
   __syncthreads();
   if (*abort_flag != 0) {
+    // a wait gave up: let copies that are still in flight land before the CTA retires
+    const unsigned long long t0 = global_timer_ns();
+    while (global_timer_ns() - t0 < 2000000ull) __nanosleep(1000);
+    __syncthreads();
+  }
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, C::TMEM_COLS);
+  }
+}
+
+// ============================================================================================ backward
+// dQ, dK, dV of causal attention from q, k, v, dO, the forward's log-sum-exp and delta_i = sum_d O_id dO_id.  With
+// S = scale * Q K^T, P = exp(S - lse):
+//   dV = P^T dO,  dP = dO V^T,  dS = P o (dP - delta) * scale,  dQ = dS K,  dK = dS^T Q.
+// Two kernels, neither needs atomics: attn_bwd_dq_kernel loops over the kv tiles of a query tile, attn_bwd_dkv_kernel over
+// the query tiles of a kv tile and over the query heads that share the kv head.  P and dS are rebuilt in registers from S
+// and dP and handed to the next MMA as bf16 through tensor memory.
+
+struct AttnBwdParams {
+  __nv_bfloat16* dq;
+  __nv_bfloat16* dk;
+  __nv_bfloat16* dv;
+  const float* neg_lse2;   // see attn_delta_kernel
+  const float* neg_delta;
+  int B, T, H, Hkv;
+  WorkPlan q_plan, kv_plan;
+  FastDiv by_heads, by_kv_heads, by_group;
+  float scale, scale_log2;
+  int* status;
+};
+
+// What the backward kernels take per query row, laid out [B, H, T rounded up to 128]:
+//   neg_lse2 = -lse * log2(e) (-inf beyond the sequence: P is zero there),  neg_delta = -scale * sum_d O_d dO_d.
+// D / 8 lanes per row, 16 bytes per lane, two rows per lane; a block takes consecutive rows of one head, so that what it
+// writes is contiguous (64 x 1024 rows of 12 heads of 64: 45 us with the rows of a block spread over the heads).
+constexpr int kDeltaRows = 2;  // per lane
+template <int D>
+__global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __restrict__ o,
+                                                        const __nv_bfloat16* __restrict__ d_o,
+                                                        const float* __restrict__ lse, float* __restrict__ neg_lse2,
+                                                        float* __restrict__ neg_delta, int T, int H, int t_pad,
+                                                        FastDiv by_heads, float scale) {
+  constexpr int LPR = D / 8;  // lanes per row: 16 (D = 128) or 8 (D = 64)
+  constexpr int ROWS = 256 / LPR;
+  const int sub = threadIdx.x % LPR;
+  const int bh = (int)blockIdx.x, b = by_heads(bh), h = bh - b * H;
+  const int t0 = (int)blockIdx.y * (ROWS * kDeltaRows) + threadIdx.x / LPR;
+  uint4 a[kDeltaRows], g[kDeltaRows];
+#pragma unroll
+  for (int r = 0; r < kDeltaRows; ++r) {
+    const int t = t0 + r * ROWS;
+    const long long src = (((long long)b * T + t) * H + h) * D + sub * 8;
+    a[r] = t < T ? *reinterpret_cast<const uint4*>(o + src) : make_uint4(0, 0, 0, 0);
+    g[r] = t < T ? *reinterpret_cast<const uint4*>(d_o + src) : make_uint4(0, 0, 0, 0);
+  }
+#pragma unroll
+  for (int r = 0; r < kDeltaRows; ++r) {
+    const int t = t0 + r * ROWS;
+    const __nv_bfloat162* ah = reinterpret_cast<const __nv_bfloat162*>(&a[r]);
+    const __nv_bfloat162* gh = reinterpret_cast<const __nv_bfloat162*>(&g[r]);
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 x = __bfloat1622float2(ah[i]), y = __bfloat1622float2(gh[i]);
+      s = fmaf(x.x, y.x, fmaf(x.y, y.y, s));
+    }
+#pragma unroll
+    for (int off = LPR / 2; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+    if (sub == 0 && t < t_pad) {
+      const long long dst = (long long)bh * t_pad + t;
+      neg_delta[dst] = t < T ? -s * scale : 0.f;
+      neg_lse2[dst] = t < T ? -lse[(long long)bh * T + t] * 1.4426950408889634f : -INFINITY;
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------------- dQ
+constexpr int kDqThreads = 32 * 12;  // TMA; S, dP; dQ; a spare; eight softmax warps (two per lane quadrant, 64 columns each)
+
+template <int D>
+struct BwdQCfg {
+  static constexpr int PANELS = D / 64;
+  static constexpr int TILE_BYTES = kBM * D * 2;  // 128 rows of Q, dO, K or V
+  static constexpr int K_STAGES = D == 128 ? 3 : 4, V_STAGES = D == 128 ? 2 : 4;
+  static constexpr int SMEM = (2 + K_STAGES + V_STAGES) * TILE_BYTES + 256;
+  // tensor memory: S, dP, two buffers of dS, dQ; D = 64 has room for Q and dO too (as A operands they leave half of the
+  // shared memory's bandwidth to the rest)
+  static constexpr bool Q_IN_TMEM = D == 64;
+  static constexpr int S_COL = 0, DP_COL = kBM, DS_COL = 2 * kBM, DQ_COL = 3 * kBM;
+  static constexpr int Q_COL = DQ_COL + D, DO_COL = Q_COL + D / 2;
+  static constexpr int TMEM_COLS = 512;
+  static_assert((Q_IN_TMEM ? DO_COL + D / 2 : DQ_COL + D) <= TMEM_COLS && SMEM <= 232448, "one CTA per SM");
+};
+
+// One CTA per SM runs through (query tile of 128 rows) x (kv tiles of 128 rows that it sees).  The softmax warps load S
+// and dP of a tile into registers at once and release both, so the next tile's products run under the 1024 cycles that the
+// exponentials of this one take; dS alternates between two buffers, and the products of tile i + 1 are issued after
+// dQ += dS K of tile i - 1, so whoever sees S of tile i + 1 may overwrite the dS of tile i - 1.
+template <int D>
+__global__ void __launch_bounds__(kDqThreads, 1)
+attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_do,
+                   const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
+                   const AttnBwdParams p) {
+  using C = BwdQCfg<D>;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  uint8_t* sQ = smem;
+  uint8_t* sDO = sQ + C::TILE_BYTES;
+  uint8_t* sK = sDO + C::TILE_BYTES;
+  uint8_t* sV = sK + C::K_STAGES * C::TILE_BYTES;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sV + C::V_STAGES * C::TILE_BYTES);
+  uint64_t* q_full = bars;       // Q and dO
+  uint64_t* q_empty = bars + 1;
+  uint64_t* sdp_full = bars + 2;
+  uint64_t* sdp_free = bars + 3;  // softmax warps: S and dP are in registers
+  uint64_t* ds_full = bars + 4;   // softmax warps
+  uint64_t* dq_full = bars + 5;
+  uint64_t* k_full = bars + 6;    // K_STAGES each
+  uint64_t* k_empty = k_full + C::K_STAGES;
+  uint64_t* v_full = k_empty + C::K_STAGES;  // V_STAGES each
+  uint64_t* v_empty = v_full + C::V_STAGES;
+  uint64_t* bars_end = v_empty + C::V_STAGES;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars_end);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = (int)warp_uniform(threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  const int tiles = (p.T + kBM - 1) / kBM;
+  WorkList work(p.q_plan);          // level 0 = the last query tile, which sees all kv tiles
+  if (smem_u32(smem) & 1023) {      // the 128-byte swizzle repeats every 1024 bytes
+    if (threadIdx.x == 0 && p.status) atomicCAS(p.status, 0, kStatusBadArgument);
+    return;
+  }
+
+  if (threadIdx.x == 0) {
+    tma_prefetch_desc(&tmap_q);
+    tma_prefetch_desc(&tmap_do);
+    tma_prefetch_desc(&tmap_k);
+    tma_prefetch_desc(&tmap_v);
+    for (uint64_t* b = bars; b < bars_end; ++b) mbar_init(b, (b == sdp_free || b == ds_full) ? 8 : 1);
+    *abort_flag = 0;
+    mbar_fence_init();
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, C::TMEM_COLS);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
+
+  if (warp < 4) {
+    give_registers<72, 216>();
+    if (warp == 0) {
+      // ---------------------------------------------------------------- TMA producer
+      if (lane == 0) {
+        bool ok = true;
+        Ring<C::K_STAGES> ks;
+        Ring<C::V_STAGES> vs;
+        auto load = [&](uint8_t* dst, const CUtensorMap* map, uint64_t* bar, int col, int row, int seq) {
+#pragma unroll
+          for (int c = 0; c < C::PANELS; ++c) tma_load_3d(dst + c * (kBM * 128), map, bar, col + c * 64, row, seq);
+        };
+        for (int r = 0; ok && work.valid; ++r, work.next()) {
+          const int qt = tiles - 1 - work.level, b = p.by_heads(work.head), h = work.head - b * p.H, hk = p.by_group(h);
+          ok = mbar_wait(q_empty, (r & 1) ^ 1u, abort_flag);
+          if (!ok) break;
+          mbar_arrive_expect_tx(q_full, 2 * C::TILE_BYTES);
+          load(sQ, &tmap_q, q_full, h * D, qt * kBM, b);
+          load(sDO, &tmap_do, q_full, h * D, qt * kBM, b);
+          for (int j = 0; j <= qt; ++j) {
+            ok = mbar_wait(&k_empty[ks.s], ks.ph ^ 1u, abort_flag);
+            if (!ok) break;
+            mbar_arrive_expect_tx(&k_full[ks.s], C::TILE_BYTES);
+            load(sK + ks.s * C::TILE_BYTES, &tmap_k, &k_full[ks.s], hk * D, j * kBM, b);
+            ok = mbar_wait(&v_empty[vs.s], vs.ph ^ 1u, abort_flag);
+            if (!ok) break;
+            mbar_arrive_expect_tx(&v_full[vs.s], C::TILE_BYTES);
+            load(sV + vs.s * C::TILE_BYTES, &tmap_v, &v_full[vs.s], hk * D, j * kBM, b);
+            ks.next();
+            vs.next();
+          }
+        }
+        if (!ok) {
+          *abort_flag = 1;
+          if (p.status) atomicCAS(p.status, 0, kStatusProducerTimeout);
+        }
+      }
+    } else if (warp == 1) {
+      // ---------------------------------------------------------------- S = Q K^T, dP = dO V^T, dQ += dS K
+      if (elect_one()) {
+        constexpr uint32_t idesc_dq = make_instr_desc(1, kMajorK, kMajorMN, kBM, D);
+        const DescHalves dq_ = desc_halves(smem_u32(sQ), 16, 1024), ddo_ = desc_halves(smem_u32(sDO), 16, 1024);
+        const DescHalves dk_ = desc_halves(smem_u32(sK), 16, 1024), dv_ = desc_halves(smem_u32(sV), 16, 1024);
+        const DescHalves dkm_ = desc_halves(smem_u32(sK), kBM * 128, 1024);  // K as [kv rows (K)] x [D (N)], MN-major
+        bool ok = true;
+        Ring<C::K_STAGES> ks, ka;  // S; dQ
+        Ring<C::V_STAGES> vs;
+        uint32_t ph = 0, ph_a = 0;
+        // dQ of the tile before: its dS lies in buffer ph_a
+        auto accumulate = [&](bool fresh, bool last) -> bool {
+          if (!mbar_wait(ds_full, ph_a, abort_flag)) return false;
+          tc_fence_after();
+#pragma unroll
+          for (int kk = 0; kk < kBM / 16; ++kk)
+            umma_ts_h(tmem_base + C::DQ_COL, tmem_base + C::DS_COL + ph_a * 64 + kk * 8, dkm_,
+                      ka.s * C::TILE_BYTES + kk * (16 * 128), idesc_dq, (!fresh || kk > 0) ? 1u : 0u);
+          umma_commit(&k_empty[ka.s]);
+          if (last) umma_commit(dq_full);
+          ka.next();
+          ph_a ^= 1u;
+          return true;
+        };
+        int behind = 0;  // kv tiles of the query tile before whose dQ is outstanding: its last one
+        bool behind_fresh = false;
+        for (int r = 0; ok && work.valid; ++r, work.next()) {
+          const int n = tiles - work.level;
+          for (int j = 0; j < n; ++j) {
+            ok = (j > 0 || mbar_wait(q_full, r & 1, abort_flag)) && mbar_wait(&k_full[ks.s], ks.ph, abort_flag) &&
+                 mbar_wait(&v_full[vs.s], vs.ph, abort_flag) && mbar_wait(sdp_free, ph ^ 1u, abort_flag);
+            if (!ok) break;
+            tc_fence_after();
+            if (C::Q_IN_TMEM && j == 0) {  // the S and dP before these have been read
+              keep_tile<D>(tmem_base + C::Q_COL, dq_);
+              keep_tile<D>(tmem_base + C::DO_COL, ddo_);
+              umma_commit(q_empty);
+            }
+            scores<D, C::Q_IN_TMEM>(tmem_base + C::S_COL, dq_, tmem_base + C::Q_COL, dk_, ks.s * C::TILE_BYTES);
+            scores<D, C::Q_IN_TMEM>(tmem_base + C::DP_COL, ddo_, tmem_base + C::DO_COL, dv_, vs.s * C::TILE_BYTES);
+            umma_commit(sdp_full);
+            umma_commit(&v_empty[vs.s]);
+            if (!C::Q_IN_TMEM && j == n - 1) umma_commit(q_empty);
+            ks.next();
+            vs.next();
+            ph ^= 1u;
+            if (behind) {
+              ok = accumulate(behind_fresh, j == 0);
+              if (!ok) break;
+            }
+            behind = 1;
+            behind_fresh = j == 0;
+          }
+        }
+        if (ok && behind) ok = accumulate(behind_fresh, true);
+        if (!ok) {
+          *abort_flag = 1;
+          if (p.status) atomicCAS(p.status, 0, kStatusMmaTimeout);
+        }
+      }
+    }
+  } else {
+    // ------------------------------------------------------------------ softmax, stores
+    // Quadrant = warp & 3 (query rows), half = which 64 of the 128 kv columns.  A wait that gives up raises the abort flag
+    // for all roles and the warp goes on (its lanes stay together); nothing is stored then.
+    take_registers<72, 216>();
+    const int quad = warp & 3;
+    const int half = (warp - 4) >> 2;
+    const int row_in_tile = quad * 32 + lane;
+    const uint32_t lane_base = tmem_base + ((uint32_t)(quad * 32) << 16);
+    const f32x2 scale2 = pack2(p.scale_log2, p.scale_log2), out_scale2 = pack2(p.scale, p.scale);
+    auto wait = [&](uint64_t* bar, uint32_t parity) {
+      if (!mbar_wait(bar, parity, abort_flag)) *abort_flag = 1;
+    };
+    uint32_t ph = 0;
+    for (int r = 0; work.valid; ++r) {
+      const int qt = tiles - 1 - work.level, b = p.by_heads(work.head), h = work.head - b * p.H;
+      const long long stat = (long long)work.head * tiles * kBM + qt * kBM + row_in_tile;
+      const float nl = p.neg_lse2[stat], nd = p.neg_delta[stat];
+      const f32x2 nl2 = pack2(nl, nl), nd2 = pack2(nd, nd);
+      for (int j = 0; j <= qt; ++j) {
+        wait(sdp_full, ph);
+        tc_fence_after();
+        float sc[64], dp[64];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          tmem_ld_32x32(lane_base + C::S_COL + half * 64 + q * 32, *reinterpret_cast<float(*)[32]>(&sc[q * 32]));
+          tmem_ld_32x32(lane_base + C::DP_COL + half * 64 + q * 32, *reinterpret_cast<float(*)[32]>(&dp[q * 32]));
+        }
+        tmem_ld_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(sdp_free);
+        // dS = P o (dP - delta) * scale
+        float pk[32];
+        auto columns = [&](auto masked) {
+#pragma unroll
+          for (int c = 0; c < 64; c += 2) {
+            float p0, p1, d0, d1;
+            unpack2(fma2(pack2(sc[c], sc[c + 1]), scale2, nl2), p0, p1);
+            p0 = fast_exp2(p0);
+            p1 = fast_exp2(p1);
+            if constexpr (decltype(masked)::value) {
+              if (half * 64 + c > row_in_tile) p0 = 0.f;
+              if (half * 64 + c + 1 > row_in_tile) p1 = 0.f;
+            }
+            unpack2(mul2(pack2(p0, p1), fma2(pack2(dp[c], dp[c + 1]), out_scale2, nd2)), d0, d1);
+            pk[c >> 1] = __uint_as_float(pack_bf16x2(d0, d1));
+          }
+        };
+        if (j == qt) columns(std::true_type());
+        else columns(std::false_type());
+        tmem_st_32x32(lane_base + C::DS_COL + ph * 64 + half * 32, pk);
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(ds_full);
+        ph ^= 1u;
+      }
+      work.next();
+      wait(dq_full, r & 1);
+      tc_fence_after();
+      if (__any_sync(0xffffffffu, *abort_flag != 0)) break;
+      // half of the columns each; the next query tile's first product overwrites dQ only after these warps delivered its dS
+      store_rows<D / 2>(tmem_base + C::DQ_COL + half * (D / 2), quad, lane,
+                        p.dq + (((long long)b * p.T + qt * kBM) * p.H + h) * D + half * (D / 2), (long long)p.H * D,
+                        p.T - qt * kBM);
+    }
+    if (*abort_flag != 0 && lane == 0 && p.status) atomicCAS(p.status, 0, kStatusEpilogueTimeout);
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (*abort_flag != 0) {
+    // a wait gave up: let copies that are still in flight land before the CTA retires
     const unsigned long long t0 = global_timer_ns();
     while (global_timer_ns() - t0 < 2000000ull) __nanosleep(1000);
     __syncthreads();
@@ -767,79 +980,86 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
 }
 
 // ---------------------------------------------------------------------------------- dK, dV
-constexpr int kKvThreads = 64 + 32 * 8;  // TMA warp, MMA warp, eight softmax warps (two per lane quadrant)
-constexpr int kBQ = 64;                  // query rows per iteration
+constexpr int kSoftmaxWarps = 16;                  // four per lane quadrant, each with 32 of a tile's 128 columns
+constexpr int kBwdThreads = 32 * (4 + kSoftmaxWarps);  // TMA; S^T; dV, dK; dP^T; softmax
 
 template <int D>
 struct BwdKvCfg {
   static constexpr int PANELS = D / 64;
-  static constexpr int KV_BYTES = kBM * D * 2;         // K or V tile: 128 kv rows
-  static constexpr int Q_BYTES = kBQ * D * 2;          // Q_i or dO_i tile: 64 query rows
-  static constexpr int STAT_BYTES = kBQ * 4;           // lse_i or delta_i
-  static constexpr int TILE_BYTES = 2 * Q_BYTES;                   // Q_i and dO_i of one stage
-  static constexpr int STAGE_BYTES = TILE_BYTES + 2 * STAT_BYTES;  // what one stage's barrier receives
-  static constexpr int STAGES = 3;                                  // query-side tiles in flight
-  static constexpr int SMEM = 2 * KV_BYTES + STAGES * STAGE_BYTES + 256 + 1024;
-  // D = 128: S^T / dP^T double buffered, one CTA per SM (512 columns).  D = 64: single buffers and
-  // 256 columns, so that two CTAs share an SM and cover each other's prologue, epilogue and waits.
-  static constexpr int NBUF = D == 128 ? 2 : 1;
-  static constexpr int ST_COL = 0;                   // NBUF buffers of 64 columns
-  static constexpr int DPT_COL = NBUF * kBQ;         // NBUF buffers of 64 columns
-  static constexpr int DV_COL = 2 * NBUF * kBQ;
+  static constexpr int TILE_BYTES = kBM * D * 2;    // 128 rows of K, V, Q or dO
+  static constexpr int STAT_BYTES = kBM * 4;        // one fp32 per query row
+  static constexpr int Q_STAGES = D == 128 ? 3 : 4;   // query-side tiles in flight
+  static constexpr int DO_STAGES = D == 128 ? 2 : 4;
+  static constexpr int SMEM = (2 + Q_STAGES + DO_STAGES) * TILE_BYTES + (Q_STAGES + DO_STAGES) * STAT_BYTES + 256;
+  // Tensor memory.  D = 64 keeps K and V there too (as A operands they leave half of the shared memory's bandwidth to
+  // the rest) and P^T beside S^T; at D = 128 dV and dK take half of it, P^T is written over S^T.
+  static constexpr bool KV_IN_TMEM = D == 64;
+  static constexpr int S_COL = 0, DP_COL = kBM;
+  static constexpr int P_COL = KV_IN_TMEM ? 2 * kBM : S_COL;
+  static constexpr int P_STEP = KV_IN_TMEM ? 16 : 32;  // columns from the P^T of 32 query rows to that of the next 32
+  static constexpr int DV_COL = KV_IN_TMEM ? 2 * kBM + 64 : 2 * kBM;
   static constexpr int DK_COL = DV_COL + D;
-  static constexpr int TMEM_COLS = D == 128 ? 512 : 256;
-  static constexpr int CTAS_PER_SM = D == 128 ? 1 : 2;
+  static constexpr int K_COL = DK_COL + D, V_COL = K_COL + D / 2;
+  static constexpr int TMEM_COLS = 512;
+  static_assert((KV_IN_TMEM ? V_COL + D / 2 : DK_COL + D) <= TMEM_COLS && SMEM <= 232448, "one CTA per SM");
 };
 
+// One CTA per SM runs through (kv tile of 128 rows) x (query tiles of 128 rows that see it, over the query heads of the
+// kv head).  Per pair of tiles the tensor core multiplies for 1024 cycles (D = 64; 2048 at D = 128) and the special
+// function unit takes 1024 for the exponentials; the order below keeps both fed: while the softmax warps turn S^T of one
+// tile into P^T, the tensor core runs dK and dP^T of the tile before, and dV and the next S^T while they form dS^T.
+// P^T and dS^T go back over the columns that the same thread read, so no warp waits for another.  The next kv tile's
+// loads and first products run under the last tile of the one before; only the store of dV and dK stands alone.
 template <int D>
-__global__ void __launch_bounds__(kKvThreads, BwdKvCfg<D>::CTAS_PER_SM)
+__global__ void __launch_bounds__(kBwdThreads, 1)
 attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_do,
                     const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
                     const AttnBwdParams p) {
   using C = BwdKvCfg<D>;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
-                                             ~static_cast<uintptr_t>(1023));
+  extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* sK = smem;
-  uint8_t* sV = sK + C::KV_BYTES;
-  uint8_t* sStage = sV + C::KV_BYTES;           // per stage: Q_i, dO_i (1024-byte aligned tiles)
-  uint8_t* sStat = sStage + C::STAGES * C::TILE_BYTES;  // per stage: lse_i, delta_i
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sStat + C::STAGES * 2 * C::STAT_BYTES);
-  uint64_t* kv_full = bars;          // 1
-  uint64_t* qdo_full = bars + 1;     // 3
-  uint64_t* qdo_empty = bars + 4;    // 3
-  uint64_t* sdp_full = bars + 7;     // 2
-  uint64_t* pds_full = bars + 9;     // 2 (eight warps arrive)
-  uint64_t* acc_full = bars + 11;    // 1
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 12);
+  uint8_t* sV = sK + C::TILE_BYTES;
+  uint8_t* sQ = sV + C::TILE_BYTES;
+  uint8_t* sDO = sQ + C::Q_STAGES * C::TILE_BYTES;
+  float* sLse = reinterpret_cast<float*>(sDO + C::DO_STAGES * C::TILE_BYTES);  // -lse * log2(e) of each stage's rows
+  float* sDelta = sLse + C::Q_STAGES * kBM;                                    // -delta * scale
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sDelta + C::DO_STAGES * kBM);
+  uint64_t* k_full = bars;       // 1
+  uint64_t* k_empty = bars + 1;  // 1
+  uint64_t* v_full = bars + 2;   // 1
+  uint64_t* v_empty = bars + 3;  // 1
+  uint64_t* s_full = bars + 4;
+  uint64_t* s_free = bars + 5;   // softmax warps: S^T is in registers (KV_IN_TMEM)
+  uint64_t* p_full = bars + 6;   // softmax warps
+  uint64_t* dp_full = bars + 7;
+  uint64_t* ds_full = bars + 8;  // softmax warps
+  uint64_t* dv_done = bars + 9;  // P^T has been multiplied
+  uint64_t* dk_done = bars + 10;  // dS^T has been multiplied
+  uint64_t* acc_full = bars + 11;
+  uint64_t* q_full = bars + 12;   // Q_STAGES each
+  uint64_t* q_empty = q_full + C::Q_STAGES;
+  uint64_t* do_full = q_empty + C::Q_STAGES;  // DO_STAGES each
+  uint64_t* do_empty = do_full + C::DO_STAGES;  // both MMA warps
+  uint64_t* bars_end = do_empty + C::DO_STAGES;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars_end);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = (int)warp_uniform(threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
-  const int kv_tile = blockIdx.x;                 // light (late) kv tiles last
-  const int bhk = blockIdx.y;
-  const int b = bhk / p.Hkv, hk = bhk - b * p.Hkv;
+  const int tiles = (p.T + kBM - 1) / kBM;
   const int group = p.H / p.Hkv;
-  const int kv0 = kv_tile * kBM;
-  const int i_first = kv0 / kBQ;                  // first query tile that sees this kv tile
-  const int n_q = p.T / kBQ - i_first;            // query tiles per head
-  const int n_it = n_q * group;
+  WorkList work(p.kv_plan);  // level = kv tile: the first one is seen by all query tiles
+  if (smem_u32(smem) & 1023) {  // the 128-byte swizzle repeats every 1024 bytes
+    if (threadIdx.x == 0 && p.status) atomicCAS(p.status, 0, kStatusBadArgument);
+    return;
+  }
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmap_q);
     tma_prefetch_desc(&tmap_do);
     tma_prefetch_desc(&tmap_k);
     tma_prefetch_desc(&tmap_v);
-    mbar_init(kv_full, 1);
-    for (int s = 0; s < C::STAGES; ++s) {
-      mbar_init(&qdo_full[s], 1);
-      mbar_init(&qdo_empty[s], 1);
-    }
-    for (int s = 0; s < 2; ++s) {
-      mbar_init(&sdp_full[s], 1);
-      mbar_init(&pds_full[s], 8);
-    }
-    mbar_init(acc_full, 1);
+    for (uint64_t* b = bars; b < bars_end; ++b) mbar_init(b, (b == ds_full || b == p_full || b == s_free) ? kSoftmaxWarps : b >= do_empty ? 2 : 1);
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -850,37 +1070,48 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
 
   if (warp == 0) {
+    // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
-      mbar_arrive_expect_tx(kv_full, 2 * C::KV_BYTES);
-#pragma unroll
-      for (int c = 0; c < C::PANELS; ++c) {
-        tma_load_2d(sK + c * (kBM * 128), &tmap_k, kv_full, hk * D + c * 64, b * p.T + kv0);
-        tma_load_2d(sV + c * (kBM * 128), &tmap_v, kv_full, hk * D + c * 64, b * p.T + kv0);
-      }
       bool ok = true;
-      for (int it = 0; it < n_it && ok; ++it) {
-        const int s = it % C::STAGES;
-        const int g = it / n_q, i = i_first + (it - g * n_q);
-        const int h = hk * group + g;
-        if (!mbar_wait(&qdo_empty[s], ((it / C::STAGES) & 1) ^ 1u, abort_flag)) {
-          ok = false;
-          break;
-        }
-        uint8_t* st = sStage + s * C::TILE_BYTES;
-        uint8_t* stat_s = sStat + s * 2 * C::STAT_BYTES;
-        mbar_arrive_expect_tx(&qdo_full[s], C::STAGE_BYTES);
-        const int row = b * p.T + i * kBQ;
+      Ring<C::Q_STAGES> qs;
+      Ring<C::DO_STAGES> os;
+      auto load = [&](uint8_t* dst, const CUtensorMap* map, uint64_t* bar, int col, int row, int seq) {
 #pragma unroll
-        for (int c = 0; c < C::PANELS; ++c) {
-          tma_load_2d(st + c * (kBQ * 128), &tmap_q, &qdo_full[s], h * D + c * 64, row);
-          tma_load_2d(st + C::Q_BYTES + c * (kBQ * 128), &tmap_do, &qdo_full[s], h * D + c * 64, row);
+        for (int c = 0; c < C::PANELS; ++c) tma_load_3d(dst + c * (kBM * 128), map, bar, col + c * 64, row, seq);
+      };
+      for (int r = 0; ok && work.valid; ++r, work.next()) {
+        const int kt = work.level, b = p.by_kv_heads(work.head), hk = work.head - b * p.Hkv;
+        ok = mbar_wait(k_empty, (r & 1) ^ 1u, abort_flag);
+        if (!ok) break;
+        mbar_arrive_expect_tx(k_full, C::TILE_BYTES);
+        load(sK, &tmap_k, k_full, hk * D, kt * kBM, b);
+        for (int g = 0; g < group && ok; ++g) {
+          const int h = hk * group + g;
+          const long long stat0 = ((long long)b * p.H + h) * ((long long)tiles * kBM);
+          for (int i = kt; i < tiles && ok; ++i) {
+            ok = mbar_wait(&q_empty[qs.s], qs.ph ^ 1u, abort_flag);
+            if (!ok) break;
+            mbar_arrive_expect_tx(&q_full[qs.s], C::TILE_BYTES + C::STAT_BYTES);
+            load(sQ + qs.s * C::TILE_BYTES, &tmap_q, &q_full[qs.s], h * D, i * kBM, b);
+            bulk_load_1d(sLse + qs.s * kBM, p.neg_lse2 + stat0 + i * kBM, C::STAT_BYTES, &q_full[qs.s]);
+            if (g == 0 && i == kt) {
+              ok = mbar_wait(v_empty, (r & 1) ^ 1u, abort_flag);
+              if (!ok) break;
+              mbar_arrive_expect_tx(v_full, C::TILE_BYTES);
+              load(sV, &tmap_v, v_full, hk * D, kt * kBM, b);
+            }
+            ok = mbar_wait(&do_empty[os.s], os.ph ^ 1u, abort_flag);
+            if (!ok) break;
+            mbar_arrive_expect_tx(&do_full[os.s], C::TILE_BYTES + C::STAT_BYTES);
+            load(sDO + os.s * C::TILE_BYTES, &tmap_do, &do_full[os.s], h * D, i * kBM, b);
+            bulk_load_1d(sDelta + os.s * kBM, p.neg_delta + stat0 + i * kBM, C::STAT_BYTES, &do_full[os.s]);
+            qs.next();
+            os.next();
+          }
         }
-        const long long stat = ((long long)b * p.H + h) * p.T + i * kBQ;
-        bulk_load_1d(stat_s, p.lse + stat, C::STAT_BYTES, &qdo_full[s]);
-        bulk_load_1d(stat_s + C::STAT_BYTES, p.delta + stat, C::STAT_BYTES, &qdo_full[s]);
       }
       if (!ok) {
         *abort_flag = 1;
@@ -888,164 +1119,213 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc_s = make_instr_desc(1, kMajorK, kMajorK, kBM, kBQ);
-      constexpr uint32_t idesc_acc = make_instr_desc(1, kMajorK, kMajorMN, kBM, D);
-      const DescHalves dk_ = desc_halves(smem_u32(sK), 16, 1024), dv_ = desc_halves(smem_u32(sV), 16, 1024);
-      // stage 0 of the query-side tiles, K-major (for S^T, dP^T) and MN-major (for dV, dK)
-      const DescHalves dq_ = desc_halves(smem_u32(sStage), 16, 1024),
-                       ddo_ = desc_halves(smem_u32(sStage + C::Q_BYTES), 16, 1024);
-      const DescHalves dqm_ = desc_halves(smem_u32(sStage), kBQ * 128, 1024),
-                       ddom_ = desc_halves(smem_u32(sStage + C::Q_BYTES), kBQ * 128, 1024);
-      bool ok = mbar_wait(kv_full, 0, abort_flag);
-      // S^T = K Q_i^T and dP^T = V dO_i^T into buffer it & 1
-      auto issue_sdp = [&](int it) -> bool {
-        const int s = it % C::NBUF, st = it % C::STAGES;
-        if (!mbar_wait(&qdo_full[st], (it / C::STAGES) & 1, abort_flag)) return false;
-        tc_fence_after();
-        const uint32_t st_off = st * C::TILE_BYTES;
-#pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-          const uint32_t off_a = (kk >> 2) * (kBM * 128) + (kk & 3) * 32;
-          const uint32_t off_b = (kk >> 2) * (kBQ * 128) + (kk & 3) * 32;
-          umma_ss_h(tmem_base + C::ST_COL + s * kBQ, dk_, off_a, dq_, st_off + off_b, idesc_s, kk > 0 ? 1u : 0u);
+    // ------------------------------------------------------------------ S^T = K Q^T
+    if (elect_one()) {
+      const DescHalves dk_ = desc_halves(smem_u32(sK), 16, 1024), dq_ = desc_halves(smem_u32(sQ), 16, 1024);
+      bool ok = true;
+      Ring<C::Q_STAGES> qs;
+      uint32_t ph = 0;
+      for (int r = 0; ok && work.valid; ++r, work.next()) {
+        const int n = (tiles - work.level) * group;
+        for (int i = 0; i < n; ++i) {
+          ok = (i > 0 || mbar_wait(k_full, r & 1, abort_flag)) && mbar_wait(&q_full[qs.s], qs.ph, abort_flag) &&
+               mbar_wait(C::KV_IN_TMEM ? s_free : dv_done, ph ^ 1u, abort_flag);
+          if (!ok) break;
+          tc_fence_after();
+          if (C::KV_IN_TMEM && i == 0) {
+            keep_tile<D>(tmem_base + C::K_COL, dk_);  // the S^T before this one has been read
+            umma_commit(k_empty);
+          }
+          scores<D, C::KV_IN_TMEM>(tmem_base + C::S_COL, dk_, tmem_base + C::K_COL, dq_, qs.s * C::TILE_BYTES);
+          umma_commit(s_full);
+          if (!C::KV_IN_TMEM && i == n - 1) umma_commit(k_empty);
+          ph ^= 1u;
+          qs.next();
         }
-#pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-          const uint32_t off_a = (kk >> 2) * (kBM * 128) + (kk & 3) * 32;
-          const uint32_t off_b = (kk >> 2) * (kBQ * 128) + (kk & 3) * 32;
-          umma_ss_h(tmem_base + C::DPT_COL + s * kBQ, dv_, off_a, ddo_, st_off + off_b, idesc_s, kk > 0 ? 1u : 0u);
-        }
-        umma_commit(&sdp_full[s]);
-        return true;
-      };
-      if (ok) ok = issue_sdp(0);
-      if (ok && C::NBUF > 1 && n_it > 1) ok = issue_sdp(1);
-      for (int it = 0; it < n_it && ok; ++it) {
-        const int s = it % C::NBUF;
-        if (!mbar_wait(&pds_full[s], (it / C::NBUF) & 1, abort_flag)) {
-          ok = false;
-          break;
-        }
-        tc_fence_after();
-        const int st = it % C::STAGES;
-        const uint32_t st_off = st * C::TILE_BYTES;
-#pragma unroll
-        for (int kk = 0; kk < kBQ / 16; ++kk) {
-          // dV += P^T dO_i and dK += dS^T Q_i: A from tensor memory (bf16 pairs, 8 columns per step),
-          // B = the query-side tile read as [64 rows (K) x D (N)], MN-major
-          umma_ts_h(tmem_base + C::DV_COL, tmem_base + C::ST_COL + s * kBQ + kk * 8, ddom_, st_off + kk * (16 * 128),
-                    idesc_acc, (it > 0 || kk > 0) ? 1u : 0u);
-          umma_ts_h(tmem_base + C::DK_COL, tmem_base + C::DPT_COL + s * kBQ + kk * 8, dqm_, st_off + kk * (16 * 128),
-                    idesc_acc, (it > 0 || kk > 0) ? 1u : 0u);
-        }
-        umma_commit(&qdo_empty[st]);
-        if (it + C::NBUF < n_it) ok = issue_sdp(it + C::NBUF);
       }
-      if (ok) umma_commit(acc_full);
-      else {
+      if (!ok) {
         *abort_flag = 1;
         if (p.status) atomicCAS(p.status, 0, kStatusMmaTimeout);
       }
     }
-  } else {
-    // eight warps: quadrant = warp & 3 (kv rows), half = which 32 of the 64 query columns
-    const int quad = warp & 3;
-    const int half = (warp - 2) >> 2;
-    const int row_in_tile = quad * 32 + lane;
-    const int kv_pos = kv0 + row_in_tile;
-    const uint32_t lane_base = tmem_base + ((uint32_t)(quad * 32) << 16);
-    const f32x2 scale2 = pack2(p.scale_log2, p.scale_log2), neg_log2e = pack2(-1.4426950408889634f, -1.4426950408889634f),
-                minus1 = pack2(-1.f, -1.f), out_scale2 = pack2(p.scale, p.scale);
-    bool ok = true;
-    // A failed wait clears `ok` but the loop keeps its shape: both warps of a quadrant must reach
-    // the named barrier the same number of times.
-    for (int it = 0; it < n_it; ++it) {
-      const int s = it % C::NBUF;
-      const int g = it / n_q, i = i_first + (it - g * n_q);
-      if (ok && !mbar_wait(&sdp_full[s], (it / C::NBUF) & 1, abort_flag)) ok = false;
-      tc_fence_after();
-      const float* lse_s = reinterpret_cast<const float*>(sStat + (it % C::STAGES) * 2 * C::STAT_BYTES) + half * 32;
-      const float* dlt_s = lse_s + kBQ;
-      float sc[32], dp[32];
-      if (ok) {
-        tmem_ld_32x32(lane_base + C::ST_COL + s * kBQ + half * 32, sc);
-        tmem_ld_32x32(lane_base + C::DPT_COL + s * kBQ + half * 32, dp);
-        tmem_ld_wait();
-      } else {
-#pragma unroll
-        for (int c = 0; c < 32; ++c) sc[c] = dp[c] = 0.f;
-      }
-      const int qcol0 = i * kBQ + half * 32;           // sequence position of this thread's first column
-      const bool diag = qcol0 < kv0 + kBM;             // some query of this block precedes some kv row
-      uint32_t pp[16], dd[16];
-      // P and dS = P o (dP - delta) * scale
-      auto columns = [&](auto masked) {
-#pragma unroll
-        for (int c = 0; c < 32; c += 4) {
-          const float4 l4 = *reinterpret_cast<const float4*>(lse_s + c);
-          const float4 d4 = *reinterpret_cast<const float4*>(dlt_s + c);
-#pragma unroll
-          for (int t = 0; t < 4; t += 2) {
-            const f32x2 neg_lse2 = mul2(t ? pack2(l4.z, l4.w) : pack2(l4.x, l4.y), neg_log2e);
-            float e0, e1, g0, g1;
-            unpack2(fma2(pack2(sc[c + t], sc[c + t + 1]), scale2, neg_lse2), e0, e1);
-            e0 = fast_exp2(e0);
-            e1 = fast_exp2(e1);
-            if constexpr (decltype(masked)::value) {
-              if (qcol0 + c + t < kv_pos) e0 = 0.f;
-              if (qcol0 + c + t + 1 < kv_pos) e1 = 0.f;
-            }
-            const f32x2 d = fma2(t ? pack2(d4.z, d4.w) : pack2(d4.x, d4.y), minus1, pack2(dp[c + t], dp[c + t + 1]));
-            unpack2(mul2(mul2(pack2(e0, e1), d), out_scale2), g0, g1);
-            pp[(c + t) >> 1] = pack_bf16x2(e0, e1);
-            dd[(c + t) >> 1] = pack_bf16x2(g0, g1);
+  } else if (warp == 3) {
+    // ------------------------------------------------------------------ dP^T = V dO^T
+    if (elect_one()) {
+      const DescHalves dv_ = desc_halves(smem_u32(sV), 16, 1024), ddo_ = desc_halves(smem_u32(sDO), 16, 1024);
+      bool ok = true;
+      Ring<C::DO_STAGES> os;
+      uint32_t ph = 0;
+      for (int r = 0; ok && work.valid; ++r, work.next()) {
+        const int n = (tiles - work.level) * group;
+        for (int i = 0; i < n; ++i) {
+          ok = (i > 0 || mbar_wait(v_full, r & 1, abort_flag)) && mbar_wait(&do_full[os.s], os.ph, abort_flag) &&
+               mbar_wait(dk_done, ph ^ 1u, abort_flag);
+          if (!ok) break;
+          tc_fence_after();
+          if (C::KV_IN_TMEM && i == 0) {
+            keep_tile<D>(tmem_base + C::V_COL, dv_);
+            umma_commit(v_empty);
           }
+          scores<D, C::KV_IN_TMEM>(tmem_base + C::DP_COL, dv_, tmem_base + C::V_COL, ddo_, os.s * C::TILE_BYTES);
+          umma_commit(dp_full);
+          umma_commit(&do_empty[os.s]);
+          if (!C::KV_IN_TMEM && i == n - 1) umma_commit(v_empty);
+          ph ^= 1u;
+          os.next();
         }
+      }
+      if (!ok) {
+        *abort_flag = 1;
+        if (p.status) atomicCAS(p.status, 0, kStatusMmaTimeout);
+      }
+    }
+  } else if (warp == 2) {
+    // ------------------------------------------------------------------ accumulators: dV += P^T dO, dK += dS^T Q
+    if (elect_one()) {
+      constexpr uint32_t idesc = make_instr_desc(1, kMajorK, kMajorMN, kBM, D);
+      const DescHalves dq_ = desc_halves(smem_u32(sQ), kBM * 128, 1024), ddo_ = desc_halves(smem_u32(sDO), kBM * 128, 1024);
+      // A: bf16 pairs in tensor memory, 32 query rows every a_step columns
+      auto accumulate = [&](uint32_t col, uint32_t a_col, uint32_t a_step, DescHalves b, uint32_t b_off, bool fresh) {
+#pragma unroll
+        for (int kk = 0; kk < kBM / 16; ++kk)
+          umma_ts_h(tmem_base + col, tmem_base + a_col + (kk >> 1) * a_step + (kk & 1) * 8, b, b_off + kk * (16 * 128), idesc,
+                    (!fresh || kk > 0) ? 1u : 0u);
       };
-      if (diag) columns(std::true_type());
-      else columns(std::false_type());
-      // both warps of a quadrant must have read S^T / dP^T before either overwrites its part: the
-      // packed halves land in columns [0, 32) of the buffers, which the other warp may still be loading
-      pair_barrier(quad);
-      if (!__all_sync(0xffffffffu, ok)) {
-        ok = false;
-        continue;
-      }
-      tmem_st_32x16(lane_base + C::ST_COL + s * kBQ + half * 16, pp);
-      tmem_st_32x16(lane_base + C::DPT_COL + s * kBQ + half * 16, dd);
-      tmem_st_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&pds_full[s]);
-    }
-    if (ok && !mbar_wait(acc_full, 0, abort_flag)) ok = false;
-    if (ok) {
-      tc_fence_after();
-      // warp `half` 0 writes dV, `half` 1 writes dK
-      __nv_bfloat16* base = (half == 0 ? p.dv : p.dk) + ((long long)(b * p.T + kv_pos) * p.Hkv + hk) * D;
-      const uint32_t col = half == 0 ? C::DV_COL : C::DK_COL;
-#pragma unroll 1
-      for (int c = 0; c < D / 32; ++c) {
-        float o[32];
-        tmem_ld_32x32(lane_base + col + c * 32, o);
-        tmem_ld_wait();
-        if (kv_pos < p.T) {
-#pragma unroll
-          for (int i = 0; i < 32; i += 8) {
-            uint4 q;
-            q.x = pack_bf16x2(o[i], o[i + 1]);
-            q.y = pack_bf16x2(o[i + 2], o[i + 3]);
-            q.z = pack_bf16x2(o[i + 4], o[i + 5]);
-            q.w = pack_bf16x2(o[i + 6], o[i + 7]);
-            *reinterpret_cast<uint4*>(base + c * 32 + i) = q;
-          }
+      bool ok = true;
+      Ring<C::Q_STAGES> qs;
+      Ring<C::DO_STAGES> os;
+      uint32_t ph = 0;
+      for (; ok && work.valid; work.next()) {
+        const int n = (tiles - work.level) * group;
+        for (int i = 0; i < n; ++i) {
+          ok = mbar_wait(&do_full[os.s], os.ph, abort_flag) && mbar_wait(p_full, ph, abort_flag);
+          if (!ok) break;
+          tc_fence_after();
+          accumulate(C::DV_COL, C::P_COL, C::P_STEP, ddo_, os.s * C::TILE_BYTES, i == 0);
+          umma_commit(dv_done);
+          umma_commit(&do_empty[os.s]);
+          ok = mbar_wait(ds_full, ph, abort_flag);
+          if (!ok) break;
+          tc_fence_after();
+          accumulate(C::DK_COL, C::DP_COL, 32, dq_, qs.s * C::TILE_BYTES, i == 0);
+          umma_commit(dk_done);
+          umma_commit(&q_empty[qs.s]);
+          if (i == n - 1) umma_commit(acc_full);
+          ph ^= 1u;
+          qs.next();
+          os.next();
         }
       }
-    } else {
-      *abort_flag = 1;
-      if (p.status) atomicCAS(p.status, 0, kStatusEpilogueTimeout);
+      if (!ok) {
+        *abort_flag = 1;
+        if (p.status) atomicCAS(p.status, 0, kStatusMmaTimeout);
+      }
     }
+  } else if (warp >= 4) {
+    // ------------------------------------------------------------------ softmax, stores
+    // Quadrant = warp & 3 (kv rows), part = which 32 of the 128 query columns.  A wait that gives up raises the abort flag
+    // for all roles and the warp goes on (its lanes stay together); nothing is stored then.
+    const int quad = warp & 3;
+    const int part = (warp - 4) >> 2;
+    const int row_in_tile = quad * 32 + lane;
+    const uint32_t lane_base = tmem_base + ((uint32_t)(quad * 32) << 16);
+    const f32x2 scale2 = pack2(p.scale_log2, p.scale_log2), out_scale2 = pack2(p.scale, p.scale);
+    auto wait = [&](uint64_t* bar, uint32_t parity) {
+      if (!mbar_wait(bar, parity, abort_flag)) *abort_flag = 1;
+    };
+    Ring<C::Q_STAGES> qs;
+    Ring<C::DO_STAGES> os;
+    uint32_t ph = 0;
+    for (int r = 0; work.valid; ++r) {
+      const int kt = work.level, b = p.by_kv_heads(work.head), hk = work.head - b * p.Hkv;
+      for (int g = 0; g < group; ++g) {
+        for (int i = kt; i < tiles; ++i) {
+          // P = exp(S * scale - lse), kept in registers for dS
+          wait(s_full, ph);
+          tc_fence_after();
+          float pr[32];
+          tmem_ld_32x32(lane_base + C::S_COL + part * 32, pr);
+          tmem_ld_wait();
+          if (C::KV_IN_TMEM) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(s_free);
+          }
+          const float* lse_s = sLse + qs.s * kBM + part * 32;
+          {
+            uint32_t pk[16];
+            auto columns = [&](auto masked) {
+#pragma unroll
+              for (int c = 0; c < 32; c += 4) {
+                const float4 l4 = *reinterpret_cast<const float4*>(lse_s + c);
+#pragma unroll
+                for (int t = 0; t < 4; t += 2) {
+                  float e0, e1;
+                  unpack2(fma2(pack2(pr[c + t], pr[c + t + 1]), scale2, t ? pack2(l4.z, l4.w) : pack2(l4.x, l4.y)), e0, e1);
+                  e0 = fast_exp2(e0);
+                  e1 = fast_exp2(e1);
+                  if constexpr (decltype(masked)::value) {
+                    if (part * 32 + c + t < row_in_tile) e0 = 0.f;
+                    if (part * 32 + c + t + 1 < row_in_tile) e1 = 0.f;
+                  }
+                  pr[c + t] = e0;
+                  pr[c + t + 1] = e1;
+                  pk[(c + t) >> 1] = pack_bf16x2(e0, e1);
+                }
+              }
+            };
+            if (i == kt) columns(std::true_type());
+            else columns(std::false_type());
+            if (C::KV_IN_TMEM) wait(dv_done, ph ^ 1u);  // the P^T before this one
+            tmem_st_32x16(lane_base + C::P_COL + part * C::P_STEP, pk);
+          }
+          tmem_st_wait();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(p_full);
+          // dS = P o (dP - delta) * scale
+          wait(dp_full, ph);
+          tc_fence_after();
+          {
+            const float* dlt_s = sDelta + os.s * kBM + part * 32;
+            float dp[32];
+            uint32_t dk[16];
+            tmem_ld_32x32(lane_base + C::DP_COL + part * 32, dp);
+            tmem_ld_wait();
+#pragma unroll
+            for (int c = 0; c < 32; c += 4) {
+              const float4 d4 = *reinterpret_cast<const float4*>(dlt_s + c);
+#pragma unroll
+              for (int t = 0; t < 4; t += 2) {
+                const f32x2 d = fma2(pack2(dp[c + t], dp[c + t + 1]), out_scale2, t ? pack2(d4.z, d4.w) : pack2(d4.x, d4.y));
+                float g0, g1;
+                unpack2(mul2(pack2(pr[c + t], pr[c + t + 1]), d), g0, g1);
+                dk[(c + t) >> 1] = pack_bf16x2(g0, g1);
+              }
+            }
+            tmem_st_32x16(lane_base + C::DP_COL + part * 32, dk);
+          }
+          tmem_st_wait();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(ds_full);
+          ph ^= 1u;
+          qs.next();
+          os.next();
+        }
+      }
+      work.next();
+      wait(acc_full, r & 1);
+      tc_fence_after();
+      if (__any_sync(0xffffffffu, *abort_flag != 0)) break;
+      // Parts 0 and 1 write dV, 2 and 3 dK, half of the columns each.  The next kv tile's products overwrite both only
+      // after these warps delivered its first P^T and dS^T, which they do after the reads here.
+      const int c0 = (part & 1) * (D / 2);
+      __nv_bfloat16* base = (part < 2 ? p.dv : p.dk) + (((long long)b * p.T + kt * kBM) * p.Hkv + hk) * D + c0;
+      store_rows<D / 2>(tmem_base + (part < 2 ? C::DV_COL : C::DK_COL) + c0, quad, lane, base, (long long)p.Hkv * D,
+                        p.T - kt * kBM);
+    }
+    if (*abort_flag != 0 && lane == 0 && p.status) atomicCAS(p.status, 0, kStatusEpilogueTimeout);
   }
 
   tc_fence_before();
@@ -1078,18 +1358,30 @@ EncodeFn attn_encode_fn() {
   return fn;
 }
 
-// [rows, cols] bf16 row-major with pitch `ld` elements; box = 64 columns x box_rows rows, 128-byte swizzle
-bool attn_tmap(CUtensorMap* map, const void* base, uint64_t cols, uint64_t rows, uint64_t ld, uint32_t box_rows) {
+// [seqs, T, cols] bf16, contiguous; box = 64 columns x kBM rows of one sequence (rows beyond T read as zeros), 128-byte swizzle
+bool attn_tmap_seq(CUtensorMap* map, const void* base, uint64_t cols, uint64_t T, uint64_t seqs) {
   EncodeFn fn = attn_encode_fn();
-  if (!fn) return false;
-  if ((reinterpret_cast<uintptr_t>(base) & 15) || ((ld * 2) & 15)) return false;
-  cuuint64_t dims[2] = {cols, rows};
-  cuuint64_t strides[1] = {ld * 2};
-  cuuint32_t box[2] = {64, box_rows};
-  cuuint32_t estr[2] = {1, 1};
-  return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
+  if (!fn || (reinterpret_cast<uintptr_t>(base) & 15)) return false;
+  cuuint64_t dims[3] = {cols, T, seqs};
+  cuuint64_t strides[2] = {cols * 2, T * cols * 2};
+  cuuint32_t box[3] = {64, kBM, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// CTAs of a persistent kernel with one CTA per SM
+int attn_grid(long long items) {
+  static std::atomic<int> known[64];  // per device; the count does not change
+  int dev = 0;
+  cudaGetDevice(&dev);
+  int sms = dev < 64 ? known[dev].load(std::memory_order_relaxed) : 0;
+  if (sms == 0) {
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
+    if (dev < 64) known[dev].store(sms, std::memory_order_relaxed);
+  }
+  return (int)(items < sms ? items : sms);
 }
 
 template <int D>
@@ -1097,14 +1389,15 @@ cudaError_t attn_fwd_launch_d(const void* q, const void* k, const void* v, void*
                               int Hkv, float scale, int* status, cudaStream_t stream) {
   using C = AttnCfg<D>;
   CUtensorMap tq, tk, tv;
-  const uint64_t rows = (uint64_t)B * T;
-  if (!attn_tmap(&tq, q, (uint64_t)H * D, rows, (uint64_t)H * D, kBM) ||
-      !attn_tmap(&tk, k, (uint64_t)Hkv * D, rows, (uint64_t)Hkv * D, kBN) ||
-      !attn_tmap(&tv, v, (uint64_t)Hkv * D, rows, (uint64_t)Hkv * D, kBN))
+  if (!attn_tmap_seq(&tq, q, (uint64_t)H * D, T, B) || !attn_tmap_seq(&tk, k, (uint64_t)Hkv * D, T, B) ||
+      !attn_tmap_seq(&tv, v, (uint64_t)Hkv * D, T, B))
     return cudaErrorInvalidValue;
   auto kernel = attn_fwd_kernel<D>;
   static bool attr_set = false;
   if (!attr_set) {
+    cudaFuncAttributes fa;
+    // the register shares of the kernel's warps add up to what it is launched with, or the larger one waits forever
+    if (cudaFuncGetAttributes(&fa, kernel) != cudaSuccess || fa.numRegs != 168) return cudaErrorInvalidConfiguration;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
     if (e != cudaSuccess) return e;
     attr_set = true;
@@ -1112,69 +1405,89 @@ cudaError_t attn_fwd_launch_d(const void* q, const void* k, const void* v, void*
   AttnParams p;
   p.out = reinterpret_cast<__nv_bfloat16*>(out);
   p.lse = lse;
+  p.B = B;
   p.T = T;
   p.H = H;
   p.Hkv = Hkv;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.status = status;
-  dim3 grid((T + kBM - 1) / kBM, B * H);
-  kernel<<<grid, kAttnThreads, C::SMEM, stream>>>(tq, tk, tv, p);
+  const int tiles = (T + kBM - 1) / kBM;
+  const int heads = B * H, sms = attn_grid(1 << 20);
+  p.pair = (long long)heads * tiles > sms ? 2 : 1;
+  const int items = (tiles + p.pair - 1) / p.pair, ctas = attn_grid((long long)heads * items);
+  p.plan = WorkPlan(items, heads, ctas);
+  p.by_heads = FastDiv(H);
+  p.by_group = FastDiv(H / Hkv);
+  kernel<<<ctas, kFwdThreads, C::SMEM, stream>>>(tq, tk, tv, p);
   return cudaGetLastError();
 }
 
 template <int D>
 cudaError_t attn_bwd_launch_d(const void* q, const void* k, const void* v, const void* o, const void* d_o,
-                              const float* lse, float* delta, void* dq, void* dk, void* dv, int B, int T, int H,
+                              const float* lse, float* stats, void* dq, void* dk, void* dv, int B, int T, int H,
                               int Hkv, float scale, int* status, cudaStream_t stream) {
-  const uint64_t rows = (uint64_t)B * T;
-  CUtensorMap q128, do128, k64, v64, q64, do64, k128, v128;
+  CUtensorMap qs, dos, ks, vs;
   const uint64_t wq = (uint64_t)H * D, wk = (uint64_t)Hkv * D;
-  if (!attn_tmap(&q128, q, wq, rows, wq, kBM) || !attn_tmap(&do128, d_o, wq, rows, wq, kBM) ||
-      !attn_tmap(&k64, k, wk, rows, wk, kBN) || !attn_tmap(&v64, v, wk, rows, wk, kBN) ||
-      !attn_tmap(&q64, q, wq, rows, wq, kBQ) || !attn_tmap(&do64, d_o, wq, rows, wq, kBQ) ||
-      !attn_tmap(&k128, k, wk, rows, wk, kBM) || !attn_tmap(&v128, v, wk, rows, wk, kBM))
+  if (!attn_tmap_seq(&qs, q, wq, T, B) || !attn_tmap_seq(&dos, d_o, wq, T, B) || !attn_tmap_seq(&ks, k, wk, T, B) ||
+      !attn_tmap_seq(&vs, v, wk, T, B))
     return cudaErrorInvalidValue;
   auto kq = attn_bwd_dq_kernel<D>;
   auto kkv = attn_bwd_dkv_kernel<D>;
   static bool attr_set = false;
   if (!attr_set) {
+    cudaFuncAttributes fa;
+    // the register shares of the kernel's warps add up to what it is launched with, or the larger one waits forever
+    if (cudaFuncGetAttributes(&fa, kq) != cudaSuccess || fa.numRegs != 168) return cudaErrorInvalidConfiguration;
     cudaError_t e = cudaFuncSetAttribute(kq, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdQCfg<D>::SMEM);
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(kkv, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdKvCfg<D>::SMEM);
     if (e != cudaSuccess) return e;
     attr_set = true;
   }
-  const long long nrows = (long long)B * T * H;
-  attn_delta_kernel<D><<<(unsigned)((nrows * (D / 8) + 255) / 256), 256, 0, stream>>>(
-      reinterpret_cast<const __nv_bfloat16*>(o), reinterpret_cast<const __nv_bfloat16*>(d_o), delta, nrows, T, H);
+  const int tiles = (T + kBM - 1) / kBM, t_pad = tiles * kBM;
+  float* neg_lse2 = stats;
+  float* neg_delta = stats + (long long)B * H * t_pad;
+  const FastDiv by_heads(H);
+  constexpr int rows = 256 / (D / 8) * kDeltaRows;  // per block
+  if ((t_pad + rows - 1) / rows > 65535) return cudaErrorInvalidValue;
+  attn_delta_kernel<D><<<dim3(B * H, (t_pad + rows - 1) / rows), 256, 0, stream>>>(
+      reinterpret_cast<const __nv_bfloat16*>(o), reinterpret_cast<const __nv_bfloat16*>(d_o), lse, neg_lse2, neg_delta, T, H,
+      t_pad, by_heads, scale);
+  const int kv_ctas = attn_grid((long long)B * Hkv * tiles), q_ctas = attn_grid((long long)B * H * tiles);
   AttnBwdParams p;
   p.dq = reinterpret_cast<__nv_bfloat16*>(dq);
   p.dk = reinterpret_cast<__nv_bfloat16*>(dk);
   p.dv = reinterpret_cast<__nv_bfloat16*>(dv);
-  p.lse = lse;
-  p.delta = delta;
+  p.neg_lse2 = neg_lse2;
+  p.neg_delta = neg_delta;
+  p.q_plan = WorkPlan(tiles, B * H, q_ctas);
+  p.kv_plan = WorkPlan(tiles, B * Hkv, kv_ctas);
+  p.by_heads = by_heads;
+  p.by_kv_heads = FastDiv(Hkv);
+  p.by_group = FastDiv(H / Hkv);
+  p.B = B;
   p.T = T;
   p.H = H;
   p.Hkv = Hkv;
   p.scale = scale;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.status = status;
-  kkv<<<dim3(T / kBM, B * Hkv), kKvThreads, BwdKvCfg<D>::SMEM, stream>>>(q64, do64, k128, v128, p);
-  kq<<<dim3(T / kBM, B * H), kAttnThreads, BwdQCfg<D>::SMEM, stream>>>(q128, do128, k64, v64, p);
+  kkv<<<kv_ctas, kBwdThreads, BwdKvCfg<D>::SMEM, stream>>>(qs, dos, ks, vs, p);
+  kq<<<q_ctas, kDqThreads, BwdQCfg<D>::SMEM, stream>>>(qs, dos, ks, vs, p);
   return cudaGetLastError();
 }
 
 }  // namespace
 
 cudaError_t attn_bwd_launch(const void* q, const void* k, const void* v, const void* o, const void* d_o,
-                            const float* lse, float* delta, void* dq, void* dk, void* dv, int B, int T, int H, int Hkv,
+                            const float* lse, float* stats, void* dq, void* dk, void* dv, int B, int T, int H, int Hkv,
                             int D, float scale, int* status, cudaStream_t stream) {
   if (B <= 0 || T <= 0 || H <= 0 || Hkv <= 0 || H % Hkv != 0 || B * H > 65535 || T % kBM != 0)
     return cudaErrorInvalidValue;
   if (D == 128)
-    return attn_bwd_launch_d<128>(q, k, v, o, d_o, lse, delta, dq, dk, dv, B, T, H, Hkv, scale, status, stream);
+    return attn_bwd_launch_d<128>(q, k, v, o, d_o, lse, stats, dq, dk, dv, B, T, H, Hkv, scale, status, stream);
   if (D == 64)
-    return attn_bwd_launch_d<64>(q, k, v, o, d_o, lse, delta, dq, dk, dv, B, T, H, Hkv, scale, status, stream);
+    return attn_bwd_launch_d<64>(q, k, v, o, d_o, lse, stats, dq, dk, dv, B, T, H, Hkv, scale, status, stream);
   return cudaErrorInvalidValue;
 }
 

@@ -1118,19 +1118,19 @@ Tensor gpt_block_fwd(const Tensor& x, const Tensor& wq, const Tensor& wk, const 
 }
 
 void attn_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& d_o, const Tensor& lse,
-              Tensor delta, Tensor dq, Tensor dk, Tensor dv, double scale, Tensor status) {
+              Tensor stats, Tensor dq, Tensor dk, Tensor dv, double scale, Tensor status) {
   const c10::cuda::CUDAGuard guard(q.device());
   for (const Tensor* t : std::initializer_list<const Tensor*>{&q, &k, &v, &o, &d_o, &dq, &dk, &dv})
     TORCH_CHECK(t->dim() == 4 && t->scalar_type() == at::kBFloat16 && t->is_contiguous(),
                 "attention tensors must be contiguous bf16 [B, T, H, D]");
-  TORCH_CHECK(lse.scalar_type() == at::kFloat && delta.scalar_type() == at::kFloat && lse.is_contiguous() &&
-              delta.is_contiguous() && delta.numel() == lse.numel());
   const int64_t B = q.size(0), T = q.size(1), H = q.size(2), D = q.size(3), Hkv = k.size(2);
+  TORCH_CHECK(lse.scalar_type() == at::kFloat && stats.scalar_type() == at::kFloat && lse.is_contiguous() &&
+              stats.is_contiguous() && stats.numel() >= 2 * B * H * ((T + 127) / 128 * 128));
   TORCH_CHECK(o.sizes() == q.sizes() && d_o.sizes() == q.sizes() && dq.sizes() == q.sizes() && v.sizes() == k.sizes() &&
               dk.sizes() == k.sizes() && dv.sizes() == k.sizes() && lse.numel() == B * H * T);
   g_launches += 3;
   DION_CUDA_CHECK(dion::attn_bwd_launch(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), d_o.data_ptr(),
-                                        lse.data_ptr<float>(), delta.data_ptr<float>(), dq.data_ptr(), dk.data_ptr(),
+                                        lse.data_ptr<float>(), stats.data_ptr<float>(), dq.data_ptr(), dk.data_ptr(),
                                         dv.data_ptr(), (int)B, (int)T, (int)H, (int)Hkv, (int)D, (float)scale,
                                         status.data_ptr<int>(), at::cuda::getCurrentCUDAStream()));
 }
@@ -1305,7 +1305,7 @@ TORCH_LIBRARY(dion_b200, m) {
   m.def("split_tf32(Tensor x, Tensor(a!) hi, Tensor(b!) lo) -> ()");
   m.def("attn_fwd(Tensor q, Tensor k, Tensor v, Tensor(a!) out, Tensor(b!) lse, float scale, Tensor(c!) status) -> ()");
   m.def(
-      "attn_bwd(Tensor q, Tensor k, Tensor v, Tensor o, Tensor d_o, Tensor lse, Tensor(a!) delta, Tensor(b!) dq, "
+      "attn_bwd(Tensor q, Tensor k, Tensor v, Tensor o, Tensor d_o, Tensor lse, Tensor(a!) stats, Tensor(b!) dq, "
       "Tensor(c!) dk, Tensor(d!) dv, float scale, Tensor(e!) status) -> ()");
   m.def("refine_prep(Tensor G, Tensor(a!) C, Tensor(b!) d, float dead_below, Tensor? skip, bool fold=False) -> ()");
   m.def(

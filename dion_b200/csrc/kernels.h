@@ -135,9 +135,10 @@ cudaError_t col_sumsq_launch(const void* X, int x_type, float* out, int batch, l
 cudaError_t attn_fwd_launch(const void* q, const void* k, const void* v, void* out, float* lse, int B, int T, int H,
                             int Hkv, int D, float scale, int* status, cudaStream_t stream);
 // Backward of the same attention: dq [B*T, H*D], dk / dv [B*T, Hkv*D] (bf16) from q, k, v, the forward's
-// output `o` and log-sum-exp `lse`, and the output gradient `d_o`; `delta` is a [B, H, T] fp32 workspace.
+// output `o` and log-sum-exp `lse`, and the output gradient `d_o`; `stats` is a workspace of 2 x B x H x (T rounded up to
+// 128) fp32 values.
 cudaError_t attn_bwd_launch(const void* q, const void* k, const void* v, const void* o, const void* d_o,
-                            const float* lse, float* delta, void* dq, void* dk, void* dv, int B, int T, int H, int Hkv,
+                            const float* lse, float* stats, void* dq, void* dk, void* dv, int B, int T, int H, int Hkv,
                             int D, float scale, int* status, cudaStream_t stream);
 // Pieces of the blocked Cholesky-inverse: W = D G D with d = rsqrt(diag G) (contiguous W [batch][r][r], d
 // [batch][r]); and the placement of a diagonal block's inverse factor Zd ([batch][nb][nb]) into Z at (k0, k0)

@@ -701,8 +701,8 @@ def flash_attention_backward(q, k, v, out, lse, d_out, scale: Optional[float] = 
     if scale is None:
         scale = 1.0 / math.sqrt(D)
     dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-    delta = torch.empty_like(lse)
-    torch.ops.dion_b200.attn_bwd(q, k, v, out, d_out.contiguous(), lse, delta, dq, dk, dv, float(scale),
+    stats = torch.empty(2, B, H, (T + 127) // 128 * 128, dtype=torch.float32, device=q.device)
+    torch.ops.dion_b200.attn_bwd(q, k, v, out, d_out.contiguous(), lse, stats, dq, dk, dv, float(scale),
                                  runtime.status_tensor(q.device))
     return dq, dk, dv
 

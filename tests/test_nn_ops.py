@@ -328,6 +328,39 @@ def test_flash_attention_backward_matches_fp32_reference(shape):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("shape", [
+    (150, 128, 1, 1, 128),  # one tile per head; a head for every CTA and two left over
+    (40, 256, 4, 4, 64),    # pairs of query tiles, 160 heads
+    (5, 640, 40, 8, 64),    # an odd number of tiles: the last pair is a single one; grouped kv heads
+    (1, 384, 2, 2, 128),    # fewer tiles than SMs: one query tile per work item
+    (2, 896, 24, 2, 128),   # leftover heads over several rounds, back and forth over the CTAs
+])
+def test_flash_attention_work_split(shape):
+    """Every (head, tile) of the persistent kernels is worked on exactly once, forward and backward.  Outputs are bf16
+    (2^-9 of values up to about 4.5) of products with bf16 probabilities: 2e-2, as for the shapes above."""
+    from dion_b200 import ops
+    from dion_b200.ops.nn import flash_attention_backward, flash_attention_forward
+
+    B, T, H, Hkv, D = shape
+    g = torch.Generator(device="cuda").manual_seed(17)
+    q, k, v, d_out = (torch.randn(B, T, h, D, device="cuda", generator=g).to(torch.bfloat16) for h in (H, Hkv, Hkv, H))
+    out, lse = flash_attention_forward(q, k, v)
+    grads = flash_attention_backward(q, k, v, out, lse, d_out)
+    ops.check_status()
+    qf, kf, vf = (t.float().requires_grad_() for t in (q, k, v))
+    kr, vr = (t.transpose(1, 2).repeat_interleave(H // Hkv, dim=1) for t in (kf, vf))
+    s = (qf.transpose(1, 2) @ kr.transpose(-1, -2)) / D ** 0.5
+    s = s.masked_fill(torch.triu(torch.ones(T, T, device="cuda", dtype=torch.bool), 1), float("-inf"))
+    ref = (torch.softmax(s, dim=-1) @ vr).transpose(1, 2)
+    ref.backward(d_out.float())
+    assert (out.float() - ref).abs().max().item() < 2e-2
+    torch.testing.assert_close(lse, torch.logsumexp(s, dim=-1), rtol=1e-3, atol=1e-3)
+    for name, got, want in zip(("dq", "dk", "dv"), grads, (qf.grad, kf.grad, vf.grad)):
+        err = (got.float() - want).abs().max().item() / want.abs().max().item()
+        assert err < 2e-2, (name, err)
+
+
+@pytest.mark.gpu
 def test_linear_fanout_matches_separate_linears():
     x = torch.randn(640, 256, device="cuda").to(torch.bfloat16).requires_grad_()
     ws = [torch.nn.Parameter(torch.randn(n, 256, device="cuda") * 0.05) for n in (256, 128, 384)]

@@ -25,6 +25,7 @@
 
 #include "gemm.h"
 #include "kernels.h"
+#include "pdl.cuh"
 #include "umma.cuh"
 
 namespace dion {
@@ -398,6 +399,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     *abort_flag = 0;
     mbar_fence_init();
   }
+  pdl_trigger();
+  pdl_wait();
   if (warp == 1) {
     tmem_alloc(tmem_slot, C::TMEM_COLS);
     tmem_relinquish();
@@ -687,6 +690,8 @@ __global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __
                                                         const float* __restrict__ lse, float* __restrict__ neg_lse2,
                                                         float* __restrict__ neg_delta, int T, int H, int t_pad,
                                                         FastDiv by_heads, float scale) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int LPR = D / 8;  // lanes per row: 16 (D = 128) or 8 (D = 64)
   constexpr int ROWS = 256 / LPR;
   const int sub = threadIdx.x % LPR;
@@ -787,6 +792,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     *abort_flag = 0;
     mbar_fence_init();
   }
+  pdl_trigger();
+  pdl_wait();
   if (warp == 1) {
     tmem_alloc(tmem_slot, C::TMEM_COLS);
     tmem_relinquish();
@@ -1063,6 +1070,8 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     *abort_flag = 0;
     mbar_fence_init();
   }
+  pdl_trigger();
+  pdl_wait();
   if (warp == 1) {
     tmem_alloc(tmem_slot, C::TMEM_COLS);
     tmem_relinquish();
@@ -1418,7 +1427,7 @@ cudaError_t attn_fwd_launch_d(const void* q, const void* k, const void* v, void*
   p.plan = WorkPlan(items, heads, ctas);
   p.by_heads = FastDiv(H);
   p.by_group = FastDiv(H / Hkv);
-  kernel<<<ctas, kFwdThreads, C::SMEM, stream>>>(tq, tk, tv, p);
+  launch_pdl(kernel, dim3(ctas), dim3(kFwdThreads), C::SMEM, stream, 0, tq, tk, tv, p);
   return cudaGetLastError();
 }
 
@@ -1450,9 +1459,9 @@ cudaError_t attn_bwd_launch_d(const void* q, const void* k, const void* v, const
   const FastDiv by_heads(H);
   constexpr int rows = 256 / (D / 8) * kDeltaRows;  // per block
   if ((t_pad + rows - 1) / rows > 65535) return cudaErrorInvalidValue;
-  attn_delta_kernel<D><<<dim3(B * H, (t_pad + rows - 1) / rows), 256, 0, stream>>>(
-      reinterpret_cast<const __nv_bfloat16*>(o), reinterpret_cast<const __nv_bfloat16*>(d_o), lse, neg_lse2, neg_delta, T, H,
-      t_pad, by_heads, scale);
+  launch_pdl(attn_delta_kernel<D>, dim3(B * H, (t_pad + rows - 1) / rows), dim3(256), 0, stream, 0,
+             reinterpret_cast<const __nv_bfloat16*>(o), reinterpret_cast<const __nv_bfloat16*>(d_o), lse, neg_lse2, neg_delta, T,
+             H, t_pad, by_heads, scale);
   const int kv_ctas = attn_grid((long long)B * Hkv * tiles), q_ctas = attn_grid((long long)B * H * tiles);
   AttnBwdParams p;
   p.dq = reinterpret_cast<__nv_bfloat16*>(dq);
@@ -1472,8 +1481,8 @@ cudaError_t attn_bwd_launch_d(const void* q, const void* k, const void* v, const
   p.scale = scale;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.status = status;
-  kkv<<<kv_ctas, kBwdThreads, BwdKvCfg<D>::SMEM, stream>>>(qs, dos, ks, vs, p);
-  kq<<<q_ctas, kDqThreads, BwdQCfg<D>::SMEM, stream>>>(qs, dos, ks, vs, p);
+  launch_pdl(kkv, dim3(kv_ctas), dim3(kBwdThreads), BwdKvCfg<D>::SMEM, stream, 0, qs, dos, ks, vs, p);
+  launch_pdl(kq, dim3(q_ctas), dim3(kDqThreads), BwdQCfg<D>::SMEM, stream, 0, qs, dos, ks, vs, p);
   return cudaGetLastError();
 }
 

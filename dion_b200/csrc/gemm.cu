@@ -29,6 +29,7 @@
 #include <mutex>
 #include <string>
 
+#include "pdl.cuh"
 #include "umma.cuh"
 
 namespace dion {
@@ -442,6 +443,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     }
     *abort_flag = 0;
     mbar_fence_init();
+  }
+  if constexpr (!kGather) {
+    pdl_trigger();
+    pdl_wait();
   }
   if (warp == 1) {
     if constexpr (kPair) {
@@ -1550,24 +1555,14 @@ cudaError_t launch_cfg(const GemmArgs& a, const KernelParams& kp, cudaStream_t s
     grid /= cluster;  // one tile per cluster at a time
     if (grid > kp.total_tiles || kClusterK) grid = kp.total_tiles;
     if (grid < 1) grid = 1;
-    cudaLaunchConfig_t cfg;
-    memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3(cluster * grid, 1, 1);
-    cfg.blockDim = dim3(kThreads, 1, 1);
-    cfg.dynamicSmemBytes = C::SMEM_BYTES;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = cluster;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, ta, tb, ta_lo, tb_lo, tm, kp);
+    return launch_pdl(kernel, dim3(cluster * grid), dim3(kThreads), C::SMEM_BYTES, stream, cluster, ta, tb, ta_lo, tb_lo, tm, kp);
   } else {
     if (grid > kp.total_tiles) grid = kp.total_tiles;
-    kernel<<<grid, kThreads, C::SMEM_BYTES, stream>>>(ta, tb, ta_lo, tb_lo, tm, kp);
-    return cudaGetLastError();
+    if constexpr (kGather) {  // waits for other ranks' kernels: launched when the kernels before it are done
+      kernel<<<grid, kThreads, C::SMEM_BYTES, stream>>>(ta, tb, ta_lo, tb_lo, tm, kp);
+      return cudaGetLastError();
+    }
+    return launch_pdl(kernel, dim3(grid), dim3(kThreads), C::SMEM_BYTES, stream, 0, ta, tb, ta_lo, tb_lo, tm, kp);
   }
 }
 

@@ -21,6 +21,7 @@
 #include <string.h>
 
 #include "kernels.h"
+#include "pdl.cuh"
 #include "umma.cuh"
 
 namespace dion {
@@ -249,6 +250,8 @@ chol_inverse_kernel(const float* __restrict__ Gall, float* __restrict__ Zall, fl
 __global__ void __launch_bounds__(256) col_sumsq_kernel(const void* __restrict__ X, int x_type,
                                                        float* __restrict__ out, long long rows, int cols,
                                                        long long ldx, long long batch_stride) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ float red[8][33];
   const int b = blockIdx.y;
   const int col = blockIdx.x * 32 + (threadIdx.x & 31);
@@ -800,6 +803,8 @@ __global__ void __launch_bounds__(256) split_tf32_kernel(const float4* __restric
                                                         float4* __restrict__ lo, long long nvec,
                                                         const float* __restrict__ xs, float* __restrict__ his,
                                                         float* __restrict__ los, long long ntail) {
+  pdl_trigger();
+  pdl_wait();
   auto split = [](float v, float& h, float& l) {
     h = __int_as_float(__float_as_int(v) & 0xffffe000);
     l = v - h;
@@ -827,6 +832,8 @@ __global__ void __launch_bounds__(256) split_tf32_kernel(const float4* __restric
 __global__ void __launch_bounds__(256) refine_prep_kernel(const float* __restrict__ G, float* __restrict__ C,
                                                          float* __restrict__ d, int r, float dead_below,
                                                          const int* __restrict__ skip, int fold) {
+  pdl_trigger();
+  pdl_wait();
   const long long b = blockIdx.y;
   // matrices flagged in `skip` get C = 0: they are only rescaled, not corrected
   const bool no_correction = skip != nullptr && skip[b] != 0;
@@ -941,7 +948,7 @@ cudaError_t col_sumsq_launch(const void* X, int x_type, float* out, int batch, l
                              long long ldx, long long batch_stride, cudaStream_t s) {
   if (batch == 0 || cols == 0) return cudaSuccess;
   dim3 grid((cols + 31) / 32, batch);
-  col_sumsq_kernel<<<grid, 256, 0, s>>>(X, x_type, out, rows, cols, ldx, batch_stride);
+  launch_pdl(col_sumsq_kernel, dim3(grid), dim3(256), 0, s, 0, X, x_type, out, rows, cols, ldx, batch_stride);
   return cudaGetLastError();
 }
 
@@ -949,6 +956,8 @@ cudaError_t col_sumsq_launch(const void* X, int x_type, float* out, int batch, l
 __global__ void __launch_bounds__(256) split_tf32_rows_kernel(const float* __restrict__ x, float* __restrict__ hi,
                                                              float* __restrict__ lo, long long rows_total, int rows,
                                                              int cols, long long ld, long long bs) {
+  pdl_trigger();
+  pdl_wait();
   const int vpr = cols >> 2;  // float4 per row (cols is a multiple of 4)
   const long long nvec = rows_total * vpr;
   for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < nvec; v += (long long)gridDim.x * blockDim.x) {
@@ -976,6 +985,8 @@ __global__ void __launch_bounds__(256) split_tf32_rows_kernel(const float* __res
 __global__ void __launch_bounds__(256) jacobi_scale_kernel(const float* __restrict__ G, float* __restrict__ W,
                                                           float* __restrict__ d, int r, long long ldg,
                                                           long long g_batch_stride) {
+  pdl_trigger();
+  pdl_wait();
   const long long b = blockIdx.y;
   const float* g = G + b * g_batch_stride;
   float* w = W + b * (long long)r * r;
@@ -997,6 +1008,8 @@ __global__ void __launch_bounds__(256) jacobi_scale_kernel(const float* __restri
 __global__ void __launch_bounds__(256) place_block_kernel(const float* __restrict__ Zd, const float* __restrict__ mask,
                                                          float* __restrict__ Z, float* __restrict__ Zm, int nb, int r,
                                                          int k0) {
+  pdl_trigger();
+  pdl_wait();
   const long long b = blockIdx.y;
   const int row = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (row >= nb) return;
@@ -1016,7 +1029,7 @@ cudaError_t jacobi_scale_launch(const float* G, float* W, float* d, int batch, i
                                 long long g_batch_stride, cudaStream_t s) {
   if (batch == 0 || r == 0) return cudaSuccess;
   if (batch > 65535) return cudaErrorInvalidValue;
-  jacobi_scale_kernel<<<dim3((r + 7) / 8, batch), 256, 0, s>>>(G, W, d, r, ldg, g_batch_stride);
+  launch_pdl(jacobi_scale_kernel, dim3((r + 7) / 8, batch), dim3(256), 0, s, 0, G, W, d, r, ldg, g_batch_stride);
   return cudaGetLastError();
 }
 
@@ -1024,7 +1037,7 @@ cudaError_t place_block_launch(const float* Zd, const float* mask, float* Z, flo
                                cudaStream_t s) {
   if (batch == 0 || nb == 0) return cudaSuccess;
   if (batch > 65535 || k0 < 0 || k0 + nb > r) return cudaErrorInvalidValue;
-  place_block_kernel<<<dim3((nb + 7) / 8, batch), 256, 0, s>>>(Zd, mask, Z, Zm, nb, r, k0);
+  launch_pdl(place_block_kernel, dim3((nb + 7) / 8, batch), dim3(256), 0, s, 0, Zd, mask, Z, Zm, nb, r, k0);
   return cudaGetLastError();
 }
 
@@ -1038,7 +1051,7 @@ cudaError_t split_tf32_rows_launch(const float* x, float* hi, float* lo, int bat
   const long long nvec = rows_total * (cols >> 2);
   long long grid = (nvec + 255) / 256;
   if (grid > 148 * 16) grid = 148 * 16;
-  split_tf32_rows_kernel<<<(int)grid, 256, 0, s>>>(x, hi, lo, rows_total, rows, cols, ld, bs);
+  launch_pdl(split_tf32_rows_kernel, dim3((int)grid), dim3(256), 0, s, 0, x, hi, lo, rows_total, rows, cols, ld, bs);
   return cudaGetLastError();
 }
 
@@ -1050,7 +1063,7 @@ cudaError_t split_tf32_launch(const float* x, float* hi, float* lo, long long nu
   long long grid = (nvec + 255) / 256;
   if (grid > 148 * 16) grid = 148 * 16;
   if (grid < 1) grid = 1;
-  split_tf32_kernel<<<(int)grid, 256, 0, s>>>(reinterpret_cast<const float4*>(x), reinterpret_cast<float4*>(hi),
+  launch_pdl(split_tf32_kernel, dim3((int)grid), dim3(256), 0, s, 0, reinterpret_cast<const float4*>(x), reinterpret_cast<float4*>(hi),
                                               reinterpret_cast<float4*>(lo), nvec, x + nvec * 4, hi + nvec * 4,
                                               lo + nvec * 4, ntail);
   return cudaGetLastError();
@@ -1060,7 +1073,7 @@ cudaError_t refine_prep_launch(const float* G, float* C, float* d, int batch, in
                                const int* skip, bool fold, cudaStream_t s) {
   if (batch == 0 || r == 0) return cudaSuccess;
   if (batch > 65535) return cudaErrorInvalidValue;
-  refine_prep_kernel<<<dim3((r + 7) / 8, batch), 256, 0, s>>>(G, C, d, r, dead_below, skip, fold ? 1 : 0);
+  launch_pdl(refine_prep_kernel, dim3((r + 7) / 8, batch), dim3(256), 0, s, 0, G, C, d, r, dead_below, skip, fold ? 1 : 0);
   return cudaGetLastError();
 }
 

@@ -5,6 +5,7 @@
 #include <cuda_bf16.h>
 
 #include "kernels.h"
+#include "pdl.cuh"
 
 namespace dion {
 
@@ -52,6 +53,8 @@ __global__ void __launch_bounds__(256) rmsnorm_gain_fwd_kernel(const bf16* __res
                                                               int gain_type, bf16* __restrict__ y,
                                                               float* __restrict__ rstd, long long rows, int dim,
                                                               float eps) {
+  pdl_trigger();
+  pdl_wait();
   const long long row = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (row >= rows) return;
   const int lane = threadIdx.x & 31;
@@ -101,6 +104,8 @@ __global__ void __launch_bounds__(256) rmsnorm_gain_bwd_kernel(const bf16* __res
                                                               const void* __restrict__ gain, int gain_type,
                                                               bf16* __restrict__ dx, float* __restrict__ partial,
                                                               long long rows, int dim, long long rows_per_block) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ float red[2][kGainRows][8];
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -188,6 +193,8 @@ __global__ void __launch_bounds__(256) rmsnorm_gain_bwd_kernel(const bf16* __res
 // h = silu(g) * u
 __global__ void __launch_bounds__(256) swiglu_fwd_kernel(const uint4* __restrict__ g, const uint4* __restrict__ u,
                                                         uint4* __restrict__ h, long long nvec) {
+  pdl_trigger();
+  pdl_wait();
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nvec; i += (long long)gridDim.x * blockDim.x) {
     float a[8], b[8], o[8];
     unpack8(g[i], a);
@@ -201,6 +208,8 @@ __global__ void __launch_bounds__(256) swiglu_fwd_kernel(const uint4* __restrict
 __global__ void __launch_bounds__(256) swiglu_bwd_kernel(const uint4* __restrict__ dh, const uint4* __restrict__ g,
                                                         const uint4* __restrict__ u, uint4* __restrict__ dg,
                                                         uint4* __restrict__ du, long long nvec) {
+  pdl_trigger();
+  pdl_wait();
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nvec; i += (long long)gridDim.x * blockDim.x) {
     float d[8], a[8], b[8], og[8], ou[8];
     unpack8(dh[i], d);
@@ -230,7 +239,7 @@ cudaError_t rmsnorm_gain_fwd_launch(const void* x, const void* gain, int gain_ty
   if (!norm_args_ok(gain, gain_type, dim)) return cudaErrorInvalidValue;
   const unsigned grid = (unsigned)((rows + 7) / 8);
 #define DION_GAIN_FWD(V)                                                                                          \
-  rmsnorm_gain_fwd_kernel<V><<<grid, 256, 0, s>>>(reinterpret_cast<const bf16*>(x), gain, gain_type,                 \
+  launch_pdl(rmsnorm_gain_fwd_kernel<V>, dim3(grid), dim3(256), 0, s, 0, reinterpret_cast<const bf16*>(x), gain, gain_type,                 \
                                                   reinterpret_cast<bf16*>(y), rstd, rows, dim, eps)
   if (dim <= 4 * 256) DION_GAIN_FWD(4);
   else if (dim <= 8 * 256) DION_GAIN_FWD(8);
@@ -255,7 +264,7 @@ cudaError_t rmsnorm_gain_bwd_launch(const void* dy, const void* x, const float* 
   const int per_thread = nvec > 256 ? 2 : 1;
   const int threads = ((nvec + per_thread - 1) / per_thread + 31) / 32 * 32;
   const auto kernel = per_thread == 2 ? rmsnorm_gain_bwd_kernel<2> : rmsnorm_gain_bwd_kernel<1>;
-  kernel<<<blocks, threads, 0, s>>>(reinterpret_cast<const bf16*>(dy), reinterpret_cast<const bf16*>(x), rstd, gain,
+  launch_pdl(kernel, dim3(blocks), dim3(threads), 0, s, 0, reinterpret_cast<const bf16*>(dy), reinterpret_cast<const bf16*>(x), rstd, gain,
                                     gain_type, reinterpret_cast<bf16*>(dx), partial, rows, dim, rpb);
   return cudaGetLastError();
 }
@@ -267,7 +276,7 @@ cudaError_t swiglu_fwd_launch(const void* g, const void* u, void* h, long long n
   const long long nvec = n / 8;
   long long grid = (nvec + 255) / 256;
   if (grid > 148 * 16) grid = 148 * 16;
-  swiglu_fwd_kernel<<<(int)grid, 256, 0, s>>>(reinterpret_cast<const uint4*>(g), reinterpret_cast<const uint4*>(u),
+  launch_pdl(swiglu_fwd_kernel, dim3((int)grid), dim3(256), 0, s, 0, reinterpret_cast<const uint4*>(g), reinterpret_cast<const uint4*>(u),
                                               reinterpret_cast<uint4*>(h), nvec);
   return cudaGetLastError();
 }
@@ -281,7 +290,7 @@ cudaError_t swiglu_bwd_launch(const void* dh, const void* g, const void* u, void
   const long long nvec = n / 8;
   long long grid = (nvec + 255) / 256;
   if (grid > 148 * 16) grid = 148 * 16;
-  swiglu_bwd_kernel<<<(int)grid, 256, 0, s>>>(reinterpret_cast<const uint4*>(dh), reinterpret_cast<const uint4*>(g),
+  launch_pdl(swiglu_bwd_kernel, dim3((int)grid), dim3(256), 0, s, 0, reinterpret_cast<const uint4*>(dh), reinterpret_cast<const uint4*>(g),
                                               reinterpret_cast<const uint4*>(u), reinterpret_cast<uint4*>(dg),
                                               reinterpret_cast<uint4*>(du), nvec);
   return cudaGetLastError();

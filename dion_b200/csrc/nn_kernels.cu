@@ -10,6 +10,7 @@
 #include <initializer_list>
 
 #include "kernels.h"
+#include "pdl.cuh"
 
 namespace dion {
 
@@ -56,6 +57,8 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const bf16* __restrict
                                                          bf16* __restrict__ x_out, bf16* __restrict__ y,
                                                          float* __restrict__ rstd, long long rows, int dim,
                                                          float eps) {
+  pdl_trigger();
+  pdl_wait();
   const long long row = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (row >= rows) return;
   const int lane = threadIdx.x & 31;
@@ -108,6 +111,8 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd_kernel(const bf16* __restrict
                                                          const float* __restrict__ rstd,
                                                          const bf16* __restrict__ dx_add, bf16* __restrict__ dx,
                                                          long long rows, int dim) {
+  pdl_trigger();
+  pdl_wait();
   const long long row = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (row >= rows) return;
   const int lane = threadIdx.x & 31;
@@ -189,6 +194,8 @@ __global__ void __launch_bounds__(256) rope_qknorm_fwd_kernel(const bf16* __rest
                                                              const bf16* __restrict__ sinb, long long tokens,
                                                              int seq_len, int heads, long long in_pitch,
                                                              long long out_pitch, float eps) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int HALF = HD / 2;
   constexpr int LPR = HD / 8;  // lanes per row
   const long long gid = (long long)blockIdx.x * 256 + threadIdx.x;
@@ -239,6 +246,8 @@ __global__ void __launch_bounds__(256) rope_qknorm_bwd_kernel(const bf16* __rest
                                                              const bf16* __restrict__ sinb, long long tokens,
                                                              int seq_len, int heads, long long in_pitch,
                                                              long long out_pitch, float eps) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int HALF = HD / 2;
   constexpr int LPR = HD / 8;
   const long long gid = (long long)blockIdx.x * 256 + threadIdx.x;
@@ -316,6 +325,8 @@ __global__ void __launch_bounds__(256) rope_qknorm_fwd_wide_kernel(const bf16* _
                                                                   const bf16* __restrict__ sinb, long long tokens,
                                                                   int seq_len, int heads, long long in_pitch,
                                                                   long long out_pitch, float eps) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int HALF = HD / 2;
   constexpr int LPR = HD / 16;  // lanes per (token, head)
   const long long gid = (long long)blockIdx.x * 256 + threadIdx.x;
@@ -408,6 +419,8 @@ __global__ void __launch_bounds__(256) rope_qknorm_bwd_wide_kernel(const bf16* _
                                                                   const bf16* __restrict__ sinb, long long tokens,
                                                                   int seq_len, int heads, long long in_pitch,
                                                                   long long out_pitch, float eps) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int HALF = HD / 2;
   constexpr int LPR = HD / 16;
   const long long gid = (long long)blockIdx.x * 256 + threadIdx.x;
@@ -454,6 +467,8 @@ __global__ void __launch_bounds__(256) rope_qknorm_bwd_wide_kernel(const bf16* _
 // ------------------------------------------------------------------ ReLU^2
 __global__ void __launch_bounds__(256) relu2_fwd_kernel(const uint4* __restrict__ x, uint4* __restrict__ h,
                                                        long long nvec) {
+  pdl_trigger();
+  pdl_wait();
   const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
   if (i >= nvec) return;
   float f[8];
@@ -467,6 +482,8 @@ __global__ void __launch_bounds__(256) relu2_fwd_kernel(const uint4* __restrict_
 }
 __global__ void __launch_bounds__(256) relu2_bwd_kernel(const uint4* __restrict__ dh, const uint4* __restrict__ x,
                                                        uint4* __restrict__ dx, long long nvec) {
+  pdl_trigger();
+  pdl_wait();
   const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
   if (i >= nvec) return;
   float f[8], g[8];
@@ -503,6 +520,8 @@ __global__ void __launch_bounds__(kCeThreads) cross_entropy_kernel(bf16* __restr
                                                                   const float* __restrict__ scale_ptr,
                                                                   int vocab, long long pitch, float grad_scale,
                                                                   long long ignore_index, int write_grad) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ float red_m[kCeThreads / 32], red_s[kCeThreads / 32];
   const long long row = blockIdx.x;
   const long long tgt = targets[row];
@@ -571,6 +590,8 @@ __global__ void __launch_bounds__(kCeThreads) cross_entropy_kernel(bf16* __restr
 template <bool kBf16>
 __global__ void __launch_bounds__(256) scale_by_scalar_kernel(const void* x, void* y, long long n, int vec,
                                                              const float* __restrict__ scale) {
+  pdl_trigger();
+  pdl_wait();
   const float s = kBf16 ? __bfloat162float(__float2bfloat16(*scale)) : *scale;
   if (x == y && s == 1.f) return;
   const long long t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -602,6 +623,8 @@ __global__ void __launch_bounds__(256) scale_by_scalar_kernel(const void* x, voi
 __global__ void __launch_bounds__(256) embedding_fwd_kernel(const void* __restrict__ table, int table_type,
                                                            const long long* __restrict__ idx, bf16* __restrict__ out,
                                                            long long tokens, int dim) {
+  pdl_trigger();
+  pdl_wait();
   const long long tok = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (tok >= tokens) return;
   const int lane = threadIdx.x & 31;
@@ -625,6 +648,8 @@ __global__ void __launch_bounds__(256) embedding_fwd_kernel(const void* __restri
 __global__ void __launch_bounds__(256) embedding_bwd_kernel(const bf16* __restrict__ dout,
                                                            const long long* __restrict__ idx,
                                                            float* __restrict__ dtable, long long tokens, int dim) {
+  pdl_trigger();
+  pdl_wait();
   const long long tok = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (tok >= tokens) return;
   const int lane = threadIdx.x & 31;
@@ -646,7 +671,7 @@ cudaError_t rmsnorm_fwd_launch(const void* x, const void* residual, void* x_out,
   if (dim % 8 != 0 || dim > kNormMaxVec * 256) return cudaErrorInvalidValue;
   const unsigned grid = (unsigned)((rows + 7) / 8);
 #define DION_NORM_FWD(V)                                                                                          \
-  rmsnorm_fwd_kernel<V><<<grid, 256, 0, s>>>(reinterpret_cast<const bf16*>(x), reinterpret_cast<const bf16*>(residual), \
+  launch_pdl(rmsnorm_fwd_kernel<V>, dim3(grid), dim3(256), 0, s, 0, reinterpret_cast<const bf16*>(x), reinterpret_cast<const bf16*>(residual), \
                                              reinterpret_cast<bf16*>(x_out), reinterpret_cast<bf16*>(y), rstd, rows, \
                                              dim, eps)
   if (dim <= 4 * 256) DION_NORM_FWD(4);
@@ -661,7 +686,7 @@ cudaError_t rmsnorm_bwd_launch(const void* dy, const void* x, const float* rstd,
   if (dim % 8 != 0 || dim > kNormMaxVec * 256) return cudaErrorInvalidValue;
   const unsigned grid = (unsigned)((rows + 7) / 8);
 #define DION_NORM_BWD(V)                                                                                          \
-  rmsnorm_bwd_kernel<V><<<grid, 256, 0, s>>>(reinterpret_cast<const bf16*>(dy), reinterpret_cast<const bf16*>(x), rstd, \
+  launch_pdl(rmsnorm_bwd_kernel<V>, dim3(grid), dim3(256), 0, s, 0, reinterpret_cast<const bf16*>(dy), reinterpret_cast<const bf16*>(x), rstd, \
                                              reinterpret_cast<const bf16*>(dx_add), reinterpret_cast<bf16*>(dx), rows, dim)
   if (dim <= 4 * 256) DION_NORM_BWD(4);
   else if (dim <= 8 * 256) DION_NORM_BWD(8);
@@ -693,7 +718,7 @@ cudaError_t rope_qknorm_fwd_launch(const void* q, const void* k, void* q_out, vo
   const unsigned grid = wide ? (unsigned)((tokens * heads * (head_dim / 16) + 255) / 256)
                              : (unsigned)((nrows * (head_dim / 8) + 255) / 256);
 #define DION_ROPE_FWD(KERNEL, HD)                                                                                 \
-  KERNEL<HD><<<grid, 256, 0, s>>>(                                                                                \
+  launch_pdl(KERNEL<HD>, dim3(grid), dim3(256), 0, s, 0, \
       reinterpret_cast<const bf16*>(q), reinterpret_cast<const bf16*>(k), reinterpret_cast<bf16*>(q_out),         \
       reinterpret_cast<bf16*>(k_out), reinterpret_cast<const bf16*>(cos), reinterpret_cast<const bf16*>(sin),     \
       tokens, seq_len, heads, in_pitch, out_pitch, eps)
@@ -719,7 +744,7 @@ cudaError_t rope_qknorm_bwd_launch(const void* dq_out, const void* dk_out, const
   const unsigned grid = wide ? (unsigned)((tokens * heads * (head_dim / 16) + 255) / 256)
                              : (unsigned)((nrows * (head_dim / 8) + 255) / 256);
 #define DION_ROPE_BWD(KERNEL, HD)                                                                                 \
-  KERNEL<HD><<<grid, 256, 0, s>>>(                                                                                \
+  launch_pdl(KERNEL<HD>, dim3(grid), dim3(256), 0, s, 0, \
       reinterpret_cast<const bf16*>(dq_out), reinterpret_cast<const bf16*>(dk_out),                               \
       reinterpret_cast<const bf16*>(q), reinterpret_cast<const bf16*>(k), reinterpret_cast<bf16*>(dq),            \
       reinterpret_cast<bf16*>(dk), reinterpret_cast<const bf16*>(cos), reinterpret_cast<const bf16*>(sin),        \
@@ -739,7 +764,7 @@ cudaError_t relu2_fwd_launch(const void* x, void* h, long long n, cudaStream_t s
   if (n == 0) return cudaSuccess;
   if (n % 8 != 0) return cudaErrorInvalidValue;
   const long long nvec = n / 8;
-  relu2_fwd_kernel<<<(unsigned)((nvec + 255) / 256), 256, 0, s>>>(reinterpret_cast<const uint4*>(x),
+  launch_pdl(relu2_fwd_kernel, dim3((unsigned)((nvec + 255) / 256)), dim3(256), 0, s, 0, reinterpret_cast<const uint4*>(x),
                                                                  reinterpret_cast<uint4*>(h), nvec);
   return cudaGetLastError();
 }
@@ -747,8 +772,7 @@ cudaError_t relu2_bwd_launch(const void* dh, const void* x, void* dx, long long 
   if (n == 0) return cudaSuccess;
   if (n % 8 != 0) return cudaErrorInvalidValue;
   const long long nvec = n / 8;
-  relu2_bwd_kernel<<<(unsigned)((nvec + 255) / 256), 256, 0, s>>>(
-      reinterpret_cast<const uint4*>(dh), reinterpret_cast<const uint4*>(x), reinterpret_cast<uint4*>(dx), nvec);
+  launch_pdl(relu2_bwd_kernel, dim3((unsigned)((nvec + 255) / 256)), dim3(256), 0, s, 0, reinterpret_cast<const uint4*>(dh), reinterpret_cast<const uint4*>(x), reinterpret_cast<uint4*>(dx), nvec);
   return cudaGetLastError();
 }
 
@@ -757,7 +781,7 @@ cudaError_t cross_entropy_fwd_bwd_launch(void* logits, const long long* targets,
                                          float grad_scale, long long ignore_index, bool write_grad, cudaStream_t s) {
   if (rows == 0) return cudaSuccess;
   if (vocab % 8 != 0 || pitch % 8 != 0) return cudaErrorInvalidValue;
-  cross_entropy_kernel<<<(unsigned)rows, kCeThreads, 0, s>>>(reinterpret_cast<bf16*>(logits), targets, row_loss,
+  launch_pdl(cross_entropy_kernel, dim3((unsigned)rows), dim3(kCeThreads), 0, s, 0, reinterpret_cast<bf16*>(logits), targets, row_loss,
                                                             scale_ptr, vocab, pitch, grad_scale, ignore_index,
                                                             write_grad ? 1 : 0);
   return cudaGetLastError();
@@ -770,9 +794,9 @@ cudaError_t scale_by_scalar_launch(const void* x, void* y, int elem_type, long l
   long long grid = (n + 1023) / 1024;
   if (grid > 148 * 8) grid = 148 * 8;
   if (elem_type == kElemF32)
-    scale_by_scalar_kernel<false><<<(unsigned)grid, 256, 0, s>>>(x, y, n, vec, scale);
+    launch_pdl(scale_by_scalar_kernel<false>, dim3((unsigned)grid), dim3(256), 0, s, 0, x, y, n, vec, scale);
   else
-    scale_by_scalar_kernel<true><<<(unsigned)grid, 256, 0, s>>>(x, y, n, vec, scale);
+    launch_pdl(scale_by_scalar_kernel<true>, dim3((unsigned)grid), dim3(256), 0, s, 0, x, y, n, vec, scale);
   return cudaGetLastError();
 }
 
@@ -780,7 +804,7 @@ cudaError_t embedding_fwd_launch(const void* table, int table_type, const long l
                                  long long tokens, int dim, cudaStream_t s) {
   if (tokens == 0) return cudaSuccess;
   if (dim % 8 != 0) return cudaErrorInvalidValue;
-  embedding_fwd_kernel<<<(unsigned)((tokens + 7) / 8), 256, 0, s>>>(table, table_type, idx,
+  launch_pdl(embedding_fwd_kernel, dim3((unsigned)((tokens + 7) / 8)), dim3(256), 0, s, 0, table, table_type, idx,
                                                                    reinterpret_cast<bf16*>(out), tokens, dim);
   return cudaGetLastError();
 }
@@ -788,7 +812,7 @@ cudaError_t embedding_bwd_launch(const void* dout, const long long* idx, float* 
                                  cudaStream_t s) {
   if (tokens == 0) return cudaSuccess;
   if (dim % 2 != 0) return cudaErrorInvalidValue;
-  embedding_bwd_kernel<<<(unsigned)((tokens + 7) / 8), 256, 0, s>>>(reinterpret_cast<const bf16*>(dout), idx, dtable,
+  launch_pdl(embedding_bwd_kernel, dim3((unsigned)((tokens + 7) / 8)), dim3(256), 0, s, 0, reinterpret_cast<const bf16*>(dout), idx, dtable,
                                                                    tokens, dim);
   return cudaGetLastError();
 }

@@ -4,6 +4,7 @@
 #include <cuda_bf16.h>
 
 #include "kernels.h"
+#include "pdl.cuh"
 
 namespace dion {
 
@@ -84,6 +85,8 @@ __device__ __forceinline__ float sgn(float x) { return (x > 0.f) ? 1.f : ((x < 0
 
 __global__ void __launch_bounds__(kThreads) adamw_kernel(const __grid_constant__ TensorListChunk tl, int g_type,
                                                         int m_type, int v_type, int has_shadow, AdamWHyper h) {
+  pdl_trigger();
+  pdl_wait();
   const int t = find_tensor(tl, blockIdx.x);
   const long long n = tl.numel[t];
   const long long base = (long long)(blockIdx.x - tl.block_start[t]) * kBlockElems;
@@ -130,6 +133,8 @@ __global__ void __launch_bounds__(kThreads) adamw_kernel(const __grid_constant__
 
 __global__ void __launch_bounds__(kThreads) lion_kernel(const __grid_constant__ TensorListChunk tl, int g_type,
                                                        int m_type, int has_shadow, LionHyper h) {
+  pdl_trigger();
+  pdl_wait();
   const int t = find_tensor(tl, blockIdx.x);
   const long long n = tl.numel[t];
   const long long base = (long long)(blockIdx.x - tl.block_start[t]) * kBlockElems;
@@ -184,6 +189,8 @@ __device__ __forceinline__ float block_sum(float v) {
 
 __global__ void __launch_bounds__(kThreads) muon_pre_kernel(const __grid_constant__ TensorListChunk tl, int g_type,
                                                            float mu, int nesterov, float* sumsq) {
+  pdl_trigger();
+  pdl_wait();
   const int t = find_tensor(tl, blockIdx.x);
   const long long n = tl.numel[t];
   const long long base = (long long)(blockIdx.x - tl.block_start[t]) * kBlockElems;
@@ -225,6 +232,8 @@ __global__ void __launch_bounds__(kThreads) muon_pre_kernel(const __grid_constan
 
 __global__ void __launch_bounds__(kThreads) muon_post_kernel(const __grid_constant__ TensorListChunk tl,
                                                             int has_shadow, float decay, float step) {
+  pdl_trigger();
+  pdl_wait();
   const int t = find_tensor(tl, blockIdx.x);
   const long long n = tl.numel[t];
   const long long base = (long long)(blockIdx.x - tl.block_start[t]) * kBlockElems;
@@ -252,6 +261,8 @@ __global__ void __launch_bounds__(kThreads) muon_post_kernel(const __grid_consta
 
 __global__ void __launch_bounds__(kThreads) dion_accum_kernel(const __grid_constant__ TensorListChunk tl, int g_type,
                                                              int m_type, int* nonzero) {
+  pdl_trigger();
+  pdl_wait();
   const int t = find_tensor(tl, blockIdx.x);
   const long long n = tl.numel[t];
   const long long base = (long long)(blockIdx.x - tl.block_start[t]) * kBlockElems;
@@ -283,6 +294,8 @@ __global__ void __launch_bounds__(kThreads) dion_accum_kernel(const __grid_const
 
 __global__ void __launch_bounds__(kThreads) cast_kernel(const __grid_constant__ TensorListChunk tl, int src_type,
                                                        int dst_type) {
+  pdl_trigger();
+  pdl_wait();
   const int t = find_tensor(tl, blockIdx.x);
   const long long n = tl.numel[t];
   const long long base = (long long)(blockIdx.x - tl.block_start[t]) * kBlockElems;
@@ -302,6 +315,8 @@ constexpr int kFrobChunk = 16384;  // bf16 elements per block
 
 __global__ void __launch_bounds__(kThreads) frob_partial_kernel(const __nv_bfloat16* __restrict__ x,
                                                                float* __restrict__ partial, long long per, int nchunk) {
+  pdl_trigger();
+  pdl_wait();
   const long long b = blockIdx.y;
   const long long lo = (long long)blockIdx.x * kFrobChunk;
   const long long hi = min(per, lo + (long long)kFrobChunk);
@@ -336,6 +351,8 @@ __global__ void __launch_bounds__(kThreads) frob_scale_kernel(const __nv_bfloat1
                                                              __nv_bfloat16* __restrict__ out,
                                                              const float* __restrict__ partial, int npart,
                                                              const float* __restrict__ sumsq, float eps, long long per) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ float scale_s;
   const long long b = blockIdx.y;
   float acc = 0.f;
@@ -382,11 +399,11 @@ cudaError_t frob_scale_launch(const void* x, void* out, float* partial, const fl
   const int nchunk = frob_chunks(per);
   const dim3 grid(nchunk, batch);
   if (sumsq == nullptr) {
-    frob_partial_kernel<<<grid, kThreads, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(x), partial, per, nchunk);
+    launch_pdl(frob_partial_kernel, dim3(grid), dim3(kThreads), 0, s, 0, reinterpret_cast<const __nv_bfloat16*>(x), partial, per, nchunk);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
-  frob_scale_kernel<<<grid, kThreads, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(x),
+  launch_pdl(frob_scale_kernel, dim3(grid), dim3(kThreads), 0, s, 0, reinterpret_cast<const __nv_bfloat16*>(x),
                                               reinterpret_cast<__nv_bfloat16*>(out), partial, nchunk, sumsq, eps, per);
   return cudaGetLastError();
 }
@@ -394,36 +411,36 @@ cudaError_t frob_scale_launch(const void* x, void* out, float* partial, const fl
 cudaError_t adamw_multi_launch(const TensorListChunk& tl, int g_type, int m_type, int v_type, bool has_shadow,
                                const AdamWHyper& h, cudaStream_t s) {
   if (total_blocks(tl) == 0) return cudaSuccess;
-  adamw_kernel<<<total_blocks(tl), kThreads, 0, s>>>(tl, g_type, m_type, v_type, has_shadow ? 1 : 0, h);
+  launch_pdl(adamw_kernel, dim3(total_blocks(tl)), dim3(kThreads), 0, s, 0, tl, g_type, m_type, v_type, has_shadow ? 1 : 0, h);
   return cudaGetLastError();
 }
 cudaError_t lion_multi_launch(const TensorListChunk& tl, int g_type, int m_type, bool has_shadow,
                               const LionHyper& h, cudaStream_t s) {
   if (total_blocks(tl) == 0) return cudaSuccess;
-  lion_kernel<<<total_blocks(tl), kThreads, 0, s>>>(tl, g_type, m_type, has_shadow ? 1 : 0, h);
+  launch_pdl(lion_kernel, dim3(total_blocks(tl)), dim3(kThreads), 0, s, 0, tl, g_type, m_type, has_shadow ? 1 : 0, h);
   return cudaGetLastError();
 }
 cudaError_t muon_pre_multi_launch(const TensorListChunk& tl, int g_type, float mu, bool nesterov, float* sumsq,
                                   cudaStream_t s) {
   if (total_blocks(tl) == 0) return cudaSuccess;
-  muon_pre_kernel<<<total_blocks(tl), kThreads, 0, s>>>(tl, g_type, mu, nesterov ? 1 : 0, sumsq);
+  launch_pdl(muon_pre_kernel, dim3(total_blocks(tl)), dim3(kThreads), 0, s, 0, tl, g_type, mu, nesterov ? 1 : 0, sumsq);
   return cudaGetLastError();
 }
 cudaError_t muon_post_multi_launch(const TensorListChunk& tl, bool has_shadow, float decay, float step,
                                    cudaStream_t s) {
   if (total_blocks(tl) == 0) return cudaSuccess;
-  muon_post_kernel<<<total_blocks(tl), kThreads, 0, s>>>(tl, has_shadow ? 1 : 0, decay, step);
+  launch_pdl(muon_post_kernel, dim3(total_blocks(tl)), dim3(kThreads), 0, s, 0, tl, has_shadow ? 1 : 0, decay, step);
   return cudaGetLastError();
 }
 cudaError_t dion_accum_multi_launch(const TensorListChunk& tl, int g_type, int m_type, int* nonzero,
                                     cudaStream_t s) {
   if (total_blocks(tl) == 0) return cudaSuccess;
-  dion_accum_kernel<<<total_blocks(tl), kThreads, 0, s>>>(tl, g_type, m_type, nonzero);
+  launch_pdl(dion_accum_kernel, dim3(total_blocks(tl)), dim3(kThreads), 0, s, 0, tl, g_type, m_type, nonzero);
   return cudaGetLastError();
 }
 cudaError_t cast_multi_launch(const TensorListChunk& tl, int src_type, int dst_type, cudaStream_t s) {
   if (total_blocks(tl) == 0) return cudaSuccess;
-  cast_kernel<<<total_blocks(tl), kThreads, 0, s>>>(tl, src_type, dst_type);
+  launch_pdl(cast_kernel, dim3(total_blocks(tl)), dim3(kThreads), 0, s, 0, tl, src_type, dst_type);
   return cudaGetLastError();
 }
 

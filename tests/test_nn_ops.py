@@ -361,6 +361,49 @@ def test_flash_attention_work_split(shape):
 
 
 @pytest.mark.gpu
+def test_overlapping_launches_in_a_graph_and_between_streams():
+    """Kernels that start before their predecessor has ended: a chain of this library's kernels and torch's, eagerly,
+    captured in a graph and with its halves on two streams, gives the same bits."""
+    from dion_b200.ops.nn import flash_attention_forward
+
+    g = torch.Generator(device="cuda").manual_seed(3)
+    w1, w2 = (torch.randn(512, 512, device="cuda", generator=g).bfloat16() * 0.05 for _ in range(2))
+
+    def first(x, buf):
+        buf.zero_()                                    # a plain launch before, between and after
+        buf.add_(x)
+        h = N.linear(N.rms_norm(buf), w1)
+        q = h.view(2, 128, 8, 64)
+        return N.linear(flash_attention_forward(q, q, q)[0].view(256, 512), w2)
+
+    def second(y):
+        return N.linear(torch.relu(N.rms_norm(y)), w1) + y
+
+    with torch.no_grad():
+        xs = [torch.randn(256, 512, device="cuda", generator=g).bfloat16() for _ in range(3)]
+        buf = torch.empty_like(xs[0])
+        want = [second(first(x, buf)).clone() for x in xs]
+        x0 = xs[0].clone()
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            got = second(first(x0, buf))
+        for x, w in zip(xs, want):
+            x0.copy_(x)
+            graph.replay()
+            assert torch.equal(got, w)
+        side = torch.cuda.Stream()
+        for x, w in zip(xs, want):
+            y = first(x, buf)
+            side.wait_stream(torch.cuda.current_stream())
+            with torch.cuda.stream(side):
+                z = second(y)
+            torch.cuda.current_stream().wait_stream(side)
+            y.record_stream(side)
+            assert torch.equal(z, w)
+
+
+@pytest.mark.gpu
 def test_linear_fanout_matches_separate_linears():
     x = torch.randn(640, 256, device="cuda").to(torch.bfloat16).requires_grad_()
     ws = [torch.nn.Parameter(torch.randn(n, 256, device="cuda") * 0.05) for n in (256, 128, 384)]

@@ -1375,9 +1375,14 @@ bool attn_tmap_seq(CUtensorMap* map, const void* base, uint64_t cols, uint64_t T
   cuuint64_t strides[2] = {cols * 2, T * cols * 2};
   cuuint32_t box[3] = {64, kBM, 1};
   cuuint32_t estr[3] = {1, 1, 1};
-  return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+  auto encode = [&] {
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  };
+  CUresult r = encode();
+  if (r == CUDA_ERROR_INVALID_CONTEXT && bind_primary_context()) r = encode();  // the first call of a thread
+  return r == CUDA_SUCCESS;
 }
 
 // CTAs of a persistent kernel with one CTA per SM

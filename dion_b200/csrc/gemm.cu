@@ -1477,13 +1477,17 @@ bool make_tmap(CUtensorMap* map, const void* base, int dtype, uint64_t inner, ui
     slot->valid = false;
     slot->key = key;
   }
-  CUresult r = fn(map, dtype == kBF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3,
+  auto encode = [&] {
+    return fn(map, dtype == kBF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3,
                   const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                   swizzle == kSwizzleNone        ? CU_TENSOR_MAP_SWIZZLE_NONE
                   : swizzle == kSwizzle128Atom32 ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B
                                                  : CU_TENSOR_MAP_SWIZZLE_128B,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  };
+  CUresult r = encode();
+  if (r == CUDA_ERROR_INVALID_CONTEXT && bind_primary_context()) r = encode();  // the first call of a thread
   if (r != CUDA_SUCCESS) {
     char buf[160];
     snprintf(buf, sizeof(buf), "cuTensorMapEncodeTiled failed with code %d", (int)r);

@@ -142,4 +142,11 @@ void gemm_plan(const GemmArgs& args, int (&out)[4]);
 // rows per readiness counter, copy units per counter, first m-tile of the schedule, m-tiles, n-tiles}.
 bool gemm_gather_plan(const GemmArgs& args, int (&out)[8]);
 
+// Makes the current device's primary context current on the calling thread, which a driver call needs and only a runtime
+// call brings about: a backward pass may begin on a thread that has made none.
+inline bool bind_primary_context() {
+  int dev = 0;
+  return cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess;
+}
+
 }  // namespace dion

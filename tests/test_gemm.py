@@ -612,3 +612,33 @@ def test_two_streams_at_a_time_give_the_bits_of_one():
         for outs in got[i]:
             assert all(torch.equal(a, b) for a, b in zip(outs, want[i]))
     ops.check_status()
+
+
+@pytest.mark.gpu
+def test_first_call_of_a_thread():
+    """A thread that has made no CUDA call yet, as a backward pass may meet it, starts with a product or with attention."""
+    import threading
+
+    from dion_b200.ops import runtime
+
+    a, b = (torch.randn(256, 256, device="cuda").bfloat16() for _ in range(2))
+    q = torch.randn(1, 128, 2, 64, device="cuda").bfloat16()
+    lse, status = torch.empty(1, 2, 128, device="cuda"), runtime.status_tensor(a.device)
+    outs, errors = [torch.empty_like(a), torch.empty_like(q)], []
+
+    def run(f):
+        try:
+            f()
+        except Exception as e:  # noqa: BLE001 - handed to the test's thread
+            errors.append(e)
+
+    torch.cuda.synchronize()
+    for f in (lambda: gemm(a, b, out=outs[0]),
+              lambda: torch.ops.dion_b200.attn_fwd(q, q, q, outs[1], lse, 0.125, status)):
+        t = threading.Thread(target=run, args=(f,))
+        t.start()
+        t.join()
+    torch.cuda.synchronize()
+    assert not errors, errors
+    assert torch.equal(outs[0], gemm(a, b, out=torch.empty_like(a)))
+    assert outs[1].isfinite().all()

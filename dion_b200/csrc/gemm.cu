@@ -379,8 +379,10 @@ __device__ __forceinline__ bool mbar_wait_for(uint64_t* bar, uint32_t parity, vo
 // owns a 4 KB buffer, one box of 32 rows x 128 bytes: the C box is fetched into it (the first of a tile while the accumulator is
 // still being multiplied), replaced in place by the result and stored from it.  The path with generic loads and stores takes 4.6 us
 // for a 128 x 256 tile and 8.2 us with C, more than the multiply of K = 768 (5.6 us) that should hide it.
+// kF32Out (with kTmaEpi, bf16 operands, fp32 D, no C): boxes of 32 columns, stored or added to D by the copy engine
+// (kEpiAtomicAdd).  One atomic per element, a row per lane, touched 32 lines per instruction.
 template <bool kTf32, int kAMajor, int kBMajor, int kBlockN, bool kPair, bool kGather = false, bool kSplit = false,
-          bool kClusterK = false, bool kTmaEpi = false>
+          bool kClusterK = false, bool kTmaEpi = false, bool kF32Out = false>
 __global__ void __launch_bounds__(kNumThreads + (kGather ? kNumGatherThreads : 0) + (kSplit ? kNumSplitThreads : 0), 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
             const __grid_constant__ CUtensorMap tmap_a_lo, const __grid_constant__ CUtensorMap tmap_b_lo,
@@ -388,6 +390,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   // kTmaEpi: the slots of the low halves hold the maps of D and C, tmap_mirror the map of D for transposed boxes
   static_assert(!(kSplit && kGather), "the converter warps and the copier warps use the same warp slots");
   static_assert(!kTmaEpi || (!kGather && !kClusterK && kBlockN >= 128), "TMA epilogue: 128- and 256-column tiles");
+  static_assert(!kF32Out || (kTmaEpi && !kTf32), "fp32 results by TMA: of bf16 operands");
   static_assert(!kClusterK || (kSplit && kBlockN == 128), "K ranges over a cluster: splitting variants, 128-column tiles");
   using C = Cfg<kTf32, kAMajor, kBMajor, kBlockN, kPair, kSplit>;
   extern __shared__ uint8_t smem_raw[];
@@ -794,12 +797,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   } else if constexpr (kTmaEpi) {
     // ------------------------------------------------------------------ epilogue, C and D by TMA
     const int quad = warp & 3;
-    constexpr int kBoxCols = 128 / C::ES;                // C and D have the operands' element size
+    constexpr bool kF32D = kTf32 || kF32Out;
+    constexpr int kBoxCols = kF32D ? 32 : 64;            // 128 bytes of D (and C)
     constexpr int kBoxes = kBlockN / 2 / kBoxCols;       // per warp and tile
     uint8_t* st = stage_area + (warp - 2) * kStageBytes;
     uint64_t* cb = &c_bar[warp - 2];
     uint32_t c_phase = 0;
-    const bool use_c = p.C != nullptr;
+    const bool use_c = !kF32Out && p.C != nullptr;
+    const bool add = kF32Out && p.epilogue == kEpiAtomicAdd;
     auto fetch_c = [&](int col, int row, int batch) {
       if (lane == 0) {
         tma_store_wait_read();  // the box stored last has left the buffer
@@ -877,7 +882,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
 #pragma unroll
           for (int i = 0; i < kBoxCols; ++i) v[i] = apply_act(v[i], kActRelu2);
         }
-        if (use_c) {
+        if constexpr (!kF32Out) if (use_c) {
           if (!wait(cb, c_phase)) {
             ok = false;
             *abort_flag = 1;
@@ -934,7 +939,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
         // this lane's row over the C row it has just read
 #pragma unroll
         for (int s = 0; s < 8; ++s) {
-          if constexpr (kTf32) {
+          if constexpr (kF32D) {
             *reinterpret_cast<float4*>(st + stage_off(lane, s)) = make_float4(v[4 * s], v[4 * s + 1], v[4 * s + 2], v[4 * s + 3]);
           } else {
             uint4 q;
@@ -947,13 +952,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
         fence_proxy_async_shared();
         __syncwarp();
         if (lane == 0) {
-          tma_store_3d(&tmap_a_lo, st, col, row0, t.batch);
+          if (add) tma_add_f32_3d(&tmap_a_lo, st, col, row0, t.batch);
+          else tma_store_3d(&tmap_a_lo, st, col, row0, t.batch);
           tma_store_commit();
         }
-        if (mirror) {
+        if (!kF32Out && mirror) {
           // the block transposed, 64 (bf16) or 32 (fp32) rows of 32: every lane parks its row as a column
           buffer_free();
-          if constexpr (kTf32) {
+          if constexpr (kF32D) {
 #pragma unroll
             for (int i = 0; i < 32; ++i) *reinterpret_cast<float*>(st + stage_off(i, lane >> 2) + (lane & 3) * 4) = v[i];
           } else {
@@ -1513,7 +1519,7 @@ int num_sms() {
 }
 
 template <bool kTf32, int kAMajor, int kBMajor, int kBlockN, bool kPair = false, bool kGather = false, bool kSplit = false,
-          bool kClusterK = false, bool kTmaEpi = false>
+          bool kClusterK = false, bool kTmaEpi = false, bool kF32Out = false>
 cudaError_t launch_cfg(const GemmArgs& a, const KernelParams& kp, cudaStream_t stream) {
   using C = Cfg<kTf32, kAMajor, kBMajor, kBlockN, kPair, kSplit>;
   CUtensorMap ta, tb, ta_lo, tb_lo;
@@ -1536,16 +1542,17 @@ cudaError_t launch_cfg(const GemmArgs& a, const KernelParams& kp, cudaStream_t s
   }
   CUtensorMap tm = ta;  // never read
   if constexpr (kTmaEpi) {
-    if (!make_tmap(&ta_lo, a.D, dt, a.N, a.M, a.batch, a.ldd, a.d_batch_stride, 128 / C::ES, 32, kSwizzle128))
+    const int dd = kF32Out ? kF32 : dt;
+    if (!make_tmap(&ta_lo, a.D, dd, a.N, a.M, a.batch, a.ldd, a.d_batch_stride, dd == kF32 ? 32 : 64, 32, kSwizzle128))
       return cudaErrorInvalidValue;
-    if (a.C && !make_tmap(&tb_lo, a.C, dt, a.N, a.M, a.batch, a.ldc, a.c_batch_stride, 128 / C::ES, 32, kSwizzle128))
+    if (!kF32Out && a.C && !make_tmap(&tb_lo, a.C, dt, a.N, a.M, a.batch, a.ldc, a.c_batch_stride, 128 / C::ES, 32, kSwizzle128))
       return cudaErrorInvalidValue;
     if (a.B_more[0] && (!map_b(&tb_lo, a.B_more[0]) || !map_b(&tm, a.B_more[1]))) return cudaErrorInvalidValue;
-    if (!kTf32 && a.symmetric && !make_tmap(&tm, a.D, kBF16, a.N, a.M, a.batch, a.ldd, a.d_batch_stride, 32, 64, kSwizzleNone))
+    if (!kTf32 && !kF32Out && a.symmetric && !make_tmap(&tm, a.D, kBF16, a.N, a.M, a.batch, a.ldd, a.d_batch_stride, 32, 64, kSwizzleNone))
       return cudaErrorInvalidValue;
   }
 
-  auto kernel = gemm_kernel<kTf32, kAMajor, kBMajor, kBlockN, kPair, kGather, kSplit, kClusterK, kTmaEpi>;
+  auto kernel = gemm_kernel<kTf32, kAMajor, kBMajor, kBlockN, kPair, kGather, kSplit, kClusterK, kTmaEpi, kF32Out>;
   constexpr int kThreads = kNumThreads + (kGather ? kNumGatherThreads : 0) + (kSplit ? kNumSplitThreads : 0);
   static bool attr_set = false;
   if (!attr_set) {
@@ -1606,6 +1613,16 @@ bool tma_epilogue(const GemmArgs& a) {
          a.ldd >= a.N && (!a.C || a.ldc >= a.N) && a.N % (bf16 ? 8 : 4) == 0 && (!a.C || (a.c_dtype == a.ab_dtype && vec_c_ok(a))) &&
          (a.batch == 1 || (a.d_batch_stride != 0 && (!a.C || a.c_batch_stride != 0)));
 }
+// bf16 operands with fp32 results that TMA can store or add: one destination, whole 16-byte rows, no addend but D itself.
+// Weight gradients above all.  768 x 768, K = 65536 in 24 parts: 70.8 us with a row per lane and vector atomics, 63.4 us;
+// 3072 x 768 in 6 parts 218 and 215; 768 x 768, K = 1024, plain stores: 18.4 and 14.6.
+bool tma_f32_out(const GemmArgs& a) {
+  const bool adds = a.epilogue == kEpiAtomicAdd;
+  return stage_enabled() && a.ab_dtype == kBF16 && a.d_dtype == kF32 && (adds || a.epilogue == kEpiStore) && !a.symmetric && !a.A_lo &&
+         (adds || ((!a.C || a.beta == 0.f) && !a.c_ptrs)) && !a.c_col_scale && !a.d_ptrs && !a.D2 && !a.d2_ptrs && a.scatter_mode == 0 &&
+         a.gather.world == 0 && !a.B_more[0] && (a.act == 0 || (a.act == kActRelu2 && !adds)) && vec_d_ok(a) && a.D && a.ldd >= a.N &&
+         a.N % 4 == 0 && (a.batch == 1 || a.d_batch_stride != 0);
+}
 // C is read only where it counts
 KernelParams tma_params(const KernelParams& kp) {
   KernelParams kt = kp;
@@ -1621,6 +1638,13 @@ cudaError_t launch_bn(const GemmArgs& a, const KernelParams& kp, int bn, bool pa
       if (pair) return launch_cfg<kTf32, kAMajor, kBMajor, 256, true, false, false, false, true>(a, kt, s);
       if (bn == 128) return launch_cfg<kTf32, kAMajor, kBMajor, 128, false, false, false, false, true>(a, kt, s);
       return launch_cfg<kTf32, kAMajor, kBMajor, 256, false, false, false, false, true>(a, kt, s);
+    }
+  }
+  if constexpr (!kTf32 && kBMajor == kMajorMN) {
+    if (bn >= 128 && tma_f32_out(a)) {
+      if (pair) return launch_cfg<false, kAMajor, kBMajor, 256, true, false, false, false, true, true>(a, kp, s);
+      if (bn == 128) return launch_cfg<false, kAMajor, kBMajor, 128, false, false, false, false, true, true>(a, kp, s);
+      return launch_cfg<false, kAMajor, kBMajor, 256, false, false, false, false, true, true>(a, kp, s);
     }
   }
   if (pair) return launch_cfg<kTf32, kAMajor, kBMajor, 256, true>(a, kp, s);

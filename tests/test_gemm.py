@@ -615,6 +615,47 @@ def test_two_streams_at_a_time_give_the_bits_of_one():
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("M,N,K,split_k,batch", [
+    (128, 256, 64, 1, 1),        # one tile
+    (300, 260, 200, 1, 2),       # rows and columns that fill no box, batches
+    (129, 132, 1000, 3, 1),      # parts of unequal length
+    (768, 768, 4096, 4, 1),      # pairs
+    (1000, 516, 2056, 2, 1),
+    (256, 250, 512, 2, 1),       # rows of 1000 bytes: the generic epilogue
+])
+@pytest.mark.parametrize("ta", [False, True])
+@pytest.mark.parametrize("mode", ["store", "relu2", "add", "slice"])
+def test_fp32_results_of_bf16_operands_by_tma(M, N, K, split_k, batch, ta, mode):
+    """Stored or added to D by the copy engine.  Products of bf16 are exact in fp32 and the sums run in fp32: against fp64
+    K * 2^-24 of the largest partial sum bounds the error; 1e-5 of the result's largest value lies above that here."""
+    if mode in ("store", "relu2", "slice") and split_k > 1:
+        pytest.skip("parts are added")
+    if ta and M % 8:
+        pytest.skip("rows of A^T are not whole 16 bytes")
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    lead = (batch,) if batch > 1 else ()
+    n_pad = (N + 7) // 8 * 8
+    a = torch.randn(*lead, *((K, M) if ta else (M, K)), device="cuda", generator=g).bfloat16()
+    b = torch.randn(*lead, K, n_pad, device="cuda", generator=g).bfloat16()[..., :N]
+    a = a.transpose(-1, -2) if ta else a
+    want = a.double() @ b.double()
+    if mode == "add":
+        out = torch.randn(*lead, M, N, device="cuda", generator=g)
+        want = out.double() + 0.5 * want
+        gemm(a, b, out=out, alpha=0.5, accumulate=True, split_k=split_k)
+    elif mode == "slice":
+        whole = torch.full((*lead, M, N + 24), 7.0, device="cuda")
+        out = whole[..., 8:8 + N]
+        gemm(a, b, out=out)
+        assert (whole[..., :8] == 7).all() and (whole[..., 8 + N:] == 7).all()
+    else:
+        out = torch.empty(*lead, M, N, device="cuda")
+        gemm(a, b, out=out, act=None if mode == "store" else "relu2")
+        want = want if mode == "store" else want.clamp_min(0).square()
+    assert (out.double() - want).abs().max().item() <= 1e-5 * want.abs().max().item()
+
+
+@pytest.mark.gpu
 def test_first_call_of_a_thread():
     """A thread that has made no CUDA call yet, as a backward pass may meet it, starts with a product or with attention."""
     import threading

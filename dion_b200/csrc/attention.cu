@@ -544,6 +544,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     const f32x2 s2 = pack2(p.scale_log2, p.scale_log2);
     auto wait = [&](uint64_t* bar, uint32_t parity) {
       if (!mbar_wait(bar, parity, abort_flag)) *abort_flag = 1;
+      __syncwarp();  // the tensor-memory accesses that follow take the whole warp at once
     };
     uint32_t ph = 0;  // of the tile at hand: s_full, s_free, p_full, pv_done
     for (; work.valid;) {
@@ -764,9 +765,10 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   uint64_t* q_empty = bars + 1;
   uint64_t* sdp_full = bars + 2;
   uint64_t* sdp_free = bars + 3;  // softmax warps: S and dP are in registers
-  uint64_t* ds_full = bars + 4;   // softmax warps
-  uint64_t* dq_full = bars + 5;
-  uint64_t* k_full = bars + 6;    // K_STAGES each
+  uint64_t* ds_full = bars + 4;   // softmax warps; one per buffer of dS: a warp may deliver the next tile's before another
+                                  // has delivered this one's, as S and dP are released before dS is formed
+  uint64_t* dq_full = bars + 6;
+  uint64_t* k_full = bars + 7;    // K_STAGES each
   uint64_t* k_empty = k_full + C::K_STAGES;
   uint64_t* v_full = k_empty + C::K_STAGES;  // V_STAGES each
   uint64_t* v_empty = v_full + C::V_STAGES;
@@ -788,7 +790,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     tma_prefetch_desc(&tmap_do);
     tma_prefetch_desc(&tmap_k);
     tma_prefetch_desc(&tmap_v);
-    for (uint64_t* b = bars; b < bars_end; ++b) mbar_init(b, (b == sdp_free || b == ds_full) ? 8 : 1);
+    for (uint64_t* b = bars; b < bars_end; ++b) mbar_init(b, (b >= sdp_free && b < dq_full) ? 8 : 1);
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -850,19 +852,19 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         bool ok = true;
         Ring<C::K_STAGES> ks, ka;  // S; dQ
         Ring<C::V_STAGES> vs;
-        uint32_t ph = 0, ph_a = 0;
-        // dQ of the tile before: its dS lies in buffer ph_a
+        uint32_t ph = 0, n_a = 0;  // parity of the next S; dQ products so far
+        // dQ of the tile before: its dS lies in buffer n_a & 1
         auto accumulate = [&](bool fresh, bool last) -> bool {
-          if (!mbar_wait(ds_full, ph_a, abort_flag)) return false;
+          if (!mbar_wait(&ds_full[n_a & 1], (n_a >> 1) & 1, abort_flag)) return false;
           tc_fence_after();
 #pragma unroll
           for (int kk = 0; kk < kBM / 16; ++kk)
-            umma_ts_h(tmem_base + C::DQ_COL, tmem_base + C::DS_COL + ph_a * 64 + kk * 8, dkm_,
+            umma_ts_h(tmem_base + C::DQ_COL, tmem_base + C::DS_COL + (n_a & 1) * 64 + kk * 8, dkm_,
                       ka.s * C::TILE_BYTES + kk * (16 * 128), idesc_dq, (!fresh || kk > 0) ? 1u : 0u);
           umma_commit(&k_empty[ka.s]);
           if (last) umma_commit(dq_full);
           ka.next();
-          ph_a ^= 1u;
+          ++n_a;
           return true;
         };
         int behind = 0;  // kv tiles of the query tile before whose dQ is outstanding: its last one
@@ -914,6 +916,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     const f32x2 scale2 = pack2(p.scale_log2, p.scale_log2), out_scale2 = pack2(p.scale, p.scale);
     auto wait = [&](uint64_t* bar, uint32_t parity) {
       if (!mbar_wait(bar, parity, abort_flag)) *abort_flag = 1;
+      __syncwarp();  // the tensor-memory accesses that follow take the whole warp at once
     };
     uint32_t ph = 0;
     for (int r = 0; work.valid; ++r) {
@@ -957,7 +960,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(ds_full);
+        if (lane == 0) mbar_arrive(&ds_full[ph]);
         ph ^= 1u;
       }
       work.next();
@@ -1212,13 +1215,13 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
           tc_fence_after();
           accumulate(C::DV_COL, C::P_COL, C::P_STEP, ddo_, os.s * C::TILE_BYTES, i == 0);
           umma_commit(dv_done);
-          umma_commit(&do_empty[os.s]);
           ok = mbar_wait(ds_full, ph, abort_flag);
           if (!ok) break;
           tc_fence_after();
           accumulate(C::DK_COL, C::DP_COL, 32, dq_, qs.s * C::TILE_BYTES, i == 0);
           umma_commit(dk_done);
           umma_commit(&q_empty[qs.s]);
+          umma_commit(&do_empty[os.s]);  // not before: the softmax read delta_i from this stage up to its dS^T
           if (i == n - 1) umma_commit(acc_full);
           ph ^= 1u;
           qs.next();
@@ -1241,6 +1244,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     const f32x2 scale2 = pack2(p.scale_log2, p.scale_log2), out_scale2 = pack2(p.scale, p.scale);
     auto wait = [&](uint64_t* bar, uint32_t parity) {
       if (!mbar_wait(bar, parity, abort_flag)) *abort_flag = 1;
+      __syncwarp();  // the tensor-memory accesses that follow take the whole warp at once
     };
     Ring<C::Q_STAGES> qs;
     Ring<C::DO_STAGES> os;
@@ -1507,9 +1511,7 @@ cudaError_t attn_bwd_launch(const void* q, const void* k, const void* v, const v
 
 cudaError_t attn_fwd_launch(const void* q, const void* k, const void* v, void* out, float* lse, int B, int T, int H,
                             int Hkv, int D, float scale, int* status, cudaStream_t stream) {
-  if (B <= 0 || T <= 0 || H <= 0 || Hkv <= 0 || H % Hkv != 0 || B * H > 65535) return cudaErrorInvalidValue;
-  // the TMA boxes of one sequence must not run into the next one: whole kv tiles per sequence
-  if (T % kBM != 0) return cudaErrorInvalidValue;
+  if (B <= 0 || T <= 0 || H <= 0 || Hkv <= 0 || H % Hkv != 0 || B * H > 65535 || T % kBM != 0) return cudaErrorInvalidValue;
   if (D == 128) return attn_fwd_launch_d<128>(q, k, v, out, lse, B, T, H, Hkv, scale, status, stream);
   if (D == 64) return attn_fwd_launch_d<64>(q, k, v, out, lse, B, T, H, Hkv, scale, status, stream);
   return cudaErrorInvalidValue;

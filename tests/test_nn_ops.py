@@ -361,6 +361,24 @@ def test_flash_attention_work_split(shape):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(64, 384, 6, 6, 128), (64, 512, 6, 3, 64), (2, 2048, 16, 4, 128)])
+def test_flash_attention_gives_the_same_bits_in_every_run(shape):
+    """No sum depends on the order in which warps or CTAs run, so a difference between two runs is a race."""
+    from dion_b200.ops.nn import flash_attention_backward, flash_attention_forward
+
+    B, T, H, Hkv, D = shape
+    g = torch.Generator(device="cuda").manual_seed(23)
+    q, k, v, d_out = (torch.randn(B, T, h, D, device="cuda", generator=g).to(torch.bfloat16) for h in (H, Hkv, Hkv, H))
+    first = None
+    for _ in range(8):
+        out, lse = flash_attention_forward(q, k, v)
+        run = (out, lse, *flash_attention_backward(q, k, v, out, lse, d_out))
+        first = first or run
+        for name, a, b in zip(("out", "lse", "dq", "dk", "dv"), first, run):
+            assert torch.equal(a, b), name
+
+
+@pytest.mark.gpu
 def test_overlapping_launches_in_a_graph_and_between_streams():
     """Kernels that start before their predecessor has ended: a chain of this library's kernels and torch's, eagerly,
     captured in a graph and with its halves on two streams, gives the same bits."""

@@ -826,6 +826,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       bool mirror = p.symmetric && t.m_blk != t.n_blk;
       // boxes of this warp that lie inside the matrix (a box that only overlaps it is clipped by the copy)
       int boxes = row0 < p.M ? min(kBoxes, max(0, (p.N - col0 + kBoxCols - 1) / kBoxCols)) : 0;
+      // with more parts of K than blocks to go round the last ones are empty: nothing was multiplied, nothing is added
+      if (kF32Out && t.split * kb_per_split >= p.kblocks_total) boxes = 0;
       if constexpr (kSplit && kPair) {
         // On a diagonal tile the lower left quarter (the peer's rows, the first half of the columns) is the mirror of the
         // upper right one, as it is between 128 x 128 tiles: computed by itself its cross terms would be added the other

@@ -621,6 +621,8 @@ def test_two_streams_at_a_time_give_the_bits_of_one():
     (129, 132, 1000, 3, 1),      # parts of unequal length
     (768, 768, 4096, 4, 1),      # pairs
     (1000, 516, 2056, 2, 1),
+    (384, 384, 16384, 17, 1),    # 17 parts of 16 blocks for 256 blocks: the last one is empty
+    (256, 128, 1024, 7, 2),      # 6 parts of 3 blocks would do for 16
     (256, 250, 512, 2, 1),       # rows of 1000 bytes: the generic epilogue
 ])
 @pytest.mark.parametrize("ta", [False, True])

@@ -1500,7 +1500,7 @@ cudaError_t attn_bwd_launch_d(const void* q, const void* k, const void* v, const
 cudaError_t attn_bwd_launch(const void* q, const void* k, const void* v, const void* o, const void* d_o,
                             const float* lse, float* stats, void* dq, void* dk, void* dv, int B, int T, int H, int Hkv,
                             int D, float scale, int* status, cudaStream_t stream) {
-  if (B <= 0 || T <= 0 || H <= 0 || Hkv <= 0 || H % Hkv != 0 || B * H > 65535 || T % kBM != 0)
+  if (B <= 0 || T <= 0 || H <= 0 || Hkv <= 0 || H % Hkv != 0 || B * H > 65535)
     return cudaErrorInvalidValue;
   if (D == 128)
     return attn_bwd_launch_d<128>(q, k, v, o, d_o, lse, stats, dq, dk, dv, B, T, H, Hkv, scale, status, stream);
@@ -1511,7 +1511,7 @@ cudaError_t attn_bwd_launch(const void* q, const void* k, const void* v, const v
 
 cudaError_t attn_fwd_launch(const void* q, const void* k, const void* v, void* out, float* lse, int B, int T, int H,
                             int Hkv, int D, float scale, int* status, cudaStream_t stream) {
-  if (B <= 0 || T <= 0 || H <= 0 || Hkv <= 0 || H % Hkv != 0 || B * H > 65535 || T % kBM != 0) return cudaErrorInvalidValue;
+  if (B <= 0 || T <= 0 || H <= 0 || Hkv <= 0 || H % Hkv != 0 || B * H > 65535) return cudaErrorInvalidValue;
   if (D == 128) return attn_fwd_launch_d<128>(q, k, v, out, lse, B, T, H, Hkv, scale, status, stream);
   if (D == 64) return attn_fwd_launch_d<64>(q, k, v, out, lse, B, T, H, Hkv, scale, status, stream);
   return cudaErrorInvalidValue;

@@ -1098,7 +1098,7 @@ Tensor gpt_block_fwd(const Tensor& x, const Tensor& wq, const Tensor& wk, const 
     Tensor qo = at::empty_like(q), ko = at::empty_like(k);
     rope_qknorm_fwd(q, k, qo, ko, cos, sin, T, heads, D, eps);
     const Tensor q4 = qo.view({B, T, heads, D}), k4 = ko.view({B, T, heads, D}), v4 = v.view({B, T, heads, D});
-    if (kernel_attention && T % 128 == 0 && B * heads <= 65535) {
+    if (kernel_attention && T > 0 && B * heads <= 65535) {
       y = at::empty_like(q4);
       Tensor lse = at::empty({B, heads, T}, x.options().dtype(at::kFloat));
       attn_fwd(q4, k4, v4, y, lse, 1. / std::sqrt((double)D), status);

@@ -130,8 +130,7 @@ cudaError_t chol_inverse_launch(const float* G, float* Rinv, float* work, int* i
 cudaError_t col_sumsq_launch(const void* X, int x_type, float* out, int batch, long long rows, int cols,
                              long long ldx, long long batch_stride, cudaStream_t s);
 // Causal flash attention forward on tcgen05: q [B*T, H*D], k / v [B*T, Hkv*D], out [B*T, H*D] bf16,
-// lse [B, H, T] fp32 (natural log of the softmax denominator, for the backward pass); D is 64 or 128,
-// T a multiple of 128.
+// lse [B, H, T] fp32 (natural log of the softmax denominator, for the backward pass); D is 64 or 128.
 cudaError_t attn_fwd_launch(const void* q, const void* k, const void* v, void* out, float* lse, int B, int T, int H,
                             int Hkv, int D, float scale, int* status, cudaStream_t stream);
 // Backward of the same attention: dq [B*T, H*D], dk / dv [B*T, Hkv*D] (bf16) from q, k, v, the forward's

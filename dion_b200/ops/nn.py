@@ -682,9 +682,7 @@ def linear_cross_entropy(x: torch.Tensor, weight: torch.Tensor, targets: torch.T
 
 # --------------------------------------------------------------------------- attention
 
-def flash_attention_forward(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, scale: Optional[float] = None):
-    """Causal attention forward by the tcgen05 kernel.  q: [B, T, H, D], k / v: [B, T, Hkv, D], bf16,
-    contiguous, D in {64, 128}, T a multiple of 128.  Returns (out [B, T, H, D], lse [B, H, T])."""
+def _attention_forward(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, scale: Optional[float] = None):
     B, T, H, D = q.shape
     if scale is None:
         scale = 1.0 / math.sqrt(D)
@@ -693,6 +691,29 @@ def flash_attention_forward(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, s
     lse = torch.empty(B, H, T, dtype=torch.float32, device=q.device)
     torch.ops.dion_b200.attn_fwd(q, k, v, out, lse, float(scale), runtime.status_tensor(q.device))
     return out, lse
+
+
+def _attention_backward(q, k, v, out, lse, d_out, scale: Optional[float] = None):
+    B, T, H, D = q.shape
+    if scale is None:
+        scale = 1.0 / math.sqrt(D)
+    dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
+    stats = torch.empty(2, B, H, (T + 127) // 128 * 128, dtype=torch.float32, device=q.device)
+    torch.ops.dion_b200.attn_bwd(q, k, v, out, d_out.contiguous(), lse, stats, dq, dk, dv, float(scale),
+                                 runtime.status_tensor(q.device))
+    return dq, dk, dv
+
+
+def _whole_tiles(q: torch.Tensor) -> None:
+    if q.shape[1] % 128:
+        raise RuntimeError(f"flash attention takes sequences of a multiple of 128, not {q.shape[1]}; see causal_attention")
+
+
+def flash_attention_forward(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, scale: Optional[float] = None):
+    """Causal attention forward by the tcgen05 kernel.  q: [B, T, H, D], k / v: [B, T, Hkv, D], bf16,
+    contiguous, D in {64, 128}, T a multiple of 128.  Returns (out [B, T, H, D], lse [B, H, T])."""
+    _whole_tiles(q)
+    return _attention_forward(q, k, v, scale)
 
 
 def flash_attention_supported(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor) -> bool:
@@ -704,27 +725,44 @@ def flash_attention_supported(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor)
 
 def flash_attention_backward(q, k, v, out, lse, d_out, scale: Optional[float] = None):
     """Gradients of :func:`flash_attention_forward` by the tcgen05 kernels: (dq, dk, dv)."""
-    B, T, H, D = q.shape
-    if scale is None:
-        scale = 1.0 / math.sqrt(D)
-    dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-    stats = torch.empty(2, B, H, (T + 127) // 128 * 128, dtype=torch.float32, device=q.device)
-    torch.ops.dion_b200.attn_bwd(q, k, v, out, d_out.contiguous(), lse, stats, dq, dk, dv, float(scale),
-                                 runtime.status_tensor(q.device))
-    return dq, dk, dv
+    _whole_tiles(q)
+    return _attention_backward(q, k, v, out, lse, d_out, scale)
 
 
 class _FlashAttnFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, v):
-        out, lse = flash_attention_forward(q, k, v)
+        out, lse = _attention_forward(q, k, v)
         ctx.save_for_backward(q, k, v, out, lse)
         return out
 
     @staticmethod
     def backward(ctx, d_out):
         q, k, v, out, lse = ctx.saved_tensors
-        return flash_attention_backward(q, k, v, out, lse, d_out)
+        return _attention_backward(q, k, v, out, lse, d_out)
+
+
+class _FlashAttnAnyLengthFn(_FlashAttnFn):
+    """Lengths that fill no tile.  A second derivative raises, as that of the library's kernels does."""
+
+    @staticmethod
+    @torch.autograd.function.once_differentiable
+    def backward(ctx, d_out):
+        q, k, v, out, lse = ctx.saved_tensors
+        if d_out.is_contiguous() and d_out.data_ptr() % 16:
+            d_out = d_out.clone()
+        return _attention_backward(q, k, v, out, lse, d_out)
+
+
+def _any_length(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor) -> bool:
+    """Contiguous q, k, v of a length that is no multiple of 128, in a plain call: rows beyond the sequence are read as
+    zeros and masked.  What a tracer, a mode or a transform looks at, and other shapes and types, go to the library.
+    8 x 777, 12 heads of 64: 26 us against 36, with the backward pass 65 against 81; 24 tokens, 6 heads of 128: 14 against 18."""
+    B, T, H, D = q.shape
+    return (q.dtype == k.dtype == v.dtype == torch.bfloat16 and D in (64, 128) and q.numel() > 0 and k.numel() > 0
+            and k.dim() == 4 and k.shape[:2] == q.shape[:2] and k.shape[3] == D and v.shape == k.shape
+            and H % k.shape[2] == 0 and B * H <= 65535 and not torch.compiler.is_compiling() and not _observed()
+            and not any(_transformed(t) for t in (q, k, v)))
 
 
 # "kernel": the in-tree tcgen05 kernels wherever they apply; "library": always
@@ -741,6 +779,9 @@ def causal_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor) -> torch
         q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
         if flash_attention_supported(q, k, v):
             return _FlashAttnFn.apply(q, k, v).view(B, T, H * Dh)
+        if T % 128 and _any_length(q, k, v):
+            q, k, v = (t.clone() if t.data_ptr() % 16 else t for t in (q, k, v))
+            return _FlashAttnAnyLengthFn.apply(q, k, v).view(B, T, H * Dh)
     qt, kt, vt = q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2)
     y = F.scaled_dot_product_attention(qt, kt, vt, is_causal=True, enable_gqa=(Hkv != H))
     return y.transpose(1, 2).reshape(B, T, H * Dh)

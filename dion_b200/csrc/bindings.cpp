@@ -92,7 +92,8 @@ bool gemm(const Tensor& a, const Tensor& b, const std::optional<Tensor>& c, Tens
           const std::optional<Tensor>& d_ptrs, const std::optional<Tensor>& d2_ptrs, double alpha, double beta,
           int64_t act, int64_t epilogue, int64_t split_k, bool symmetric, int64_t block_n, int64_t pair,
           const std::optional<Tensor>& status, int64_t d_dup, const std::optional<Tensor>& a_lo,
-          const std::optional<Tensor>& b_lo, const std::optional<Tensor>& c_col_scale, bool split3) {
+          const std::optional<Tensor>& b_lo, const std::optional<Tensor>& c_col_scale, bool split3,
+          std::vector<int64_t> x_ptrs = {}) {
   TORCH_CHECK(a.is_cuda() && b.is_cuda(), "gemm operands must be CUDA tensors");
   TORCH_CHECK(a.scalar_type() == b.scalar_type(), "gemm operands must share a dtype");
   TORCH_CHECK(a.dim() == b.dim(), "gemm operands must both be 2-D or both 3-D");
@@ -182,6 +183,11 @@ bool gemm(const Tensor& a, const Tensor& b, const std::optional<Tensor>& c, Tens
     }
     g.D2 = t.data_ptr();
     g.ldd2 = t.stride(-2);
+  }
+  if (!x_ptrs.empty()) {
+    TORCH_CHECK(d_ptrs.has_value() && c_ptrs.has_value() && (int64_t)x_ptrs.size() == g.batch && g.C == g.D,
+                "x_ptrs: the addresses of c_ptrs and d_ptrs, one per batch element");
+    g.x_ptrs = x_ptrs.data();
   }
   if (status.has_value()) {
     TORCH_CHECK(status->scalar_type() == at::kInt && status->is_cuda());
@@ -1256,7 +1262,7 @@ TORCH_LIBRARY(dion_b200, m) {
       "gemm(Tensor a, Tensor b, Tensor? c, Tensor(a!) d, Tensor(b!)? d2, Tensor? c_ptrs, Tensor? d_ptrs, "
       "Tensor? d2_ptrs, float alpha, float beta, int act, int epilogue, int split_k, bool symmetric, "
       "int block_n, int pair, Tensor? status, int d_dup=1, Tensor? a_lo=None, Tensor? b_lo=None, "
-      "Tensor? c_col_scale=None, bool split3=False) -> bool");
+      "Tensor? c_col_scale=None, bool split3=False, int[] x_ptrs=[]) -> bool");
   m.def(
       "newton_schulz_steps(Tensor X, Tensor? sumsq, float eps, float[] coeffs, bool tall, Tensor status) -> Tensor");
   m.def(

@@ -381,16 +381,26 @@ __device__ __forceinline__ bool mbar_wait_for(uint64_t* bar, uint32_t parity, vo
 // for a 128 x 256 tile and 8.2 us with C, more than the multiply of K = 768 (5.6 us) that should hide it.
 // kF32Out (with kTmaEpi, bf16 operands, fp32 D, no C): boxes of 32 columns, stored or added to D by the copy engine
 // (kEpiAtomicAdd).  One atomic per element, a row per lane, touched 32 lines per instruction.
+// kPtrs (with kTmaEpi, fp32 C and D in one place): every batch element is a matrix of its own allocation with its own map.
+constexpr int kMaxMaps = 32;
+template <bool kPtrs>
+struct MapTable {
+  CUtensorMap m[kPtrs ? kMaxMaps : 1];
+};
+template <>
+struct MapTable<false> {};
+
 template <bool kTf32, int kAMajor, int kBMajor, int kBlockN, bool kPair, bool kGather = false, bool kSplit = false,
-          bool kClusterK = false, bool kTmaEpi = false, bool kF32Out = false>
+          bool kClusterK = false, bool kTmaEpi = false, bool kF32Out = false, bool kPtrs = false>
 __global__ void __launch_bounds__(kNumThreads + (kGather ? kNumGatherThreads : 0) + (kSplit ? kNumSplitThreads : 0), 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
             const __grid_constant__ CUtensorMap tmap_a_lo, const __grid_constant__ CUtensorMap tmap_b_lo,
-            const __grid_constant__ CUtensorMap tmap_mirror, const KernelParams p) {
+            const __grid_constant__ CUtensorMap tmap_mirror, const __grid_constant__ MapTable<kPtrs> maps, const KernelParams p) {
   // kTmaEpi: the slots of the low halves hold the maps of D and C, tmap_mirror the map of D for transposed boxes
   static_assert(!(kSplit && kGather), "the converter warps and the copier warps use the same warp slots");
   static_assert(!kTmaEpi || (!kGather && !kClusterK && kBlockN >= 128), "TMA epilogue: 128- and 256-column tiles");
   static_assert(!kF32Out || (kTmaEpi && !kTf32), "fp32 results by TMA: of bf16 operands");
+  static_assert(!kPtrs || (kTmaEpi && (kTf32 || kF32Out)), "matrices of their own: fp32, by TMA");
   static_assert(!kClusterK || (kSplit && kBlockN == 128), "K ranges over a cluster: splitting variants, 128-column tiles");
   using C = Cfg<kTf32, kAMajor, kBMajor, kBlockN, kPair, kSplit>;
   extern __shared__ uint8_t smem_raw[];
@@ -803,13 +813,17 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     uint8_t* st = stage_area + (warp - 2) * kStageBytes;
     uint64_t* cb = &c_bar[warp - 2];
     uint32_t c_phase = 0;
-    const bool use_c = !kF32Out && p.C != nullptr;
+    const bool use_c = p.C != nullptr;
     const bool add = kF32Out && p.epilogue == kEpiAtomicAdd;
+    auto d_map = [&](int batch) -> const CUtensorMap* {
+      if constexpr (kPtrs) return &maps.m[batch];
+      else return &tmap_a_lo;
+    };
     auto fetch_c = [&](int col, int row, int batch) {
       if (lane == 0) {
         tma_store_wait_read();  // the box stored last has left the buffer
         mbar_arrive_expect_tx(cb, kStageBytes);
-        tma_load_3d(st, &tmap_b_lo, cb, col, row, batch);
+        tma_load_3d(st, kPtrs ? d_map(batch) : &tmap_b_lo, cb, col, row, kPtrs ? 0 : batch);
       }
     };
     auto buffer_free = [&] {
@@ -884,7 +898,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
 #pragma unroll
           for (int i = 0; i < kBoxCols; ++i) v[i] = apply_act(v[i], kActRelu2);
         }
-        if constexpr (!kF32Out) if (use_c) {
+        if (use_c) {
           if (!wait(cb, c_phase)) {
             ok = false;
             *abort_flag = 1;
@@ -892,11 +906,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
             break;
           }
           c_phase ^= 1u;
-          if constexpr (kTf32) {
+          if constexpr (kF32D) {
             // every lane reads the same factors (a broadcast load per factor); the splitting variants have no registers to
             // spare for them and leave such products to the generic epilogue
             const float* cs =
-                !kSplit && p.c_col_scale != nullptr ? p.c_col_scale + (long long)t.batch * p.N + col : nullptr;
+                kTf32 && !kSplit && p.c_col_scale != nullptr ? p.c_col_scale + (long long)t.batch * p.N + col : nullptr;
 #pragma unroll
             for (int s = 0; s < 8; ++s) {
               const float4 q = *reinterpret_cast<const float4*>(st + stage_off(lane, s));
@@ -955,8 +969,23 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
         __syncwarp();
         if (lane == 0) {
           if (add) tma_add_f32_3d(&tmap_a_lo, st, col, row0, t.batch);
-          else tma_store_3d(&tmap_a_lo, st, col, row0, t.batch);
+          else tma_store_3d(d_map(t.batch), st, col, row0, kPtrs ? 0 : t.batch);
           tma_store_commit();
+        }
+        if constexpr (kPtrs) {
+          if (p.d2_ptrs != nullptr) {  // the bf16 copy of the box
+            __nv_bfloat16* d2 = reinterpret_cast<__nv_bfloat16*>(p.d2_ptrs[t.batch]);
+            if (col + 32 <= p.N && p.vec_d2) {
+              buffer_free();
+              stage_put_bf16(st, lane, 0, v);
+              __syncwarp();
+              stage_flush<4>(st, lane, row0, p.M, [&](int grow) { return reinterpret_cast<char*>(d2 + (long long)grow * p.ldd2 + col); });
+              fence_proxy_async_shared();  // the next box may be fetched over what was just read
+              __syncwarp();
+            } else if (row0 + lane < p.M) {
+              store_chunk_bf16(d2 + (long long)(row0 + lane) * p.ldd2 + col, v, false, p.N - col);
+            }
+          }
         }
         if (!kF32Out && mirror) {
           // the block transposed, 64 (bf16) or 32 (fp32) rows of 32: every lane parks its row as a column
@@ -1521,7 +1550,7 @@ int num_sms() {
 }
 
 template <bool kTf32, int kAMajor, int kBMajor, int kBlockN, bool kPair = false, bool kGather = false, bool kSplit = false,
-          bool kClusterK = false, bool kTmaEpi = false, bool kF32Out = false>
+          bool kClusterK = false, bool kTmaEpi = false, bool kF32Out = false, bool kPtrs = false>
 cudaError_t launch_cfg(const GemmArgs& a, const KernelParams& kp, cudaStream_t stream) {
   using C = Cfg<kTf32, kAMajor, kBMajor, kBlockN, kPair, kSplit>;
   CUtensorMap ta, tb, ta_lo, tb_lo;
@@ -1545,16 +1574,24 @@ cudaError_t launch_cfg(const GemmArgs& a, const KernelParams& kp, cudaStream_t s
   CUtensorMap tm = ta;  // never read
   if constexpr (kTmaEpi) {
     const int dd = kF32Out ? kF32 : dt;
-    if (!make_tmap(&ta_lo, a.D, dd, a.N, a.M, a.batch, a.ldd, a.d_batch_stride, dd == kF32 ? 32 : 64, 32, kSwizzle128))
+    if (!kPtrs && !make_tmap(&ta_lo, a.D, dd, a.N, a.M, a.batch, a.ldd, a.d_batch_stride, dd == kF32 ? 32 : 64, 32, kSwizzle128))
       return cudaErrorInvalidValue;
-    if (!kF32Out && a.C && !make_tmap(&tb_lo, a.C, dt, a.N, a.M, a.batch, a.ldc, a.c_batch_stride, 128 / C::ES, 32, kSwizzle128))
+    if (!kF32Out && !kPtrs && a.C && !make_tmap(&tb_lo, a.C, dt, a.N, a.M, a.batch, a.ldc, a.c_batch_stride, 128 / C::ES, 32, kSwizzle128))
       return cudaErrorInvalidValue;
     if (a.B_more[0] && (!map_b(&tb_lo, a.B_more[0]) || !map_b(&tm, a.B_more[1]))) return cudaErrorInvalidValue;
     if (!kTf32 && !kF32Out && a.symmetric && !make_tmap(&tm, a.D, kBF16, a.N, a.M, a.batch, a.ldd, a.d_batch_stride, 32, 64, kSwizzleNone))
       return cudaErrorInvalidValue;
   }
 
-  auto kernel = gemm_kernel<kTf32, kAMajor, kBMajor, kBlockN, kPair, kGather, kSplit, kClusterK, kTmaEpi, kF32Out>;
+  MapTable<kPtrs> maps;
+  if constexpr (kPtrs) {
+    for (int i = 0; i < a.batch; ++i)
+      if (!make_tmap(&maps.m[i], reinterpret_cast<const void*>(a.x_ptrs[i]), kF32, a.N, a.M, 1, a.ldd, 0, 32, 32, kSwizzle128))
+        return cudaErrorInvalidValue;
+    for (int i = a.batch; i < kMaxMaps; ++i) maps.m[i] = maps.m[0];  // never read
+  }
+
+  auto kernel = gemm_kernel<kTf32, kAMajor, kBMajor, kBlockN, kPair, kGather, kSplit, kClusterK, kTmaEpi, kF32Out, kPtrs>;
   constexpr int kThreads = kNumThreads + (kGather ? kNumGatherThreads : 0) + (kSplit ? kNumSplitThreads : 0);
   static bool attr_set = false;
   if (!attr_set) {
@@ -1568,30 +1605,30 @@ cudaError_t launch_cfg(const GemmArgs& a, const KernelParams& kp, cudaStream_t s
     grid /= cluster;  // one tile per cluster at a time
     if (grid > kp.total_tiles || kClusterK) grid = kp.total_tiles;
     if (grid < 1) grid = 1;
-    return launch_pdl(kernel, dim3(cluster * grid), dim3(kThreads), C::SMEM_BYTES, stream, cluster, ta, tb, ta_lo, tb_lo, tm, kp);
+    return launch_pdl(kernel, dim3(cluster * grid), dim3(kThreads), C::SMEM_BYTES, stream, cluster, ta, tb, ta_lo, tb_lo, tm, maps, kp);
   } else {
     if (grid > kp.total_tiles) grid = kp.total_tiles;
     if constexpr (kGather) {  // waits for other ranks' kernels: launched when the kernels before it are done
-      kernel<<<grid, kThreads, C::SMEM_BYTES, stream>>>(ta, tb, ta_lo, tb_lo, tm, kp);
+      kernel<<<grid, kThreads, C::SMEM_BYTES, stream>>>(ta, tb, ta_lo, tb_lo, tm, maps, kp);
       return cudaGetLastError();
     }
-    return launch_pdl(kernel, dim3(grid), dim3(kThreads), C::SMEM_BYTES, stream, 0, ta, tb, ta_lo, tb_lo, tm, kp);
+    return launch_pdl(kernel, dim3(grid), dim3(kThreads), C::SMEM_BYTES, stream, 0, ta, tb, ta_lo, tb_lo, tm, maps, kp);
   }
 }
 
 bool aligned16(const void* p, long long ld, int es) {
   return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && ((ld * es) & 15) == 0;
 }
-// 16-byte vector access to C and D: aligned bases and pitches.  Per-batch pointer arrays and scattered blocks satisfy
-// this by contract (checked by the Python wrapper).
+// 16-byte vector access to C and D: aligned bases and pitches.  The addresses in per-batch pointer arrays and those of
+// scattered blocks satisfy this by contract (checked by the Python wrapper); their pitch need not.
 bool vec_c_ok(const GemmArgs& a) {
   const int es = a.c_dtype == kBF16 ? 2 : 4;
-  return (a.c_ptrs || aligned16(a.C, a.ldc, es)) && (a.c_batch_stride * es) % 16 == 0;
+  return aligned16(a.c_ptrs ? nullptr : a.C, a.ldc, es) && (a.c_batch_stride * es) % 16 == 0;
 }
 bool vec_d_ok(const GemmArgs& a) {
   const int es = a.d_dtype == kBF16 ? 2 : 4;
   if (a.scatter_mode != 0) return (a.ldd * es) % 16 == 0;
-  return (a.d_ptrs || aligned16(a.D, a.ldd, es)) && (a.d_batch_stride * es) % 16 == 0;
+  return aligned16(a.d_ptrs ? nullptr : a.D, a.ldd, es) && (a.d_batch_stride * es) % 16 == 0;
 }
 // DION_B200_GEMM_STAGE=0: every epilogue with direct accesses
 bool stage_enabled() {
@@ -1625,6 +1662,19 @@ bool tma_f32_out(const GemmArgs& a) {
          a.gather.world == 0 && !a.B_more[0] && (a.act == 0 || (a.act == kActRelu2 && !adds)) && vec_d_ok(a) && a.D && a.ldd >= a.N &&
          a.N % 4 == 0 && (a.batch == 1 || a.d_batch_stride != 0);
 }
+// Matrices that are allocations of their own, updated in place (X = beta X + alpha A B, GemmArgs::x_ptrs): a map per matrix lets
+// TMA move them too, with the same bits.  4 x 14336 x 4096, rank 512: 710 us by staged loads and stores, 540; with bf16 factors
+// 705 and 404; 48 x 768 x 768, rank 96, bf16 factors and copies: 104 and 75; 12 x 3072 x 768, rank 96: 89 and 59.
+bool tma_ptrs(const GemmArgs& a) {
+  if (!a.x_ptrs || !stage_enabled() || a.d_dtype != kF32 || a.epilogue != kEpiStore || a.act != 0 || a.symmetric || a.split_k != 1 ||
+      a.A_lo || a.split3 || a.scatter_mode != 0 || a.gather.world > 0 || a.c_col_scale || a.B_more[0] || a.a_major != kMajorK ||
+      a.b_major != kMajorK || a.N % 4 != 0 || a.N <= 64 || (a.block_n != 0 && a.block_n < 128) || a.d_dup > 1 || a.ldd < a.N ||
+      a.ldd % 4 != 0 || (a.C && (a.c_dtype != kF32 || a.ldc != a.ldd)) || (a.D2 != nullptr) != (a.d2_ptrs != nullptr))
+    return false;
+  for (int i = 0; i < a.batch; ++i)
+    if (a.x_ptrs[i] & 15) return false;
+  return true;
+}
 // C is read only where it counts
 KernelParams tma_params(const KernelParams& kp) {
   KernelParams kt = kp;
@@ -1642,11 +1692,21 @@ cudaError_t launch_bn(const GemmArgs& a, const KernelParams& kp, int bn, bool pa
       return launch_cfg<kTf32, kAMajor, kBMajor, 256, false, false, false, false, true>(a, kt, s);
     }
   }
+  if constexpr (kAMajor == kMajorK && kBMajor == kMajorK) {
+    if (bn >= 128 && tma_ptrs(a)) {
+      const KernelParams kt = tma_params(kp);
+      if (pair) return launch_cfg<kTf32, kAMajor, kBMajor, 256, true, false, false, false, true, !kTf32, true>(a, kt, s);
+      if (bn == 128) return launch_cfg<kTf32, kAMajor, kBMajor, 128, false, false, false, false, true, !kTf32, true>(a, kt, s);
+      return launch_cfg<kTf32, kAMajor, kBMajor, 256, false, false, false, false, true, !kTf32, true>(a, kt, s);
+    }
+  }
   if constexpr (!kTf32 && kBMajor == kMajorMN) {
     if (bn >= 128 && tma_f32_out(a)) {
-      if (pair) return launch_cfg<false, kAMajor, kBMajor, 256, true, false, false, false, true, true>(a, kp, s);
-      if (bn == 128) return launch_cfg<false, kAMajor, kBMajor, 128, false, false, false, false, true, true>(a, kp, s);
-      return launch_cfg<false, kAMajor, kBMajor, 256, false, false, false, false, true, true>(a, kp, s);
+      KernelParams kt = kp;
+      kt.C = nullptr;
+      if (pair) return launch_cfg<false, kAMajor, kBMajor, 256, true, false, false, false, true, true>(a, kt, s);
+      if (bn == 128) return launch_cfg<false, kAMajor, kBMajor, 128, false, false, false, false, true, true>(a, kt, s);
+      return launch_cfg<false, kAMajor, kBMajor, 256, false, false, false, false, true, true>(a, kt, s);
     }
   }
   if (pair) return launch_cfg<kTf32, kAMajor, kBMajor, 256, true>(a, kp, s);
@@ -1901,6 +1961,23 @@ bool gemm_gather_plan(const GemmArgs& a, int (&out)[8]) {
 }
 
 cudaError_t gemm_launch(const GemmArgs& a, cudaStream_t stream) {
+  if (a.batch > kMaxMaps && tma_ptrs(a)) {  // the maps of a launch travel with its parameters
+    const long long es = a.ab_dtype == kF32 ? 4 : 2;
+    for (int b0 = 0; b0 < a.batch; b0 += kMaxMaps) {
+      GemmArgs part = a;
+      part.batch = a.batch - b0 < kMaxMaps ? a.batch - b0 : kMaxMaps;
+      part.A = static_cast<const char*>(a.A) + b0 * a.a_batch_stride * es;
+      part.B = static_cast<const char*>(a.B) + b0 * a.b_batch_stride * es;
+      part.x_ptrs = a.x_ptrs + b0;
+      if (a.c_ptrs) part.c_ptrs = a.c_ptrs + b0;
+      if (a.d_ptrs) part.d_ptrs = a.d_ptrs + b0;
+      if (a.d2_ptrs) part.d2_ptrs = a.d2_ptrs + b0;
+      const cudaError_t e = gemm_launch(part, stream);
+      if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+  }
+
   g_last_error.clear();
   if (a.M <= 0 || a.N <= 0 || a.K <= 0 || a.batch <= 0 || a.split_k <= 0) {
     g_last_error = "GEMM sizes must be positive";
@@ -2007,7 +2084,7 @@ cudaError_t gemm_launch(const GemmArgs& a, cudaStream_t stream) {
   kp.status = a.status;
   kp.vec_c = vec_c_ok(a);
   kp.vec_d = vec_d_ok(a);
-  kp.vec_d2 = (a.d2_ptrs || aligned16(a.D2, a.ldd2, 2)) && ((a.d2_batch_stride * 2) % 16 == 0);
+  kp.vec_d2 = aligned16(a.d2_ptrs ? nullptr : a.D2, a.ldd2, 2) && ((a.d2_batch_stride * 2) % 16 == 0);
   kp.stage = stage_enabled();
 
   if (a.gather.world > 0) {

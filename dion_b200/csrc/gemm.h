@@ -90,6 +90,8 @@ struct GemmArgs {
   int scatter_block = 0;
   int scatter_dests = 0;
   void* const* scatter_ptrs = nullptr;
+  // Host copy of the addresses in c_ptrs and d_ptrs where both name the same matrices (X updated in place)
+  const int64_t* x_ptrs = nullptr;
   int block_n = 0;  // 0 = choose automatically (64 / 128 / 256)
   int max_ctas = 0;  // 0 = one CTA per SM
   // Three products of one A with three matrices laid out like B (bf16, K-major both, no C): batch is 3, B belongs to batch

@@ -80,7 +80,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, c: Optional[torch.Tensor] = None, 
          block_n: int = 0, pair: int = 0, out_ptrs: Optional[torch.Tensor] = None, c_ptrs: Optional[torch.Tensor] = None,
          shadow_ptrs: Optional[torch.Tensor] = None, out_dup: int = 1, a_lo: Optional[torch.Tensor] = None,
          b_lo: Optional[torch.Tensor] = None, c_col_scale: Optional[torch.Tensor] = None,
-         split3: bool = False) -> torch.Tensor:
+         split3: bool = False, host_ptrs: Optional[list] = None) -> torch.Tensor:
     """``out = act(alpha * a @ b + beta * c)``.
 
     a: ``[B,] M, K``; b: ``[B,] K, N``; each may be a transposed view (one unit stride in
@@ -91,6 +91,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, c: Optional[torch.Tensor] = None, 
     one device address per batch element, for outputs that are separate allocations.
     With ``out_dup = k > 1`` every batch element is stored to k destinations, ``out_ptrs[b * k + j]``
     (for instance one slot of a symmetric buffer on each rank of a group).
+    ``host_ptrs``: the addresses of ``out_ptrs`` as a list, where ``c_ptrs`` is the same table (matrices updated in place);
+    the kernel then moves them with TMA.
     ``a_lo`` / ``b_lo`` (fp32, laid out like ``a`` / ``b``): ``a`` and ``b`` are then the tf32-exact high
     halves of split operands and the product is ``a @ b + a_lo @ b + a @ b_lo`` accumulated in one pass
     over three K-segments - a 3xTF32 product in a single launch.
@@ -135,7 +137,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, c: Optional[torch.Tensor] = None, 
 
     if torch.ops.dion_b200.gemm(a, b, c, out, shadow, c_ptrs, out_ptrs, shadow_ptrs, float(alpha), float(beta),
                                 _ACT[act], 1 if accumulate else 0, int(split_k), bool(symmetric), int(block_n), int(pair),
-                                runtime.status_tensor(a.device), int(out_dup), a_lo, b_lo, c_col_scale, bool(split3)):
+                                runtime.status_tensor(a.device), int(out_dup), a_lo, b_lo, c_col_scale, bool(split3),
+                                host_ptrs if host_ptrs is not None and c_ptrs is out_ptrs and out is c else []):
         return out
     # shapes TMA cannot address (pitch not a multiple of 16 bytes): library GEMM
     if out_ptrs is not None or c_ptrs is not None or shadow_ptrs is not None:

@@ -196,8 +196,9 @@ def foreach_baddbmm_(X: List[Tensor], A: Tensor, B: Tensor, alpha: float = 1.0, 
             and a_op.dtype in (torch.float32, torch.bfloat16)
             and all(x.is_contiguous() and x.data_ptr() % 16 == 0 for x in Xl) and (x0.shape[-1] * 4) % 16 == 0)
     if fast:
-        ptrs = torch.tensor([x.data_ptr() for x in Xl], dtype=torch.int64, device=x0.device)
-        ops.gemm(a_op, b_op, c=x0, out=x0, c_ptrs=ptrs, out_ptrs=ptrs, alpha=float(alpha), beta=float(beta))
+        addresses = [x.data_ptr() for x in Xl]
+        ptrs = torch.tensor(addresses, dtype=torch.int64, device=x0.device)
+        ops.gemm(a_op, b_op, c=x0, out=x0, c_ptrs=ptrs, out_ptrs=ptrs, alpha=float(alpha), beta=float(beta), host_ptrs=addresses)
         return
     prod = ops.gemm(a_op, b_op, out_dtype=torch.float32) if a_op.is_cuda and a_op.dtype == b_op.dtype else \
         torch.matmul(a_op.float(), b_op.float())

@@ -658,6 +658,40 @@ def test_fp32_results_of_bf16_operands_by_tma(M, N, K, split_k, batch, ta, mode)
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("B,M,N,K", [(1, 128, 256, 64), (3, 131, 260, 96), (33, 256, 132, 40), (40, 96, 768, 200), (2, 520, 1000, 64),
+                                     (2, 300, 64, 64)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("copies", [False, True])
+def test_updates_in_place_through_maps_of_their_own(B, M, N, K, dtype, copies):
+    """More matrices than one launch has maps for, sizes that fill no box, bf16 copies whose rows are not 16 bytes wide, an
+    address TMA cannot take, beta = 0 over NaN: the bits of the path with staged loads and stores."""
+    g = torch.Generator(device="cuda").manual_seed(B + M + N + K)
+    P, R = (torch.randn(B, n, K, device="cuda", generator=g).to(dtype) for n in (M, N))
+    start = torch.randn(B, M, N, device="cuda", generator=g)
+
+    def run(host, beta, shift=0):
+        X = [torch.empty(M * N + 4, device="cuda")[shift:shift + M * N].view(M, N).copy_(x if beta else float("nan") * x)
+             for x in start]
+        S = [torch.zeros(M, N, device="cuda", dtype=torch.bfloat16) for _ in X]
+        addresses = [x.data_ptr() for x in X]
+        ptrs = torch.tensor(addresses, device="cuda")
+        kw = dict(shadow=S[0], shadow_ptrs=torch.tensor([s.data_ptr() for s in S], device="cuda")) if copies else {}
+        gemm(P, R.transpose(1, 2), c=X[0], out=X[0], c_ptrs=ptrs, out_ptrs=ptrs, alpha=-0.3, beta=beta,
+             host_ptrs=addresses if host else None, **kw)
+        return X + (S if copies else [])
+
+    for beta, shift in ((0.9, 0), (0.0, 0), (0.9, 1)):
+        if shift and (N * 4) % 16 == 0:
+            shift = 4  # still aligned: other addresses than the first time
+        for a, b in zip(run(True, beta, shift), run(False, beta, shift)):
+            assert torch.equal(a, b) and a.isfinite().all()
+    want = 0.9 * start.double() - 0.3 * (P.double() @ R.double().transpose(1, 2))
+    bound = 1e-5 if dtype == torch.bfloat16 else 2.0 ** -9  # tf32 operands: 10 bits
+    for a, w in zip(run(True, 0.9), want):
+        assert (a.double() - w).abs().max().item() <= bound * w.abs().max().item()
+
+
+@pytest.mark.gpu
 def test_first_call_of_a_thread():
     """A thread that has made no CUDA call yet, as a backward pass may meet it, starts with a product or with attention."""
     import threading

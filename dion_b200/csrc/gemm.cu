@@ -421,7 +421,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   volatile int* gather_word = abort_flag + 1;  // broadcast slot of the copier warps
   uint8_t* stage_area = bar_area + 1024;  // 128B-swizzled boxes start on 1024 bytes
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = (int)warp_uniform(threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   // CTA pair: rank 0 leads (issues the MMAs, owns the full / tmem_empty barriers in use)
   uint32_t cta_rank = 0;
@@ -474,7 +474,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   __syncthreads();
   if constexpr (kPair) cluster_sync_all();  // both CTAs' barriers and TMEM exist before either is used
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
   // debug build: the allocation lies inside the 512 columns of tensor memory
   if (threadIdx.x == 0) (void)DION_DBG_OK((tmem_base & 0xffffu) + C::TMEM_COLS <= 512u, p.status);
 
@@ -490,7 +490,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
 
   if (warp == 0) {
     // ------------------------------------------------------------------ producer
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -580,8 +580,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0 && cta_rank == 0) {
+    if (cta_rank == 0 && elect_one()) {
       constexpr uint32_t idesc = make_instr_desc(kTf32 ? 2 : 1, kAMajor, kBMajor, C::TILE_M, kBlockN);
+      // Descriptors of stage 0; the others differ in the address field alone (units of 16 bytes, no carry below 256 KB).  Put
+      // together afresh for every MMA they took longer than the splitting variants' multiplies.
+      const uint64_t desc_a0 = make_smem_desc(smem_u32(smem), C::A_LBO, C::A_SBO, C::A_LAYOUT);
+      const uint64_t desc_b0 = make_smem_desc(smem_u32(smem), C::B_LBO, C::B_SBO, C::B_LAYOUT);
       int stage = 0;
       uint32_t phase = 0;
       int it = 0;
@@ -623,15 +627,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
             break;
           }
           tc_fence_after();
-          const uint32_t sa = smem_u32(smem + stage * C::STAGE_STRIDE);
-          const uint32_t sb = sa + b_off;
+          const uint64_t desc_a = desc_a0 + (uint32_t)((stage * C::STAGE_STRIDE) >> 4);
+          const uint64_t desc_b = desc_b0 + (uint32_t)((stage * C::STAGE_STRIDE + b_off) >> 4);
 #pragma unroll
           for (int j = 0; j < C::KSTEPS; ++j) {
-            const uint64_t da = make_smem_desc(sa + j * C::A_KSTEP, C::A_LBO, C::A_SBO, C::A_LAYOUT);
-            const uint64_t db = make_smem_desc(sb + j * C::B_KSTEP, C::B_LBO, C::B_SBO, C::B_LAYOUT);
+            const uint64_t da = desc_a + ((j * C::A_KSTEP) >> 4);
+            const uint64_t db = desc_b + ((j * C::B_KSTEP) >> 4);
             if constexpr (kSplit) {
-              const uint64_t da_lo = make_smem_desc(sa + C::LO_OFFSET + j * C::A_KSTEP, C::A_LBO, C::A_SBO, C::A_LAYOUT);
-              const uint64_t db_lo = make_smem_desc(sb + C::LO_OFFSET + j * C::B_KSTEP, C::B_LBO, C::B_SBO, C::B_LAYOUT);
+              const uint64_t da_lo = da + (C::LO_OFFSET >> 4);
+              const uint64_t db_lo = db + (C::LO_OFFSET >> 4);
               const uint32_t first = (!fresh || j > 0) ? 1u : 0u;
               auto mma = [&](uint32_t d, uint64_t x, uint64_t y, uint32_t accumulate) {
                 if constexpr (kPair) umma_ss_pair<true>(d, x, y, idesc, accumulate);

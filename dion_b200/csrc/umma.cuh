@@ -123,6 +123,17 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
   }
 }
 
+// One lane of a converged warp.  tcgen05.mma takes its descriptors from uniform registers: issued by a thread of a
+// divergent branch (`if (lane == 0)`) every MMA costs about 63 cycles, whatever its shape; with the whole warp running
+// the loop and one elected lane issuing, 8 MMAs of 128 x 64 x 16 go out in 285 cycles (48 each when both operands
+// come from shared memory, 32 when A comes from tensor memory: the rates of the tensor core itself).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(p));
+  return p != 0;
+}
+// a value that is the same in all lanes, in a form the compiler can keep in a uniform register
+__device__ __forceinline__ uint32_t warp_uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
 // ----------------------------------------------------------------------------
 // TMA (tiled bulk tensor loads, never multicast)
 // ----------------------------------------------------------------------------

@@ -201,6 +201,51 @@ bool gemm(const Tensor& a, const Tensor& b, const std::optional<Tensor>& c, Tens
 }
 
 
+// Gram matrices X_i^T X_i (3xTF32, every sum in one pass) of several batches X_i [B_i, rows_i, r] fp32 into G [sum B_i, r, r]:
+// one launch where that can take them, false where it cannot (nothing is launched then).
+bool gram_many(std::vector<Tensor> xs, Tensor G, Tensor status) {
+  TORCH_CHECK(xs.size() >= 1 && xs.size() <= 4, "gram_many takes up to four batches");
+  TORCH_CHECK(G.is_cuda() && G.scalar_type() == at::kFloat && G.dim() == 3 && G.is_contiguous() && G.size(1) == G.size(2));
+  const c10::cuda::CUDAGuard guard(G.device());
+  dion::GemmArgs g;
+  g.ab_dtype = dion::kF32;
+  g.split3 = g.symmetric = 1;
+  g.pair = dion::kPairInOrder;
+  g.M = g.N = (int)G.size(1);
+  g.batch = (int)G.size(0);
+  g.D = G.data_ptr();
+  g.ldd = g.N;
+  g.d_batch_stride = (int64_t)g.N * g.N;
+  int64_t total = 0;
+  for (size_t i = 0; i < xs.size(); ++i) {
+    const Tensor& x = xs[i];
+    TORCH_CHECK(x.device() == G.device() && x.scalar_type() == at::kFloat && x.dim() == 3 && x.size(2) == G.size(1), "gram_many: fp32 [B, rows, r]");
+    total += x.size(0);
+    if (!x.is_contiguous() || !tma_addressable(x) || x.numel() == 0) return false;
+    if (i == 0) {
+      g.A = g.B = x.data_ptr();
+      g.a_major = g.b_major = dion::kMajorMN;
+      g.lda = g.ldb = x.size(2);
+      g.a_batch_stride = g.b_batch_stride = x.stride(0);
+      g.K = (int)x.size(1);
+    } else {
+      auto& m = g.more[g.more_count++];
+      m.A = x.data_ptr();
+      m.lda = x.size(2);
+      m.a_batch_stride = x.stride(0);
+      m.K = (int)x.size(1);
+      m.batch = (int)x.size(0);
+    }
+  }
+  TORCH_CHECK(total == G.size(0), "gram_many: one result per matrix");
+  g.status = status.data_ptr<int>();
+  if (!dion::gemm_takes_groups(g)) return false;
+  const cudaError_t e = dion::gemm_launch(g, at::cuda::getCurrentCUDAStream());
+  TORCH_CHECK(e == cudaSuccess, "Gram matrices: ", cudaGetErrorString(e), " ", dion::gemm_last_error());
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  return true;
+}
+
 // host only: how such a product would run, {tile columns, CTA pairs, CTAs that share a tile's K, C and D moved by TMA}; the tensors
 // give types, sizes, strides and alignment and may lie on the CPU
 std::vector<int64_t> gemm_plan(const Tensor& a, const Tensor& b, const std::optional<Tensor>& c, const Tensor& d, double beta,
@@ -1309,6 +1354,7 @@ TORCH_LIBRARY(dion_b200, m) {
   m.def("place_block(Tensor Zd, Tensor mask, Tensor(a!) Z, Tensor(b!) Zm, int k0) -> ()");
   m.def("col_sumsq(Tensor X, Tensor(a!) out) -> ()");
   m.def("split_tf32(Tensor x, Tensor(a!) hi, Tensor(b!) lo) -> ()");
+  m.def("gram_many(Tensor[] xs, Tensor(a!) G, Tensor status) -> bool");
   m.def("attn_fwd(Tensor q, Tensor k, Tensor v, Tensor(a!) out, Tensor(b!) lse, float scale, Tensor(c!) status) -> ()");
   m.def(
       "attn_bwd(Tensor q, Tensor k, Tensor v, Tensor o, Tensor d_o, Tensor lse, Tensor(a!) stats, Tensor(b!) dq, "
@@ -1360,6 +1406,7 @@ TORCH_LIBRARY_IMPL(dion_b200, CUDA, m) {
   m.impl("split_tf32_rows", &split_tf32_rows);
   m.impl("jacobi_scale", &jacobi_scale);
   m.impl("place_block", &place_block);
+  m.impl("gram_many", &gram_many);
   m.impl("attn_fwd", &attn_fwd);
   m.impl("attn_bwd", &attn_bwd);
   m.impl("refine_prep", &refine_prep);

@@ -89,6 +89,8 @@ struct KernelParams {
   int stage;                 // turn epilogue accesses through shared memory (coalesced)
   int b_is_a;                // symmetric product of one matrix with itself: diagonal tiles need one operand only
   int b_separate;            // kTmaEpi: one A, the B of batch elements 1 and 2 in the map slots of C and of mirrored boxes
+  int groups;                // kSplit: batches of several operands (GemmArgs::more), 0 or 1: one
+  int group_end[4], group_kb[4];  // batch element behind each group's last, K blocks of its operand
   int cluster_k;             // kClusterK: CTAs of a cluster that share one output tile (each a K range)
   int* status;
   GatherParams g;            // used by the kGather instantiations only
@@ -482,6 +484,22 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   // diagonal tile of x^T x with the same rows on both sides: B is A's tile, loaded and split once
   // (in a pair each CTA's half of B are its own rows of A)
   auto one_operand = [&](const TileCoord& t) -> bool { return kSplit && kBlockN == C::TILE_M && p.b_is_a && t.m_blk == t.n_blk; };
+  // K blocks of a tile: its part of the whole, or all those of its group's operand (`z`: batch element within the group)
+  constexpr bool kGroups = kSplit && !kPair && !kClusterK && !kTmaEpi && kBlockN == 128 && kAMajor == kMajorMN && kBMajor == kMajorMN;
+  struct Range {
+    int kb0, kb1, z, group;
+  };
+  auto range_of = [&](const TileCoord& t) -> Range {
+    if constexpr (kGroups) {
+      if (p.groups > 1) {
+        int g = 0;
+        while (g + 1 < p.groups && t.batch >= p.group_end[g]) ++g;
+        return Range{0, p.group_kb[g], t.batch - (g > 0 ? p.group_end[g - 1] : 0), g};
+      }
+    }
+    const int kb0_ = (kClusterK ? k_rank : t.split) * kb_per_split;
+    return Range{kb0_, min(kb0_ + kb_per_split, p.kblocks_total), kTmaEpi && p.b_separate ? 0 : t.batch, 0};
+  };
   // every wait inside the pipeline; the all-gather variant allows for the time another GPU may take
   auto wait = [&](uint64_t* bar, uint32_t parity) -> bool {
     if constexpr (kGather) return mbar_wait_for(bar, parity, abort_flag, kWaitBudgetNs + p.g.budget_ns);
@@ -499,8 +517,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
         const TileCoord t = decode_tile<kGather>(p, tile);
         const int m0 = t.m_blk * C::TILE_M + (int)cta_rank * kBlockM;
         const int n0 = t.n_blk * kBlockN + (int)cta_rank * (kPair ? C::B_ROWS : 0);
-        const int kb0 = (kClusterK ? k_rank : t.split) * kb_per_split;
-        const int kb1 = min(kb0 + kb_per_split, p.kblocks_total);
+        const Range kr = range_of(t);
+        const int kb0 = kr.kb0, kb1 = kr.kb1;
         const bool skip_b = one_operand(t);
         if constexpr (kGather) {
           // the rows of this tile are in place once every unit of their chunk has been counted
@@ -534,7 +552,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
           if (!kJoint || cta_rank == 0)
             mbar_arrive_expect_tx(&full_bar[stage], skip_b ? C::A_BYTES : kJoint ? C::TX_BYTES : C::STAGE_BYTES);
           const uint32_t bar = kJoint ? mapa_shared(smem_u32(&full_bar[stage]), 0) : smem_u32(&full_bar[stage]);
-          const int z = kTmaEpi && p.b_separate ? 0 : t.batch;
+          const int z = kr.z;
           auto load = [&](void* dst, const CUtensorMap* map, int c0, int c1) {
             if constexpr (kJoint) tma_load_3d_pair(dst, map, bar, c0, c1, z);
             else tma_load_3d(dst, map, &full_bar[stage], c0, c1, z);
@@ -544,12 +562,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
           // hi / lo operands: the K range is walked three times, as A B, A_lo B and A B_lo
           const CUtensorMap* map_a = &tmap_a;
           const CUtensorMap* map_b = &tmap_b;
+          if constexpr (kGroups) {  // the groups after the first lie in the slots of other variants' maps
+            if (kr.group > 0) map_a = map_b = kr.group == 1 ? &tmap_a_lo : kr.group == 2 ? &tmap_b_lo : &tmap_mirror;
+          }
           if constexpr (kTmaEpi) {
             if (p.b_separate && t.batch > 0) map_b = t.batch == 1 ? &tmap_b_lo : &tmap_mirror;
           }
           int kk = kb;
           if constexpr (kTf32) {
-            if (kb >= p.kblocks_seg) {
+            if (!kSplit && kb >= p.kblocks_seg) {
               const int seg = kb / p.kblocks_seg;
               kk = kb - seg * p.kblocks_seg;
               if (seg == 1) map_a = &tmap_a_lo;
@@ -592,8 +613,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       bool ok = true;
       for (int tile = worker; tile < p.total_tiles && ok; tile += num_workers, ++it) {
         const TileCoord t = decode_tile<kGather>(p, tile);
-        const int kb0 = (kClusterK ? k_rank : t.split) * kb_per_split;
-        const int kb1 = min(kb0 + kb_per_split, p.kblocks_total);
+        const Range kr = range_of(t);
+        const int kb0 = kr.kb0, kb1 = kr.kb1;
         const int b_off = one_operand(t) ? 0 : C::A_BYTES;
         const int acc = C::acc_of(it);
         const uint32_t acc_phase = C::acc_phase_of(it);
@@ -610,7 +631,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
           // segments to the second one, which starts from zero at the first of them
           uint32_t d_tmem = d_main;
           bool fresh = kb == kb0;
-          if constexpr (C::CROSS_ACC) {
+          if constexpr (C::CROSS_ACC && !kSplit) {
             if (kb >= p.kblocks_seg) {
               d_tmem = d_main + kBlockN;
               fresh = kb == p.kblocks_seg;
@@ -672,8 +693,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     bool ok = true;
     for (int tile = worker; tile < p.total_tiles && ok; tile += num_workers) {
       const TileCoord t = decode_tile<false>(p, tile);
-      const int kb0 = (kClusterK ? k_rank : t.split) * kb_per_split;
-      const int kb1 = min(kb0 + kb_per_split, p.kblocks_total);
+      const Range kr = range_of(t);
+      const int kb0 = kr.kb0, kb1 = kr.kb1;
       const int nbytes = one_operand(t) ? C::A_BYTES : C::STAGE_BYTES;
       for (int kb = kb0; kb < kb1; ++kb) {
         if (!wait(&full_bar[stage], phase)) {
@@ -1031,8 +1052,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       const int n0 = t.n_blk * kBlockN;
       const int acc = C::acc_of(it);
       const uint32_t acc_phase = C::acc_phase_of(it);
-      const int kb0 = (kClusterK ? k_rank : t.split) * kb_per_split;
-      const bool has_work = kb0 < p.kblocks_total;
+      const Range kr = range_of(t);
+      const bool has_work = kr.kb0 < kr.kb1;
       if constexpr (kClusterK) {
         // park this CTA's partial tile in the pipeline's shared memory (every load and multiply is done with it);
         // the sum over the cluster follows behind the barrier at the end of the kernel
@@ -1559,7 +1580,8 @@ cudaError_t launch_cfg(const GemmArgs& a, const KernelParams& kp, cudaStream_t s
   using C = Cfg<kTf32, kAMajor, kBMajor, kBlockN, kPair, kSplit>;
   CUtensorMap ta, tb, ta_lo, tb_lo;
   const int dt = kTf32 ? kF32 : kBF16;
-  const int batch = a.B_more[0] ? 1 : a.batch;  // of the operands' maps
+  int batch = a.B_more[0] ? 1 : a.batch;  // of the operands' maps
+  for (int g = 0; g < a.more_count; ++g) batch -= a.more[g].batch;
   auto map_a = [&](CUtensorMap* m, const void* base) {
     if (kAMajor == kMajorK) return make_tmap(m, base, dt, a.K, a.M, batch, a.lda, a.a_batch_stride, C::BK, kBlockM, kSwizzle128);
     return make_tmap(m, base, dt, a.M, a.K, batch, a.lda, a.a_batch_stride, C::CH, C::BK, C::A_ATOM32 ? kSwizzle128Atom32 : kSwizzle128);
@@ -1576,6 +1598,13 @@ cudaError_t launch_cfg(const GemmArgs& a, const KernelParams& kp, cudaStream_t s
     tb_lo = tb;
   }
   CUtensorMap tm = ta;  // never read
+  if constexpr (kSplit && !kTmaEpi && kAMajor == kMajorMN) {
+    CUtensorMap* slots[3] = {&ta_lo, &tb_lo, &tm};
+    for (int g = 0; g < a.more_count; ++g)
+      if (!make_tmap(slots[g], a.more[g].A, kF32, a.M, a.more[g].K, a.more[g].batch, a.more[g].lda, a.more[g].a_batch_stride, C::CH,
+                     C::BK, C::A_ATOM32 ? kSwizzle128Atom32 : kSwizzle128))
+        return cudaErrorInvalidValue;
+  }
   if constexpr (kTmaEpi) {
     const int dd = kF32Out ? kF32 : dt;
     if (!kPtrs && !make_tmap(&ta_lo, a.D, dd, a.N, a.M, a.batch, a.ldd, a.d_batch_stride, dd == kF32 ? 32 : 64, 32, kSwizzle128))
@@ -1788,7 +1817,7 @@ bool split_pair(const GemmArgs& a) {
 }
 
 cudaError_t launch_split(const GemmArgs& a, const KernelParams& kp, int bn, cudaStream_t s) {
-  const int ck = bn == 256 ? 1 : choose_cluster_k(a, bn, kp.total_tiles, kp.kblocks_total);
+  const int ck = bn == 256 || a.more_count > 0 ? 1 : choose_cluster_k(a, bn, kp.total_tiles, kp.kblocks_total);
   if (ck > 1) {
     KernelParams kc = kp;
     kc.cluster_k = ck;
@@ -1964,6 +1993,19 @@ bool gemm_gather_plan(const GemmArgs& a, int (&out)[8]) {
   return true;
 }
 
+// All tiles of all groups run at the same time (one per SM): the launch takes as long as its longest sum, where a launch per
+// group adds them up.  48 x 768, 12 x 3072 and 12 x 3072 rows of rank 96: 218 us in three launches, 95 in one.  With more
+// tiles than SMs the groups fill the chip by themselves.
+bool gemm_takes_groups(const GemmArgs& a) {
+  if (a.more_count < 0 || a.more_count > 3 || !a.split3 || !a.symmetric || a.A != a.B || a.a_major != kMajorMN || a.b_major != kMajorMN ||
+      a.ab_dtype != kF32 || a.d_dtype != kF32 || a.epilogue != kEpiStore || a.act != 0 || a.pair != kPairInOrder || a.C || a.c_ptrs ||
+      a.d_ptrs || a.D2 || a.scatter_mode != 0 || a.gather.world > 0 || a.block_n != 0 || a.max_ctas > 0 || a.split_k != 1 || a.M != a.N ||
+      split_pair(a))
+    return false;
+  const long long t = (a.N + kBlockM - 1) / kBlockM;
+  return t * (t + 1) / 2 * a.batch <= num_sms();
+}
+
 cudaError_t gemm_launch(const GemmArgs& a, cudaStream_t stream) {
   if (a.batch > kMaxMaps && tma_ptrs(a)) {  // the maps of a launch travel with its parameters
     const long long es = a.ab_dtype == kF32 ? 4 : 2;
@@ -2080,6 +2122,17 @@ cudaError_t gemm_launch(const GemmArgs& a, cudaStream_t stream) {
   kp.b_is_a = a.symmetric && a.A == a.B && a.a_major == kMajorMN && a.b_major == kMajorMN && a.lda == a.ldb &&
               a.a_batch_stride == a.b_batch_stride;
   kp.cluster_k = 1;
+  kp.groups = a.more_count > 0 ? a.more_count + 1 : 0;
+  if (a.more_count > 0) {
+    int end = a.batch;
+    for (int g = 0; g < a.more_count; ++g) end -= a.more[g].batch;
+    kp.group_end[0] = end;
+    kp.group_kb[0] = kp.kblocks_total;
+    for (int g = 0; g < a.more_count; ++g) {
+      kp.group_end[g + 1] = end += a.more[g].batch;
+      kp.group_kb[g + 1] = (a.more[g].K + bk - 1) / bk;
+    }
+  }
   kp.b_separate = a.B_more[0] != nullptr;
   kp.scatter_mode = a.scatter_mode;
   kp.scatter_block = a.scatter_block;
@@ -2110,6 +2163,10 @@ cudaError_t gemm_launch(const GemmArgs& a, cudaStream_t stream) {
     if (pair) return launch_cfg<false, kMajorK, kMajorK, 256, true, true>(a, kp, stream);
     if (bn == 128) return launch_cfg<false, kMajorK, kMajorK, 128, false, true>(a, kp, stream);
     return launch_cfg<false, kMajorK, kMajorK, 256, false, true>(a, kp, stream);
+  }
+  if (a.more_count > 0 && !gemm_takes_groups(a)) {
+    g_last_error = "batches of several operands: split3 Gram products in order, on unpaired tiles";
+    return cudaErrorInvalidValue;
   }
   if (a.split3) return launch_split(a, kp, bn, stream);
   return tf32 ? launch_major<true>(a, kp, bn, pair, stream) : launch_major<false>(a, kp, bn, pair, stream);

@@ -97,6 +97,15 @@ struct GemmArgs {
   // Three products of one A with three matrices laid out like B (bf16, K-major both, no C): batch is 3, B belongs to batch
   // element 0, these to 1 and 2, and D holds the three results d_batch_stride apart.
   const void* B_more[2] = {nullptr, nullptr};
+  // Gram matrices X^T X of several batches in one launch (split3, symmetric, MN-major A == B, one rank N, fp32 D contiguous
+  // over all of them): A / lda / a_batch_stride / K describe the first, these the others in the order of their results; `batch`
+  // counts the matrices of all.
+  struct Group {
+    const void* A = nullptr;
+    int64_t lda = 0, a_batch_stride = 0;
+    int K = 0, batch = 0;
+  } more[3];
+  int more_count = 0;
   // CTA pairs (256-row tiles): 0 = choose automatically, 1 = force (needs block_n 256), -1 = never, and no K range shared by a
   // cluster either; kPairInOrder = choose automatically, but every K sum is taken in one pass (no sharing by a cluster)
   int pair = 0;
@@ -134,6 +143,9 @@ const char* gemm_last_error();
 
 // Host only, no launch: can one launch take the three products of `args` (GemmArgs::B_more)?
 bool gemm_takes_three(const GemmArgs& args);
+
+// Host only, no launch: can one launch take the batches of `args` (GemmArgs::more, with `batch` counting all of them)?
+bool gemm_takes_groups(const GemmArgs& args);
 
 // Host only, no launch: how gemm_launch would run `args`.  out = {tile columns, CTA pairs (0 / 1), CTAs that share a tile's K,
 // C and D moved by TMA (0 / 1)}.

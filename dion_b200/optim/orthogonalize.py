@@ -77,6 +77,22 @@ def gram(P: Tensor, reduce_group=None, out: Optional[Tensor] = None, in_order: b
     return ops.gemm(hi.transpose(-1, -2), hi, out=out, symmetric=True, a_lo=lo.transpose(-1, -2), b_lo=lo)
 
 
+def _grams_together(Xs, idxs, row_groups, in_order, out: Optional[Tensor] = None) -> Optional[Tensor]:
+    """The Gram matrices of the batches ``Xs[i]``, i in `idxs`, one behind the other, from one launch: for batches whose sums
+    stay in order (one CTA per tile whatever the number of rows) and which together have fewer tiles than there are SMs.
+    None where that does not apply."""
+    X0 = Xs[idxs[0]]
+    if not (2 <= len(idxs) <= 4 and X0.is_cuda and SPLIT_IN_KERNEL and GRAM_PRECISION != "tf32" and all(in_order[i] for i in idxs)
+            and all(Xs[i].dtype == torch.float32 and Xs[i].is_contiguous() and Xs[i].numel() > 0 for i in idxs)
+            and all(row_groups[i] is None or dist.get_world_size(row_groups[i]) == 1 for i in idxs)):
+        return None
+    r = X0.shape[-1]
+    if out is None:
+        out = torch.empty((sum(Xs[i].shape[0] for i in idxs), r, r), dtype=torch.float32, device=X0.device)
+    ops.runtime.use_cuda_kernels(X0)
+    return out if torch.ops.dion_b200.gram_many([Xs[i] for i in idxs], out, ops.runtime.status_tensor(X0.device)) else None
+
+
 def apply_right(P: Tensor, Z: Tensor) -> Tensor:
     """``P @ Z^T`` for ``P: [B, a, r]`` fp32 and lower-triangular ``Z: [B, r, r]``."""
     Zt = Z.transpose(-1, -2)
@@ -114,14 +130,15 @@ def orthonormalize_cholqr(P: Tensor, row_group: Optional[dist.ProcessGroup] = No
 
 
 def _refine(X: Tensor, row_group: Optional[dist.ProcessGroup], gave_up: Optional[Tensor] = None,
-            out_dtype: Optional[torch.dtype] = None, in_order: bool = False) -> Tensor:
+            out_dtype: Optional[torch.dtype] = None, in_order: bool = False, G: Optional[Tensor] = None) -> Tensor:
     """One triangular Newton correction of an almost orthonormal X: with the column-scaled
     Gram matrix D G D = I + E, the Cholesky factor's inverse is I - stril(E) to first order,
     so X <- (X D) (I - stril(E))^T squares the orthogonality error while keeping the column
-    spans nested exactly like a QR factorisation does."""
-    G = gram(X, row_group, in_order=in_order)
-    if row_group is not None and dist.get_world_size(row_group) > 1:
-        symm.all_reduce(G, row_group)
+    spans nested exactly like a QR factorisation does.  ``G``: the Gram matrices, where they are known already."""
+    if G is None:
+        G = gram(X, row_group, in_order=in_order)
+        if row_group is not None and dist.get_world_size(row_group) > 1:
+            symm.all_reduce(G, row_group)
     # d = rsqrt(diag G), C = stril(D G D) = stril(E); columns the factorisation gave up on (squared norm
     # far below 1) are dropped instead of being blown up to unit length
     # a matrix whose factorisation gave up on some pivot (`gave_up`, int32 per matrix) is far from
@@ -291,12 +308,15 @@ def _orthonormalize_many(Ps, row_groups, refine_passes, pivot_floor, shard_group
             if len(idxs) > 1:
                 total = sum(Xs[i].shape[0] for i in idxs)
                 Gcats[r] = torch.empty((total, r, r), dtype=torch.float32, device=Xs[idxs[0]].device)
+            together = _grams_together(Xs, idxs, row_groups, in_order, Gcats.get(r)) is not None
             off = 0
             for i in idxs:
                 b = Xs[i].shape[0]
                 g = row_groups[i]
                 sharded_rows = g is not None and dist.get_world_size(g) > 1
-                if r in Gcats and not sharded_rows:
+                if together:
+                    Gs[i] = Gcats[r][off:off + b]
+                elif r in Gcats and not sharded_rows:
                     Gs[i] = gram(Xs[i], out=Gcats[r][off:off + b], in_order=in_order[i])
                 else:
                     Gs[i] = gram(Xs[i], g, in_order=in_order[i])
@@ -333,12 +353,17 @@ def _orthonormalize_many(Ps, row_groups, refine_passes, pivot_floor, shard_group
     # that to the 1e-6 level.  After a single pass the error can be 1e-1, which takes two corrections.
     passes = [max(1, refine_passes - 1) if (rb and refine_passes > 0) else refine_passes for rb in robust]
     for k in range(refine_passes):
-        for i in range(n):
-            if k >= passes[i]:
-                continue
+        todo = [i for i in range(n) if k < passes[i]]
+        known = {}
+        for r in {Xs[i].shape[-1] for i in todo}:
+            idxs = [i for i in todo if Xs[i].shape[-1] == r]
+            G = _grams_together(Xs, idxs, row_groups, in_order)
+            if G is not None:
+                known.update(zip(idxs, G.split([Xs[i].shape[0] for i in idxs])))
+        for i in todo:
             # the last correction writes the result in the dtype its consumer multiplies with
             last = k == passes[i] - 1
-            Xs[i] = _refine(Xs[i], row_groups[i], last_info[i], dtypes[i] if last else None, in_order[i])
+            Xs[i] = _refine(Xs[i], row_groups[i], last_info[i], dtypes[i] if last else None, in_order[i], known.get(i))
     return [X.to(dt) for X, dt in zip(Xs, dtypes)]
 
 

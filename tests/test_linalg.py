@@ -235,3 +235,32 @@ def test_chol_inverse_takes_the_blocked_path_for_large_ranks():
     Zr, _ = ops.chol_inverse_reference(G.double())
     assert ((Z.double() - Zr.double()).norm() / Zr.double().norm()).item() < 1e-4
     assert int(info.sum()) == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("r,batches", [
+    (96, [(48, 768), (12, 3072), (12, 3072)]),
+    (200, [(3, 500), (2, 2056), (7, 1992), (1, 16)]),  # off-diagonal tiles, rows that fill no block, four operands
+    (8, [(1, 64), (1, 31)]),
+    (256, [(40, 100), (10, 300)]),                     # 150 tiles: more than SMs, one launch per batch
+])
+def test_gram_matrices_of_several_batches_in_one_launch(r, batches):
+    from dion_b200.ops import runtime
+    from dion_b200.optim.orthogonalize import _grams_together, gram
+
+    g = torch.Generator(device="cuda").manual_seed(r)
+    Xs = [torch.randn(b, m, r, device="cuda", generator=g) for b, m in batches]
+    out = torch.full((sum(b for b, _ in batches), r, r), float("nan"), device="cuda")
+    got = _grams_together(Xs, list(range(len(Xs))), [None] * len(Xs), [True] * len(Xs), out)
+    tiles = -(-r // 128)
+    few = tiles * (tiles + 1) // 2 * len(out) <= 148
+    assert (got is not None) == few
+    if few:
+        assert torch.equal(got, torch.cat([gram(X, in_order=True) for X in Xs]))
+    else:
+        assert out.isnan().all()
+    assert int(runtime.status_tensor(out.device).item()) == 0
+    # batches whose sums may be taken in parts, other types and strided rows keep their own launches
+    assert _grams_together(Xs, [0, 1], [None] * 2, [True, False]) is None
+    assert _grams_together([Xs[0].double(), Xs[1].double()], [0, 1], [None] * 2, [True, True]) is None
+    assert _grams_together([Xs[0][:, ::2], Xs[1]], [0, 1], [None] * 2, [True, True]) is None

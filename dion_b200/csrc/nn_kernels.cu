@@ -495,14 +495,51 @@ __global__ void __launch_bounds__(256) relu2_bwd_kernel(const uint4* __restrict_
 }
 
 // ------------------------------------------------------------------ cross entropy
-// One 256-thread block per row.  Pass 1 streams the bf16 row once and keeps an online
-// (max, sum-exp) pair per thread; pass 2 re-reads the row and writes the gradient in place.  Nothing
-// is kept in registers, so any vocabulary size works and eight rows are resident per SM.  For
-// 50304-wide rows the second read mostly comes from DRAM again (1.4x the algorithmic traffic); a
-// variant that kept the row in shared memory instead was slower, because with two exponentials per
-// element the kernel is bound as much by the special-function unit as by DRAM and needs many small
-// blocks per SM to overlap the two.
-constexpr int kCeThreads = 256;
+// One block per row.  Pass 1 streams the bf16 row once and keeps an online (max, sum-exp) pair per thread; pass 2 re-reads
+// the row and writes the gradient in place.  Nothing is kept in registers, so any vocabulary size works.
+//
+// Two things bound it: DRAM, and two exponentials per logit on the special-function unit (8192 x 50304: 250 us for one read
+// and one write, 184 us for the exponentials).  Hence
+//  * the rows in flight have to stay in the L2 for pass 2, and a block takes the more threads the longer its row is: with
+//    2048 threads per SM there are 1184 rows in flight at 256 threads (119 MB of 50304-wide rows), 592 at 512, 296 at 1024.
+//    A row kept in shared memory instead was slower (8192 x 50304: 406 us): it holds back the blocks that cover one block's
+//    reductions with another's loads.
+//  * everything around the exponential is packed: additions and multiplications of two values each, the maximum on the
+//    bf16 pairs themselves, one rescaling of the sum per 16 logits.  The exponential is the flush-to-zero form, as in the
+//    attention kernels: probabilities below 2^-126 come out as zero.
+// 8192 x 50304: 407 -> 296 us; 4096 x 128256: 539 -> 401; 8192 x 32000: 224 -> 188; 8192 x 4096: 48 -> 39.
+
+__device__ __forceinline__ float exp2_ftz(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float2 add_pair(float2 a, float2 b) {
+  float2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(reinterpret_cast<unsigned long long&>(r))
+      : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)));
+  return r;
+}
+__device__ __forceinline__ float2 mul_pair(float2 a, float2 b) {
+  float2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(reinterpret_cast<unsigned long long&>(r))
+      : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)));
+  return r;
+}
+
+// exp(x - base) of two logits.  x - base is rounded before the scaling, as a plain exp(x - base) does: folded into one
+// fused step, log2(e) * base would carry its rounding into every term.
+__device__ __forceinline__ float2 exp_pair(__nv_bfloat162 x, float base) {
+  constexpr float kLog2e = 1.4426950408889634f;
+  const float2 t = mul_pair(add_pair(__bfloat1622float2(x), make_float2(-base, -base)), make_float2(kLog2e, kLog2e));
+  return make_float2(exp2_ftz(t.x), exp2_ftz(t.y));
+}
+
+__device__ __forceinline__ float max8(const uint4& q) {  // NaN is passed over here; the sum takes it up
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
+  const __nv_bfloat162 m = __hmax2(__hmax2(h[0], h[1]), __hmax2(h[2], h[3]));
+  return fmaxf(__low2float(m), __high2float(m));
+}
 
 __device__ __forceinline__ void online_merge(float& m, float& s, float m2, float s2) {
   const float mx = fmaxf(m, m2);
@@ -514,15 +551,36 @@ __device__ __forceinline__ void online_merge(float& m, float& s, float m2, float
   m = mx;
 }
 
-__global__ void __launch_bounds__(kCeThreads) cross_entropy_kernel(bf16* __restrict__ logits,
-                                                                  const long long* __restrict__ targets,
-                                                                  float* __restrict__ row_loss,
-                                                                  const float* __restrict__ scale_ptr,
-                                                                  int vocab, long long pitch, float grad_scale,
-                                                                  long long ignore_index, int write_grad) {
+// The running maximum, and sums of exp(x - maximum) of the even and the odd logits, of kNum vectors more.
+template <int kNum>
+__device__ __forceinline__ void online_add(const uint4 (&q)[kNum], float& m, float2& sum) {
+  float mx = m;
+#pragma unroll
+  for (int u = 0; u < kNum; ++u) mx = fmaxf(mx, max8(q[u]));
+  const float base = mx == -INFINITY ? 0.f : mx;  // nothing but -inf so far: exp(-inf) adds nothing
+  const float c = __expf(m - base);
+  sum.x *= c;
+  sum.y *= c;
+  m = mx;
+#pragma unroll
+  for (int u = 0; u < kNum; ++u) {
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q[u]);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) sum = add_pair(sum, exp_pair(h[j], base));
+  }
+}
+
+constexpr int kCeVec = 2;  // 16-byte loads in flight per thread
+
+template <int kThreads>
+__global__ void __launch_bounds__(kThreads, 2048 / kThreads)
+    cross_entropy_kernel(bf16* __restrict__ logits, const long long* __restrict__ targets, float* __restrict__ row_loss,
+                         const float* __restrict__ scale_ptr, int vocab, long long pitch, float grad_scale,
+                         long long ignore_index, int write_grad) {
   pdl_trigger();
   pdl_wait();
-  __shared__ float red_m[kCeThreads / 32], red_s[kCeThreads / 32];
+  constexpr int kWarps = kThreads / 32;
+  __shared__ float red_m[kWarps], red_s[kWarps];
   const long long row = blockIdx.x;
   const long long tgt = targets[row];
   uint4* lr = reinterpret_cast<uint4*>(logits + row * pitch);
@@ -531,25 +589,25 @@ __global__ void __launch_bounds__(kCeThreads) cross_entropy_kernel(bf16* __restr
     if (threadIdx.x == 0) row_loss[row] = 0.f;
     if (write_grad) {
       const uint4 z = make_uint4(0, 0, 0, 0);
-      for (int v = threadIdx.x; v < nvec; v += kCeThreads) lr[v] = z;
+      for (int v = threadIdx.x; v < nvec; v += kThreads) lr[v] = z;
     }
     return;
   }
   // pass 1: online softmax statistics
-  float m = -INFINITY, ssum = 0.f;
-  for (int v = threadIdx.x; v < nvec; v += kCeThreads) {
-    float f[8];
-    unpack8(lr[v], f);
-    float mv = f[0];
+  float m = -INFINITY;
+  float2 sum = make_float2(0.f, 0.f);
+  int v = threadIdx.x;
+  for (; v + (kCeVec - 1) * kThreads < nvec; v += kCeVec * kThreads) {
+    uint4 q[kCeVec];
 #pragma unroll
-    for (int j = 1; j < 8; ++j) mv = fmaxf(mv, f[j]);
-    const float mx = fmaxf(m, mv);
-    float acc = ssum * __expf(m - mx);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) acc += __expf(f[j] - mx);
-    ssum = acc;
-    m = mx;
+    for (int u = 0; u < kCeVec; ++u) q[u] = lr[v + u * kThreads];
+    online_add(q, m, sum);
   }
+  for (; v < nvec; v += kThreads) {
+    const uint4 q[1] = {lr[v]};
+    online_add(q, m, sum);
+  }
+  float ssum = sum.x + sum.y;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     const float m2 = __shfl_xor_sync(0xffffffffu, m, o);
@@ -560,27 +618,45 @@ __global__ void __launch_bounds__(kCeThreads) cross_entropy_kernel(bf16* __restr
     red_m[threadIdx.x >> 5] = m;
     red_s[threadIdx.x >> 5] = ssum;
   }
-  __syncthreads();
-  m = red_m[0];
-  ssum = red_s[0];
-#pragma unroll
-  for (int w = 1; w < kCeThreads / 32; ++w) online_merge(m, ssum, red_m[w], red_s[w]);
   const float tl = __bfloat162float(logits[row * pitch + tgt]);
-  if (threadIdx.x == 0) row_loss[row] = m + __logf(ssum) - tl;
+  __syncthreads();  // also: every thread has read the target logit before the row is overwritten
+  m = red_m[threadIdx.x % kWarps];
+  ssum = red_s[threadIdx.x % kWarps];
+#pragma unroll
+  for (int o = kWarps / 2; o > 0; o >>= 1) {
+    const float m2 = __shfl_xor_sync(0xffffffffu, m, o);
+    const float s2 = __shfl_xor_sync(0xffffffffu, ssum, o);
+    online_merge(m, ssum, m2, s2);
+  }
+  if (threadIdx.x == 0) row_loss[row] = (m - tl) + __logf(ssum);
   if (!write_grad) return;
-  __syncthreads();  // every thread has read the target logit before the row is overwritten
   // pass 2: gradient, in place
   const float gs = grad_scale * (scale_ptr ? *scale_ptr : 1.f);
   const float inv = gs / ssum;
   const int tv = (int)(tgt >> 3), tj = (int)(tgt & 7);
-  for (int v = threadIdx.x; v < nvec; v += kCeThreads) {
+  const auto gradient = [&](const uint4& q, int at) {
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
     float f[8];
-    unpack8(lr[v], f);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) f[j] = __expf(f[j] - m) * inv;
-    if (v == tv) f[tj] -= gs;
-    lr[v] = pack8(f);
+    for (int j = 0; j < 4; ++j) {
+      const float2 p = mul_pair(exp_pair(h[j], m), make_float2(inv, inv));
+      f[2 * j] = p.x;
+      f[2 * j + 1] = p.y;
+    }
+    if (at == tv) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) f[j] -= j == tj ? gs : 0.f;
+    }
+    lr[at] = pack8(f);
+  };
+  for (v = threadIdx.x; v + (kCeVec - 1) * kThreads < nvec; v += kCeVec * kThreads) {
+    uint4 q[kCeVec];
+#pragma unroll
+    for (int u = 0; u < kCeVec; ++u) q[u] = lr[v + u * kThreads];
+#pragma unroll
+    for (int u = 0; u < kCeVec; ++u) gradient(q[u], v + u * kThreads);
   }
+  for (; v < nvec; v += kThreads) gradient(lr[v], v);
 }
 
 // ------------------------------------------------------------------ scaling by a device scalar
@@ -781,9 +857,14 @@ cudaError_t cross_entropy_fwd_bwd_launch(void* logits, const long long* targets,
                                          float grad_scale, long long ignore_index, bool write_grad, cudaStream_t s) {
   if (rows == 0) return cudaSuccess;
   if (vocab % 8 != 0 || pitch % 8 != 0) return cudaErrorInvalidValue;
-  launch_pdl(cross_entropy_kernel, dim3((unsigned)rows), dim3(kCeThreads), 0, s, 0, reinterpret_cast<bf16*>(logits), targets, row_loss,
-                                                            scale_ptr, vocab, pitch, grad_scale, ignore_index,
-                                                            write_grad ? 1 : 0);
+  // Threads per row, us at 256 / 512 / 1024 threads: 4096 x 128256 497 / 474 / 400, 4096 x 100352 384 / 365 / 308,
+  // 4096 x 65536 253 / 214 / 208, 8192 x 50304 368 / 296 / 337, 8192 x 32000 208 / 188 / 231, 8192 x 24576 146 / 148 / 205,
+  // 8192 x 16384 97 / 110 / 152.
+  const auto kernel = vocab >= 65536 ? cross_entropy_kernel<1024> : vocab > 24576 ? cross_entropy_kernel<512>
+                                                                                  : cross_entropy_kernel<256>;
+  const unsigned threads = vocab >= 65536 ? 1024 : vocab > 24576 ? 512 : 256;
+  launch_pdl(kernel, dim3((unsigned)rows), dim3(threads), 0, s, 0, reinterpret_cast<bf16*>(logits), targets, row_loss,
+             scale_ptr, vocab, pitch, grad_scale, ignore_index, write_grad ? 1 : 0);
   return cudaGetLastError();
 }
 

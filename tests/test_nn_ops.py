@@ -206,6 +206,42 @@ def test_linear_cross_entropy(vocab):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("vocab", [8, 2056, 24576, 24584, 32760, 65528, 65536, 100008, 131072])
+@pytest.mark.parametrize("write_grad", [True, False])
+def test_cross_entropy_rows(vocab, write_grad):
+    """Every number of threads per row, at lengths that end in whole groups of vectors and in between."""
+    torch.manual_seed(vocab)
+    rows, pitch = 37, vocab + 8
+    x = torch.full((rows, pitch), 7.0, device="cuda", dtype=torch.bfloat16)
+    x[:, :vocab] = 3 * torch.randn(rows, vocab, device="cuda")
+    x[3, : vocab // 2] = -float("inf")              # a masked vocabulary
+    x[4, : vocab // 2] = torch.finfo(torch.bfloat16).min
+    x[5, :vocab] = 1e4
+    t = torch.randint(vocab // 2, vocab, (rows,), device="cuda")
+    t[0], t[1], t[2] = vocab - 1, vocab // 2, -1
+    ref = x[:, :vocab].double()
+    logits, loss = x.clone(), torch.empty(rows, device="cuda")
+    scale = torch.tensor([0.25], device="cuda")
+    assert N.runtime.use_cuda_kernels(x)
+    torch.ops.dion_b200.cross_entropy_fwd_bwd(logits[:, :vocab], t, loss, scale, 3.0, -1, write_grad)
+    want = F.cross_entropy(ref, t, ignore_index=-1, reduction="none")
+    # maximum minus target rounds once (2^-24 of it), the sum of a thread has up to 128 terms, each exponential 2 ulp
+    torch.testing.assert_close(loss.double(), want, rtol=2.0 ** -22, atol=128 * 2.0 ** -24 + 1e-5)
+    if write_grad:
+        p = 0.75 * (torch.softmax(ref, 1) - F.one_hot(t.clamp_min(0), vocab))
+        p[t == -1] = 0
+        # bf16: half of 2^-8; the target's p - 1 can cancel, to within the rounding of fp32
+        torch.testing.assert_close(logits[:, :vocab].double(), p, rtol=2.0 ** -8, atol=1e-6 * float(p.abs().amax()))
+    else:
+        assert torch.equal(logits, x)
+    assert bool((logits[:, vocab:] == 7.0).all())
+    bad = x.clone()
+    bad[0, vocab // 3], bad[1, 0], bad[6, vocab - 1] = float("nan"), float("inf"), float("nan")
+    torch.ops.dion_b200.cross_entropy_fwd_bwd(bad[:, :vocab], t, loss, scale, 3.0, -1, write_grad)
+    assert torch.equal(loss.isnan(), torch.isin(torch.arange(rows, device="cuda"), torch.tensor([0, 1, 6], device="cuda")))
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("tokens,chunk", [(256, 8192), (300, 128)])
 def test_linear_cross_entropy_backward_twice_and_scaled(tokens, chunk):
     """The gradients kept by the forward pass are scaled in place only when nobody needs them again: a kept graph gives

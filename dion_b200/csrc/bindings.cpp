@@ -1085,6 +1085,17 @@ Tensor newton_schulz_steps(const Tensor& X0, const std::optional<Tensor>& sumsq,
   Tensor X = at::empty_like(X0), Y = at::empty_like(X0);
   frob_scale(X0, X, sumsq, eps);
   Tensor A = at::empty({B, k, k}, X0.options()), P = at::empty_like(A);
+  const int64_t L = tall ? X0.size(1) : X0.size(2);
+  const int steps = (int)std::min<size_t>(coeffs.size() / 3, 1 << 20);
+  if (dion::newton_schulz_takes(B, k, L, steps)) {
+    const int64_t pitch = tall ? (L + 7) / 8 * 8 : L;
+    const Tensor rows = tall ? at::empty({B, k, pitch}, X0.options()) : X, t0 = tall ? X : at::empty({B, L, k}, X0.options());
+    const std::vector<float> c(coeffs.begin(), coeffs.end());
+    DION_CUDA_CHECK(dion::newton_schulz_launch(rows.data_ptr(), A.data_ptr(), P.data_ptr(), t0.data_ptr(),
+                                               (tall ? Y : at::empty_like(t0)).data_ptr(), (int)B, (int)k, (int)L, (int)pitch,
+                                               c.data(), steps, tall, status.data_ptr<int>(), at::cuda::getCurrentCUDAStream()));
+    return tall && steps % 2 == 1 ? Y : X;
+  }
   for (size_t i = 0; i < coeffs.size(); i += 3) {
     if (tall) product(X.transpose(1, 2), X, {}, A, 1., 0., true, status);
     else product(X, X.transpose(1, 2), {}, A, 1., 0., true, status);

@@ -1960,6 +1960,12 @@ bool plan_gather(const GemmArgs& a, const Tiling& tl, GatherParams* g) {
 
 }  // namespace
 
+bool bf16_tile_map(void* map, const void* base, unsigned long long inner, unsigned long long rows, unsigned long long batch,
+                   unsigned long long pitch, unsigned long long batch_stride, unsigned box_inner, unsigned box_rows) {
+  return make_tmap(static_cast<CUtensorMap*>(map), base, kBF16, inner, rows, batch, pitch, batch_stride, box_inner, box_rows,
+                   kSwizzle128);
+}
+
 const char* gemm_last_error() { return g_last_error.c_str(); }
 
 void gemm_plan(const GemmArgs& a, int (&out)[4]) {

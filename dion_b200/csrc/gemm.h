@@ -156,6 +156,11 @@ void gemm_plan(const GemmArgs& args, int (&out)[4]);
 // rows per readiness counter, copy units per counter, first m-tile of the schedule, m-tiles, n-tiles}.
 bool gemm_gather_plan(const GemmArgs& args, int (&out)[8]);
 
+// Tensor map (CUtensorMap*) over a row-major bf16 array [batch][rows][inner] with a 128-byte swizzled box of box_inner x
+// box_rows; false with a message in gemm_last_error() where the driver refuses it.
+bool bf16_tile_map(void* map, const void* base, unsigned long long inner, unsigned long long rows, unsigned long long batch,
+                   unsigned long long pitch, unsigned long long batch_stride, unsigned box_inner, unsigned box_rows);
+
 // Makes the current device's primary context current on the calling thread, which a driver call needs and only a runtime
 // call brings about: a backward pass may begin on a thread that has made none.
 inline bool bind_primary_context() {

@@ -57,6 +57,12 @@ int multi_tensor_block_elems();
 // a first launch writes per-chunk partial sums to `partial` (batch * frob_chunks(per) floats), which the
 // scaling launch adds up in a fixed order.
 int frob_chunks(long long per);
+// A whole Newton-Schulz iteration of small matrices (newton_schulz.cu); host only, no launch: are they small enough?
+bool newton_schulz_takes(long long batch, long long k, long long L, int steps);
+// X [batch][k][pitch], A and P [batch][k][k], Xt0 and Xt1 [batch][L][k], all bf16.  The input lies in X, with `tall` transposed
+// in Xt0; the result in X, with `tall` in Xt0 for an even number of steps and in Xt1 for an odd one.
+cudaError_t newton_schulz_launch(void* X, void* A, void* P, void* Xt0, void* Xt1, int batch, int k, int L, int pitch,
+                                 const float* coeffs, int steps, bool tall, int* status, cudaStream_t stream);
 cudaError_t frob_scale_launch(const void* x, void* out, float* partial, const float* sumsq, float eps, int batch,
                               long long per, cudaStream_t s);
 

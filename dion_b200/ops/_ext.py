@@ -25,7 +25,7 @@ DEBUG = os.environ.get("DION_B200_DEBUG", "0") == "1"
 _BUILD_DIR = _PKG_DIR / ("_C_debug" if DEBUG else "_C")
 _LIB_NAME = "dion_b200_C_debug" if DEBUG else "dion_b200_C"
 _SOURCES = ["bindings.cpp", "gemm.cu", "optim_kernels.cu", "nn_kernels.cu", "linalg.cu", "comm_kernels.cu",
-            "noalloc.cu", "attention.cu", "dion_fused.cu", "llama_kernels.cu"]
+            "noalloc.cu", "attention.cu", "dion_fused.cu", "llama_kernels.cu", "newton_schulz.cu"]
 
 _lock = threading.Lock()
 _loaded: Optional[bool] = None

@@ -125,3 +125,61 @@ def test_symmetric_helpers_on_cpu():
     S = torch.randn(16, 16)
     S = S + S.T
     torch.testing.assert_close(ns_line_2(S, 0.5, 2.0), 0.5 * (S @ S.T) + 2.0 * S)
+
+
+def _one_launch_per_product(g, coeffs, tall):
+    """Scaling and products of ``newton_schulz``, each in a launch of its own; sides of a multiple of eight."""
+    from dion_b200 import ops
+
+    X = torch.empty_like(g)
+    torch.ops.dion_b200.frob_scale(g, X, None, 1e-7)
+    for a, b, c in coeffs:
+        A = ops.gemm(X.mT, X, symmetric=True) if tall else ops.gemm(X, X.mT, symmetric=True)
+        P = ops.gemm(A, A.mT, c=A, alpha=c, beta=b, symmetric=True)
+        X = ops.gemm(X, P, c=X, beta=a) if tall else ops.gemm(P, X, c=X, beta=a)
+    return X
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("steps", [1, 2, 5])
+@pytest.mark.parametrize("shape", [(1, 8, 8), (2, 8, 1024), (1, 72, 64), (5, 64, 72), (1, 128, 128), (3, 200, 264), (2, 264, 200),
+                                   (1, 1003, 56), (12, 256, 512), (2, 511, 256), (13, 136, 128), (24, 128, 256), (25, 64, 256),
+                                   (64, 128, 128), (65, 128, 128), (128, 64, 64), (129, 64, 64), (1, 256, 768)])
+def test_small_matrices_take_one_launch_for_all_products(shape, steps):
+    """Every number of CTAs per matrix, edges of the 128 x 64 tiles, both orientations, odd and even numbers of steps (the
+    transposes change places), and sizes just beyond: the sums and roundings are those of single products."""
+    from dion_b200.ops import runtime
+
+    torch.manual_seed(sum(shape))
+    g = torch.randn(*shape, device="cuda").bfloat16()
+    tall = shape[1] > shape[2]
+    before = runtime.launch_count()
+    want = _one_launch_per_product(g, NS_COEFFS[:steps], tall)
+    between = runtime.launch_count()
+    out = newton_schulz(g, coeffs=NS_COEFFS[:steps])
+    small = shape not in ((129, 64, 64), (1, 256, 768))
+    assert runtime.launch_count() - between == between - before - (3 * steps - 1 if small else 0)
+    assert torch.equal(out, want)
+    runtime.check_status()
+
+
+@pytest.mark.gpu
+def test_small_matrices_under_capture_and_on_two_streams():
+    gs = [torch.randn(3, 200, 264, device="cuda").bfloat16() for _ in range(2)]
+    want = [newton_schulz(g) for g in gs]
+    streams = [torch.cuda.Stream() for _ in gs]
+    torch.cuda.synchronize()
+    got = [[], []]
+    for _ in range(10):
+        for i, s in enumerate(streams):
+            with torch.cuda.stream(s):
+                got[i].append(newton_schulz(gs[i]))
+    torch.cuda.synchronize()
+    assert all(torch.equal(o, want[i]) for i in range(2) for o in got[i])
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = newton_schulz(gs[0])
+    gs[0].copy_(gs[1])
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, want[1])

@@ -712,7 +712,7 @@ __global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __
 }
 
 // ---------------------------------------------------------------------------------- dQ
-constexpr int kDqThreads = 32 * 12;  // TMA; S, dP; dQ; a spare; eight softmax warps (two per lane quadrant, 64 columns each)
+constexpr int kDqThreads = 32 * 12;  // TMA; S, dP and dQ; two spare; eight softmax warps (two per lane quadrant, 64 columns each)
 
 template <int D>
 struct BwdQCfg {
@@ -1002,8 +1002,8 @@ struct BwdKvCfg {
 // kv head).  Per pair of tiles the tensor core multiplies for 1024 cycles (D = 64; 2048 at D = 128) and the special
 // function unit takes 1024 for the exponentials; the order below keeps both fed: while the softmax warps turn S^T of one
 // tile into P^T, the tensor core runs dK and dP^T of the tile before, and dV and the next S^T while they form dS^T.
-// P^T and dS^T go back over the columns that the same thread read, so no warp waits for another.  The next kv tile's
-// loads and first products run under the last tile of the one before; only the store of dV and dK stands alone.
+// P^T and dS^T go back over the columns that the same thread read (D = 64 has room for P^T beside S^T), so no warp waits for
+// another.  The next kv tile's loads and first products run under the last tile of the one before; only the store of dV and dK stands alone.
 template <int D>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_do,

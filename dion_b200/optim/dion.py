@@ -551,9 +551,13 @@ class Dion(Optimizer):
         cfg = self._get_dion_param_config(params[0])
         if cls is not None and len(cls.params) == len(params) and all(a is b for a, b in zip(cls.params, params)):
             intact = True
+            # the address of M[i] and Q[i], without a view for each (a class of 48: 100 us of every step)
+            m_at, q_at = cls.M.data_ptr(), cls.Q.data_ptr()
+            m_step = cls.M.stride(0) * cls.M.element_size() if cls.M.numel() else 0
+            q_step = cls.Q.stride(0) * cls.Q.element_size() if cls.Q.numel() else 0
             for i, s in enumerate(states):
                 m_loc, q_loc = to_local(s["momentum"]), to_local(s["Q"])
-                if m_loc.data_ptr() != cls.M[i].data_ptr() or q_loc.data_ptr() != cls.Q[i].data_ptr() \
+                if m_loc.data_ptr() != m_at + i * m_step or q_loc.data_ptr() != q_at + i * q_step \
                         or m_loc.dtype != cls.M.dtype or q_loc.dtype != cls.Q.dtype:
                     intact = False
                     break

@@ -9,6 +9,7 @@ missing build.  ``build()`` cross-compiles and works without a GPU.
 from __future__ import annotations
 
 import os
+import subprocess
 import threading
 from pathlib import Path
 from typing import Optional
@@ -45,9 +46,20 @@ def _is_stale() -> bool:
     if not lib.exists():
         return True
     t = lib.stat().st_mtime
-    deps = list(_SRC_DIR.glob("*.cu")) + list(_SRC_DIR.glob("*.cuh")) + list(_SRC_DIR.glob("*.h")) + list(
+    deps = [Path(__file__)] + list(_SRC_DIR.glob("*.cu")) + list(_SRC_DIR.glob("*.cuh")) + list(_SRC_DIR.glob("*.h")) + list(
         _SRC_DIR.glob("*.cpp"))
     return any(p.stat().st_mtime > t for p in deps)
+
+
+def _libstdcxx() -> list[str]:
+    """The C++ library that the process already has, named to the linker.  A compiler that finds no ``libstdc++.so`` takes the
+    archive instead; that second copy has locale tables of its own, and a check whose message prints an integer (a size, a
+    stride) ends the process with a segmentation fault where it should raise."""
+    from torch.utils import cpp_extension
+
+    found = subprocess.run([cpp_extension.get_cxx_compiler(), "-print-file-name=libstdc++.so.6"], capture_output=True, text=True)
+    path = found.stdout.strip()
+    return [path] if os.path.isabs(path) and os.path.exists(path) else []
 
 
 def build(verbose: bool = False, force: bool = False) -> Path:
@@ -66,6 +78,7 @@ def build(verbose: bool = False, force: bool = False) -> Path:
             "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
             "--expt-relaxed-constexpr", "-Xptxas", "-v",
         ] + (["-DDION_B200_DEBUG"] if DEBUG else []),
+        extra_ldflags=_libstdcxx(),
         build_directory=str(_BUILD_DIR),
         is_python_module=False,
         verbose=verbose,

@@ -159,3 +159,28 @@ def test_openmp_compiler_selection(tmp_path, monkeypatch):
         assert chosen != str(broken) and os.environ["CXX"] == chosen and compilers.can_openmp(chosen)
         monkeypatch.setenv("CXX", chosen)
         assert compilers.ensure_openmp_cxx() == chosen
+
+
+def test_a_refused_call_raises_a_message_with_numbers_in_it():
+    """In a process of its own: with a second C++ library in the extension, printing the strides ends it with a signal."""
+    import subprocess
+    import sys
+
+    from dion_b200.ops import _ext
+
+    if not _ext.load(required=False):
+        pytest.skip("extension not built")
+    code = """
+import torch
+from dion_b200.ops import _ext
+_ext.load(required=False)
+x = torch.zeros(8, 8)
+try:
+    torch.ops.dion_b200.gemm_plan(torch.zeros(16, 16)[::2, ::2], x, None, x)
+except RuntimeError as e:
+    assert "strides = [32, 2]" in str(e), e
+    print("raised")
+"""
+    done = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300,
+                          cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert done.returncode == 0 and done.stdout.strip() == "raised", (done.returncode, done.stderr[-500:])

@@ -1047,8 +1047,16 @@ void dion_q_norm(const Tensor& R32, const Tensor& ss, const Tensor& Qm, double e
   DION_CUDA_CHECK(dion::q_norm_launch(a, at::cuda::getCurrentCUDAStream()));
 }
 
+// The attention kernels take bare addresses: one of another device would be read as if it were of this one.
+void check_attention_devices(const Tensor& q, std::initializer_list<const Tensor*> others) {
+  TORCH_CHECK(q.is_cuda(), "attention operands must be CUDA tensors");
+  for (const Tensor* t : others)
+    TORCH_CHECK(t->device() == q.device(), "attention operands must be on one device, not on ", q.device(), " and ", t->device());
+}
+
 // q [B, T, H, D], k / v [B, T, Hkv, D] (contiguous bf16) -> out [B, T, H, D], lse [B, H, T]
 void attn_fwd(const Tensor& q, const Tensor& k, const Tensor& v, Tensor out, Tensor lse, double scale, Tensor status) {
+  check_attention_devices(q, {&k, &v, &out, &lse, &status});
   const c10::cuda::CUDAGuard guard(q.device());
   TORCH_CHECK(q.dim() == 4 && k.dim() == 4 && v.dim() == 4, "attention operands must be [B, T, H, D]");
   TORCH_CHECK(q.scalar_type() == at::kBFloat16 && k.scalar_type() == at::kBFloat16 &&
@@ -1181,6 +1189,7 @@ Tensor gpt_block_fwd(const Tensor& x, const Tensor& wq, const Tensor& wk, const 
 
 void attn_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& d_o, const Tensor& lse,
               Tensor stats, Tensor dq, Tensor dk, Tensor dv, double scale, Tensor status) {
+  check_attention_devices(q, {&k, &v, &o, &d_o, &lse, &stats, &dq, &dk, &dv, &status});
   const c10::cuda::CUDAGuard guard(q.device());
   for (const Tensor* t : std::initializer_list<const Tensor*>{&q, &k, &v, &o, &d_o, &dq, &dk, &dv})
     TORCH_CHECK(t->dim() == 4 && t->scalar_type() == at::kBFloat16 && t->is_contiguous(),

@@ -718,7 +718,7 @@ def flash_attention_forward(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, s
 
 def flash_attention_supported(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor) -> bool:
     B, T, H, D = q.shape
-    return (q.is_cuda and q.dtype == torch.bfloat16 and k.dtype == torch.bfloat16 and v.dtype == torch.bfloat16
+    return (q.is_cuda and q.device == k.device == v.device and q.dtype == torch.bfloat16 and k.dtype == torch.bfloat16 and v.dtype == torch.bfloat16
             and D in (64, 128) and T % 128 == 0 and H % k.shape[2] == 0 and B * H <= 65535
             and q.is_contiguous() and k.is_contiguous() and v.is_contiguous())
 
@@ -759,7 +759,7 @@ def _any_length(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor) -> bool:
     zeros and masked.  What a tracer, a mode or a transform looks at, and other shapes and types, go to the library.
     8 x 777, 12 heads of 64: 26 us against 36, with the backward pass 65 against 81; 24 tokens, 6 heads of 128: 14 against 18."""
     B, T, H, D = q.shape
-    return (q.dtype == k.dtype == v.dtype == torch.bfloat16 and D in (64, 128) and q.numel() > 0 and k.numel() > 0
+    return (q.device == k.device == v.device and q.dtype == k.dtype == v.dtype == torch.bfloat16 and D in (64, 128) and q.numel() > 0 and k.numel() > 0
             and k.dim() == 4 and k.shape[:2] == q.shape[:2] and k.shape[3] == D and v.shape == k.shape
             and H % k.shape[2] == 0 and B * H <= 65535 and not torch.compiler.is_compiling() and not _observed()
             and not any(_transformed(t) for t in (q, k, v)))

@@ -456,6 +456,42 @@ def test_attention_of_other_lengths_keeps_what_the_library_takes_and_refuses():
         grad.float().sum().backward()
 
 
+def test_attention_takes_operands_of_one_device_only(monkeypatch):
+    """The questions that come before the kernels, asked of tensors without memory."""
+    from torch._subclasses.fake_tensor import FakeTensorMode
+
+    with FakeTensorMode():
+        tiles, ragged = ({d: torch.empty(2, T, 4, 64, dtype=torch.bfloat16, device=d) for d in ("cuda:0", "cuda:1", "cpu")}
+                         for T in (128, 100))
+    monkeypatch.setattr(N, "_transformed", lambda t: False)  # a stand-in is a subclass
+    for ask, t in ((N.flash_attention_supported, tiles), (N._any_length, ragged)):
+        q = t["cuda:0"]
+        assert ask(q, q, q)
+        for other in (t["cuda:1"], t["cpu"]):
+            assert not ask(q, other, q) and not ask(q, q, other)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T", [128, 100])
+def test_attention_refuses_operands_of_another_device(T):
+    from dion_b200.ops import runtime
+
+    q, far = torch.zeros(1, T, 2, 64, device="cuda").bfloat16(), torch.zeros(1, T, 2, 64).bfloat16()
+    lse, stats, status = torch.zeros(1, 2, T, device="cuda"), torch.zeros(2, 1, 2, 128, device="cuda"), runtime.status_tensor(q.device)
+    for k, v in ((far, far), (far, q), (q, far)):
+        with pytest.raises(RuntimeError):
+            N.causal_attention(q, k, v)
+    op = torch.ops.dion_b200
+    for args in ((q, far, q, q, lse), (q, q, far, q, lse), (q, q, q, far, lse), (q, q, q, q, lse.cpu()), (far, q, q, q, lse)):
+        with pytest.raises(RuntimeError, match="attention operands must be"):
+            op.attn_fwd(*args, 0.125, status)
+    good = [q, q, q, q, q, lse, stats, q.clone(), q.clone(), q.clone()]
+    for i in range(len(good)):
+        args = good[:i] + [good[i].cpu()] + good[i + 1:]
+        with pytest.raises(RuntimeError, match="attention operands must be"):
+            op.attn_bwd(*args, 0.125, status)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("shape", [(64, 384, 6, 6, 128), (64, 512, 6, 3, 64), (2, 2048, 16, 4, 128), (64, 333, 6, 6, 128)])
 def test_flash_attention_gives_the_same_bits_in_every_run(shape):

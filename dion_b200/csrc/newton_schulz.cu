@@ -97,6 +97,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     sh.abort = 0;
     mbar_fence_init();
   }
+  pdl_wait();  // before tensor memory is taken, which a kernel ahead of this one may still be waiting for
   if (warp == 8) {
     tmem_alloc(&sh.tmem, kTmemCols);
     tmem_relinquish();
@@ -106,7 +107,6 @@ __global__ void __launch_bounds__(kThreads, 1)
   tc_fence_after();
   const uint32_t tmem = warp_uniform(sh.tmem);
   volatile int* abort_flag = &sh.abort;
-  pdl_wait();
 
   const int k = p.k, L = p.L, pitch = p.pitch;
   bf16* X = p.X + (long long)batch * k * pitch;

@@ -5,12 +5,13 @@
 // The rules that every kernel launched this way keeps:
 //  * all its threads that touch global memory call pdl_wait() before they do, in every CTA.  It returns when the kernels
 //    before this one have completed and their writes are visible, so that chains of such kernels stay ordered;
-//  * tensor memory is allocated after pdl_wait(): CTAs that wait must not hold what the kernel before them needs;
+//  * tensor memory is allocated after pdl_wait(): CTAs that wait must not hold what the kernel before them needs.  Sharing an
+//    SM, the two would wait for each other;
 //  * no thread waits for another kernel's CTA.
-//  * a kernel that wants its CTAs on SMs of their own is too large for two of them on one: early CTAs gather on the SMs that
-//    are free first (the Cholesky inverse of a few matrices: 5 % of an optimizer step of the 8B shape, so it starts plainly).
-// Newton-Schulz of one 256 x 256 matrix (17 kernels) 130 -> 103 us, a Muon step on ragged matrices (61)
-// 992 -> 910, logits of 8 x 777 tokens (100) 1842 -> 1728.
+// A kernel that wants its CTAs on SMs of their own, but is small enough for two of them on one, is launched plainly: early CTAs
+// gather on the SMs that are free first (the Cholesky inverse in an optimizer step of the 8B shape: 8142 us, launched early 8192).
+// Newton-Schulz of one 256 x 256 matrix as 17 kernels 130 -> 103 us (it is one kernel now), a Muon step on ragged matrices (61)
+// 992 -> 910, logits of 8 x 777 tokens (100) 1842 -> 1708.
 // pdl_trigger() lets the next kernel of the stream start as soon as every CTA of this one has called it (or exited).
 #pragma once
 

@@ -184,3 +184,34 @@ except RuntimeError as e:
     done = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300,
                           cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
     assert done.returncode == 0 and done.stdout.strip() == "raised", (done.returncode, done.stderr[-500:])
+
+
+def _kernels():
+    """(file, name, body) of every kernel in the sources."""
+    import re
+
+    from dion_b200.ops import _ext
+
+    for path in _ext.sources():
+        text = path.read_text()
+        for m in re.finditer(r"__global__ void(?:\s+__launch_bounds__\((?:[^()]|\([^()]*\))*\))?\s+(\w+)\s*\(", text):
+            start = text.index("{", m.end())
+            depth, end = 1, start + 1
+            while depth:
+                depth += {"{": 1, "}": -1}.get(text[end], 0)
+                end += 1
+            yield path.name, m.group(1), text[start:end]
+
+
+def test_kernels_that_start_early_wait_before_they_take_tensor_memory():
+    """A CTA that holds tensor memory while it waits for the kernel before it could keep that kernel from its own."""
+    seen = set()
+    for file, name, body in _kernels():
+        if "pdl_trigger();" not in body:
+            continue
+        seen.add(name)
+        assert body.count("pdl_wait();") == 1, (file, name)
+        if "tmem_alloc" in body:
+            assert body.index("pdl_wait();") < body.index("tmem_alloc"), (file, name)
+    assert {"gemm_kernel", "attn_fwd_kernel", "attn_bwd_dq_kernel", "attn_bwd_dkv_kernel", "newton_schulz_kernel",
+            "cross_entropy_kernel", "adamw_kernel"} <= seen

@@ -26,6 +26,7 @@
 #include "gemm.h"
 #include "kernels.h"
 #include "pdl.cuh"
+#include "per_device.h"
 #include "umma.cuh"
 
 namespace dion {
@@ -1395,15 +1396,14 @@ cudaError_t attn_fwd_launch_d(const void* q, const void* k, const void* v, void*
       !attn_tmap_seq(&tv, v, (uint64_t)Hkv * D, T, B))
     return cudaErrorInvalidValue;
   auto kernel = attn_fwd_kernel<D>;
-  static bool attr_set = false;
-  if (!attr_set) {
+  static std::atomic<unsigned long long> granted{0};
+  const cudaError_t e = once_per_device(granted, [&] {
     cudaFuncAttributes fa;
     // the register shares of the kernel's warps add up to what it is launched with, or the larger one waits forever
     if (cudaFuncGetAttributes(&fa, kernel) != cudaSuccess || fa.numRegs != 168) return cudaErrorInvalidConfiguration;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
-    if (e != cudaSuccess) return e;
-    attr_set = true;
-  }
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
+  });
+  if (e != cudaSuccess) return e;
   AttnParams p;
   p.out = reinterpret_cast<__nv_bfloat16*>(out);
   p.lse = lse;
@@ -1435,17 +1435,15 @@ cudaError_t attn_bwd_launch_d(const void* q, const void* k, const void* v, const
     return cudaErrorInvalidValue;
   auto kq = attn_bwd_dq_kernel<D>;
   auto kkv = attn_bwd_dkv_kernel<D>;
-  static bool attr_set = false;
-  if (!attr_set) {
+  static std::atomic<unsigned long long> granted{0};
+  const cudaError_t e = once_per_device(granted, [&] {
     cudaFuncAttributes fa;
     // the register shares of the kernel's warps add up to what it is launched with, or the larger one waits forever
     if (cudaFuncGetAttributes(&fa, kq) != cudaSuccess || fa.numRegs != 168) return cudaErrorInvalidConfiguration;
-    cudaError_t e = cudaFuncSetAttribute(kq, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdQCfg<D>::SMEM);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(kkv, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdKvCfg<D>::SMEM);
-    if (e != cudaSuccess) return e;
-    attr_set = true;
-  }
+    const cudaError_t set = cudaFuncSetAttribute(kq, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdQCfg<D>::SMEM);
+    return set != cudaSuccess ? set : cudaFuncSetAttribute(kkv, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdKvCfg<D>::SMEM);
+  });
+  if (e != cudaSuccess) return e;
   const int tiles = (T + kBM - 1) / kBM, t_pad = tiles * kBM;
   float* neg_lse2 = stats;
   float* neg_delta = stats + (long long)B * H * t_pad;

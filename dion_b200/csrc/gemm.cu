@@ -30,6 +30,7 @@
 #include <string>
 
 #include "pdl.cuh"
+#include "per_device.h"
 #include "umma.cuh"
 
 namespace dion {
@@ -1626,12 +1627,10 @@ cudaError_t launch_cfg(const GemmArgs& a, const KernelParams& kp, cudaStream_t s
 
   auto kernel = gemm_kernel<kTf32, kAMajor, kBMajor, kBlockN, kPair, kGather, kSplit, kClusterK, kTmaEpi, kF32Out, kPtrs>;
   constexpr int kThreads = kNumThreads + (kGather ? kNumGatherThreads : 0) + (kSplit ? kNumSplitThreads : 0);
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
-    if (e != cudaSuccess) return e;
-    attr_set = true;
-  }
+  static std::atomic<unsigned long long> granted{0};
+  const cudaError_t e = once_per_device(
+      granted, [&] { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES); });
+  if (e != cudaSuccess) return e;
   int grid = a.max_ctas > 0 ? a.max_ctas : num_sms();
   if constexpr (kPair || kClusterK) {
     const int cluster = kPair ? 2 : kp.cluster_k;

@@ -19,6 +19,7 @@
 #include "gemm.h"
 #include "kernels.h"
 #include "pdl.cuh"
+#include "per_device.h"
 #include "umma.cuh"
 
 namespace dion {
@@ -339,16 +340,10 @@ cudaError_t newton_schulz_launch(void* X, void* A, void* P, void* Xt0, void* Xt1
   p.X = (bf16*)X, p.A = (bf16*)A, p.Xt[0] = (bf16*)Xt0, p.Xt[1] = (bf16*)Xt1;
   p.k = k, p.L = L, p.pitch = pitch, p.steps = steps, p.tall = tall, p.status = status;
   for (int i = 0; i < 3 * kMaxSteps; ++i) p.coeffs[i] = i < 3 * steps ? coeffs[i] : 0.f;
-  static std::atomic<unsigned long long> granted{0};  // a bit per device
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
+  static std::atomic<unsigned long long> granted{0};
+  const cudaError_t e = once_per_device(
+      granted, [] { return cudaFuncSetAttribute(newton_schulz_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes); });
   if (e != cudaSuccess) return e;
-  const unsigned long long bit = 1ull << (dev & 63);
-  if (!(granted.load(std::memory_order_acquire) & bit)) {
-    e = cudaFuncSetAttribute(newton_schulz_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-    if (e != cudaSuccess) return e;
-    granted.fetch_or(bit, std::memory_order_release);
-  }
   const unsigned c = cluster_size(batch, k, L);
   if (c == 0) return cudaErrorInvalidValue;
   return launch_pdl(newton_schulz_kernel, dim3(c, batch), dim3(kThreads), kSmemBytes, stream, c, mx, ma, mp, m0, m1, p);

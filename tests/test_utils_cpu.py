@@ -215,3 +215,50 @@ def test_kernels_that_start_early_wait_before_they_take_tensor_memory():
             assert body.index("pdl_wait();") < body.index("tmem_alloc"), (file, name)
     assert {"gemm_kernel", "attn_fwd_kernel", "attn_bwd_dq_kernel", "attn_bwd_dkv_kernel", "newton_schulz_kernel",
             "cross_entropy_kernel", "adamw_kernel"} <= seen
+
+
+def test_what_a_kernel_needs_once_per_device(tmp_path):
+    """The helper behind every opt-in to large shared memory, against a runtime that only names the current device."""
+    import re
+    import shutil
+    import subprocess
+
+    from dion_b200.ops import _ext
+
+    src = _ext.sources()[0].parent
+    for path in src.glob("*.cu"):  # the opt-in belongs to a device: one flag for all of them skips it on the second
+        assert not re.search(r"static bool \w+ = false;", path.read_text()), path.name
+    cxx, cuda = os.environ.get("CXX", "g++"), os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    if not (shutil.which(cxx) and os.path.exists(os.path.join(cuda, "include", "cuda_runtime.h"))):
+        pytest.skip("no compiler")
+    (tmp_path / "t.cpp").write_text(r"""
+#include "per_device.h"
+#include <stdio.h>
+#include <thread>
+static thread_local int current = 0;
+extern "C" cudaError_t cudaGetDevice(int* d) { *d = current; return current < 0 ? cudaErrorNoDevice : cudaSuccess; }
+int main() {
+  std::atomic<unsigned long long> done{0};
+  std::atomic<int> calls[80] = {};
+  bool fail = true;
+  auto on = [&](int dev) {
+    current = dev;
+    return dion::once_per_device(done, [&] { ++calls[current]; return fail ? cudaErrorInvalidValue : cudaSuccess; });
+  };
+  bool ok = on(3) == cudaErrorInvalidValue && on(3) == cudaErrorInvalidValue;  // a failure is not remembered
+  fail = false;
+  for (int round = 0; round < 2; ++round)
+    for (int dev : {0, 1, 3, 63, 64, 70}) ok = ok && on(dev) == cudaSuccess;
+  ok = ok && calls[0] == 1 && calls[1] == 1 && calls[3] == 3 && calls[63] == 1 && calls[64] == 2 && calls[70] == 2;
+  ok = ok && on(-1) == cudaErrorNoDevice;
+  std::thread ts[8];
+  std::atomic<bool> all{true};
+  for (auto& t : ts) t = std::thread([&] { if (on(5) != cudaSuccess || calls[5] == 0) all = false; });
+  for (auto& t : ts) t.join();
+  puts(ok && all && calls[5] >= 1 ? "ok" : "wrong");
+}
+""")
+    exe = tmp_path / "t"
+    subprocess.run([cxx, "-std=c++17", "-pthread", f"-I{src}", f"-I{cuda}/include", str(tmp_path / "t.cpp"), "-o", str(exe)],
+                   check=True, capture_output=True)
+    assert subprocess.run([str(exe)], capture_output=True, text=True).stdout.strip() == "ok"

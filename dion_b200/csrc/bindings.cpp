@@ -1195,6 +1195,7 @@ Tensor gpt_block_fwd(const Tensor& x, const Tensor& wq, const Tensor& wk, const 
 
 void attn_bwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& o_, const Tensor& d_o_, const Tensor& lse,
               Tensor stats, Tensor dq, Tensor dk, Tensor dv, double scale, Tensor status) {
+  TORCH_CHECK(k.size(0) == B && k.size(1) == T && k.size(3) == D, "attention: k ", k.sizes(), " does not go with q ", q.sizes());
   check_attention_devices(q_, {&k_, &v_, &o_, &d_o_, &lse, &stats, &dq, &dk, &dv, &status});
   const c10::cuda::CUDAGuard guard(q_.device());
   const Tensor q = aligned(q_), k = aligned(k_), v = aligned(v_), o = aligned(o_), d_o = aligned(d_o_);

@@ -1054,10 +1054,16 @@ void check_attention_devices(const Tensor& q, std::initializer_list<const Tensor
     TORCH_CHECK(t->device() == q.device(), "attention operands must be on one device, not on ", q.device(), " and ", t->device());
 }
 
+bool on_16_bytes(const Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0; }
+// an operand where TMA and 16-byte loads can take it
+Tensor aligned(const Tensor& t) { return on_16_bytes(t) ? t : t.clone(); }
+
 // q [B, T, H, D], k / v [B, T, Hkv, D] (contiguous bf16) -> out [B, T, H, D], lse [B, H, T]
-void attn_fwd(const Tensor& q, const Tensor& k, const Tensor& v, Tensor out, Tensor lse, double scale, Tensor status) {
-  check_attention_devices(q, {&k, &v, &out, &lse, &status});
-  const c10::cuda::CUDAGuard guard(q.device());
+void attn_fwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, Tensor out, Tensor lse, double scale, Tensor status) {
+  check_attention_devices(q_, {&k_, &v_, &out, &lse, &status});
+  const c10::cuda::CUDAGuard guard(q_.device());
+  const Tensor q = aligned(q_), k = aligned(k_), v = aligned(v_);
+  TORCH_CHECK(on_16_bytes(out), "attention results must start on 16 bytes");
   TORCH_CHECK(q.dim() == 4 && k.dim() == 4 && v.dim() == 4, "attention operands must be [B, T, H, D]");
   TORCH_CHECK(q.scalar_type() == at::kBFloat16 && k.scalar_type() == at::kBFloat16 &&
               v.scalar_type() == at::kBFloat16 && out.scalar_type() == at::kBFloat16 && lse.scalar_type() == at::kFloat);
@@ -1187,10 +1193,12 @@ Tensor gpt_block_fwd(const Tensor& x, const Tensor& wq, const Tensor& wk, const 
   return linear(u, wproj, x3, 0).view({B, T, C});
 }
 
-void attn_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& d_o, const Tensor& lse,
+void attn_bwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& o_, const Tensor& d_o_, const Tensor& lse,
               Tensor stats, Tensor dq, Tensor dk, Tensor dv, double scale, Tensor status) {
-  check_attention_devices(q, {&k, &v, &o, &d_o, &lse, &stats, &dq, &dk, &dv, &status});
-  const c10::cuda::CUDAGuard guard(q.device());
+  check_attention_devices(q_, {&k_, &v_, &o_, &d_o_, &lse, &stats, &dq, &dk, &dv, &status});
+  const c10::cuda::CUDAGuard guard(q_.device());
+  const Tensor q = aligned(q_), k = aligned(k_), v = aligned(v_), o = aligned(o_), d_o = aligned(d_o_);
+  for (const Tensor* t : {&stats, &dq, &dk, &dv}) TORCH_CHECK(on_16_bytes(*t), "attention results must start on 16 bytes");
   for (const Tensor* t : std::initializer_list<const Tensor*>{&q, &k, &v, &o, &d_o, &dq, &dk, &dv})
     TORCH_CHECK(t->dim() == 4 && t->scalar_type() == at::kBFloat16 && t->is_contiguous(),
                 "attention tensors must be contiguous bf16 [B, T, H, D]");

@@ -748,10 +748,7 @@ class _FlashAttnAnyLengthFn(_FlashAttnFn):
     @staticmethod
     @torch.autograd.function.once_differentiable
     def backward(ctx, d_out):
-        q, k, v, out, lse = ctx.saved_tensors
-        if d_out.is_contiguous() and d_out.data_ptr() % 16:
-            d_out = d_out.clone()
-        return _attention_backward(q, k, v, out, lse, d_out)
+        return _FlashAttnFn.backward(ctx, d_out)
 
 
 def _any_length(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor) -> bool:

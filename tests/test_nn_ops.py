@@ -472,6 +472,25 @@ def test_attention_takes_operands_of_one_device_only(monkeypatch):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("T", [100, 128, 384])
+def test_attention_of_tensors_on_odd_addresses(T):
+    """q, k, v and the gradient that comes in, contiguous but shifted by one element: the bits of aligned copies."""
+    def shifted(*shape):
+        n = torch.Size(shape).numel()
+        return torch.randn(n + 1, device="cuda").bfloat16()[1:].view(shape)
+
+    def run(q, k, v, dy):
+        q, k, v = (t.detach().requires_grad_() for t in (q, k, v))
+        y = N.causal_attention(q, k, v)
+        return (y, *torch.autograd.grad(y, (q, k, v), dy))
+
+    ts = shifted(2, T, 4, 64), shifted(2, T, 2, 64), shifted(2, T, 2, 64), shifted(2, T, 256)
+    assert all(t.data_ptr() % 16 and t.is_contiguous() for t in ts)
+    for got, want in zip(run(*ts), run(*(t.clone() for t in ts))):
+        assert torch.equal(got, want)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("T", [128, 100])
 def test_attention_refuses_operands_of_another_device(T):
     from dion_b200.ops import runtime

@@ -1205,6 +1205,7 @@ void attn_bwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor
   const int64_t B = q.size(0), T = q.size(1), H = q.size(2), D = q.size(3), Hkv = k.size(2);
   TORCH_CHECK(lse.scalar_type() == at::kFloat && stats.scalar_type() == at::kFloat && lse.is_contiguous() &&
               stats.is_contiguous() && stats.numel() >= 2 * B * H * ((T + 127) / 128 * 128));
+  TORCH_CHECK(k.size(0) == B && k.size(1) == T && k.size(3) == D, "attention: k ", k.sizes(), " does not go with q ", q.sizes());
   TORCH_CHECK(o.sizes() == q.sizes() && d_o.sizes() == q.sizes() && dq.sizes() == q.sizes() && v.sizes() == k.sizes() &&
               dk.sizes() == k.sizes() && dv.sizes() == k.sizes() && lse.numel() == B * H * T);
   g_launches += 3;

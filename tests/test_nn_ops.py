@@ -364,6 +364,17 @@ def test_flash_attention_backward_matches_fp32_reference(shape):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(1, 128, 2, 64), (2, 64, 2, 64), (2, 256, 2, 64), (2, 128, 2, 128)])
+def test_attention_backward_refuses_keys_of_other_sizes(shape):
+    """Sequences, rows or columns that q does not have: the kernels would read k and v where they are not."""
+    from dion_b200.ops.nn import flash_attention_backward
+
+    q, k = torch.zeros(2, 128, 4, 64, device="cuda").bfloat16(), torch.zeros(shape, device="cuda").bfloat16()
+    with pytest.raises(RuntimeError, match="does not go with q"):
+        flash_attention_backward(q, k, k, q, torch.zeros(2, 4, 128, device="cuda"), q)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("shape", [
     (150, 128, 1, 1, 128),  # one tile per head; a head for every CTA and two left over
     (40, 256, 4, 4, 64),    # pairs of query tiles, 160 heads

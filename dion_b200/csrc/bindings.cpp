@@ -420,6 +420,7 @@ void for_each_chunk(std::initializer_list<std::pair<int, at::TensorList>> lists,
   }
 }
 
+// checks a launch and counts it
 #define DION_CUDA_CHECK(expr)                                                           \
   do {                                                                                  \
     cudaError_t _e = (expr);                                                            \
@@ -512,10 +513,9 @@ void frob_scale(const Tensor& x, Tensor out, const std::optional<Tensor>& sumsq,
   if (sumsq.has_value()) {
     TORCH_CHECK(sumsq->scalar_type() == at::kFloat && sumsq->is_contiguous() && sumsq->numel() >= B);
     ss = sumsq->data_ptr<float>();
-    g_launches += 1;
   } else {
     partial = at::empty({B * dion::frob_chunks(per)}, x.options().dtype(at::kFloat));
-    g_launches += 2;
+    g_launches += 1;  // the partial sums
   }
   DION_CUDA_CHECK(dion::frob_scale_launch(x.data_ptr(), out.data_ptr(), ss ? nullptr : partial.data_ptr<float>(), ss,
                                           (float)eps, (int)B, per, at::cuda::getCurrentCUDAStream()));
@@ -603,7 +603,6 @@ void rmsnorm_gain_fwd(const Tensor& x, const Tensor& gain, Tensor y, Tensor rstd
   const int64_t rows = x.numel() / dim;
   TORCH_CHECK(x.is_contiguous() && y.is_contiguous() && gain.is_contiguous() && gain.numel() == dim);
   TORCH_CHECK(rstd.scalar_type() == at::kFloat && rstd.numel() == rows);
-  ++g_launches;
   DION_CUDA_CHECK(dion::rmsnorm_gain_fwd_launch(x.data_ptr(), gain.data_ptr(), elem_type(gain, "gain"), y.data_ptr(),
                                                 rstd.data_ptr<float>(), rows, dim, (float)eps,
                                                 at::cuda::getCurrentCUDAStream()));
@@ -620,7 +619,6 @@ Tensor rmsnorm_gain_bwd(const Tensor& dy, const Tensor& x, const Tensor& rstd, c
   TORCH_CHECK(dy.is_contiguous() && x.is_contiguous() && dx.is_contiguous() && gain.is_contiguous() && gain.numel() == dim);
   const int blocks = dion::rmsnorm_gain_bwd_blocks(rows);
   Tensor partial = at::empty({blocks, dim}, x.options().dtype(at::kFloat));
-  ++g_launches;
   DION_CUDA_CHECK(dion::rmsnorm_gain_bwd_launch(dy.data_ptr(), x.data_ptr(), rstd.data_ptr<float>(), gain.data_ptr(),
                                                 elem_type(gain, "gain"), dx.data_ptr(), partial.data_ptr<float>(), blocks,
                                                 rows, dim, at::cuda::getCurrentCUDAStream()));
@@ -633,7 +631,6 @@ void swiglu_fwd(const Tensor& g, const Tensor& u, Tensor h) {
   check_bf16(h, "h");
   const c10::cuda::CUDAGuard guard(g.device());
   TORCH_CHECK(g.is_contiguous() && u.is_contiguous() && h.is_contiguous() && u.numel() == g.numel() && h.numel() == g.numel());
-  ++g_launches;
   DION_CUDA_CHECK(dion::swiglu_fwd_launch(g.data_ptr(), u.data_ptr(), h.data_ptr(), g.numel(), at::cuda::getCurrentCUDAStream()));
 }
 
@@ -646,7 +643,6 @@ void swiglu_bwd(const Tensor& dh, const Tensor& g, const Tensor& u, Tensor dg, T
   const c10::cuda::CUDAGuard guard(g.device());
   TORCH_CHECK(dh.is_contiguous() && g.is_contiguous() && u.is_contiguous() && dg.is_contiguous() && du.is_contiguous());
   TORCH_CHECK(dh.numel() == g.numel() && u.numel() == g.numel() && dg.numel() == g.numel() && du.numel() == g.numel());
-  ++g_launches;
   DION_CUDA_CHECK(dion::swiglu_bwd_launch(dh.data_ptr(), g.data_ptr(), u.data_ptr(), dg.data_ptr(), du.data_ptr(), g.numel(),
                                           at::cuda::getCurrentCUDAStream()));
 }
@@ -732,7 +728,6 @@ void scale_by_scalar(const Tensor& x, Tensor y, const Tensor& scale) {
               "scale_by_scalar: contiguous tensors of one size and type");
   TORCH_CHECK(scale.numel() == 1 && scale.scalar_type() == at::kFloat && scale.device() == x.device(),
               "scale_by_scalar: the scale is one fp32 value on the same device");
-  ++g_launches;
   DION_CUDA_CHECK(dion::scale_by_scalar_launch(x.data_ptr(), y.data_ptr(), elem_type(x, "x"), x.numel(),
                                                scale.data_ptr<float>(), at::cuda::getCurrentCUDAStream()));
 }
@@ -915,7 +910,6 @@ void slot_reduce(const Tensor& slots, const std::optional<Tensor>& out, const st
   a.ndest = (int)dests.size();
   for (size_t i = 0; i < dests.size(); ++i) a.dest[i] = reinterpret_cast<float*>(dests[i]);
   a.status = status.data_ptr<int>();
-  ++g_launches;
   DION_CUDA_CHECK(dion::slot_reduce_launch(a, at::cuda::getCurrentCUDAStream()));
 }
 
@@ -939,7 +933,6 @@ void slot_reduce_bf16(const Tensor& slots, Tensor out, const std::optional<Tenso
     a.residual = residual->data_ptr();
   }
   a.status = status.data_ptr<int>();
-  ++g_launches;
   DION_CUDA_CHECK(dion::slot_reduce_bf16_launch(a, at::cuda::getCurrentCUDAStream()));
 }
 
@@ -1009,7 +1002,6 @@ void dion_r_post(const Tensor& slots, double scale, const std::optional<Tensor>&
     a.qs_cols = (int)Qs->size(2);
   }
   a.status = status.data_ptr<int>();
-  ++g_launches;
   DION_CUDA_CHECK(dion::r_post_launch(a, at::cuda::getCurrentCUDAStream()));
 }
 
@@ -1043,7 +1035,6 @@ void dion_q_norm(const Tensor& R32, const Tensor& ss, const Tensor& Qm, double e
     a.qs_col0 = (int)qs_col0;
     a.qs_cols = (int)Qs->size(2);
   }
-  ++g_launches;
   DION_CUDA_CHECK(dion::q_norm_launch(a, at::cuda::getCurrentCUDAStream()));
 }
 
@@ -1071,7 +1062,6 @@ void attn_fwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, Tensor out, 
   const int64_t B = q.size(0), T = q.size(1), H = q.size(2), D = q.size(3), Hkv = k.size(2);
   TORCH_CHECK(k.size(0) == B && k.size(1) == T && k.size(3) == D && v.sizes() == k.sizes() && out.sizes() == q.sizes());
   TORCH_CHECK(lse.numel() == B * H * T);
-  ++g_launches;
   DION_CUDA_CHECK(dion::attn_fwd_launch(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr<float>(),
                                         (int)B, (int)T, (int)H, (int)Hkv, (int)D, (float)scale, status.data_ptr<int>(),
                                         at::cuda::getCurrentCUDAStream()));
@@ -1208,7 +1198,7 @@ void attn_bwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor
   TORCH_CHECK(k.size(0) == B && k.size(1) == T && k.size(3) == D, "attention: k ", k.sizes(), " does not go with q ", q.sizes());
   TORCH_CHECK(o.sizes() == q.sizes() && d_o.sizes() == q.sizes() && dq.sizes() == q.sizes() && v.sizes() == k.sizes() &&
               dk.sizes() == k.sizes() && dv.sizes() == k.sizes() && lse.numel() == B * H * T);
-  g_launches += 3;
+  g_launches += 2;  // row sums, dK and dV; then dQ
   DION_CUDA_CHECK(dion::attn_bwd_launch(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), d_o.data_ptr(),
                                         lse.data_ptr<float>(), stats.data_ptr<float>(), dq.data_ptr(), dk.data_ptr(),
                                         dv.data_ptr(), (int)B, (int)T, (int)H, (int)Hkv, (int)D, (float)scale,
@@ -1220,7 +1210,6 @@ void split_tf32(const Tensor& x, Tensor hi, Tensor lo) {
   TORCH_CHECK(x.scalar_type() == at::kFloat && hi.scalar_type() == at::kFloat && lo.scalar_type() == at::kFloat);
   TORCH_CHECK(x.is_contiguous() && hi.is_contiguous() && lo.is_contiguous() && hi.numel() == x.numel() &&
               lo.numel() == x.numel());
-  ++g_launches;
   DION_CUDA_CHECK(dion::split_tf32_launch(x.data_ptr<float>(), hi.data_ptr<float>(), lo.data_ptr<float>(), x.numel(),
                                           at::cuda::getCurrentCUDAStream()));
 }
@@ -1231,7 +1220,6 @@ void jacobi_scale(const Tensor& G, Tensor W, Tensor d) {
   const int64_t B = G.size(0), r = G.size(1);
   TORCH_CHECK(W.scalar_type() == at::kFloat && W.is_contiguous() && W.numel() == B * r * r);
   TORCH_CHECK(d.scalar_type() == at::kFloat && d.is_contiguous() && d.numel() == B * r);
-  ++g_launches;
   DION_CUDA_CHECK(dion::jacobi_scale_launch(G.data_ptr<float>(), W.data_ptr<float>(), d.data_ptr<float>(), (int)B, (int)r,
                                             G.stride(1), G.stride(0), at::cuda::getCurrentCUDAStream()));
 }
@@ -1244,7 +1232,6 @@ void place_block(const Tensor& Zd, const Tensor& mask, Tensor Z, Tensor Zm, int6
   TORCH_CHECK(Z.scalar_type() == at::kFloat && Z.dim() == 3 && Z.is_contiguous() && Z.size(0) == B && Z.size(1) == Z.size(2));
   TORCH_CHECK(Zm.scalar_type() == at::kFloat && Zm.is_contiguous() && Zm.numel() == Zd.numel());
   TORCH_CHECK(mask.scalar_type() == at::kFloat && mask.is_contiguous() && mask.numel() == B * nb);
-  ++g_launches;
   DION_CUDA_CHECK(dion::place_block_launch(Zd.data_ptr<float>(), mask.data_ptr<float>(), Z.data_ptr<float>(),
                                            Zm.data_ptr<float>(), (int)B, (int)nb, (int)Z.size(1), (int)k0,
                                            at::cuda::getCurrentCUDAStream()));
@@ -1256,7 +1243,6 @@ void split_tf32_rows(const Tensor& x, Tensor hi, Tensor lo) {
   TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kFloat && x.dim() == 3 && x.stride(2) == 1);
   TORCH_CHECK(hi.scalar_type() == at::kFloat && lo.scalar_type() == at::kFloat && hi.is_contiguous() &&
               lo.is_contiguous() && hi.numel() == x.numel() && lo.numel() == x.numel());
-  ++g_launches;
   DION_CUDA_CHECK(dion::split_tf32_rows_launch(x.data_ptr<float>(), hi.data_ptr<float>(), lo.data_ptr<float>(),
                                                (int)x.size(0), (int)x.size(1), (int)x.size(2), x.stride(1), x.stride(0),
                                                at::cuda::getCurrentCUDAStream()));
@@ -1271,7 +1257,6 @@ void refine_prep(const Tensor& G, Tensor C, Tensor d, double dead_below, const s
   if (skip.has_value())
     TORCH_CHECK(skip->scalar_type() == at::kInt && skip->is_cuda() && skip->is_contiguous() && skip->numel() == G.size(0),
                 "skip must be one int32 per matrix");
-  ++g_launches;
   DION_CUDA_CHECK(dion::refine_prep_launch(G.data_ptr<float>(), C.data_ptr<float>(), d.data_ptr<float>(),
                                            (int)G.size(0), (int)G.size(1), (float)dead_below,
                                            skip.has_value() ? skip->data_ptr<int>() : nullptr, fold,
@@ -1284,7 +1269,6 @@ void symm_all_gather(const Tensor& inp, Tensor out, at::IntArrayRef peers, int64
   const c10::cuda::CUDAGuard guard(inp.device());
   TORCH_CHECK(inp.is_contiguous() && out.is_contiguous() && inp.scalar_type() == out.scalar_type());
   TORCH_CHECK(out.numel() == inp.numel() * (int64_t)peers.size(), "all-gather output must hold every rank's input");
-  ++g_launches;
   DION_CUDA_CHECK(dion::symm_all_gather_launch(peer_table(peers), flag_off, slot_off, inp.data_ptr(), out.data_ptr(),
                                                inp.numel() * inp.element_size(), (int)rank, (int)peers.size(),
                                                (unsigned)epoch, (int)channel,
@@ -1301,7 +1285,6 @@ void symm_reduce_scatter(const Tensor& inp, Tensor out, at::IntArrayRef peers, i
   TORCH_CHECK(inp.numel() == out.numel() * (int64_t)peers.size(), "reduce-scatter input must hold one slice per rank");
   TORCH_CHECK(reinterpret_cast<int64_t>(inp.data_ptr()) == peers[rank] + data_off,
               "input is not at the stated offset of this rank's arena");
-  ++g_launches;
   DION_CUDA_CHECK(dion::symm_reduce_scatter_launch(
       peer_table(peers), flag_off, data_off, reinterpret_cast<void*>(mc_base), elem_type(inp, "input"), out.data_ptr(),
       out.numel(), (float)scale, (int)rank, (int)peers.size(), (unsigned)epoch, (int)ch_start, (int)ch_end,

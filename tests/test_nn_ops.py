@@ -843,3 +843,39 @@ def test_halved_input_gradient_of_the_loss():
     want = (p / T) @ wb
     # logits of about 0.55, the probabilities and dx are rounded to bf16 once each (2^-9 relative)
     assert ((runs[0][0].float() - want).norm() / want.norm()).item() < 3 * 2.0 ** -9
+
+
+@pytest.mark.gpu
+def test_every_launch_is_counted_once():
+    """The count of a training step, and of Newton-Schulz with and without norms in hand, against a profile of the same."""
+    from torch.profiler import ProfilerActivity, profile
+
+    from dion_b200 import Dion, ops
+    from dion_b200.models import GPT, GPTConfig
+    from dion_b200.optim.newton_schulz import newton_schulz
+
+    with torch.device("cuda"):
+        model = GPT(GPTConfig(sequence_len=128, vocab_size=1024, n_layer=2, n_head=4, n_embd=256))
+    model.init_weights()
+    hidden = [p for p in model.parameters() if p.dim() == 2 and p.shape[0] <= 1024 and p.shape != (1024, 256)]
+    rest = [p for p in model.parameters() if all(p is not h for h in hidden)]
+    opt = Dion([dict(params=hidden), dict(params=rest, algorithm="lion")], lr=1e-3, rank_fraction=0.25)
+    idx = torch.randint(0, 1024, (2, 128), device="cuda")
+    g = torch.randn(2, 300, 520, device="cuda").bfloat16()
+
+    def step():
+        model(idx, idx).backward()
+        opt.step()
+        opt.zero_grad()
+        newton_schulz(g)
+        newton_schulz(g, sumsq=g.float().square().sum((1, 2)))
+
+    for _ in range(2):
+        step()
+    torch.cuda.synchronize()
+    before = ops.launch_count()
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        step()
+        torch.cuda.synchronize()
+    kernels = [e.name for e in prof.events() if e.device_type == torch.autograd.DeviceType.CUDA and "dion::" in e.name]
+    assert ops.launch_count() - before == len(kernels) > 100

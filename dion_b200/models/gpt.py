@@ -157,8 +157,10 @@ class Block(nn.Module):
         if any(w.data_ptr() % 16 for w in shadows) or not (weights[0].shape == weights[1].shape == weights[2].shape):
             return None
         cos, sin = attn.rotary.tables(x.shape[1], x.device)
-        return torch.ops.dion_b200.gpt_block_fwd(x, *shadows, cos, sin, attn.head_dim, K.RMS_EPS,
-                                                 K.ATTENTION_IMPL == "kernel", K.runtime.status_tensor(x.device))
+        heads = weights[0].shape[0] // attn.head_dim
+        on_kernels = K.attention_on_kernels(x.shape[0], x.shape[1], heads, heads, attn.head_dim, grad=False)
+        return torch.ops.dion_b200.gpt_block_fwd(x, *shadows, cos, sin, attn.head_dim, K.RMS_EPS, on_kernels,
+                                                 K.runtime.status_tensor(x.device))
 
     def forward(self, x: torch.Tensor, bt=None) -> torch.Tensor:
         if bt is None and not torch.is_grad_enabled():

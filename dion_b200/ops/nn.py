@@ -23,6 +23,7 @@ from . import runtime
 from .gemm import gemm
 from .multi_tensor import cast_copy
 
+SMS = 148  # of a B200
 RMS_EPS = 1.1920929e-07  # torch.finfo(torch.float32).eps, what F.rms_norm(eps=None) uses
 
 
@@ -753,8 +754,7 @@ class _FlashAttnAnyLengthFn(_FlashAttnFn):
 
 def _any_length(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor) -> bool:
     """Contiguous q, k, v of a length that is no multiple of 128, in a plain call: rows beyond the sequence are read as
-    zeros and masked.  What a tracer, a mode or a transform looks at, and other shapes and types, go to the library.
-    8 x 777, 12 heads of 64: 26 us against 36, with the backward pass 65 against 81; 24 tokens, 6 heads of 128: 14 against 18."""
+    zeros and masked.  What a tracer, a mode or a transform looks at, and other shapes and types, go to the library."""
     B, T, H, D = q.shape
     return (q.device == k.device == v.device and q.dtype == k.dtype == v.dtype == torch.bfloat16 and D in (64, 128) and q.numel() > 0 and k.numel() > 0
             and k.dim() == 4 and k.shape[:2] == q.shape[:2] and k.shape[3] == D and v.shape == k.shape
@@ -767,6 +767,36 @@ def _any_length(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor) -> bool:
 ATTENTION_IMPL = os.environ.get("DION_B200_ATTENTION", "kernel")
 
 
+def _ragged_on_kernels(B: int, T: int, H: int, Hkv: int, D: int, grad: bool) -> bool:
+    """Is a length that is no multiple of 128 faster on the kernels than in the library?  (B x T, H heads of D; GPU time, us here /
+    library; SMS CTAs run at a time, each with two tiles of queries where there are more tiles than that.)
+
+    Up to 64 rows a tile is at most half full, 1 x 24, 6 heads of 128: 5.5 / 3.5, with the backward pass 19 / 15.  Such a call
+    waits for the host (20 / 21, with the backward pass 130 / 137, in a block without gradients 18 us less than with the
+    library) unless there are many heads: 64 x 17, 12 of 64 18.6 / 11.8.
+    Forward: heads of 64 win up to about 2048 rows (8 x 777, 12 heads 24 / 33; 8 x 2000 79 / 88; 2 x 8100 260 / 248), a few of them
+    only while each tile has a CTA (12 heads: 1 x 1300 1.34 times as fast, 1 x 1700 0.97); heads of 128 up to 448 (64 x 333, 6
+    heads 41 / 51; 32 x 500 31.7 / 30.4; 8 x 1000 24.7 / 22.1; 1 x 2000, 32 heads 45 / 35), and to 1300 while each tile has a
+    CTA (1 x 1300, 12 heads 1.04 times as fast, 1 x 1700 0.78).
+    With the backward pass: heads of 64 up to 2048 (32 x 777, 12 heads 307 / 406), of 128 up to 768 (32 x 700, 6 heads
+    207 / 222; 32 x 1000 350 / 331).  dK and dV of grouped heads are one CTA's work for all heads of a group, so there have to be
+    kv heads enough: 8 x 32 heads of 64 on 8 at 1300 rows 1.30 times as fast, 1 x 32 on 8 0.86 (of 128, 700 rows: 85 / 57)."""
+    heads = B * H
+    if T <= 64:
+        return heads <= 4 * SMS
+    if grad:
+        return T <= (2048 if D == 64 else 768) and (T <= 128 or Hkv == H or B * Hkv >= 64)
+    spare = heads * ((T + 127) // 128) <= SMS
+    if D == 64:
+        return T <= (2048 if spare or heads >= 32 else 1300)
+    return T <= (1300 if spare else 448)
+
+
+def attention_on_kernels(B: int, T: int, H: int, Hkv: int, D: int, grad: bool) -> bool:
+    """Does causal attention of these sizes run on the kernels, where they take them?"""
+    return ATTENTION_IMPL == "kernel" and (T % 128 == 0 or _ragged_on_kernels(B, T, H, Hkv, D, grad))
+
+
 def causal_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor) -> torch.Tensor:
     """Causal self-attention; q, k, v: [B, T, H, Dh] -> [B, T, H*Dh].  Supports grouped
     KV heads (H_kv dividing H)."""
@@ -776,9 +806,10 @@ def causal_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor) -> torch
         q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
         if flash_attention_supported(q, k, v):
             return _FlashAttnFn.apply(q, k, v).view(B, T, H * Dh)
-        if T % 128 and _any_length(q, k, v):
-            q, k, v = (t.clone() if t.data_ptr() % 16 else t for t in (q, k, v))
-            return _FlashAttnAnyLengthFn.apply(q, k, v).view(B, T, H * Dh)
+        grad = torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad)
+        if T % 128 and _ragged_on_kernels(B, T, H, Hkv, Dh, grad) and _any_length(q, k, v):
+            y = _FlashAttnAnyLengthFn.apply(q, k, v) if grad else _attention_forward(q, k, v)[0]
+            return y.view(B, T, H * Dh)
     qt, kt, vt = q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2)
     y = F.scaled_dot_product_attention(qt, kt, vt, is_causal=True, enable_gqa=(Hkv != H))
     return y.transpose(1, 2).reshape(B, T, H * Dh)

@@ -845,6 +845,50 @@ def test_halved_input_gradient_of_the_loss():
     assert ((runs[0][0].float() - want).norm() / want.norm()).item() < 3 * 2.0 ** -9
 
 
+@pytest.mark.parametrize("sizes,kernels", [
+    ((8, 777, 12, 12, 64, False), True),
+    ((32, 1000, 12, 12, 64, True), True),
+    ((1, 2000, 12, 12, 64, False), False),     # few heads, more tiles than SMs
+    ((2, 8100, 12, 12, 64, True), False),
+    ((8, 8100, 12, 12, 64, False), False),
+    ((64, 333, 6, 6, 128, False), True),
+    ((32, 500, 6, 6, 128, False), False),
+    ((1, 1000, 6, 6, 128, False), True),       # a CTA for every tile
+    ((32, 700, 6, 6, 128, True), True),
+    ((32, 1000, 6, 6, 128, True), False),
+    ((1, 2000, 32, 8, 128, False), False),
+    ((1, 300, 32, 8, 128, True), False),       # a group's dK and dV are one CTA's
+    ((8, 700, 32, 8, 128, True), True),
+    ((1, 100, 32, 8, 128, True), True),
+    ((1, 24, 6, 6, 128, False), True),         # waits for the host
+    ((64, 17, 12, 12, 64, False), False),      # does not
+])
+def test_which_ragged_lengths_run_on_the_kernels(sizes, kernels, monkeypatch):
+    """Where the library measured faster, the call goes to the library as it did before the kernels took every length."""
+    assert N._ragged_on_kernels(*sizes) == kernels
+    assert N.attention_on_kernels(*sizes) == kernels
+    assert N.attention_on_kernels(sizes[0], 128 * (1 + sizes[1] // 128), *sizes[2:])  # whole tiles are never asked about
+    monkeypatch.setattr(N, "ATTENTION_IMPL", "library")
+    assert not N.attention_on_kernels(*sizes)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape,grad,kernels", [((1, 1700, 12, 12, 64), False, False), ((1, 1200, 12, 12, 64), False, True),
+                                                ((1, 300, 8, 2, 128), True, False), ((1, 300, 8, 2, 128), False, True)])
+def test_ragged_attention_takes_the_path_that_was_chosen(shape, grad, kernels):
+    from dion_b200 import ops
+
+    B, T, H, Hkv, D = shape
+    q, k, v = (torch.randn(B, T, h, D, device="cuda").bfloat16().requires_grad_(grad) for h in (H, Hkv, Hkv))
+    before = ops.launch_count()
+    y = N.causal_attention(q, k, v)
+    assert ops.launch_count() - before == int(kernels) and y.requires_grad == grad
+    kr, vr = (t.detach().double().transpose(1, 2).repeat_interleave(H // Hkv, dim=1) for t in (k, v))
+    ref = F.scaled_dot_product_attention(q.detach().double().transpose(1, 2), kr, vr, is_causal=True).transpose(1, 2)
+    # bf16 values up to about 4.5 of products with bf16 probabilities
+    assert (y.detach().view(B, T, H, D).double() - ref).abs().max().item() < 2e-2
+
+
 @pytest.mark.gpu
 def test_every_launch_is_counted_once():
     """The count of a training step, and of Newton-Schulz with and without norms in hand, against a profile of the same."""

@@ -74,6 +74,15 @@ def _tma_ok(t: torch.Tensor) -> bool:
     return True
 
 
+def worth_a_map_each(x: torch.Tensor) -> bool:
+    """Should matrices like `x`, allocations of their own that are updated in place, each get a tensor map (``host_ptrs``)?
+    Reading an address list and making the maps takes the host 0.17 us per matrix, and a launch holds 32 of them.  Products on
+    the GPU / calls on the host, us, without and with maps: 100 x 64 x 256 13 / 11 and 20 / 27, 33 x 256 x 128 8.4 / 11 and 11 / 16,
+    100 x 256 x 256 24 / 11 and 23 / 27, 64 x 128 x 512 14 / 11 and 12 / 19; from 131072 elements on they pay: 24 x 384 x 384
+    15 / 11 and 9.6 / 13, 8 x 256 x 1024 9.0 / 11 and 6.3 / 12, 100 x 512 x 512 81 / 11 and 66 / 28."""
+    return x.numel() >= 131072
+
+
 def gemm(a: torch.Tensor, b: torch.Tensor, *, c: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None,
          alpha: float = 1.0, beta: float = 0.0, act: Optional[str] = None, out_dtype: Optional[torch.dtype] = None,
          accumulate: bool = False, split_k: int = 1, symmetric: bool = False, shadow: Optional[torch.Tensor] = None,
@@ -92,7 +101,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, c: Optional[torch.Tensor] = None, 
     With ``out_dup = k > 1`` every batch element is stored to k destinations, ``out_ptrs[b * k + j]``
     (for instance one slot of a symmetric buffer on each rank of a group).
     ``host_ptrs``: the addresses of ``out_ptrs`` as a list, where ``c_ptrs`` is the same table (matrices updated in place);
-    the kernel then moves them with TMA.
+    the kernel then moves them with TMA (see ``worth_a_map_each``).
     ``a_lo`` / ``b_lo`` (fp32, laid out like ``a`` / ``b``): ``a`` and ``b`` are then the tf32-exact high
     halves of split operands and the product is ``a @ b + a_lo @ b + a @ b_lo`` accumulated in one pass
     over three K-segments - a 3xTF32 product in a single launch.

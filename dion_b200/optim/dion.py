@@ -1001,7 +1001,8 @@ class Dion(Optimizer):
                     cls.shadow_ptrs = torch.tensor(sp_list, dtype=torch.int64, device=x0.device)
                 shadow0, shadow_ptrs = shadows[0], cls.shadow_ptrs
             ops.gemm(a_op, b_op, c=x0, out=x0, c_ptrs=cls.x_ptrs, out_ptrs=cls.x_ptrs, shadow=shadow0,
-                     shadow_ptrs=shadow_ptrs, alpha=alpha, beta=beta, host_ptrs=ptr_list)
+                     shadow_ptrs=shadow_ptrs, alpha=alpha, beta=beta,
+                     host_ptrs=ptr_list if ops.worth_a_map_each(x0) else None)
             for p in params:
                 if shadow0 is not None:
                     nn_ops.mark_shadow_fresh(p)

@@ -198,7 +198,8 @@ def foreach_baddbmm_(X: List[Tensor], A: Tensor, B: Tensor, alpha: float = 1.0, 
     if fast:
         addresses = [x.data_ptr() for x in Xl]
         ptrs = torch.tensor(addresses, dtype=torch.int64, device=x0.device)
-        ops.gemm(a_op, b_op, c=x0, out=x0, c_ptrs=ptrs, out_ptrs=ptrs, alpha=float(alpha), beta=float(beta), host_ptrs=addresses)
+        ops.gemm(a_op, b_op, c=x0, out=x0, c_ptrs=ptrs, out_ptrs=ptrs, alpha=float(alpha), beta=float(beta),
+                 host_ptrs=addresses if ops.worth_a_map_each(x0) else None)
         return
     prod = ops.gemm(a_op, b_op, out_dtype=torch.float32) if a_op.is_cuda and a_op.dtype == b_op.dtype else \
         torch.matmul(a_op.float(), b_op.float())

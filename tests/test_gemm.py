@@ -692,6 +692,24 @@ def test_updates_in_place_through_maps_of_their_own(B, M, N, K, dtype, copies):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("N,maps", [(128, False), (508, False), (512, True), (768, True)])
+def test_matrices_below_512_kb_are_updated_without_maps(N, maps, monkeypatch):
+    """Where a tensor map per matrix costs the host more than it saves; 256 x N, the limit lies at N = 512.  Operands in tf32: 10 bits."""
+    from dion_b200 import ops
+    from dion_b200.optim.functional import foreach_baddbmm_
+
+    X = [torch.randn(256, N, device="cuda") for _ in range(3)]
+    A, B = torch.randn(3, 256, 32, device="cuda"), torch.randn(3, N, 32, device="cuda")
+    want = [0.9 * x.double() - 0.3 * (a.double() @ b.double().t()) for x, a, b in zip(X, A, B)]
+    seen, plain = [], ops.gemm
+    monkeypatch.setattr(ops, "gemm", lambda *args, **kw: (seen.append(kw.get("host_ptrs")), plain(*args, **kw))[1])
+    foreach_baddbmm_(X, A, B, alpha=-0.3, beta=0.9)
+    assert seen == [[x.data_ptr() for x in X] if maps else None]
+    for x, w in zip(X, want):
+        assert (x.double() - w).abs().max().item() <= 2.0 ** -9 * w.abs().max().item()
+
+
+@pytest.mark.gpu
 def test_first_call_of_a_thread():
     """A thread that has made no CUDA call yet, as a backward pass may meet it, starts with a product or with attention."""
     import threading

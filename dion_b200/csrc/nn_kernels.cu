@@ -857,13 +857,15 @@ cudaError_t cross_entropy_fwd_bwd_launch(void* logits, const long long* targets,
                                          float grad_scale, long long ignore_index, bool write_grad, cudaStream_t s) {
   if (rows == 0) return cudaSuccess;
   if (vocab % 8 != 0 || pitch % 8 != 0) return cudaErrorInvalidValue;
-  // Threads per row, us at 256 / 512 / 1024 threads: 4096 x 128256 497 / 474 / 400, 4096 x 100352 384 / 365 / 308,
-  // 4096 x 65536 253 / 214 / 208, 8192 x 50304 368 / 296 / 337, 8192 x 32000 208 / 188 / 231, 8192 x 24576 146 / 148 / 205,
-  // 8192 x 16384 97 / 110 / 152.
-  const auto kernel = vocab >= 65536 ? cross_entropy_kernel<1024> : vocab > 24576 ? cross_entropy_kernel<512>
-                                                                                  : cross_entropy_kernel<256>;
-  const unsigned threads = vocab >= 65536 ? 1024 : vocab > 24576 ? 512 : 256;
-  launch_pdl(kernel, dim3((unsigned)rows), dim3(threads), 0, s, 0, reinterpret_cast<bf16*>(logits), targets, row_loss,
+  // Threads per row.  With a gradient, us at 256 / 512 / 1024 threads: 4096 x 128256 492 / 469 / 399, 4096 x 100352
+  // 381 / 360 / 305, 4096 x 65536 247 / 207 / 208, 8192 x 50304 364 / 293 / 340, 8192 x 32000 201 / 184 / 231, 8192 x 24584
+  // 147 / 150 / 215, 8192 x 8192 53 / 70 / 127.  The loss alone reads each row once, so that nothing has to stay in the L2:
+  // 4096 x 128256 161 / 164 / 185, 8192 x 65536 167 / 176 / 229, 8192 x 50304 130 / 144 / 197, 8192 x 24584 70 / 86 / 140;
+  // more threads only where the rows do not fill the chip by themselves: 2048 x 65536 50 / 49 / 60, 1024 x 50304
+  // 24 / 22 / 27, 600 x 65536 24 / 17 / 19, 24 x 50304 6.2 / 4.8 / 4.9.
+  const int threads = vocab <= 24576 ? 256 : !write_grad ? (rows < 2048 ? 512 : 256) : vocab < 65536 ? 512 : 1024;
+  const auto kernel = threads == 1024 ? cross_entropy_kernel<1024> : threads == 512 ? cross_entropy_kernel<512> : cross_entropy_kernel<256>;
+  launch_pdl(kernel, dim3((unsigned)rows), dim3((unsigned)threads), 0, s, 0, reinterpret_cast<bf16*>(logits), targets, row_loss,
              scale_ptr, vocab, pitch, grad_scale, ignore_index, write_grad ? 1 : 0);
   return cudaGetLastError();
 }

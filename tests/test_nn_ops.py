@@ -375,6 +375,21 @@ def test_attention_backward_refuses_keys_of_other_sizes(shape):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("rows", [2047, 2048])
+@pytest.mark.parametrize("vocab", [24576, 24584])
+def test_the_loss_alone_of_many_rows(rows, vocab):
+    """Both numbers of threads per row of a pass without a gradient.  A thread adds up to 97 exponentials of 2 ulp each."""
+    torch.manual_seed(rows)
+    x = 3 * torch.randn(rows, vocab, device="cuda").bfloat16()
+    t, loss, before = torch.randint(0, vocab, (rows,), device="cuda"), torch.empty(rows, device="cuda"), x.clone()
+    assert N.runtime.use_cuda_kernels(x)
+    torch.ops.dion_b200.cross_entropy_fwd_bwd(x, t, loss, None, 1.0, -1, False)
+    torch.testing.assert_close(loss.double(), F.cross_entropy(x.double(), t, reduction="none"), rtol=2.0 ** -22,
+                               atol=97 * 2.0 ** -24 + 1e-5)
+    assert torch.equal(x, before)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("shape", [
     (150, 128, 1, 1, 128),  # one tile per head; a head for every CTA and two left over
     (40, 256, 4, 4, 64),    # pairs of query tiles, 160 heads

@@ -507,9 +507,21 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     else return mbar_wait(bar, parity, abort_flag);
   };
 
+  // Loads and MMAs come from one elected lane, except where a tile's two operands are split, MN-major and on a single CTA (Gram
+  // matrices): bound by shared memory, which converters and MMAs share, those take longer the faster they are issued.  With lane 0
+  // of a divergent branch and descriptors put together for every MMA, elected lane and stepped descriptors: sums in order of
+  // 8 x 14336 x 512 564 and 601 us, 2 x 20000 x 256 757 and 783; over a cluster 8 x 14336 x 512 401 and 414, 4 x 14336 x 512
+  // 216 and 221.  One tile, which is one operand, goes the other way by less: 12 x 3072 x 96 94.8 and 92.9, over a cluster
+  // 18.4 and 17.7.
+  constexpr bool kLane0 = kSplit && !kPair && kAMajor == kMajorMN;
+  auto issues = [&]() -> bool {
+    if constexpr (kLane0) return lane == 0;
+    else return elect_one();
+  };
+
   if (warp == 0) {
     // ------------------------------------------------------------------ producer
-    if (elect_one()) {
+    if (issues()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -571,7 +583,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
           }
           int kk = kb;
           if constexpr (kTf32) {
-            if (!kSplit && kb >= p.kblocks_seg) {
+            if ((!kSplit || kClusterK) && kb >= p.kblocks_seg) {  // kClusterK: see below
               const int seg = kb / p.kblocks_seg;
               kk = kb - seg * p.kblocks_seg;
               if (seg == 1) map_a = &tmap_a_lo;
@@ -602,7 +614,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (cta_rank == 0 && elect_one()) {
+    if (cta_rank == 0 && issues()) {
       constexpr uint32_t idesc = make_instr_desc(kTf32 ? 2 : 1, kAMajor, kBMajor, C::TILE_M, kBlockN);
       // Descriptors of stage 0; the others differ in the address field alone (units of 16 bytes, no carry below 256 KB).  Put
       // together afresh for every MMA they took longer than the splitting variants' multiplies.
@@ -632,7 +644,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
           // segments to the second one, which starts from zero at the first of them
           uint32_t d_tmem = d_main;
           bool fresh = kb == kb0;
-          if constexpr (C::CROSS_ACC && !kSplit) {
+          // (kClusterK: never, but without the question 4 x 14336 x 512 takes 225 us, with it 216; see kLane0)
+          if constexpr (C::CROSS_ACC && (!kSplit || kClusterK)) {
             if (kb >= p.kblocks_seg) {
               d_tmem = d_main + kBlockN;
               fresh = kb == p.kblocks_seg;
@@ -651,13 +664,22 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
           tc_fence_after();
           const uint64_t desc_a = desc_a0 + (uint32_t)((stage * C::STAGE_STRIDE) >> 4);
           const uint64_t desc_b = desc_b0 + (uint32_t)((stage * C::STAGE_STRIDE + b_off) >> 4);
+          const uint32_t sa = smem_u32(smem + stage * C::STAGE_STRIDE);
+          auto desc_of_a = [&](uint32_t off) -> uint64_t {
+            if constexpr (kLane0) return make_smem_desc(sa + off, C::A_LBO, C::A_SBO, C::A_LAYOUT);
+            else return desc_a + (off >> 4);
+          };
+          auto desc_of_b = [&](uint32_t off) -> uint64_t {
+            if constexpr (kLane0) return make_smem_desc(sa + b_off + off, C::B_LBO, C::B_SBO, C::B_LAYOUT);
+            else return desc_b + (off >> 4);
+          };
 #pragma unroll
           for (int j = 0; j < C::KSTEPS; ++j) {
-            const uint64_t da = desc_a + ((j * C::A_KSTEP) >> 4);
-            const uint64_t db = desc_b + ((j * C::B_KSTEP) >> 4);
+            const uint64_t da = desc_of_a(j * C::A_KSTEP);
+            const uint64_t db = desc_of_b(j * C::B_KSTEP);
             if constexpr (kSplit) {
-              const uint64_t da_lo = da + (C::LO_OFFSET >> 4);
-              const uint64_t db_lo = db + (C::LO_OFFSET >> 4);
+              const uint64_t da_lo = desc_of_a(C::LO_OFFSET + j * C::A_KSTEP);
+              const uint64_t db_lo = desc_of_b(C::LO_OFFSET + j * C::B_KSTEP);
               const uint32_t first = (!fresh || j > 0) ? 1u : 0u;
               auto mma = [&](uint32_t d, uint64_t x, uint64_t y, uint32_t accumulate) {
                 if constexpr (kPair) umma_ss_pair<true>(d, x, y, idesc, accumulate);

@@ -443,9 +443,13 @@ def test_attention_of_any_length(shape):
     ref.backward(d_out.detach().float())
     assert (y.view_as(ref).float() - ref).abs().max().item() < 2e-2
     for name, got, want in (("dq", q.grad, qf.grad), ("dk", k.grad, kf.grad), ("dv", v.grad, vf.grad)):
-        # a single key has no gradient through its score: what is left is the rounding of dO . O, up to 2^-8 of |dO||O|
+        if T == 1 and name != "dv":
+            # P is 1 and O is V bit for bit, so dP - delta is the difference of one sum taken in two orders: up to
+            # 2 D 2^-24 of sum |dO||V| < 100, times |k| or |q| < 5, over sqrt(D) = 8: 4.8e-4 at worst, 1e-6 as a rule
+            assert got.float().abs().max().item() < 1e-4, name
+            continue
         err = (got.float() - want).abs().max().item() / max(want.abs().max().item(), 1.0)
-        assert err < 2e-2 if T > 1 else err < 0.3, (name, err)
+        assert err < 2e-2, (name, err)
     if B > 1:  # the first sequence alone gives the same, and is not touched by NaN in the second
         with torch.no_grad():
             alone = N.causal_attention(q[:1], k[:1], v[:1])

@@ -196,7 +196,7 @@ bool gemm(const Tensor& a, const Tensor& b, const std::optional<Tensor>& c, Tens
   cudaError_t e = dion::gemm_launch(g, at::cuda::getCurrentCUDAStream());
   TORCH_CHECK(e == cudaSuccess, "dion_b200 gemm launch failed: ", cudaGetErrorString(e), " ",
               dion::gemm_last_error());
-  g_launches.fetch_add(1, std::memory_order_relaxed);
+  g_launches.fetch_add(dion::gemm_launches(g), std::memory_order_relaxed);
   return true;
 }
 

@@ -2033,8 +2033,10 @@ bool gemm_takes_groups(const GemmArgs& a) {
   return t * (t + 1) / 2 * a.batch <= num_sms();
 }
 
+int gemm_launches(const GemmArgs& a) { return a.batch > kMaxMaps && tma_ptrs(a) ? (a.batch + kMaxMaps - 1) / kMaxMaps : 1; }
+
 cudaError_t gemm_launch(const GemmArgs& a, cudaStream_t stream) {
-  if (a.batch > kMaxMaps && tma_ptrs(a)) {  // the maps of a launch travel with its parameters
+  if (gemm_launches(a) > 1) {  // the maps of a launch travel with its parameters
     const long long es = a.ab_dtype == kF32 ? 4 : 2;
     for (int b0 = 0; b0 < a.batch; b0 += kMaxMaps) {
       GemmArgs part = a;

@@ -139,6 +139,8 @@ struct GemmArgs {
 // Returns cudaSuccess or the launch error; argument errors return cudaErrorInvalidValue
 // and write a message retrievable with gemm_last_error().
 cudaError_t gemm_launch(const GemmArgs& args, cudaStream_t stream);
+// Host only: how many launches gemm_launch takes for `args` (updates through GemmArgs::x_ptrs: one per 32 matrices).
+int gemm_launches(const GemmArgs& args);
 const char* gemm_last_error();
 
 // Host only, no launch: can one launch take the three products of `args` (GemmArgs::B_more)?

@@ -710,6 +710,21 @@ def test_matrices_below_512_kb_are_updated_without_maps(N, maps, monkeypatch):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("B,launches", [(1, 1), (32, 1), (33, 2), (70, 3)])
+def test_updates_of_more_matrices_than_a_launch_has_maps_are_counted(B, launches):
+    from dion_b200 import ops
+    from dion_b200.optim.functional import foreach_baddbmm_
+
+    X = list(torch.zeros(B, 256, 512, device="cuda").unbind())
+    A, P = torch.randn(B, 256, 16, device="cuda"), torch.randn(B, 512, 16, device="cuda")
+    before = ops.launch_count()
+    foreach_baddbmm_(X, A, P)
+    assert ops.launch_count() - before == launches
+    # tf32 operands: 10 bits
+    assert all((x - a @ p.t()).abs().max() <= 2.0 ** -9 * x.abs().max() for x, a, p in zip(X, A, P))
+
+
+@pytest.mark.gpu
 def test_first_call_of_a_thread():
     """A thread that has made no CUDA call yet, as a backward pass may meet it, starts with a product or with attention."""
     import threading

@@ -236,8 +236,8 @@ __device__ __forceinline__ void quad_transpose(uint32_t (&v)[4], int lane) {
   }
 }
 // 32 accumulator rows (lane quadrant `quad`, COLS fp32 columns from `taddr`) to `out` as bf16, row r at out + (quad * 32 + r) *
-// pitch, rows from `rows` on left out; kScaled: times the factor that the lane of the row holds.  Eight rows of 64 bytes per store instruction: with a row per lane each one touches
-// 32 lines, and the stores of dV and dK took 3000 cycles per kv tile.
+// pitch, rows from `rows` on left out; kScaled: times the factor that the lane of the row holds.  Eight rows of 64 bytes per
+// store instruction: with a row per lane each one touches 32 lines, and the stores of dV and dK took 3000 cycles per kv tile.
 template <int COLS, bool kScaled = false>
 __device__ __forceinline__ void store_rows(uint32_t taddr, int quad, int lane, __nv_bfloat16* out, long long pitch, int rows,
                                            float scale_of_lane = 1.f) {
@@ -380,7 +380,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     tma_prefetch_desc(&tmap_q);
     tma_prefetch_desc(&tmap_k);
     tma_prefetch_desc(&tmap_v);
-    for (uint64_t* b = bars; b < bars_end; ++b) mbar_init(b, (b >= s_free && b < pv_done) ? 4 : ((b >= k_empty && b < v_full) || b >= v_empty) ? 2 : 1);
+    for (uint64_t* b = bars; b < bars_end; ++b)
+      mbar_init(b, (b >= s_free && b < pv_done) ? 4 : ((b >= k_empty && b < v_full) || b >= v_empty) ? 2 : 1);
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -1004,7 +1005,8 @@ struct BwdKvCfg {
 // function unit takes 1024 for the exponentials; the order below keeps both fed: while the softmax warps turn S^T of one
 // tile into P^T, the tensor core runs dK and dP^T of the tile before, and dV and the next S^T while they form dS^T.
 // P^T and dS^T go back over the columns that the same thread read (D = 64 has room for P^T beside S^T), so no warp waits for
-// another.  The next kv tile's loads and first products run under the last tile of the one before; only the store of dV and dK stands alone.
+// another.  The next kv tile's loads and first products run under the last tile of the one before; only the store of dV and dK
+// stands alone.
 template <int D>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_do,
@@ -1054,7 +1056,8 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     tma_prefetch_desc(&tmap_do);
     tma_prefetch_desc(&tmap_k);
     tma_prefetch_desc(&tmap_v);
-    for (uint64_t* b = bars; b < bars_end; ++b) mbar_init(b, (b == ds_full || b == p_full || b == s_free) ? kSoftmaxWarps : b >= do_empty ? 2 : 1);
+    for (uint64_t* b = bars; b < bars_end; ++b)
+      mbar_init(b, (b == ds_full || b == p_full || b == s_free) ? kSoftmaxWarps : b >= do_empty ? 2 : 1);
     *abort_flag = 0;
     mbar_fence_init();
   }

@@ -1063,9 +1063,9 @@ cudaError_t split_tf32_launch(const float* x, float* hi, float* lo, long long nu
   long long grid = (nvec + 255) / 256;
   if (grid > 148 * 16) grid = 148 * 16;
   if (grid < 1) grid = 1;
-  launch_pdl(split_tf32_kernel, dim3((int)grid), dim3(256), 0, s, 0, reinterpret_cast<const float4*>(x), reinterpret_cast<float4*>(hi),
-                                              reinterpret_cast<float4*>(lo), nvec, x + nvec * 4, hi + nvec * 4,
-                                              lo + nvec * 4, ntail);
+  launch_pdl(split_tf32_kernel, dim3((int)grid), dim3(256), 0, s, 0, reinterpret_cast<const float4*>(x),
+             reinterpret_cast<float4*>(hi), reinterpret_cast<float4*>(lo), nvec, x + nvec * 4, hi + nvec * 4, lo + nvec * 4,
+             ntail);
   return cudaGetLastError();
 }
 

@@ -239,8 +239,8 @@ cudaError_t rmsnorm_gain_fwd_launch(const void* x, const void* gain, int gain_ty
   if (!norm_args_ok(gain, gain_type, dim)) return cudaErrorInvalidValue;
   const unsigned grid = (unsigned)((rows + 7) / 8);
 #define DION_GAIN_FWD(V)                                                                                          \
-  launch_pdl(rmsnorm_gain_fwd_kernel<V>, dim3(grid), dim3(256), 0, s, 0, reinterpret_cast<const bf16*>(x), gain, gain_type,                 \
-                                                  reinterpret_cast<bf16*>(y), rstd, rows, dim, eps)
+  launch_pdl(rmsnorm_gain_fwd_kernel<V>, dim3(grid), dim3(256), 0, s, 0, reinterpret_cast<const bf16*>(x), gain,  \
+             gain_type, reinterpret_cast<bf16*>(y), rstd, rows, dim, eps)
   if (dim <= 4 * 256) DION_GAIN_FWD(4);
   else if (dim <= 8 * 256) DION_GAIN_FWD(8);
   else DION_GAIN_FWD(16);
@@ -264,8 +264,8 @@ cudaError_t rmsnorm_gain_bwd_launch(const void* dy, const void* x, const float* 
   const int per_thread = nvec > 256 ? 2 : 1;
   const int threads = ((nvec + per_thread - 1) / per_thread + 31) / 32 * 32;
   const auto kernel = per_thread == 2 ? rmsnorm_gain_bwd_kernel<2> : rmsnorm_gain_bwd_kernel<1>;
-  launch_pdl(kernel, dim3(blocks), dim3(threads), 0, s, 0, reinterpret_cast<const bf16*>(dy), reinterpret_cast<const bf16*>(x), rstd, gain,
-                                    gain_type, reinterpret_cast<bf16*>(dx), partial, rows, dim, rpb);
+  launch_pdl(kernel, dim3(blocks), dim3(threads), 0, s, 0, reinterpret_cast<const bf16*>(dy), reinterpret_cast<const bf16*>(x),
+             rstd, gain, gain_type, reinterpret_cast<bf16*>(dx), partial, rows, dim, rpb);
   return cudaGetLastError();
 }
 
@@ -276,8 +276,8 @@ cudaError_t swiglu_fwd_launch(const void* g, const void* u, void* h, long long n
   const long long nvec = n / 8;
   long long grid = (nvec + 255) / 256;
   if (grid > 148 * 16) grid = 148 * 16;
-  launch_pdl(swiglu_fwd_kernel, dim3((int)grid), dim3(256), 0, s, 0, reinterpret_cast<const uint4*>(g), reinterpret_cast<const uint4*>(u),
-                                              reinterpret_cast<uint4*>(h), nvec);
+  launch_pdl(swiglu_fwd_kernel, dim3((int)grid), dim3(256), 0, s, 0, reinterpret_cast<const uint4*>(g),
+             reinterpret_cast<const uint4*>(u), reinterpret_cast<uint4*>(h), nvec);
   return cudaGetLastError();
 }
 
@@ -290,9 +290,9 @@ cudaError_t swiglu_bwd_launch(const void* dh, const void* g, const void* u, void
   const long long nvec = n / 8;
   long long grid = (nvec + 255) / 256;
   if (grid > 148 * 16) grid = 148 * 16;
-  launch_pdl(swiglu_bwd_kernel, dim3((int)grid), dim3(256), 0, s, 0, reinterpret_cast<const uint4*>(dh), reinterpret_cast<const uint4*>(g),
-                                              reinterpret_cast<const uint4*>(u), reinterpret_cast<uint4*>(dg),
-                                              reinterpret_cast<uint4*>(du), nvec);
+  launch_pdl(swiglu_bwd_kernel, dim3((int)grid), dim3(256), 0, s, 0, reinterpret_cast<const uint4*>(dh),
+             reinterpret_cast<const uint4*>(g), reinterpret_cast<const uint4*>(u), reinterpret_cast<uint4*>(dg),
+             reinterpret_cast<uint4*>(du), nvec);
   return cudaGetLastError();
 }
 

@@ -300,8 +300,8 @@ __global__ void __launch_bounds__(kThreads, 1)
 
 int tiles_of(int rows, int cols) { return (rows + kTileM - 1) / kTileM * ((cols + kTileN - 1) / kTileN); }
 
-// CTAs per matrix: as many as have a tile each, if all clusters run at once (one CTA per SM; 12 clusters of eight, 24 of four
-// and 64 of two do, 16, 36 and 128 do not: 16 x 256 x 256 63 -> 118 us), 0 if no size does.
+// CTAs per matrix: as many as have a tile each, if all clusters run at once on the SMs of a B200 (one CTA per SM; 12 clusters
+// of eight, 24 of four and 64 of two do, 16, 36 and 128 do not: 16 x 256 x 256 63 -> 118 us), 0 if no size does.
 int cluster_size(int batch, int k, int L) {
   const int room = batch <= 12 ? 8 : batch <= 24 ? 4 : batch <= 64 ? 2 : batch <= 128 ? 1 : 0;
   int c = 1;

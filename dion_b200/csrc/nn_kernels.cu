@@ -747,9 +747,9 @@ cudaError_t rmsnorm_fwd_launch(const void* x, const void* residual, void* x_out,
   if (dim % 8 != 0 || dim > kNormMaxVec * 256) return cudaErrorInvalidValue;
   const unsigned grid = (unsigned)((rows + 7) / 8);
 #define DION_NORM_FWD(V)                                                                                          \
-  launch_pdl(rmsnorm_fwd_kernel<V>, dim3(grid), dim3(256), 0, s, 0, reinterpret_cast<const bf16*>(x), reinterpret_cast<const bf16*>(residual), \
-                                             reinterpret_cast<bf16*>(x_out), reinterpret_cast<bf16*>(y), rstd, rows, \
-                                             dim, eps)
+  launch_pdl(rmsnorm_fwd_kernel<V>, dim3(grid), dim3(256), 0, s, 0, reinterpret_cast<const bf16*>(x),             \
+             reinterpret_cast<const bf16*>(residual), reinterpret_cast<bf16*>(x_out), reinterpret_cast<bf16*>(y), \
+             rstd, rows, dim, eps)
   if (dim <= 4 * 256) DION_NORM_FWD(4);
   else if (dim <= 8 * 256) DION_NORM_FWD(8);
   else DION_NORM_FWD(16);
@@ -762,8 +762,9 @@ cudaError_t rmsnorm_bwd_launch(const void* dy, const void* x, const float* rstd,
   if (dim % 8 != 0 || dim > kNormMaxVec * 256) return cudaErrorInvalidValue;
   const unsigned grid = (unsigned)((rows + 7) / 8);
 #define DION_NORM_BWD(V)                                                                                          \
-  launch_pdl(rmsnorm_bwd_kernel<V>, dim3(grid), dim3(256), 0, s, 0, reinterpret_cast<const bf16*>(dy), reinterpret_cast<const bf16*>(x), rstd, \
-                                             reinterpret_cast<const bf16*>(dx_add), reinterpret_cast<bf16*>(dx), rows, dim)
+  launch_pdl(rmsnorm_bwd_kernel<V>, dim3(grid), dim3(256), 0, s, 0, reinterpret_cast<const bf16*>(dy),            \
+             reinterpret_cast<const bf16*>(x), rstd, reinterpret_cast<const bf16*>(dx_add),                       \
+             reinterpret_cast<bf16*>(dx), rows, dim)
   if (dim <= 4 * 256) DION_NORM_BWD(4);
   else if (dim <= 8 * 256) DION_NORM_BWD(8);
   else DION_NORM_BWD(16);
@@ -794,7 +795,7 @@ cudaError_t rope_qknorm_fwd_launch(const void* q, const void* k, void* q_out, vo
   const unsigned grid = wide ? (unsigned)((tokens * heads * (head_dim / 16) + 255) / 256)
                              : (unsigned)((nrows * (head_dim / 8) + 255) / 256);
 #define DION_ROPE_FWD(KERNEL, HD)                                                                                 \
-  launch_pdl(KERNEL<HD>, dim3(grid), dim3(256), 0, s, 0, \
+  launch_pdl(KERNEL<HD>, dim3(grid), dim3(256), 0, s, 0,                                                          \
       reinterpret_cast<const bf16*>(q), reinterpret_cast<const bf16*>(k), reinterpret_cast<bf16*>(q_out),         \
       reinterpret_cast<bf16*>(k_out), reinterpret_cast<const bf16*>(cos), reinterpret_cast<const bf16*>(sin),     \
       tokens, seq_len, heads, in_pitch, out_pitch, eps)
@@ -820,7 +821,7 @@ cudaError_t rope_qknorm_bwd_launch(const void* dq_out, const void* dk_out, const
   const unsigned grid = wide ? (unsigned)((tokens * heads * (head_dim / 16) + 255) / 256)
                              : (unsigned)((nrows * (head_dim / 8) + 255) / 256);
 #define DION_ROPE_BWD(KERNEL, HD)                                                                                 \
-  launch_pdl(KERNEL<HD>, dim3(grid), dim3(256), 0, s, 0, \
+  launch_pdl(KERNEL<HD>, dim3(grid), dim3(256), 0, s, 0,                                                          \
       reinterpret_cast<const bf16*>(dq_out), reinterpret_cast<const bf16*>(dk_out),                               \
       reinterpret_cast<const bf16*>(q), reinterpret_cast<const bf16*>(k), reinterpret_cast<bf16*>(dq),            \
       reinterpret_cast<bf16*>(dk), reinterpret_cast<const bf16*>(cos), reinterpret_cast<const bf16*>(sin),        \
@@ -841,14 +842,15 @@ cudaError_t relu2_fwd_launch(const void* x, void* h, long long n, cudaStream_t s
   if (n % 8 != 0) return cudaErrorInvalidValue;
   const long long nvec = n / 8;
   launch_pdl(relu2_fwd_kernel, dim3((unsigned)((nvec + 255) / 256)), dim3(256), 0, s, 0, reinterpret_cast<const uint4*>(x),
-                                                                 reinterpret_cast<uint4*>(h), nvec);
+             reinterpret_cast<uint4*>(h), nvec);
   return cudaGetLastError();
 }
 cudaError_t relu2_bwd_launch(const void* dh, const void* x, void* dx, long long n, cudaStream_t s) {
   if (n == 0) return cudaSuccess;
   if (n % 8 != 0) return cudaErrorInvalidValue;
   const long long nvec = n / 8;
-  launch_pdl(relu2_bwd_kernel, dim3((unsigned)((nvec + 255) / 256)), dim3(256), 0, s, 0, reinterpret_cast<const uint4*>(dh), reinterpret_cast<const uint4*>(x), reinterpret_cast<uint4*>(dx), nvec);
+  launch_pdl(relu2_bwd_kernel, dim3((unsigned)((nvec + 255) / 256)), dim3(256), 0, s, 0, reinterpret_cast<const uint4*>(dh),
+             reinterpret_cast<const uint4*>(x), reinterpret_cast<uint4*>(dx), nvec);
   return cudaGetLastError();
 }
 
@@ -864,9 +866,11 @@ cudaError_t cross_entropy_fwd_bwd_launch(void* logits, const long long* targets,
   // more threads only where the rows do not fill the chip by themselves: 2048 x 65536 50 / 49 / 60, 1024 x 50304
   // 24 / 22 / 27, 600 x 65536 24 / 17 / 19, 24 x 50304 6.2 / 4.8 / 4.9.
   const int threads = vocab <= 24576 ? 256 : !write_grad ? (rows < 2048 ? 512 : 256) : vocab < 65536 ? 512 : 1024;
-  const auto kernel = threads == 1024 ? cross_entropy_kernel<1024> : threads == 512 ? cross_entropy_kernel<512> : cross_entropy_kernel<256>;
-  launch_pdl(kernel, dim3((unsigned)rows), dim3((unsigned)threads), 0, s, 0, reinterpret_cast<bf16*>(logits), targets, row_loss,
-             scale_ptr, vocab, pitch, grad_scale, ignore_index, write_grad ? 1 : 0);
+  const auto kernel = threads == 1024  ? cross_entropy_kernel<1024>
+                      : threads == 512 ? cross_entropy_kernel<512>
+                                       : cross_entropy_kernel<256>;
+  launch_pdl(kernel, dim3((unsigned)rows), dim3((unsigned)threads), 0, s, 0, reinterpret_cast<bf16*>(logits), targets,
+             row_loss, scale_ptr, vocab, pitch, grad_scale, ignore_index, write_grad ? 1 : 0);
   return cudaGetLastError();
 }
 
@@ -888,15 +892,15 @@ cudaError_t embedding_fwd_launch(const void* table, int table_type, const long l
   if (tokens == 0) return cudaSuccess;
   if (dim % 8 != 0) return cudaErrorInvalidValue;
   launch_pdl(embedding_fwd_kernel, dim3((unsigned)((tokens + 7) / 8)), dim3(256), 0, s, 0, table, table_type, idx,
-                                                                   reinterpret_cast<bf16*>(out), tokens, dim);
+             reinterpret_cast<bf16*>(out), tokens, dim);
   return cudaGetLastError();
 }
 cudaError_t embedding_bwd_launch(const void* dout, const long long* idx, float* dtable, long long tokens, int dim,
                                  cudaStream_t s) {
   if (tokens == 0) return cudaSuccess;
   if (dim % 2 != 0) return cudaErrorInvalidValue;
-  launch_pdl(embedding_bwd_kernel, dim3((unsigned)((tokens + 7) / 8)), dim3(256), 0, s, 0, reinterpret_cast<const bf16*>(dout), idx, dtable,
-                                                                   tokens, dim);
+  launch_pdl(embedding_bwd_kernel, dim3((unsigned)((tokens + 7) / 8)), dim3(256), 0, s, 0,
+             reinterpret_cast<const bf16*>(dout), idx, dtable, tokens, dim);
   return cudaGetLastError();
 }
 

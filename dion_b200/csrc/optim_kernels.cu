@@ -399,12 +399,13 @@ cudaError_t frob_scale_launch(const void* x, void* out, float* partial, const fl
   const int nchunk = frob_chunks(per);
   const dim3 grid(nchunk, batch);
   if (sumsq == nullptr) {
-    launch_pdl(frob_partial_kernel, dim3(grid), dim3(kThreads), 0, s, 0, reinterpret_cast<const __nv_bfloat16*>(x), partial, per, nchunk);
+    launch_pdl(frob_partial_kernel, grid, dim3(kThreads), 0, s, 0, reinterpret_cast<const __nv_bfloat16*>(x), partial, per,
+               nchunk);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
-  launch_pdl(frob_scale_kernel, dim3(grid), dim3(kThreads), 0, s, 0, reinterpret_cast<const __nv_bfloat16*>(x),
-                                              reinterpret_cast<__nv_bfloat16*>(out), partial, nchunk, sumsq, eps, per);
+  launch_pdl(frob_scale_kernel, grid, dim3(kThreads), 0, s, 0, reinterpret_cast<const __nv_bfloat16*>(x),
+             reinterpret_cast<__nv_bfloat16*>(out), partial, nchunk, sumsq, eps, per);
   return cudaGetLastError();
 }
 

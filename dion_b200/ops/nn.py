@@ -129,18 +129,18 @@ def mark_shadow_stale(w: torch.Tensor) -> None:
 
 def _split_k_for(M: int, N: int, K: int) -> int:
     """Split the contraction so that a skinny weight-gradient GEMM fills the GPU: parts for about four waves of 128 x 128
-    tiles, and from there up to twice as many parts where that leaves the last wave of 256 x 256 tiles (74 at a time, on CTA
-    pairs) fuller.  More parts also keep the sums shorter.  K = 65536, 768 x 768: 17 parts are three waves of a 17th
+    tiles, and from there up to twice as many parts where that leaves the last wave of 256 x 256 tiles (one per pair of SMs)
+    fuller.  More parts also keep the sums shorter.  K = 65536, 768 x 768: 17 parts are three waves of a 17th
     (2.07 filled), 24 three of a 24th: 73 and 63 us; 3072 x 768: 5 and 6 parts, 233 and 215 us."""
     tiles = ((M + 127) // 128) * ((N + 127) // 128)
-    if tiles >= 148 or K < 2048:
+    if tiles >= SMS or K < 2048:
         return 1
-    want = max(1, (4 * 148 + tiles - 1) // tiles)
+    want = max(1, (4 * SMS + tiles - 1) // tiles)
     parts = int(max(1, min(want, K // 512, 32)))
     wide = ((M + 255) // 256) * ((N + 255) // 256)
     if K // parts < 1024 or M < 256 or N < 256:  # short parts do not run on pairs
         return parts
-    return min(range(parts, min(2 * parts, K // 1024) + 1), key=lambda n: (-(-n * wide // 74) / n, n), default=parts)
+    return min(range(parts, min(2 * parts, K // 1024) + 1), key=lambda n: (-(-n * wide // (SMS // 2)) / n, n), default=parts)
 
 
 class _LinearFn(torch.autograd.Function):

@@ -4,10 +4,12 @@ Same iteration and coefficient schedule as the reference (dion/muon.py:620-647;
 dion/newton_schulz_triton.py:336-374): ``X <- a X + (b A + c A A) X`` with ``A = X X^T``,
 five steps with per-step coefficients, input scaled to Frobenius norm <= 1.
 
-On CUDA the three products of a step are tcgen05 GEMMs: ``A`` and ``b A + c A A`` are
-symmetric, so only the upper-triangular tiles are computed and mirrored in the epilogue,
-which also fuses the ``b A`` / ``a X`` additions.  Tall inputs are handled by multiplying
-from the right (``A = X^T X``), so nothing is ever transposed in memory.
+On CUDA there are two paths, with the same sums and roundings.  In general the three products of a step are a tcgen05 launch
+each: ``A`` and ``b A + c A A`` are symmetric, so only the upper-triangular tiles are computed and mirrored in the
+epilogue, which also fuses the ``b A`` / ``a X`` additions; tall inputs are handled by multiplying from the right
+(``A = X^T X``), so nothing is transposed in memory.  Small matrices (``newton_schulz_takes``, csrc/newton_schulz.cu: sides that one
+cluster per matrix works through faster than the launches take) go through all steps in one launch, which computes every
+tile of the symmetric products and keeps X together with its transpose.
 """
 
 from __future__ import annotations

@@ -158,7 +158,7 @@ class Block(nn.Module):
             return None
         cos, sin = attn.rotary.tables(x.shape[1], x.device)
         heads = weights[0].shape[0] // attn.head_dim
-        on_kernels = K.attention_on_kernels(x.shape[0], x.shape[1], heads, heads, attn.head_dim, grad=False)
+        on_kernels = K.attention_on_kernels(x.shape[0], x.shape[1], heads, heads, attn.head_dim)
         return torch.ops.dion_b200.gpt_block_fwd(x, *shadows, cos, sin, attn.head_dim, K.RMS_EPS, on_kernels,
                                                  K.runtime.status_tensor(x.device))
 

@@ -767,34 +767,38 @@ def _any_length(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor) -> bool:
 ATTENTION_IMPL = os.environ.get("DION_B200_ATTENTION", "kernel")
 
 
-def _ragged_on_kernels(B: int, T: int, H: int, Hkv: int, D: int, grad: bool) -> bool:
-    """Is a length that is no multiple of 128 faster on the kernels than in the library?  (B x T, H heads of D; GPU time, us here /
-    library; SMS CTAs run at a time, each with two tiles of queries where there are more tiles than that.)
+def _ragged_on_kernels(B: int, T: int, H: int, Hkv: int, D: int) -> bool:
+    """Is a length that is no multiple of 128 better off on the kernels than in the library?  (B x T, H heads of D; GPU time, us
+    here / library; SMS CTAs run at a time, each with two tiles of queries where there are more tiles than that.)  One answer for
+    passes with and without gradients, so that evaluation and a recomputed forward pass have the bits of training.
 
     Up to 64 rows a tile is at most half full, 1 x 24, 6 heads of 128: 5.5 / 3.5, with the backward pass 19 / 15.  Such a call
     waits for the host (20 / 21, with the backward pass 130 / 137, in a block without gradients 18 us less than with the
     library) unless there are many heads: 64 x 17, 12 of 64 18.6 / 11.8.
-    Forward: heads of 64 win up to about 2048 rows (8 x 777, 12 heads 24 / 33; 8 x 2000 79 / 88; 2 x 8100 260 / 248), a few of them
-    only while each tile has a CTA (12 heads: 1 x 1300 1.34 times as fast, 1 x 1700 0.97); heads of 128 up to 448 (64 x 333, 6
-    heads 41 / 51; 32 x 500 31.7 / 30.4; 8 x 1000 24.7 / 22.1; 1 x 2000, 32 heads 45 / 35), and to 1300 while each tile has a
-    CTA (1 x 1300, 12 heads 1.04 times as fast, 1 x 1700 0.78).
-    With the backward pass: heads of 64 up to 2048 (32 x 777, 12 heads 307 / 406), of 128 up to 768 (32 x 700, 6 heads
-    207 / 222; 32 x 1000 350 / 331).  dK and dV of grouped heads are one CTA's work for all heads of a group, so there have to be
-    kv heads enough: 8 x 32 heads of 64 on 8 at 1300 rows 1.30 times as fast, 1 x 32 on 8 0.86 (of 128, 700 rows: 85 / 57)."""
+    From 65 to 128 rows many heads gain (64 x 100, 12 of 128: forward 1.33, with the backward pass 1.93 times as fast), few lose
+    what the host hides (1 x 100, 12 of 128 forward 6.2 / 4.8, with the backward pass 20 / 20).
+    dK and dV of grouped heads are one CTA's work for all heads of a group, so there have to be kv heads enough: with the backward
+    pass 8 x 32 heads of 64 on 8 at 1300 rows 1.30 times as fast, 1 x 32 on 8 0.86 (of 128, 700 rows: 85 / 57).
+    Heads of 64 win up to about 2048 rows (8 x 777, 12 heads 24 / 33, with the backward pass 84 / 105; 8 x 2000 79 / 88 and
+    310 / 338; 2 x 8100 forward 260 / 248), a few of them only while each tile has a CTA (forward, 12 heads: 1 x 1300 1.34 times as
+    fast, 1 x 1700 0.97).  Heads of 128 up to 448 (64 x 333, 6 heads 41 / 51 and 152 / 192; forward 32 x 500 31.7 / 30.4, 8 x 1000
+    24.7 / 22.1) and to 768 while each tile has a CTA (12 heads: 1 x 641 1.13 and 1.02 times as fast; 1 x 2000 0.80 and 0.88)."""
     heads = B * H
     if T <= 64:
         return heads <= 4 * SMS
-    if grad:
-        return T <= (2048 if D == 64 else 768) and (T <= 128 or Hkv == H or B * Hkv >= 64)
+    if T <= 128:
+        return True
+    if Hkv < H and B * Hkv < 64:
+        return False
     spare = heads * ((T + 127) // 128) <= SMS
     if D == 64:
         return T <= (2048 if spare or heads >= 32 else 1300)
-    return T <= (1300 if spare else 448)
+    return T <= (768 if spare else 448)
 
 
-def attention_on_kernels(B: int, T: int, H: int, Hkv: int, D: int, grad: bool) -> bool:
+def attention_on_kernels(B: int, T: int, H: int, Hkv: int, D: int) -> bool:
     """Does causal attention of these sizes run on the kernels, where they take them?"""
-    return ATTENTION_IMPL == "kernel" and (T % 128 == 0 or _ragged_on_kernels(B, T, H, Hkv, D, grad))
+    return ATTENTION_IMPL == "kernel" and (T % 128 == 0 or _ragged_on_kernels(B, T, H, Hkv, D))
 
 
 def causal_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor) -> torch.Tensor:
@@ -806,8 +810,8 @@ def causal_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor) -> torch
         q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
         if flash_attention_supported(q, k, v):
             return _FlashAttnFn.apply(q, k, v).view(B, T, H * Dh)
-        grad = torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad)
-        if T % 128 and _ragged_on_kernels(B, T, H, Hkv, Dh, grad) and _any_length(q, k, v):
+        if T % 128 and _ragged_on_kernels(B, T, H, Hkv, Dh) and _any_length(q, k, v):
+            grad = torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad)
             y = _FlashAttnAnyLengthFn.apply(q, k, v) if grad else _attention_forward(q, k, v)[0]
             return y.view(B, T, H * Dh)
     qt, kt, vt = q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2)

@@ -9,6 +9,7 @@ missing build.  ``build()`` cross-compiles and works without a GPU.
 from __future__ import annotations
 
 import os
+import shlex
 import subprocess
 import threading
 from pathlib import Path
@@ -57,7 +58,11 @@ def _libstdcxx() -> list[str]:
     stride) ends the process with a segmentation fault where it should raise."""
     from torch.utils import cpp_extension
 
-    found = subprocess.run([cpp_extension.get_cxx_compiler(), "-print-file-name=libstdc++.so.6"], capture_output=True, text=True)
+    try:
+        found = subprocess.run([*shlex.split(cpp_extension.get_cxx_compiler()), "-print-file-name=libstdc++.so.6"],
+                               capture_output=True, text=True)
+    except OSError:
+        return []
     path = found.stdout.strip()
     return [path] if os.path.isabs(path) and os.path.exists(path) else []
 
